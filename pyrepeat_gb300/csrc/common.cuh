@@ -185,11 +185,11 @@ class HostPool {
 constexpr double kDefaultKappaLimit = 2e5;
 
 namespace rp {
-// Tile shapes of the mixed-precision normal equations: atoms per CTA of the Phi kernel (8, 16
+// Tile shapes of the mixed-precision normal equations: most atoms per CTA of the Phi kernel (8, 16
 // or 32) and Gram points per work unit, in blocks of 64 (up to 16).  Neither changes a result: every
 // Phi value and every exact digit sum is the same whatever the tiling.
 struct TileConfig {
-    int phi_atoms = 16;
+    int phi_atoms = 32;
     int gram_split = 16;
 };
 // The autotuner's bucket of a fit: atoms, kept points, KMAX.

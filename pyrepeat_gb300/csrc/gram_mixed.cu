@@ -38,6 +38,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "df.cuh"
@@ -362,15 +363,6 @@ __device__ __forceinline__ float vscale_of(double vmax) {
 // Four 7-bit signed digits of an integer I = round(x 2^27), |x| <= 1:
 // x ~ 2^-6 (s0 + 2^-7 s1 + 2^-14 s2 + 2^-21 s3), digits rounded half up so |s| <= 64,
 // each exact in FP16.  Integer shifts only (no FP64 on the per-element path).
-// Exact warp sum of fixed-point values |I| <= 2^27: two 32-bit warp reductions of the
-// 14-bit halves (each sum stays below 2^19), recombined in 64 bits.
-__device__ __forceinline__ long long warp_sum_fixed(int I) {
-    const int hi = I >> 14, lo = I - (hi << 14);  // I = hi 2^14 + lo, lo in [0, 2^14)
-    const int shi = __reduce_add_sync(0xffffffffu, hi);
-    const int slo = __reduce_add_sync(0xffffffffu, lo);
-    return (long long)shi * 16384 + slo;
-}
-
 __device__ __forceinline__ void split4(int v, int &s0, int &s1, int &s2, int &s3) {
     s0 = (v + (1 << 20)) >> 21;
     int r = v - (s0 << 21);  // [-2^20, 2^20)
@@ -471,8 +463,85 @@ __device__ __forceinline__ float erfc_nr2(float xs) {
     return t * ex2_ftz(fmaf(-xs, xs, p));
 }
 
-constexpr int kPhiPts = 128;     // points per CTA (one per thread)
-constexpr int kPhiAtoms = 16;    // atoms per CTA by default (8 and 32 are the other tile shapes)
+// Pairs of FP32 values in one 64-bit register, for the packed instructions of this part: one
+// issue slot does the IEEE operation of both halves, each rounded as the scalar instruction
+// rounds it.  (The Phi kernel is bound by instruction issue, not by the FP32 pipe.)
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 pack2(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ f2 dup2(float a) { return pack2(a, a); }
+__device__ __forceinline__ void unpack2(f2 v, float &a, float &b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) { return fma2(b, dup2(-1.0f), a); }  // one rounding, as a - b
+// a + b as s + e exactly, both halves (dfa::two_sum)
+__device__ __forceinline__ void two_sum2(f2 a, f2 b, f2 &s, f2 &e) {
+    s = add2(a, b);
+    const f2 bb = sub2(s, a);
+    e = add2(sub2(a, sub2(s, bb)), sub2(b, bb));
+}
+
+// erfc_nr2 of two arguments: the same operations in the same order.  The polynomial is carried with
+// the opposite sign, which changes no rounding: xs^2 - p is then one packed multiply-add, and
+// the exponential instruction negates its operand.  Its steps are scalar: a packed step issues
+// once but holds its pipe as long as the two scalar ones, and its coefficients would take a
+// register pair each, where the scalar steps carry them in the instruction (302 us against
+// 308 us for 33 M pairs).
+__device__ __forceinline__ f2 erfc_nr2x2(f2 xs) {
+    float u, v, tu, tv;
+    unpack2(fma2(dup2((float)(0.5 / kSqrtLog2e)), xs, dup2(1.0f)), u, v);
+    tu = rcp_ftz(u);
+    tv = rcp_ftz(v);
+    float pu = -(float)(kLog2e * 0.17087277), pv = pu;
+    auto step = [&](float c) {
+        pu = fmaf(tu, pu, c);
+        pv = fmaf(tv, pv, c);
+    };
+    step(-(float)(kLog2e * -0.82215223));
+    step(-(float)(kLog2e * 1.48851587));
+    step(-(float)(kLog2e * -1.13520398));
+    step(-(float)(kLog2e * 0.27886807));
+    step(-(float)(kLog2e * -0.18628806));
+    step(-(float)(kLog2e * 0.09678418));
+    step(-(float)(kLog2e * 0.37409196));
+    step(-(float)(kLog2e * 1.00002368));
+    step(-(float)(kLog2e * -1.26551223));
+    unpack2(fma2(xs, xs, pack2(pu, pv)), u, v);
+    return mul2(pack2(tu, tv), pack2(ex2_ftz(-u), ex2_ftz(-v)));
+}
+// min(m, |a|, |b|): the three-operand minimum
+__device__ __forceinline__ float min3_abs(float m, float a, float b) {
+    float r;
+    asm("min.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(a), "f"(b));
+    return r;
+}
+
+constexpr int kPhiPts = 128;                  // points per CTA, two consecutive ones per thread
+constexpr int kPhiThreads = kPhiPts / 2;
+constexpr int kPhiWarps = kPhiThreads / 32;
+constexpr int kPhiAtoms = 32;    // most atoms per CTA (phi_atoms_per_cta)
+// Staged E values (KMAX 7): 60 words for the four atoms of a run (a run: consecutive points of one
+// grid row) while a tile has at most 32 runs, 28 words for two atoms up to 64 runs, else 14 for one.
+// The strides put the reads of 8 (16 for one atom) consecutive runs on distinct banks.
+constexpr int kEBytes = 7680;
 constexpr int kMaxShifts = 128;  // pruned real-space shifts (checked on the host)
 
 // The reference's FP64 cutoff decision for one (point, image) pair (repeat.py:944-966:
@@ -536,11 +605,11 @@ struct AxisDF {
     float h[9], l[9];
 };
 
-// k * (ah + al) for a small integer k, as an unevaluated pair (p, e)
-__device__ __forceinline__ void int_times_df(float k, float ah, float al, float &p, float &e) {
-    p = __fmul_rn(k, ah);
-    e = __fmaf_rn(k, ah, -p);
-    e = __fmaf_rn(k, al, e);
+// k * (ah + al) for two small integers k, each as an unevaluated pair (p, e)
+__device__ __forceinline__ void int_times_df2(f2 k, float ah, float al, f2 &p, f2 &e) {
+    p = mul2(k, dup2(ah));
+    e = fma2(k, dup2(ah), mul2(p, dup2(-1.0f)));
+    e = fma2(k, dup2(al), e);
 }
 
 // Digit output of the Phi kernel (single pass): instead of Phi_t, the kernel writes the
@@ -549,9 +618,9 @@ __device__ __forceinline__ void int_times_df(float k, float ah, float al, float 
 // rows..rows_kpad-1 get zero digits.  Exact row sums go to rowsum (one atomic per CTA
 // and row), values beyond |x| = 1 are clamped and counted in *clamped.
 struct PhiDigits {
-    __half *X0, *X1, *X2, *X3;
-    long long ldx;        // row stride of the slices
-    long long rows_kpad;  // columns written (the chunk padded to the Gram's K step)
+    __half *X;            // slice 0, rows of rows_kpad points
+    long long slice;      // elements from one slice to the next
+    long long rows_kpad;  // points per row (the chunk padded to the Gram's K step)
     const float *scale;   // per atom, a power of two
     const double *Vc;     // the chunk's centred ESP
     const double *vmax_p; // max |Vc| (the ESP row scale)
@@ -560,134 +629,262 @@ struct PhiDigits {
     int N;
 };
 
-// NC > 0: the number of n1 terms is the compile-time constant NC (KMAX = NC, the
-// reference's default 7): an atom's NC E values are loaded at the top of its iteration
-// and used after the real-space loop, which hides their L2 latency; stage C is unrolled.
-// NC = 0: any KMAX, loads in the loop.  The register cap keeps 7 CTAs per SM.
-template <int NC, bool DIG, int AT>
-__global__ void __launch_bounds__(kPhiPts, 7) phi_chunk_kernel(
+// The images of one atom that the real-space loop skipped for one point (half u of the packed
+// coordinates): decided in FP64 (fp64_pair), in table order, added to the loop's sum `acc32`.
+// Returns the sum as a double-float (s, e).  A few points in a million run it.
+__device__ __noinline__ void real_special(int f, int u, const f2 (&gh)[3], const f2 (&gl)[3], const float4 *tab,
+                                          const unsigned short *items, int nc, float fp64_below, float r2_in,
+                                          float r2_out, float saf, const double *axis, int nx, int ny,
+                                          const double *p, const double *shifts, int zero_idx, double rc, double sa,
+                                          float acc32, float &s, float &e) {
+    float h[3], lo[3];
+    for (int d = 0; d < 3; ++d) {
+        float a, b;
+        unpack2(gh[d], a, b);
+        h[d] = u ? b : a;
+        unpack2(gl[d], a, b);
+        lo[d] = u ? b : a;
+    }
+    const int row = f / nx, i = f - row * nx, l = row / ny, j = row - l * ny;
+    float x64h = 0.f, x64l = 0.f;  // rare FP64 terms, folded in as double-float pairs
+    for (int c = 0; c < nc; ++c) {
+        const float4 t0 = tab[3 * c], t1 = tab[3 * c + 1], t2 = tab[3 * c + 2];
+        const float dx = __fadd_rn(__fadd_rn(h[0], t0.x), __fadd_rn(lo[0], t1.z));
+        const float dy = __fadd_rn(__fadd_rn(h[1], t0.z), __fadd_rn(lo[1], t2.x));
+        const float dz = __fadd_rn(__fadd_rn(h[2], t1.x), __fadd_rn(lo[2], t2.z));
+        const float r2 = fmaf(dz, dz, fmaf(dx, dx, __fmul_rn(dy, dy)));
+        if (!(r2 < fp64_below || (r2 > r2_in && r2 <= r2_out))) continue;
+        float th, tl;
+        const int dec = fp64_pair(axis, i, j, l, p, shifts, items[c] & 127, zero_idx, rc, sa, r2 < fp64_below, th, tl);
+        if (dec == 1) {  // inside the cutoff: the FP32 term
+            const float rinv = rsqrt_ftz(r2);
+            acc32 = fmaf(erfc_nr2(saf * (r2 * rinv)), rinv, acc32);
+        } else if (dec == 2) {  // a point on top of an image: the large term in FP64
+            float s2, e2;
+            dfa::two_sum(x64h, th, s2, e2);
+            x64h = s2;
+            x64l = __fadd_rn(x64l, __fadd_rn(e2, tl));
+        }
+    }
+    float s_, e_;
+    dfa::two_sum(acc32, x64h, s_, e_);
+    s = s_;
+    e = __fadd_rn(e_, x64l);
+}
+
+// max(|a|, |b|), NaN if either is
+__device__ __forceinline__ float max_abs_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(fabsf(a)), "f"(fabsf(b)));
+    return r;
+}
+
+// The digits of two consecutive points of one row.  I = round(x 2^27), x = (h + l) sc, comes as
+// hi 2^14 + lo without conversion instructions (a quarter of the rate): adding 1.5 2^37 and
+// 1.5 2^23 rounds to multiples of 2^14 and of 1 (to nearest even, as rintf), and the integers
+// are read off the sums' bits; the remainder after the integer part is exact, and the low
+// part decides the last unit.  |hi|, |lo| <= 2^13 (+ 5), so with 64 (1 + 2^7) added each half
+// holds two digits as a 7-bit field below an 8-bit one, every digit 64 too large: the digits
+// of split4 up to a carry where that one gives another 64, the same value.  A field u under
+// the bits of 1024 is the FP16 number 1024 + u, and subtracting 1088 gives the digit exactly.
+// Returns the two biased sums hi, lo (without the points past the end) for the row sum.
+constexpr int kHalfBias = 64 * (1 + (1 << 7));
+__device__ __forceinline__ void digit_halves2(f2 h, f2 l, float sc, int full, bool valid0, bool valid1, int *clamped,
+                                              int &hi0, int &hi1, int &lo0, int &lo1) {
+    constexpr float kM1 = 206158430208.0f, kM0 = 12582912.0f;  // 1.5 2^37, 1.5 2^23
+    constexpr int kB1 = 0x52400000, kB0 = 0x4b400000;          // their bits
+    constexpr float kTop = 134217728.0f;                       // 2^27
+    const f2 sc2 = dup2(sc * kTop);
+    const f2 H = mul2(h, sc2), L = mul2(l, sc2);
+    const f2 a1 = add2(H, dup2(kM1));
+    const f2 r = sub2(H, add2(a1, dup2(-kM1)));
+    const f2 a0 = add2(r, dup2(kM0));
+    const f2 b0 = add2(add2(sub2(r, add2(a0, dup2(-kM0))), L), dup2(kM0));
+    float hu, hv, pu, pv, qu, qv, ru, rv;
+    unpack2(H, hu, hv);
+    unpack2(a1, pu, pv);
+    unpack2(a0, qu, qv);
+    unpack2(b0, ru, rv);
+    hi0 = __float_as_int(pu) + (kHalfBias - kB1);
+    hi1 = __float_as_int(pv) + (kHalfBias - kB1);
+    lo0 = __float_as_int(qu) + __float_as_int(ru) + (int)((unsigned)kHalfBias - 2u * (unsigned)kB0);
+    lo1 = __float_as_int(qv) + __float_as_int(rv) + (int)((unsigned)kHalfBias - 2u * (unsigned)kB0);
+    if (!full) {  // the last tile: points past the end are zero
+        if (!valid0) hi0 = lo0 = kHalfBias;
+        if (!valid1) hi1 = lo1 = kHalfBias;
+    }
+    if (!(max_abs_nan(hu, hv) <= kTop)) {  // |x| beyond 1: clamp (counted; the fit is redone); a NaN gives 0
+        if (valid0 && !(fabsf(hu) <= kTop)) {
+            hi0 = kHalfBias + (hu > 0.f ? 8192 : hu < 0.f ? -8192 : 0);
+            lo0 = kHalfBias;
+        }
+        if (valid1 && !(fabsf(hv) <= kTop)) {
+            hi1 = kHalfBias + (hv > 0.f ? 8192 : hv < 0.f ? -8192 : 0);
+            lo1 = kHalfBias;
+        }
+        const int n = (valid0 && fabsf(hu) > kTop) + (valid1 && fabsf(hv) > kTop);
+        if (n) atomicAdd(clamped, n);
+    }
+}
+__device__ __forceinline__ void store_digits2(__half *x, long long slice, int hi0, int hi1, int lo0, int lo1) {
+    const unsigned hp = __byte_perm(hi0, hi1, 0x5410), lp = __byte_perm(lo0, lo1, 0x5410);
+    const __half2 off = __half2half2(__ushort_as_half((unsigned short)0x6440));  // 1088
+    auto put = [&](int q, unsigned v) {
+        *reinterpret_cast<__half2 *>(x + q * slice) = __hsub2(*reinterpret_cast<const __half2 *>(&v), off);
+    };
+    put(0, ((hp >> 7) & 0x00ff00ffu) | 0x64006400u);
+    put(1, (hp & 0x007f007fu) | 0x64006400u);
+    put(2, ((lp >> 7) & 0x00ff00ffu) | 0x64006400u);
+    put(3, (lp & 0x007f007fu) | 0x64006400u);
+}
+// The warp's exact sum of I over its points from the biased halves (32-bit sums below 2^21)
+__device__ __forceinline__ long long warp_sum_halves2(int hi0, int hi1, int lo0, int lo1) {
+    const int shi = __reduce_add_sync(0xffffffffu, hi0 + hi1) - 64 * kHalfBias;
+    const int slo = __reduce_add_sync(0xffffffffu, lo0 + lo1) - 64 * kHalfBias;
+    return (long long)shi * 16384 + slo;
+}
+
+// x / d for 0 <= x < 2^31 by a multiplication (d's reciprocal rounded up, computed on the host)
+struct FastDiv {
+    unsigned mul;
+    int shift;
+};
+__device__ __forceinline__ int fast_div(int x, FastDiv f) {
+    return (int)(((unsigned long long)(unsigned)x * f.mul) >> f.shift);
+}
+
+// One thread handles two consecutive points (2t, 2t + 1 of the CTA's 128), packed where that
+// helps: the table loads, the loop and the digit stores serve two points and most FP32
+// operations of the real-space term issue once for both.  Each point's value is computed by
+// the same operations in the same order as one at a time.
+// What bounds it: the issue of instructions and the latencies between them (16 warps per SM at
+// 128 registers; 96 registers and 20 warps spill and took 381 us against 302).  On 273 atoms x
+// 121k points (33 M pairs): 287 us, 203 thread instructions per pair, against 360 us and 344 for
+// one point per thread with the E values loaded per point and 16 atoms per CTA.
+// NC = 7: the number of n1 terms (the reference's KMAX) is a compile-time constant: the points'
+// phases ex stay in registers, and the E values of up to four atoms at a time are copied to
+// shared memory (asynchronously, one stage ahead), once per run of points in the same grid
+// row: loaded per point, they took 112 of ~160 L1 wavefronts per 64 points and atom.
+// NC = 0: any KMAX, phases in shared memory and E read in the loop.
+template <int NC, bool DIG>
+__global__ void __launch_bounds__(kPhiThreads, 8) phi_chunk_kernel(
     const int32_t *__restrict__ kept, long long m0, long long rows, const double *__restrict__ axis, AxisDF adf,
     int nx, int ny,
-    const double *__restrict__ atoms, int N, const double *__restrict__ shifts, int S, int scap, int zero_idx,
-    double rc, double sa, float rcf, float saf_in, float near2, const float4 *__restrict__ img,
+    FastDiv dnx, FastDiv dny, const double *__restrict__ atoms, int N, const double *__restrict__ shifts, int S, int per_cta, int slots, int zero_idx,
+    double rc, double sa, float rcf, float saf, float near2, const float4 *__restrict__ img,
     const float4 *__restrict__ EX,
     const float2 *__restrict__ E, int n1c, int parts, float2 *__restrict__ phit, long long ld,
     double *__restrict__ psum, float *__restrict__ pmax, PhiDigits dg) {
-    extern __shared__ float4 dsm[];
-    float4 *img_hi = dsm;                                 // [AT][scap] (x, y, z, shift index)
-    float4 *img_lo = img_hi + (size_t)AT * scap;   // [AT][scap]
-    float2 *exs = reinterpret_cast<float2 *>(img_lo + (size_t)AT * scap);  // [n1c][kPhiPts] ex[n1][i]
-    __shared__ int ncand[AT];
-    __shared__ float bb[2][3][kPhiPts / 32];
-    __shared__ float wsum[kPhiPts / 32][AT];
-    __shared__ float wmax[kPhiPts / 32][AT];
-    __shared__ long long wrow[kPhiPts / 32][AT + 1];  // digit-row partial sums (DIG)
+    static_assert(NC == 0 || NC == 7, "the E stages are laid out for KMAX 7");
+    // Image table, `slots` entries (each warp fills one half): the negated double-float position
+    // relative to the CTA origin with every value twice, (-x, -x, -y, -y), (-z, -z, -xl, -xl),
+    // (-yl, -yl, -zl, -zl), the packed operands of both points; NC = 7: two stages of E values;
+    // NC = 0: ex[n1][i] of the points, (re, re, im, im) per pair; then the entries'
+    // (atom << 7) | shift.
+    extern __shared__ ulonglong2 dsm[];
+    ulonglong2 *tab = dsm;
+    char *es = reinterpret_cast<char *>(tab + 3 * (size_t)slots);       // NC = 7: [2][kEBytes]
+    float4 *exs = reinterpret_cast<float4 *>(tab + 3 * (size_t)slots);  // NC = 0: [n1c][kPhiThreads]
+    unsigned short *items = reinterpret_cast<unsigned short *>(
+        NC > 0 ? es + 2 * kEBytes : reinterpret_cast<char *>(exs + (size_t)n1c * kPhiThreads));
+    __shared__ int start[kPhiAtoms];        // an atom's first entry
+    __shared__ int cand[kPhiAtoms];         // (first entry << 9) | (near << 8) | entries
+    __shared__ int close[kPhiAtoms];        // an image near or inside the points' box
+    __shared__ int filled[kPhiWarps];  // end of each warp's entries
+    __shared__ float scl[kPhiAtoms];        // digit scales (DIG)
+    __shared__ float bb[2][3][kPhiWarps];
+    __shared__ float wsum[kPhiPts / 32][DIG ? 1 : kPhiAtoms];
+    __shared__ float wmax[kPhiPts / 32][DIG ? 1 : kPhiAtoms];
+    __shared__ long long wrow[kPhiWarps][kPhiAtoms + 1];  // digit-row partial sums (DIG)
+    __shared__ long long run_off[NC > 0 ? kPhiPts : 1];  // byte offset of each run's E row
+    __shared__ int wruns[kPhiWarps];
     const long long mb = (long long)blockIdx.x * kPhiPts;
-    const int a0 = blockIdx.y * AT;
-    const int na = min(AT, N - a0);
-    const int layer = nx * ny;
+    const int a0 = blockIdx.y * per_cta;
+    const int na = min(per_cta, N - a0);
+    const int Ne = (N + 1) & ~1;  // E's columns per row
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long m = mb + threadIdx.x;
-    const bool valid = m < rows;
+    const long long m = mb + 2 * threadIdx.x;
+    const bool valid0 = m < rows, valid1 = m + 1 < rows;
 
     // CTA origin: the first point of the tile (FP64 once, shared as a double-float)
     __shared__ float org[6];
     __shared__ int org_idx[3];
-    if (threadIdx.x == 0) {
-        const int f0 = kept[m0 + mb];
-        const int l0 = f0 / layer, r0 = f0 - l0 * layer, j0 = r0 / nx, i0 = r0 - j0 * nx;
-        for (int d = 0; d < 3; ++d) {
-            const double o = ((double)i0 * axis[d] + (double)j0 * axis[3 + d]) + (double)l0 * axis[6 + d];
-            org[d] = (float)o;
-            org[3 + d] = (float)(o - (double)org[d]);
-        }
-        org_idx[0] = i0;
-        org_idx[1] = j0;
-        org_idx[2] = l0;
+    if (threadIdx.x < 3) {
+        const int d = threadIdx.x, f0 = kept[m0 + mb];
+        const int q = fast_div(f0, dnx), i0 = f0 - q * nx, l0 = fast_div(q, dny), j0 = q - l0 * ny;
+        const double o = ((double)i0 * axis[d] + (double)j0 * axis[3 + d]) + (double)l0 * axis[6 + d];
+        org[d] = (float)o;
+        org[3 + d] = (float)(o - (double)org[d]);
+        org_idx[d] = d == 0 ? i0 : d == 1 ? j0 : l0;
     }
+    if (DIG && threadIdx.x < na) scl[threadIdx.x] = dg.scale[a0 + threadIdx.x];
     __syncthreads();
-    const int f = kept[m0 + (valid ? m : mb)];
-    const int l = f / layer, rem = f - l * layer, j = rem / nx, i = rem - j * nx;
+    // a point past the end repeats the tile's first point
+    const int f0 = kept[m0 + (valid0 ? m : mb)], f1 = kept[m0 + (valid1 ? m + 1 : mb)];
+    const int row0 = fast_div(f0, dnx), row1 = fast_div(f1, dnx);  // grid rows j + l ny
     // point - origin = di a0 + dj a1 + dl a2 with small integers: double-float on the FP32 pipe
-    float gh[3], gl[3], oh[3], ol[3];
+    f2 gh[3], gl[3];
     {
-        const float di = (float)(i - org_idx[0]), dj = (float)(j - org_idx[1]), dl = (float)(l - org_idx[2]);
+        const int l0 = fast_div(row0, dny), l1 = fast_div(row1, dny);
+        const f2 di = pack2((float)(f0 - row0 * nx - org_idx[0]), (float)(f1 - row1 * nx - org_idx[0])),
+                 dj = pack2((float)(row0 - l0 * ny - org_idx[1]), (float)(row1 - l1 * ny - org_idx[1])),
+                 dl = pack2((float)(l0 - org_idx[2]), (float)(l1 - org_idx[2]));
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            float p0, e0, p1, e1, p2, e2, s, t;
-            int_times_df(di, adf.h[d], adf.l[d], p0, e0);
-            int_times_df(dj, adf.h[3 + d], adf.l[3 + d], p1, e1);
-            int_times_df(dl, adf.h[6 + d], adf.l[6 + d], p2, e2);
-            dfa::two_sum(p0, p1, s, t);
-            float s2, t2;
-            dfa::two_sum(s, p2, s2, t2);
-            const float e = __fadd_rn(__fadd_rn(__fadd_rn(e0, e1), e2), __fadd_rn(t, t2));
-            gh[d] = __fadd_rn(s2, e);
-            gl[d] = __fadd_rn(e, -__fadd_rn(gh[d], -s2));
-            oh[d] = org[d];
-            ol[d] = org[3 + d];
+            f2 p0, e0, p1, e1, p2, e2, s, t, s2, t2;
+            int_times_df2(di, adf.h[d], adf.l[d], p0, e0);
+            int_times_df2(dj, adf.h[3 + d], adf.l[3 + d], p1, e1);
+            int_times_df2(dl, adf.h[6 + d], adf.l[6 + d], p2, e2);
+            two_sum2(p0, p1, s, t);
+            two_sum2(s, p2, s2, t2);
+            const f2 e = add2(add2(add2(e0, e1), e2), add2(t, t2));
+            gh[d] = add2(s2, e);
+            gl[d] = sub2(e, sub2(gh[d], s2));
+            float u, v;
+            unpack2(gh[d], u, v);
+            float mn = fminf(u, v), mx = fmaxf(u, v);
+            for (int o = 16; o > 0; o >>= 1) {
+                mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            }
+            if (lane == 0) {
+                bb[0][d][warp] = mn;
+                bb[1][d][warp] = mx;
+            }
         }
     }
+    f2 xr[NC > 0 ? NC : 1], xi[NC > 0 ? NC : 1];  // ex[n1][i] of both points (n1 > 0)
+    int slot0 = 0, slot1 = 0, nruns = 0;          // the points' runs
+    if (NC > 0) {
+        if (parts & 2) {
+            const int i0 = f0 - row0 * nx, i1 = f1 - row1 * nx;
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        float mn = gh[d], mx = gh[d];
-        for (int o = 16; o > 0; o >>= 1) {
-            mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            for (int n = 1; n < (NC > 0 ? NC : 1); ++n) {
+                const float4 x = EX[(long long)n * nx + i0], y = EX[(long long)n * nx + i1];
+                xr[n] = pack2(x.x, y.x);
+                xi[n] = pack2(x.z, y.z);
+            }
         }
-        if (lane == 0) {
-            bb[0][d][warp] = mn;
-            bb[1][d][warp] = mx;
+        int prev = __shfl_up_sync(0xffffffffu, row1, 1);
+        if (lane == 0) prev = -1;  // a warp starts a run of its own
+        const unsigned b0 = __ballot_sync(0xffffffffu, row0 != prev), b1 = __ballot_sync(0xffffffffu, row1 != row0);
+        const unsigned lt = (1u << lane) - 1u, le = lt | (1u << lane);
+        if (lane == 0) wruns[warp] = __popc(b0) + __popc(b1);
+        __syncthreads();
+        int base = 0;
+        for (int w = 0; w < kPhiWarps; ++w) {
+            if (w < warp) base += wruns[w];
+            nruns += wruns[w];
         }
-    }
-    if (parts & 2)
+        slot0 = base + __popc(b0 & le) + __popc(b1 & lt) - 1;
+        slot1 = base + __popc(b0 & le) + __popc(b1 & le) - 1;
+        if (row0 != prev) run_off[slot0] = (long long)row0 * Ne * 56;
+        if (row1 != row0) run_off[slot1] = (long long)row1 * Ne * 56;
+    } else if (parts & 2) {
+        const int i0 = f0 - row0 * nx, i1 = f1 - row1 * nx;
         for (int n = 0; n < n1c; ++n) {
-            const float4 x = EX[(long long)n * nx + i];
-            exs[n * kPhiPts + threadIdx.x] = make_float2(x.x, x.z);
-        }
-    __syncthreads();
-
-    if (parts & 1) {
-        float bmin[3], bmax[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            bmin[d] = bb[0][d][0];
-            bmax[d] = bb[1][d][0];
-            for (int w = 1; w < kPhiPts / 32; ++w) {
-                bmin[d] = fminf(bmin[d], bb[0][d][w]);
-                bmax[d] = fmaxf(bmax[d], bb[1][d][w]);
-            }
-        }
-        const float reach = rcf + 1e-3f, reach2 = reach * reach;
-        for (int a = warp; a < AT; a += kPhiPts / 32) {
-            int base = 0;
-            if (a < na) {
-                const float4 *src = img + 2 * (size_t)(a0 + a) * S;
-                for (int s0 = 0; s0 < S; s0 += 32) {
-                    const int s = s0 + lane;
-                    bool keep = false;
-                    float4 h = make_float4(0.f, 0.f, 0.f, 0.f), lo = h;
-                    if (s < S) {
-                        const float4 ph = src[2 * s], pl = src[2 * s + 1];
-                        const float2 qx = df_sub(ph.x, pl.x, oh[0], ol[0]), qy = df_sub(ph.y, pl.y, oh[1], ol[1]),
-                                     qz = df_sub(ph.z, pl.z, oh[2], ol[2]);
-                        h = make_float4(qx.x, qy.x, qz.x, ph.w);
-                        lo = make_float4(qx.y, qy.y, qz.y, 0.f);
-                        const float dx = fmaxf(fmaxf(bmin[0] - h.x, h.x - bmax[0]), 0.f);
-                        const float dy = fmaxf(fmaxf(bmin[1] - h.y, h.y - bmax[1]), 0.f);
-                        const float dz = fmaxf(fmaxf(bmin[2] - h.z, h.z - bmax[2]), 0.f);
-                        keep = dx * dx + dy * dy + dz * dz <= reach2;
-                    }
-                    const unsigned bal = __ballot_sync(0xffffffffu, keep);
-                    if (keep) {
-                        const int pos = base + __popc(bal & ((1u << lane) - 1u));
-                        img_hi[a * scap + pos] = h;
-                        img_lo[a * scap + pos] = lo;
-                    }
-                    base += __popc(bal);
-                }
-            }
-            if (lane == 0) ncand[a] = base;
+            const float4 x = EX[(long long)n * nx + i0], y = EX[(long long)n * nx + i1];
+            exs[n * kPhiThreads + threadIdx.x] = make_float4(x.x, y.x, x.z, y.z);
         }
     }
     __syncthreads();
@@ -698,133 +895,280 @@ __global__ void __launch_bounds__(kPhiPts, 7) phi_chunk_kernel(
     // r <= Rc is made in FP64 (the reference's expressions); the term itself, ~erfc(pi)/Rc
     // there, is the FP32 one.  FP64 runs at 1/64 of the FP32 rate per lane on this part,
     // and one lane in the band makes its whole warp run the FP64 code, so it stays short.
-    const float rcc = rcf * rcf, band = 4e-6f * rcc, saf = saf_in;  // sqrt(alpha log2 e), the argument scale of erfc_nr2
+    const float rcc = rcf * rcf, band = 4e-6f * rcc;  // saf: sqrt(alpha log2 e), the argument scale of erfc_nr2
+    const float r2_in = rcc - band, r2_out = rcc + band;
     const float fp64_below = fmaxf(near2, 1e-6f);
-    const long long row = f / nx;  // j + l * ny
-    const float2 *erow = E + (row * N + a0) * (NC > 0 ? NC : n1c);
-    float2 *prow = phit + (long long)a0 * ld + m;
-    for (int a = 0; a < na; ++a, erow += (NC > 0 ? NC : n1c), prow += ld) {
-        dfa::acc v{0.f, 0.f};
-        float2 ey[NC > 0 ? NC : 1];  // this atom's E values, in flight during the real-space loop
-        if (NC > 0 && valid && (parts & 2)) {
+
+    // The images of atoms r0 .. r0 + nr - 1 within Rc + 1e-3 Bohr of the points' bounding box: an
+    // FP32 test per image (1e-4 Bohr more covers its rounding), each warp over the images of half
+    // of the atoms 32 at a time, which lists the survivors, an atom's in shift order; then
+    // their table entries.  An atom with an image near or inside the box is marked: only there
+    // can a point be closer than sqrt(fp64_below) to an image.  False when a warp's list
+    // overflows its half of the table.
+    auto cull = [&](int r0, int nr) -> bool {
+        if (threadIdx.x < kPhiAtoms) close[threadIdx.x] = 0;
+        __syncthreads();
+        float bmin[3], bmax[3];
 #pragma unroll
-            for (int n = 0; n < (NC > 0 ? NC : 1); ++n) ey[n] = erow[n];
+        for (int d = 0; d < 3; ++d) {
+            bmin[d] = fminf(bb[0][d][0], bb[0][d][1]) + org[d];
+            bmax[d] = fmaxf(bb[1][d][0], bb[1][d][1]) + org[d];
         }
-        if (parts & 1) {  // every lane runs the loop (a lane past the end repeats the tile's first point)
-            const float4 *ih = img_hi + a * scap, *il = img_lo + a * scap;
-            const int nc = ncand[a];
-            float acc32 = 0.f;
+        const float reach = rcf + 1.1e-3f, reach2 = reach * reach, near = 4.f * fp64_below;
+        const int half = slots >> 1, na0 = (nr + 1) >> 1;
+        const int wa = warp ? r0 + na0 : r0, wn = warp ? nr - na0 : na0;  // the warp's atoms
+        const int step_a = 32 / S, step_s = 32 - step_a * S;
+        int a = lane / S, sh = lane - a * S, base = 0;
+        const float4 *src = img + 2 * ((size_t)(a0 + wa) * S + lane);
+        for (int k0 = 0; k0 < wn * S; k0 += 32, src += 64) {
+            bool keep = false;
+            if (a < wn) {
+                const float4 ph = *src;
+                const float dx = fmaxf(fmaxf(bmin[0] - ph.x, ph.x - bmax[0]), 0.f);
+                const float dy = fmaxf(fmaxf(bmin[1] - ph.y, ph.y - bmax[1]), 0.f);
+                const float dz = fmaxf(fmaxf(bmin[2] - ph.z, ph.z - bmax[2]), 0.f);
+                const float d2 = dx * dx + dy * dy + dz * dz;
+                keep = d2 <= reach2;
+                if (d2 <= near) close[wa + a] = 1;
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, keep);
+            const int pos = base + __popc(bal & ((1u << lane) - 1u));
+            if (sh == 0 && a < wn) start[wa + a] = warp * half + pos;
+            if (keep && pos < half) items[warp * half + pos] = (unsigned short)(((wa + a) << 7) | sh);
+            base += __popc(bal);
+            a += step_a;
+            sh += step_s;
+            if (sh >= S) {
+                sh -= S;
+                ++a;
+            }
+        }
+        if (lane == 0) filled[warp] = warp * half + base;
+        const bool ok = !__syncthreads_or(base > half);
+        if (ok) {
+            for (int t = threadIdx.x; t < nr; t += kPhiThreads) {
+                const int b = start[r0 + t];
+                const int e = t + 1 == na0 ? filled[0] : t + 1 == nr ? filled[1] : start[r0 + t + 1];
+                cand[r0 + t] = (b << 9) | (close[r0 + t] << 8) | (e - b);
+            }
+            for (int k = warp * half + lane; k < warp * half + base; k += 32) {
+                const int it = items[k];
+                const float4 *ps = img + 2 * ((size_t)(a0 + (it >> 7)) * S + (it & 127));
+                const float4 ph = ps[0], pl = ps[1];
+                const float2 qx = df_sub(ph.x, pl.x, org[0], org[3]), qy = df_sub(ph.y, pl.y, org[1], org[4]),
+                             qz = df_sub(ph.z, pl.z, org[2], org[5]);
+                ulonglong2 *t = tab + 3 * k;
+                t[0] = make_ulonglong2(dup2(-qx.x), dup2(-qy.x));
+                t[1] = make_ulonglong2(dup2(-qz.x), dup2(-qx.y));
+                t[2] = make_ulonglong2(dup2(-qy.y), dup2(-qz.y));
+            }
+        }
+        return ok;
+    };
+
+    // E values of atoms a .. a + n - 1 for every run into stage buffer b, run by run (the stride
+    // above): 16 bytes a lane, two runs of four atoms (four of two) per warp instruction; E's rows
+    // have an even number of columns, so a stage that starts at an even atom is aligned, and an
+    // odd last atom takes half of the next column along.  One atom per stage: 8 bytes a lane.
+    const int eb = nruns <= 32 ? 4 : nruns <= 64 ? 2 : 1;
+    const int e_stride = eb == 4 ? 240 : eb == 2 ? 112 : 56;
+    const int e_run = eb == 4 ? (lane >= 14) : lane / 7, e_chunk = lane - e_run * (eb == 4 ? 14 : 7);
+    const int e_runs = eb == 4 ? 2 : 4, e_run0 = warp * e_runs + e_run, e_step = kPhiWarps * e_runs;
+    const char *e_src = reinterpret_cast<const char *>(E + (long long)a0 * 7) + e_chunk * (eb > 1 ? 16 : 8);
+    const uint32_t e_dst = tc::smem_u32(es) + e_run0 * e_stride + e_chunk * (eb > 1 ? 16 : 8);
+    auto stage_e = [&](int a, int n, int b) {
+        if (lane >= 28 || (eb > 1 ? 2 * e_chunk >= 7 * n : n <= 0)) return;
+        const char *src = e_src + a * 56;
+        uint32_t dst = e_dst + b * kEBytes;
+        if (eb > 1) {
+#pragma unroll 2
+            for (int r = e_run0; r < nruns; r += e_step, dst += e_step * e_stride)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + run_off[r]) : "memory");
+        } else {
+#pragma unroll 1
+            for (int r = e_run0; r < nruns; r += e_step, dst += e_step * e_stride)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src + run_off[r]) : "memory");
+        }
+    };
+
+    int round = na;  // atoms whose images share one table
+    if ((parts & 1) && !cull(0, na)) round = 2 * ((slots >> 1) / S);
+    const float2 *erow0 = E + ((long long)row0 * Ne + a0) * n1c, *erow1 = E + ((long long)row1 * Ne + a0) * n1c;
+    const int full = mb + kPhiPts <= rows;
+    __half *xp = DIG ? dg.X + a0 * dg.rows_kpad + m : nullptr;
+    const bool stores = DIG && m < dg.rows_kpad;
+    int e_buf = 0;
+    if (NC > 0) {
+        if (parts & 2) stage_e(0, min(eb, min(round, na)), 0);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int r0 = 0; r0 < na; r0 += round) {
+        const int r1 = min(r0 + round, na);
+        __syncthreads();  // the first round's table is complete; a later round: the one before has been read
+        if (round < na && (parts & 1)) {
+            cull(r0, r1 - r0);
+            __syncthreads();
+        }
+      for (int e_lo = r0; e_lo < r1;) {
+        const int e_hi = NC > 0 ? min(e_lo + eb, r1) : r1;
+        if (NC > 0) {  // this stage has landed, and every warp is done with the buffer of the next
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();
+            if (parts & 2) stage_e(e_hi, min(eb, (e_hi < r1 ? r1 : min(r1 + round, na)) - e_hi), e_buf ^ 1);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        const char *ep = es + e_buf * kEBytes + slot0 * e_stride;
+        const int eq = (slot1 - slot0) * e_stride;
+        for (int a = e_lo; a < e_hi; ++a, ep += 56) {
+            f2 acc = 0ull;
+            float edge = 3e38f;  // the smallest | r^2 - Rc^2 |
+            bool spec = false;
+            const int ci = cand[a];
+            const ulonglong2 *t = tab + 3 * (ci >> 9);
             // Branch-free over the candidates: most of them are inside the cutoff for some lane of
             // the warp, so the term is computed for all and selected.  Images whose decision needs
             // FP64 (within the band around Rc, or on top of the point) are skipped here and taken
             // in a second pass, which a warp runs only when one of its lanes met one.  (A per-warp
             // ballot mask over the tile's candidates, which skips images out of the warp's reach,
             // measured 3 % more instructions: the mask costs more than the images it drops.)
-            bool spec_any = false;
-            for (int c = 0; c < nc; ++c) {
-                const float4 h = ih[c], lo = il[c];
-                const float hx = gh[0] - h.x, hy = gh[1] - h.y, hz = gh[2] - h.z;
-                const float dx = hx + (gl[0] - lo.x), dy = hy + (gl[1] - lo.y), dz = hz + (gl[2] - lo.z);
-                const float r2 = dx * dx + dy * dy + dz * dz;
-                const bool ok = r2 >= fp64_below && r2 <= rcc - band;
-                spec_any |= !ok && r2 <= rcc + band;
-                const float rinv = rsqrt_ftz(r2);
-                const float t = fmaf(erfc_nr2(saf * (r2 * rinv)), rinv, acc32);
-                acc32 = ok ? t : acc32;
+            auto real_space = [&](auto low) {
+                const f2 saf2 = dup2(saf), rcc2 = dup2(-rcc);
+#pragma unroll 2
+                for (int c = ci & 255; c > 0; --c, t += 3) {
+                    const ulonglong2 t0 = t[0], t1 = t[1], t2 = t[2];
+                    const f2 dx = add2(add2(gh[0], t0.x), add2(gl[0], t1.y));
+                    const f2 dy = add2(add2(gh[1], t0.y), add2(gl[1], t2.x));
+                    const f2 dz = add2(add2(gh[2], t1.x), add2(gl[2], t2.y));
+                    const f2 r2 = fma2(dz, dz, fma2(dx, dx, mul2(dy, dy)));
+                    float ra, rb, va, vb, aa, ab, da, db;
+                    unpack2(r2, ra, rb);
+                    unpack2(add2(r2, rcc2), da, db);
+                    edge = min3_abs(edge, da, db);
+                    bool oka = ra <= r2_in, okb = rb <= r2_in;
+                    if (decltype(low)::value) {
+                        oka = oka && ra >= fp64_below;
+                        okb = okb && rb >= fp64_below;
+                        spec |= ra < fp64_below || rb < fp64_below;
+                    }
+                    const f2 rinv = pack2(rsqrt_ftz(ra), rsqrt_ftz(rb));
+                    const f2 v = fma2(erfc_nr2x2(mul2(saf2, mul2(r2, rinv))), rinv, acc);
+                    unpack2(v, va, vb);
+                    unpack2(acc, aa, ab);
+                    acc = pack2(oka ? va : aa, okb ? vb : ab);
+                }
+            };
+            if (parts & 1) {
+                if (ci & 256) real_space(std::true_type{});
+                else real_space(std::false_type{});
+                spec |= edge <= band * 1.01f;  // every image of the band (r2_in, r2_out], and at most a few more
             }
-            if (__any_sync(0xffffffffu, spec_any)) {
-                float x64h = 0.f, x64l = 0.f;  // rare FP64 terms, folded in as double-float pairs
-                for (int c = 0; c < nc; ++c) {
-                    const float4 h = ih[c], lo = il[c];
-                    const float hx = gh[0] - h.x, hy = gh[1] - h.y, hz = gh[2] - h.z;
-                    const float dx = hx + (gl[0] - lo.x), dy = hy + (gl[1] - lo.y), dz = hz + (gl[2] - lo.z);
-                    const float r2 = dx * dx + dy * dy + dz * dz;
-                    if (!(r2 < fp64_below || (r2 > rcc - band && r2 <= rcc + band))) continue;
-                    float th, tl;
-                    const int dec = fp64_pair(axis, i, j, l, atoms + 3 * (a0 + a), shifts, __float_as_int(h.w),
-                                              zero_idx, rc, sa, r2 < fp64_below, th, tl);
-                    if (dec == 1) {  // inside the cutoff: the FP32 term
-                        const float rinv = rsqrt_ftz(r2);
-                        acc32 = fmaf(erfc_nr2(saf * (r2 * rinv)), rinv, acc32);
-                    } else if (dec == 2) {  // a point on top of an image: the large term in FP64
-                        float s2, e2;
-                        dfa::two_sum(x64h, th, s2, e2);
-                        x64h = s2;
-                        x64l = __fadd_rn(x64l, __fadd_rn(e2, tl));
+            float ru = 0.f, rv = 0.f;  // stage C: Re sum_n1 ex[n1][i] E[row][a][n1]
+            if (parts & 2) {
+                if (NC > 0) {
+                    const float2 *p = reinterpret_cast<const float2 *>(ep), *q = reinterpret_cast<const float2 *>(ep + eq);
+                    ru = p[0].x;  // ex[0] = 1
+                    rv = q[0].x;
+#pragma unroll
+                    for (int n = 1; n < (NC > 0 ? NC : 1); ++n) {
+                        const float2 y = p[n], z = q[n];
+                        float xa, xb, ya, yb;
+                        unpack2(xr[n], xa, xb);
+                        unpack2(xi[n], ya, yb);
+                        ru = fmaf(xa, y.x, ru);
+                        rv = fmaf(xb, z.x, rv);
+                        ru = fmaf(-ya, y.y, ru);
+                        rv = fmaf(-yb, z.y, rv);
+                    }
+                } else {
+                    const float2 *p = erow0 + (long long)a * n1c, *q = erow1 + (long long)a * n1c;
+                    for (int n = 0; n < n1c; ++n) {
+                        const float4 x = exs[n * kPhiThreads + threadIdx.x];
+                        const float2 y = p[n], z = q[n];
+                        ru = fmaf(x.x, y.x, ru);
+                        rv = fmaf(x.y, z.x, rv);
+                        ru = fmaf(-x.z, y.y, ru);
+                        rv = fmaf(-x.w, z.y, rv);
                     }
                 }
-                float s_, e_;
-                dfa::two_sum(acc32, x64h, s_, e_);
-                v.s = s_;
-                v.e = __fadd_rn(e_, x64l);
-            } else {
-                v.s = acc32;
             }
-        }
-        if (valid && (parts & 2)) {  // stage C: Re sum_n1 ex[n1][i] E[row][a][n1]
-            float rs = 0.f;
-            if (NC > 0) {
+            f2 oh, ol;  // Phi as a double-float: the sum of the two parts, exactly
+            two_sum2(acc, pack2(ru, rv), oh, ol);
+            if (__any_sync(0xffffffffu, spec)) {
+                float as[2], hh[2], ll[2];
+                unpack2(acc, as[0], as[1]);
 #pragma unroll
-                for (int n = 0; n < (NC > 0 ? NC : 1); ++n) {
-                    const float2 x = exs[n * kPhiPts + threadIdx.x];
-                    rs = fmaf(x.x, ey[n].x, rs);
-                    rs = fmaf(-x.y, ey[n].y, rs);
+                for (int u = 0; u < 2; ++u) {
+                    float s_, ve, s2, e2;
+                    real_special(u ? f1 : f0, u, gh, gl, reinterpret_cast<const float4 *>(tab + 3 * (ci >> 9)),
+                                 items + (ci >> 9), ci & 255, fp64_below, r2_in, r2_out, saf, axis, nx, ny,
+                                 atoms + 3 * (a0 + a), shifts, zero_idx, rc, sa, as[u], s_, ve);
+                    dfa::two_sum(s_, u ? rv : ru, s2, e2);
+                    const float2 o = dfa::norm(dfa::acc{s2, __fadd_rn(ve, e2)});
+                    hh[u] = o.x;
+                    ll[u] = o.y;
                 }
+                oh = pack2(hh[0], hh[1]);
+                ol = pack2(ll[0], ll[1]);
+            }
+            if (DIG) {
+                int hi0, hi1, lo0, lo1;
+                digit_halves2(oh, ol, scl[a], full, valid0, valid1, dg.clamped, hi0, hi1, lo0, lo1);
+                const long long rsum = warp_sum_halves2(hi0, hi1, lo0, lo1);
+                if (lane == 0) wrow[warp][a] = rsum;
+                if (stores) store_digits2(xp, dg.slice, hi0, hi1, lo0, lo1);
+                xp += dg.rows_kpad;
             } else {
-                for (int n = 0; n < n1c; ++n) {
-                    const float2 x = exs[n * kPhiPts + threadIdx.x], y = erow[n];
-                    rs = fmaf(x.x, y.x, rs);
-                    rs = fmaf(-x.y, y.y, rs);
+                float h0, h1, l0, l1;
+                unpack2(oh, h0, h1);
+                unpack2(ol, l0, l1);
+                float2 *p = phit + (long long)(a0 + a) * ld + m;
+                if (valid0) p[0] = make_float2(h0, l0);
+                if (valid1) p[1] = make_float2(h1, l1);
+                if (psum) {  // column statistics for the centre and the scale: FP32 is enough (any
+                             // centre is corrected exactly; the max is exact); 32 points at a time
+                    float s0 = valid0 ? h0 : 0.f, s1 = valid1 ? h1 : 0.f;
+                    float mx = fmaxf(valid0 ? fabsf(h0) : 0.f, valid1 ? fabsf(h1) : 0.f);
+                    for (int o = 8; o > 0; o >>= 1) {
+                        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+                        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+                        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                    }
+                    if ((lane & 15) == 0) {
+                        wsum[2 * warp + (lane >> 4)][a] = s0 + s1;
+                        wmax[2 * warp + (lane >> 4)][a] = mx;
+                    }
                 }
             }
-            float s_, e_;
-            dfa::two_sum(v.s, rs, s_, e_);
-            v.s = s_;
-            v.e = __fadd_rn(v.e, e_);
         }
-        const float2 out = dfa::norm(v);
-        if (DIG) {
-            int I = 0;
-            if (valid) I = x_fixed(out.x, out.y, dg.scale[a0 + a], dg.clamped);
-            const long long rs = warp_sum_fixed(I);
-            if (lane == 0) wrow[warp][a] = rs;
-            if (m < dg.rows_kpad) digits4(I, dg.X0, dg.X1, dg.X2, dg.X3, (long long)(a0 + a) * dg.ldx + m);
-        } else if (valid) {
-            *prow = out;
-        }
-        if (!DIG && psum) {  // column statistics for the centre and the scale: FP32 is enough (any
-                     // centre is corrected exactly; the max is exact)
-            float sh = valid ? out.x : 0.f, mx = valid ? fabsf(out.x) : 0.f;
-            for (int o = 16; o > 0; o >>= 1) {
-                sh += __shfl_xor_sync(0xffffffffu, sh, o);
-                mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            }
-            if (lane == 0) {
-                wsum[warp][a] = sh;
-                wmax[warp][a] = mx;
-            }
-        }
+        e_lo = e_hi;
+        e_buf ^= 1;
+      }
     }
     if (DIG) {
         // the ESP row, from the CTAs of the first atom block
         if (blockIdx.y == 0) {
-            int I = 0;
-            if (valid) {
-                const double v = dg.Vc[m];
-                const float h = (float)v;
-                I = x_fixed(h, (float)(v - (double)h), vscale_of(*dg.vmax_p), dg.clamped);
-            }
-            const long long rs = warp_sum_fixed(I);
-            if (lane == 0) wrow[warp][AT] = rs;
-            if (m < dg.rows_kpad) digits4(I, dg.X0, dg.X1, dg.X2, dg.X3, (long long)dg.N * dg.ldx + m);
+            float h[2] = {0.f, 0.f}, l[2] = {0.f, 0.f};
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+                if (u ? valid1 : valid0) {
+                    const double v = dg.Vc[m + u];
+                    h[u] = (float)v;
+                    l[u] = (float)(v - (double)h[u]);
+                }
+            int hi0, hi1, lo0, lo1;
+            digit_halves2(pack2(h[0], h[1]), pack2(l[0], l[1]), vscale_of(*dg.vmax_p), full, valid0, valid1, dg.clamped,
+                          hi0, hi1, lo0, lo1);
+            const long long rsum = warp_sum_halves2(hi0, hi1, lo0, lo1);
+            if (lane == 0) wrow[warp][kPhiAtoms] = rsum;
+            if (stores) store_digits2(dg.X + dg.N * dg.rows_kpad + m, dg.slice, hi0, hi1, lo0, lo1);
         }
         __syncthreads();
         // exact row sums (two's complement int64 atomics: order-independent), one per CTA and row
-        if (threadIdx.x < na || (blockIdx.y == 0 && threadIdx.x == AT)) {
+        if (threadIdx.x < na || (blockIdx.y == 0 && threadIdx.x == kPhiAtoms)) {
             const int a = threadIdx.x;
             long long t = 0;
-            for (int w = 0; w < kPhiPts / 32; ++w) t += wrow[w][a];
-            if (t != 0) atomicAdd(dg.rowsum + (a == AT ? dg.N : a0 + a), (unsigned long long)t);
+            for (int w = 0; w < kPhiWarps; ++w) t += wrow[w][a];
+            if (t != 0) atomicAdd(dg.rowsum + (a == kPhiAtoms ? dg.N : a0 + a), (unsigned long long)t);
         }
     } else if (psum) {
         __syncthreads();
@@ -842,38 +1186,59 @@ __global__ void __launch_bounds__(kPhiPts, 7) phi_chunk_kernel(
     }
 }
 
-size_t phi_smem_bytes(int n1c, int scap, int at) {
-    return sizeof(float4) * 2 * (size_t)at * scap + sizeof(float2) * (size_t)n1c * kPhiPts;
+// Slots of the image table: about 1.4 times the images within Rc of a tile for all the CTA's
+// atoms (a tile that reaches more goes through its atoms in rounds), at least one atom's S for
+// each warp's half.
+int phi_slots(int S, int at, double rc, double volume) {
+    const double images = std::min<double>(S, 4.18879 * (rc + 3.0) * (rc + 3.0) * (rc + 3.0) / std::max(volume, 1.0));
+    const double want = std::min(1.4 * at * images + 32.0, 640.0);
+    return 2 * (int)(std::min<double>((double)at * S, std::max<double>(2.0 * S, want)) / 2.0 + 0.5);
+}
+// d's multiplier: ceil(2^(31 + s) / d), s = ceil(log2 d), exact for dividends below 2^31
+FastDiv fast_div_of(int d) {
+    int s = 0;
+    while ((1ll << s) < d) ++s;
+    return FastDiv{(unsigned)(((1ull << (31 + s)) + d - 1) / d), 31 + s};
+}
+size_t phi_smem_bytes(int n1c, bool regs, int slots) {
+    const size_t e = regs ? 2 * (size_t)kEBytes : sizeof(float4) * (size_t)n1c * kPhiThreads;
+    return sizeof(ulonglong2) * 3 * (size_t)slots + e + (sizeof(unsigned short) * (size_t)slots + 15) / 16 * 16;
 }
 
-// The instantiation for (KMAX 7 or any, digits or staged Phi, atoms per CTA)
-using PhiKernel = decltype(&phi_chunk_kernel<7, false, 16>);
-template <int AT>
-PhiKernel phi_kernel_for(bool regs, bool dig) {
-    return dig ? (regs ? phi_chunk_kernel<7, true, AT> : phi_chunk_kernel<0, true, AT>)
-               : (regs ? phi_chunk_kernel<7, false, AT> : phi_chunk_kernel<0, false, AT>);
-}
-PhiKernel phi_kernel(bool regs, bool dig, int at) {
-    switch (at) {
-        case 8: return phi_kernel_for<8>(regs, dig);
-        case 32: return phi_kernel_for<32>(regs, dig);
-        default: return phi_kernel_for<16>(regs, dig);
-    }
+// Atoms per CTA: the largest even split of the atoms into blocks of at most `cap` (32: a CTA's
+// start costs as much as 2.5 atoms of its loop; 0.293 ms with 32 atoms, 0.308 with 16 and 0.334
+// with 8 on 273 atoms and 121k points), into more blocks, of at least 8, while the CTAs
+// would not fill the GPU four times over.
+int phi_atoms_per_cta(int N, long long tiles, int cap, int resident) {
+    int blocks = (int)ceil_div(N, cap);
+    while (tiles * blocks < 4LL * resident && (int)ceil_div(N, blocks + 1) >= 8) ++blocks;
+    const int a = (int)ceil_div(N, blocks);
+    return (a + 1) & ~1;
 }
 
-void launch_phi(const int32_t *kept, long long m0, long long rows, const double *d_axis, const double *h_axis, int nx, int ny,
+// The instantiation for (KMAX 7 or any, digits or staged Phi)
+using PhiKernel = decltype(&phi_chunk_kernel<7, false>);
+PhiKernel phi_kernel(bool regs, bool dig) {
+    return dig ? (regs ? phi_chunk_kernel<7, true> : phi_chunk_kernel<0, true>)
+               : (regs ? phi_chunk_kernel<7, false> : phi_chunk_kernel<0, false>);
+}
+
+void launch_phi(const int32_t *kept, long long m0, long long rows, const double *d_axis, const double *h_axis,
+                const double *h_box, int nx, int ny,
                 const double *d_atoms, int N, const double *d_shifts, int S, int zero_idx, double rc, double sa,
                 const float4 *img, const float4 *EX, const float2 *E, int n1c, int parts, float2 *phit, long long ld,
-                double *psum, float *pmax, const PhiDigits *dig, cudaStream_t s, int at) {
-    if (at != 8 && at != 32) at = 16;
+                double *psum, float *pmax, const PhiDigits *dig, cudaStream_t s, int cap, int sm_count) {
+    if (cap != 8 && cap != 16) cap = 32;
     RP_REQUIRE(S >= 1 && S <= kMaxShifts, "more than 128 real-space shifts after pruning (cutoff too large for the cell)");
-    const int scap = (S + 31) / 32 * 32;
     const bool regs = (n1c == 7);  // KMAX 7: the specialised kernel
-    const size_t smem = phi_smem_bytes(n1c, scap, at);
-    // the static shared memory (the statistics and row-sum tiles, ~1.3 KB) counts against
-    // the same 48 KB default, so the opt-in is raised whenever the dynamic part could cross it
+    const double *b = h_box;
+    const double vol = std::fabs(b[0] * (b[4] * b[8] - b[5] * b[7]) - b[1] * (b[3] * b[8] - b[5] * b[6]) +
+                                 b[2] * (b[3] * b[7] - b[4] * b[6]));
+    const int at = phi_atoms_per_cta(N, ceil_div(rows, kPhiPts), cap, 8 * std::max(1, sm_count));
+    const int slots = phi_slots(S, at, rc, vol);
+    const size_t smem = phi_smem_bytes(n1c, regs, slots);
     RP_REQUIRE(smem <= 192 * 1024, "phi kernel: KMAX too large for shared memory");
-    auto kern = phi_kernel(regs, dig != nullptr, at);
+    auto kern = phi_kernel(regs, dig != nullptr);
     smem_optin((const void *)kern, std::max<size_t>(smem, 96 * 1024));
     AxisDF adf;
     for (int q = 0; q < 9; ++q) {
@@ -882,9 +1247,10 @@ void launch_phi(const int32_t *kept, long long m0, long long rows, const double 
     }
     dim3 grd(ceil_div(rows, kPhiPts), ceil_div(N, at));
     const PhiDigits dg = dig ? *dig : PhiDigits{};
-    kern<<<grd, kPhiPts, smem, s>>>(kept, m0, rows, d_axis, adf, nx, ny, d_atoms, N, d_shifts, S, scap, zero_idx, rc,
-                                    sa, (float)rc, (float)(sa * kSqrtLog2e), real_near2(), img, EX, E, n1c, parts,
-                                    phit, ld, psum, pmax, dg);
+    kern<<<grd, kPhiThreads, smem, s>>>(kept, m0, rows, d_axis, adf, nx, ny, fast_div_of(nx), fast_div_of(ny), d_atoms, N, d_shifts, S, at,
+                                        slots, zero_idx, rc, sa, (float)rc,
+                                        (float)(sa * kSqrtLog2e), real_near2(), img, EX, E, n1c, parts, phit, ld, psum,
+                                        pmax, dg);
     RP_LAUNCH_CHECK();
 }
 
@@ -1273,8 +1639,9 @@ void gram_mixed(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, con
     std::vector<float> hscale;
     const bool single = rn && clamp_dev && phi_bounds(ew, S, rn, N, ctx->bound_scale, hscale);
     float2 *phit = single ? nullptr : ctx->buf_t<float2>("m_phit" + slot, (size_t)N * chunk_pad);
-    __half *X[kGSlices];
-    for (int q = 0; q < kGSlices; ++q) X[q] = ctx->buf_t<__half>("m_X" + slot + std::to_string(q), (size_t)Np * chunk_pad);
+    __half *X[kGSlices];  // one buffer: the Phi kernel addresses the slices by their distance
+    X[0] = ctx->buf_t<__half>("m_X" + slot, (size_t)kGSlices * Np * chunk_pad);
+    for (int q = 1; q < kGSlices; ++q) X[q] = X[0] + (size_t)q * Np * chunk_pad;
     int *d_clamped = ctx->status_words() + 1;  // second status word: fixed-point range overflows
     const int nblk = (int)ceil_div(chunk, kPhiPts);
     double *psum = single ? nullptr : ctx->buf_t<double>("m_psum" + slot, (size_t)N * nblk);
@@ -1317,17 +1684,17 @@ void gram_mixed(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, con
         const int nb = (int)ceil_div(rows, kPhiPts);
         if (single) {  // Phi of the chunk straight to the digits of X
             StageTimer tt(ctx, "phi", stream);
-            // the slices' row stride is the chunk's padded length, as the Gram's tensor maps read them
-            const PhiDigits dg{X[0], X[1], X[2], X[3], rows_kpad, rows_kpad, scale, Vc_dev + m0, vmax,
+            // the digits' rows hold the chunk's padded length, as the Gram's tensor maps read them
+            const PhiDigits dg{X[0], (long long)Np * chunk_pad, rows_kpad, scale, Vc_dev + m0, vmax,
                                rowsum, clamp_dev, N};
-            launch_phi(kept_idx_dev, m0, rows, d_axis, ew->grid.axis, nx, ny, d_atoms, N, d_shifts, S, zero_idx,
+            launch_phi(kept_idx_dev, m0, rows, d_axis, ew->grid.axis, ew->box, nx, ny, d_atoms, N, d_shifts, S, zero_idx,
                        ew->cutoff, ew->sqrt_alpha, img, ew->d_exf, E, n1c, 3, nullptr, chunk_pad, nullptr, nullptr,
-                       &dg, stream, tiles.phi_atoms);
+                       &dg, stream, tiles.phi_atoms, ctx->sm_count);
         } else {
             StageTimer tt(ctx, "phi", stream);
-            launch_phi(kept_idx_dev, m0, rows, d_axis, ew->grid.axis, nx, ny, d_atoms, N, d_shifts, S, zero_idx, ew->cutoff,
+            launch_phi(kept_idx_dev, m0, rows, d_axis, ew->grid.axis, ew->box, nx, ny, d_atoms, N, d_shifts, S, zero_idx, ew->cutoff,
                        ew->sqrt_alpha, img, ew->d_exf, E, n1c, 3, phit, chunk_pad, psum, pmax, nullptr, stream,
-                       tiles.phi_atoms);
+                       tiles.phi_atoms, ctx->sm_count);
         }
         // 2. centre on the first chunk, a scale per chunk, fixed-point digits of X
         if (!single) {
@@ -1586,9 +1953,9 @@ extern "C" int rp_debug_mixed_phi(rp_ctx *ctx, const rp_ewald *ew, const double 
         images_df_kernel<<<ceil_div((long long)N * S, 128), 128>>>(d_atoms, N, d_shifts, S, img);
         RP_LAUNCH_CHECK();
         float2 *ph = ctx->buf_t<float2>("dbg_phi", (size_t)N * rows);
-        launch_phi(kept_idx_dev, 0, rows, d_axis, ew->grid.axis, ew->grid.n_grid[0], ew->grid.n_grid[1], d_atoms, N, d_shifts, S,
+        launch_phi(kept_idx_dev, 0, rows, d_axis, ew->grid.axis, ew->box, ew->grid.n_grid[0], ew->grid.n_grid[1], d_atoms, N, d_shifts, S,
                    zero_idx, ew->cutoff, ew->sqrt_alpha, img, ew->d_exf, E, ew->kmax, parts, ph, rows, nullptr,
-                   nullptr, nullptr, 0, kPhiAtoms);
+                   nullptr, nullptr, 0, kPhiAtoms, ctx->sm_count);
         df_to_double_kernel<<<ceil_div((long long)N * rows, 256), 256>>>(ph, (long long)N * rows, phi_dev);
         RP_LAUNCH_CHECK();
         RP_CUDA(cudaDeviceSynchronize());

@@ -46,6 +46,7 @@ struct RecipJob {
     float2 *W, *F, *E;
     double rb[9];          // reciprocal basis (rows)
     int N, ncols, K, P, ny, nz, ab;
+    int ecols;             // columns of E's rows (recip_cols)
 };
 constexpr int kRecipJobs = 64;
 struct RecipLaunch {
@@ -236,8 +237,8 @@ __global__ void __launch_bounds__(128) recip_stage_b_kernel(const __grid_constan
                 im[2 * u + 1] = fmaf(y.w, f.x, im[2 * u + 1]);
             }
         }
-        float2 *o = J.E + (((long long)l * ny + jj * kJB) * ncols + a0) * n1c + r;
-        const long long row_stride = (long long)ncols * n1c;
+        float2 *o = J.E + (((long long)l * ny + jj * kJB) * J.ecols + a0) * n1c + r;
+        const long long row_stride = (long long)J.ecols * n1c;
 #pragma unroll
         for (int u = 0; u < kJB; ++u)
             if (jj * kJB + u < ny) o[u * row_stride] = make_float2(re[u], im[u]);
@@ -256,10 +257,14 @@ size_t stage_b_smem(int P, int ny, int ab) {
 
 }  // namespace
 
+// E's rows hold an even number of atom columns, so that every second column of a KMAX 7 row
+// starts on a 16-byte boundary for the Phi kernel's copies
+static int recip_cols(int ncols) { return (ncols + 1) & ~1; }
+
 size_t recip_rows_bytes(const rp_ewald *ew, int ncols) {
     const int P = ew->kmax - 1, n1c = P + 1;
     const long long nrows = (long long)ew->grid.n_grid[1] * ew->grid.n_grid[2];
-    return sizeof(float2) * (size_t)nrows * ncols * n1c;
+    return sizeof(float2) * (size_t)nrows * recip_cols(ncols) * n1c;
 }
 
 void recip_rows_group(rp_ctx *ctx, const std::vector<RecipRowsJob> &jobs, cudaStream_t stream,
@@ -308,6 +313,7 @@ void recip_rows_group(rp_ctx *ctx, const std::vector<RecipRowsJob> &jobs, cudaSt
             J.E = rj.E;
             for (int q = 0; q < 9; ++q) J.rb[q] = ew->rec[q];
             J.N = rj.N; J.ncols = ncols; J.K = ew->K; J.P = P; J.ny = ny; J.nz = nz; J.ab = stage_b_columns(P);
+            J.ecols = rj.d_q ? 1 : recip_cols(ncols);
             const int nb = (n1c + kN1B - 1) / kN1B;
             const int k = L.n;
             blk[0][k + 1] = blk[0][k] + (int)ceil_div((long long)rj.N * 3 * nw, 128);

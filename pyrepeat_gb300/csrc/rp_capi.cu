@@ -906,7 +906,7 @@ int rp_autotune(rp_ctx *ctx, int n, const rp_fit_desc *descs, const double *cons
                         RP_CUDA(cudaEventElapsedTime(&t, e0, e1));
                         if (rep > 0) ms = std::min(ms, t);
                     }
-                    if (at == 16 && split == 16) default_ms = ms;
+                    if (at == TileConfig{}.phi_atoms && split == TileConfig{}.gram_split) default_ms = ms;
                     if (ms < best_ms) {
                         best_ms = ms;
                         best = tc;

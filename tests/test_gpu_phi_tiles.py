@@ -1,0 +1,81 @@
+"""The Phi kernel at the edges of its tiles: 128 points per CTA in pairs, atoms in blocks, E values
+staged per run of points in one grid row (four atoms at a time up to 32 runs, two up to
+64, one beyond), an image table that a tile may overflow.  Against the oracle's FP64 Phi of the
+same points, within the 1e-6 of max|Phi| that every mixed Phi value is held to."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from conftest import load_golden
+
+pytestmark = pytest.mark.gpu
+
+
+def _phi(ctx, cube, atoms, idx, kmax, parts=3):
+    import torch
+    L = ctx.lib
+    L.rp_debug_mixed_phi.restype = ctypes.c_int
+    L.rp_debug_mixed_phi.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int,
+                                     ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, ctypes.c_void_p]
+    ew = ctx.ewald(cube.n_grid, cube.axis_vector, cube.cutoff, kmax)
+    kept = torch.from_numpy(np.ascontiguousarray(idx, dtype=np.int32)).cuda()
+    out = torch.zeros((len(atoms), len(idx)), dtype=torch.float64, device="cuda")
+    try:
+        ctx.check(L.rp_debug_mixed_phi(ctx.ptr, ew.ptr, atoms.ctypes.data, len(atoms), kept.data_ptr(), len(idx),
+                                       parts, out.data_ptr()))
+    finally:
+        ew.close()
+    return out.cpu().numpy().T
+
+
+def _reference(oracle_mod, cube, atoms, idx, kmax):
+    from pyrepeat_gb300 import synth
+    nx, ny = int(cube.n_grid[0]), int(cube.n_grid[1])
+    i, j, k = idx % nx, (idx // nx) % ny, idx // (nx * ny)
+    g = i[:, None] * cube.axis_vector[0] + j[:, None] * cube.axis_vector[1] + k[:, None] * cube.axis_vector[2]
+    box = cube.box_vectors
+    _, kv, kc = synth.kspace(box, cube.cutoff, kmax)
+    sh = synth.realspace_shifts(box, cube.cutoff)
+    zero = int(np.flatnonzero((sh == 0.0).all(axis=1))[0])
+    return oracle_mod.phi(g, atoms, kv, kc, sh, zero, cube.cutoff)
+
+
+def _check(got, ref):
+    assert np.abs(got - ref).max() <= 1e-6 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("kmax", [7, 3])
+@pytest.mark.parametrize("n,rows,order", [(1, 1, "flat"), (1, 127, "flat"), (2, 128, "shuffled"), (9, 129, "flat"),
+                                          (31, 66, "shuffled"), (33, 257, "flat"), (40, 384, "shuffled"),
+                                          (37, 250, "pairs")])
+def test_phi_at_tile_edges(n, rows, order, kmax, gpu_ctx, oracle_mod):
+    cube, g = load_golden("tricmini")
+    atoms = np.ascontiguousarray(cube.atom_pos[:n], dtype=np.float64)
+    idx = np.flatnonzero(g["mask"])
+    if order != "flat":
+        idx = np.random.default_rng(n).permutation(idx)
+    if order == "pairs":  # runs of two points: more than 32 and at most 64 or so per tile
+        idx = np.stack([idx[:rows], np.minimum(idx[:rows] + 1, cube.n_points - 1)], axis=1).ravel()
+    idx = idx[:rows]
+    _check(_phi(gpu_ctx, cube, atoms, idx, kmax), _reference(oracle_mod, cube, atoms, idx, kmax))
+
+
+@pytest.mark.parametrize("n", [7, 32])
+def test_phi_small_cell_overflows_the_image_table(n, gpu_ctx, oracle_mod):
+    """A 12 Bohr cell: ~9 of its up to 125 images per atom are within the cutoff of a point, and
+    a tile of points spread over the cell reaches several times as many."""
+    from pyrepeat_gb300 import synth
+    rng = np.random.default_rng(3)
+    ng = np.array([40, 41, 43])
+    cell = np.diag([12.0, 12.5, 13.0])
+    atoms = np.ascontiguousarray(rng.random((n, 3)) @ cell)
+    cube = synth.Cube(np.full(n, 6), atoms, ng, cell / ng[:, None], None)
+    idx = rng.permutation(cube.n_points)[:300]
+    nx, ny = int(ng[0]), int(ng[1])
+    p = np.stack([idx % nx, (idx // nx) % ny, idx // (nx * ny)], axis=1) @ cube.axis_vector
+    far = np.ones(len(idx), bool)  # points at least 1 Bohr from every image, as after a vdW filter
+    for s in synth.realspace_shifts(cell, 1.0):
+        far &= (np.linalg.norm(p[:, None] - (atoms + s)[None], axis=2) > 1.0).all(axis=1)
+    idx = idx[far]
+    _check(_phi(gpu_ctx, cube, atoms, idx, 7), _reference(oracle_mod, cube, atoms, idx, 7))
