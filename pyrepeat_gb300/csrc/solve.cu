@@ -59,7 +59,6 @@ __global__ void build_bordered_kernel(const SolveDesc *__restrict__ descs, const
         } else {
             v = 0.0;
         }
-        d.As[t] = v;
         d.A0[t] = v;
         if (c == 0) {
             double bv;
@@ -75,7 +74,32 @@ __global__ void build_bordered_kernel(const SolveDesc *__restrict__ descs, const
     }
 }
 
-constexpr int kLU = 1024;
+// A warp per row of a system to be solved in its CTA: the FP32 copy of the bordered matrix (into the
+// first half of As) and the row sums of |K| (into r) and of |A|, A the folded normal matrix
+// without the border (into x), for the solve kernel's norms.  Across the GPU because FP64
+// conversions and additions run at 1/64 of the FP32 rate: in the system's own CTA they took 45
+// (copy) + 69 + 68 us (norms) at 425 unknowns.
+__global__ void __launch_bounds__(256) prepare_kernel(const SolveDesc *__restrict__ descs) {
+    const SolveDesc d = descs[blockIdx.y];
+    const int n1 = d.n + 1, r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (d.wide64 || d.host32 || r >= n1) return;
+    const double *row = d.A0 + (size_t)r * n1;
+    float *L = reinterpret_cast<float *>(d.As) + (size_t)r * n1;
+    double s = 0.0;
+    for (int c = lane; c < n1; c += 32) {
+        const double v = row[c];
+        L[c] = (float)v;
+        s += c < d.n ? fabs(v) : 0.0;
+    }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+        d.r[r] = s + fabs(row[d.n]);
+        d.x[r] = r < d.n ? s : 0.0;
+    }
+}
+
+constexpr int kLU = 1024;    // threads of a panel CTA of the factorisation across the GPU
+constexpr int kSolve = 768;  // most threads of a solve CTA (solve_threads): 80 registers each
 
 __device__ void block_argmax(double v, int idx, double *sv, int *si, double *out_v, int *out_i) {
     // max |v| with lowest index on ties (deterministic)
@@ -88,8 +112,8 @@ __device__ void block_argmax(double v, int idx, double *sv, int *si, double *out
     if (lane == 0) { sv[w] = v; si[w] = idx; }
     __syncthreads();
     if (w == 0) {
-        v = (lane < kLU / 32) ? sv[lane] : -1.0;
-        idx = (lane < kLU / 32) ? si[lane] : 0x7fffffff;
+        v = (lane < (int)(blockDim.x >> 5)) ? sv[lane] : -1.0;
+        idx = (lane < (int)(blockDim.x >> 5)) ? si[lane] : 0x7fffffff;
         for (int o = 16; o > 0; o >>= 1) {
             double ov = __shfl_down_sync(0xffffffffu, v, o);
             int oi = __shfl_down_sync(0xffffffffu, idx, o);
@@ -98,6 +122,47 @@ __device__ void block_argmax(double v, int idx, double *sv, int *si, double *out
         if (lane == 0) { *out_v = v; *out_i = idx; }
     }
     __syncthreads();
+}
+
+// max of non-negative doubles over the block (their bits order like the values, so no FP64
+// instruction runs: one holds that pipe for 16 cycles per warp); every thread gets the
+// result.  `active`: the threads that may hold a non-zero value, a prefix.
+__device__ double block_max(double v, int active, double *sv) {
+    const int warp = threadIdx.x >> 5, nw = min((active + 31) >> 5, (int)(blockDim.x >> 5));
+    unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    auto warp_max = [](unsigned long long x) {
+        const unsigned hi = (unsigned)(x >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+        const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)x : 0u);
+        return ((unsigned long long)mh << 32) | ml;
+    };
+    unsigned long long *sb = reinterpret_cast<unsigned long long *>(sv);
+    __syncthreads();
+    if (warp < nw) {
+        b = warp_max(b);
+        if ((threadIdx.x & 31) == 0) sb[warp] = b;
+    }
+    __syncthreads();
+    b = warp_max((threadIdx.x & 31) < nw ? sb[threadIdx.x & 31] : 0ull);
+    return __longlong_as_double((long long)b);
+}
+
+// sum over the block in a fixed order; every thread gets the result.  `active` as above.
+__device__ double block_sum(double v, int active, double *sv) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31,
+              nw = min((active + 31) >> 5, (int)(blockDim.x >> 5));
+    __syncthreads();
+    if (warp < nw) {
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) sv[warp] = v;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        double t = lane < nw ? sv[lane] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) sv[32] = t;
+    }
+    __syncthreads();
+    return sv[32];
 }
 
 __device__ void lu_apply(const double *__restrict__ LU, const int *__restrict__ perm, int n1, double *__restrict__ y,
@@ -111,7 +176,7 @@ __device__ void lu_apply(const double *__restrict__ LU, const int *__restrict__ 
     __shared__ double yb[32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __syncthreads();
-    for (int t = threadIdx.x; t < n1; t += kLU) ysh[t] = y[t];
+    for (int t = threadIdx.x; t < n1; t += blockDim.x) ysh[t] = y[t];
     __syncthreads();
     if (threadIdx.x == 0) {
         int k = 0;
@@ -131,7 +196,7 @@ __device__ void lu_apply(const double *__restrict__ LU, const int *__restrict__ 
     __syncthreads();
     for (int c0 = 0; c0 < n1; c0 += 32) {  // forward: L, unit diagonal
         const int bs = min(32, n1 - c0);
-        for (int t = threadIdx.x; t < bs * 32; t += kLU) {
+        for (int t = threadIdx.x; t < bs * 32; t += blockDim.x) {
             const int r = t >> 5, c = t & 31;
             blk[r][c] = c < bs ? LU[(size_t)(c0 + r) * n1 + c0 + c] : 0.0;
         }
@@ -146,7 +211,7 @@ __device__ void lu_apply(const double *__restrict__ LU, const int *__restrict__ 
             yb[lane] = lane < bs ? yv : 0.0;
         }
         __syncthreads();
-        for (int r = c0 + bs + threadIdx.x; r < n1; r += kLU) {
+        for (int r = c0 + bs + threadIdx.x; r < n1; r += blockDim.x) {
             const double *row = LU + (size_t)r * n1 + c0;
             double t = 0.0;
             for (int c = 0; c < bs; ++c) t += row[c] * yb[c];
@@ -156,7 +221,7 @@ __device__ void lu_apply(const double *__restrict__ LU, const int *__restrict__ 
     }
     for (int c1 = n1; c1 > 0; c1 -= 32) {  // backward: U
         const int c0 = max(0, c1 - 32), bs = c1 - c0;
-        for (int t = threadIdx.x; t < bs * 32; t += kLU) {
+        for (int t = threadIdx.x; t < bs * 32; t += blockDim.x) {
             const int r = t >> 5, c = t & 31;
             blk[r][c] = c < bs ? LU[(size_t)(c0 + r) * n1 + c0 + c] : 0.0;
         }
@@ -172,7 +237,7 @@ __device__ void lu_apply(const double *__restrict__ LU, const int *__restrict__ 
             yb[lane] = lane < bs ? yv : 0.0;
         }
         __syncthreads();
-        for (int r = threadIdx.x; r < c0; r += kLU) {
+        for (int r = threadIdx.x; r < c0; r += blockDim.x) {
             const double *row = LU + (size_t)r * n1 + c0;
             double t = 0.0;
             for (int c = 0; c < bs; ++c) t += row[c] * yb[c];
@@ -180,23 +245,10 @@ __device__ void lu_apply(const double *__restrict__ LU, const int *__restrict__ 
         }
         __syncthreads();
     }
-    for (int t = threadIdx.x; t < n1; t += kLU) y[t] = ysh[t];
+    for (int t = threadIdx.x; t < n1; t += blockDim.x) y[t] = ysh[t];
     __syncthreads();
 }
 
-// max over the block (every thread gets the result)
-__device__ double block_max(double v, double *sv) {
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) sv[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double t = sv[0];
-    for (int w = 1; w < kLU / 32; ++w) t = fmax(t, sv[w]);
-    return t;
-}
-
-// FP32 LU with partial pivoting in place (row-major n1 x n1).  Returns false on a
-// zero or non-finite pivot (the same value in every thread).
 // max |v| with the lowest index on ties (deterministic), FP32: the FP32 factorisation's
 // pivot search stays off the FP64 pipe (a warp-wide FP64 compare holds that pipe for
 // 16 cycles, and every warp of the CTA runs this at every column)
@@ -210,8 +262,8 @@ __device__ void block_argmax_f(float v, int idx, float *sv, int *si, int *out_i)
     if (lane == 0) { sv[w] = v; si[w] = idx; }
     __syncthreads();
     if (w == 0) {
-        v = (lane < kLU / 32) ? sv[lane] : -1.0f;
-        idx = (lane < kLU / 32) ? si[lane] : 0x7fffffff;
+        v = (lane < (int)(blockDim.x >> 5)) ? sv[lane] : -1.0f;
+        idx = (lane < (int)(blockDim.x >> 5)) ? si[lane] : 0x7fffffff;
         for (int o = 16; o > 0; o >>= 1) {
             const float ov = __shfl_down_sync(0xffffffffu, v, o);
             const int oi = __shfl_down_sync(0xffffffffu, idx, o);
@@ -230,15 +282,15 @@ __device__ bool lu_factor_f32(float *A, int *perm, int n1, double *sv, int *si, 
     for (int k = 0; k < n1; ++k) {
         float best = -1.0f;
         int bi = 0x7fffffff;
-        for (int r = k + threadIdx.x; r < n1; r += kLU) {
+        for (int r = k + threadIdx.x; r < n1; r += blockDim.x) {
             const float v = fabsf(A[(size_t)r * n1 + k]);
             if (v > best || (v == best && r < bi)) { best = v; bi = r; }
         }
         block_argmax_f(best, bi, svf, si, piv_i);
-        const int p = *piv_i;
+        const int p = *piv_i < n1 ? *piv_i : k;  // no candidate (NaN): stay
         if (threadIdx.x == 0) perm[k] = p;
         if (p != k)
-            for (int c = threadIdx.x; c < n1; c += kLU) {
+            for (int c = threadIdx.x; c < n1; c += blockDim.x) {
                 const float t = A[(size_t)k * n1 + c];
                 A[(size_t)k * n1 + c] = A[(size_t)p * n1 + c];
                 A[(size_t)p * n1 + c] = t;
@@ -250,11 +302,11 @@ __device__ bool lu_factor_f32(float *A, int *perm, int n1, double *sv, int *si, 
         fmin_p = fminf(fmin_p, apv);
         fmax_p = fmaxf(fmax_p, apv);
         const float inv = 1.0f / pv;
-        for (int r = k + 1 + threadIdx.x; r < n1; r += kLU) A[(size_t)r * n1 + k] *= inv;
+        for (int r = k + 1 + threadIdx.x; r < n1; r += blockDim.x) A[(size_t)r * n1 + k] *= inv;
         __syncthreads();
         // rank-1 update: a warp per row, lanes along the row (coalesced, no index division)
         const float *prow = A + (size_t)k * n1;
-        for (int rr = k + 1 + (threadIdx.x >> 5); rr < n1; rr += kLU / 32) {
+        for (int rr = k + 1 + (threadIdx.x >> 5); rr < n1; rr += (int)(blockDim.x >> 5)) {
             float *row = A + (size_t)rr * n1;
             const float l = row[k];
             for (int cc = k + 1 + (threadIdx.x & 31); cc < n1; cc += 32) row[cc] -= l * prow[cc];
@@ -267,125 +319,193 @@ __device__ bool lu_factor_f32(float *A, int *perm, int n1, double *sv, int *si, 
     return true;
 }
 
-// x = (P L U)^{-1} y with the FP32 factors; y (overwritten) and x in shared memory.
-// One barrier per column: forward elimination updates y below the column, backward
-// substitution writes x[c] and updates y above it.
-// Blocked FP32 LU with partial pivoting (right-looking, panels of 32 columns), in place, for
-// n1 <= kLUBlockedMax.  Per panel: the panel's rows (32 columns, stride 33 against bank
-// conflicts) are factored in shared memory with the same partial pivoting; its row swaps
-// are applied to the other columns (one thread per column, the swaps in order); U12 is
-// solved against the panel's unit-lower block; and the trailing matrix takes one rank-32
-// update per panel, staged through a 32 x 64 tile of U12, instead of 32 rank-1 updates
-// that each re-read it from L2.  smem: n1 * 33 + 32 * 64 floats.  false on a zero pivot.
+// Blocked FP32 LU with partial pivoting (right-looking, panels of 32 columns), in place, for systems
+// of at most one row per thread; false on a zero or non-finite pivot.  Every element takes
+// its updates one column at a time in column order (as an unblocked factorisation), so the
+// factors do not depend on the blocking.
+// What bounded the first form of it (panel rows in shared memory, one output per thread in the
+// trailing update): two shared-memory reads per multiply-add and four barriers per column,
+// 3.0 us per column at 425 unknowns.  Here a thread holds its row of the panel in registers;
+// a column costs two barriers (the pivot search's partial results, then the pivot row); rows
+// change places by their position numbers only, and the panel's net permutation is applied
+// to the other columns through shared memory in one pass; the trailing update computes 8 rows x
+// 4 columns per thread (6 shared-memory reads per 32 multiply-adds).
+// orig[i]: the row of the input that ends up as row i.  work: 64 n1 floats of shared memory.
 constexpr int kLUNB = 32;
-constexpr int kLUBlockedMax = 1536;
-constexpr int kLUTile = 64;
-__device__ bool lu_factor_f32_blocked(float *A, int *perm, int n1, float *smem, float *svf, int *si, int *piv_i,
-                                      double &pmin, double &pmax) {
-    float *P = smem;                                  // [n1][33] panel rows k0..n1-1
-    float *U = smem + (size_t)n1 * (kLUNB + 1);       // [32][kLUTile] tile of U12
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+constexpr int kLUBlockedMax = kSolve;
+struct LuShared {
+    unsigned key[2][32];                 // per warp: the largest |value| of the column (bits)
+    int pos[2][32];                      // and the lowest position that has it
+    float prow[2][kLUNB];                // the pivot row
+    __align__(16) float l11[kLUNB][kLUNB + 4];  // L11 by columns
+    int src[2 * kLUNB], dst[2 * kLUNB];  // rows of the panel's net permutation
+    int moved;                           // entries beyond the first kLUNB
+};
+template <int NI>
+__device__ __forceinline__ void lu_trailing_tile(float *A, int n1, const float *L, const float *U, int nb, int r,
+                                                 int nr, int c, int nc, int ld) {
+    // rows r .. r+7 (nr of them exist), columns c + 32 i (lane-strided; nc of the warp's 32 NI exist)
+    float acc[8][NI];
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            acc[k][i] = (k < nr && lane + 32 * i < nc) ? A[(size_t)(r + k) * n1 + c + 32 * i] : 0.f;
+#pragma unroll 4
+    for (int j = 0; j < nb; ++j) {
+        const float4 la = *reinterpret_cast<const float4 *>(L + (size_t)j * ld),
+                     lb = *reinterpret_cast<const float4 *>(L + (size_t)j * ld + 4);
+        const float l[8] = {la.x, la.y, la.z, la.w, lb.x, lb.y, lb.z, lb.w};
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const float u = U[(size_t)j * ld + 32 * i];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[k][i] = fmaf(-l[k], u, acc[k][i]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k < nr && lane + 32 * i < nc) A[(size_t)(r + k) * n1 + c + 32 * i] = acc[k][i];
+}
+__device__ bool lu_factor_f32_blocked(float *A, int *orig, int n1, float *work, LuShared &sh, double &pmin,
+                                      double &pmax) {
+    const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
+    const int ld = (n1 + 3) & ~3;            // work rows: 16-byte aligned
+    float *S = work, *LT = work + (size_t)kLUNB * ld;  // [32][ld] each: the top rows / U12, and L21 by columns
     float fmin_p = 3.0e38f, fmax_p = 0.f;
+    for (int t = tid; t < n1; t += nt) orig[t] = t;
     bool ok = true;
     for (int k0 = 0; k0 < n1; k0 += kLUNB) {
-        const int nb = min(kLUNB, n1 - k0), m = n1 - k0;
-        // 1. the panel into shared memory
-        for (int t = threadIdx.x; t < m * kLUNB; t += kLU) {
-            const int r = t >> 5, c = t & 31;
-            P[r * (kLUNB + 1) + c] = c < nb ? A[(size_t)(k0 + r) * n1 + k0 + c] : 0.f;
-        }
+        const int nb = min(kLUNB, n1 - k0), m = n1 - k0, c1 = k0 + nb;
+        const bool own = tid < m;  // this thread's row of the panel: position tid at first
+        // 1. the panel's rows, coalesced through shared memory, into registers
         __syncthreads();
-        // 2. factor the panel (partial pivoting over all its rows)
-        for (int j = 0; j < nb; ++j) {
-            float best = -1.0f;
-            int bi = 0x7fffffff;
-            for (int r = j + threadIdx.x; r < m; r += kLU) {
-                const float v = fabsf(P[r * (kLUNB + 1) + j]);
-                if (v > best || (v == best && r < bi)) { best = v; bi = r; }
+        for (int r = warp; r < m; r += nw) work[r * 33 + lane] = lane < nb ? A[(size_t)(k0 + r) * n1 + k0 + lane] : 0.f;
+        __syncthreads();
+        float a[kLUNB];
+#pragma unroll
+        for (int c = 0; c < kLUNB; ++c) a[c] = own ? work[tid * 33 + c] : 0.f;
+        const int my_orig = own ? orig[k0 + tid] : 0;
+        int pos = own ? tid : 0x7fffffff;
+        // 2. factor it
+#pragma unroll
+        for (int j = 0; j < kLUNB; ++j) {
+            if (j < nb && ok) {
+                const int b = j & 1;
+                const bool in = own && pos >= j;
+                const float v = fabsf(a[j]);
+                // a NaN never wins the search, as in a comparison
+                const unsigned bits = in && v == v ? __float_as_uint(v) + 1u : 0u;  // 0: no candidate
+                unsigned best = __reduce_max_sync(0xffffffffu, bits);
+                int at = __reduce_min_sync(0xffffffffu, bits == best ? pos : 0x7fffffff);
+                if (lane == 0) {
+                    sh.key[b][warp] = best;
+                    sh.pos[b][warp] = at;
+                }
+                __syncthreads();
+                const unsigned kb = lane < nw ? sh.key[b][lane] : 0u;
+                best = __reduce_max_sync(0xffffffffu, kb);
+                at = __reduce_min_sync(0xffffffffu, kb == best && lane < nw ? sh.pos[b][lane] : 0x7fffffff);
+                const float apv = __uint_as_float(best - 1u);
+                if (best <= 1u || !(apv <= 3.402823466e38f)) {
+                    ok = false;  // uniform: zero, infinite or no pivot
+                } else {
+                    fmin_p = fminf(fmin_p, apv);
+                    fmax_p = fmaxf(fmax_p, apv);
+                    if (pos == at) {  // the pivot row: publish it, and trade places with position j
+#pragma unroll
+                        for (int c = j; c < kLUNB; ++c) sh.prow[b][c] = a[c];
+                        pos = j;
+                    } else if (pos == j) {
+                        pos = at;
+                    }
+                    __syncthreads();
+                    if (own && pos > j) {
+                        const float l = a[j] * (1.0f / sh.prow[b][j]);
+                        a[j] = l;
+#pragma unroll
+                        for (int c = j + 1; c < kLUNB; ++c) a[c] = fmaf(-l, sh.prow[b][c], a[c]);
+                    }
+                }
             }
-            block_argmax_f(best, bi, svf, si, piv_i);
-            const int p = *piv_i;
-            if (threadIdx.x == 0) perm[k0 + j] = k0 + p;
-            if (p != j && threadIdx.x < kLUNB) {
-                const float t = P[j * (kLUNB + 1) + threadIdx.x];
-                P[j * (kLUNB + 1) + threadIdx.x] = P[p * (kLUNB + 1) + threadIdx.x];
-                P[p * (kLUNB + 1) + threadIdx.x] = t;
-            }
-            __syncthreads();
-            const float pv = P[j * (kLUNB + 1) + j];
-            const float apv = fabsf(pv);
-            if (!(apv > 0.f) || !isfinite(pv)) {
-                ok = false;
-                break;  // uniform: every thread read the same pivot
-            }
-            fmin_p = fminf(fmin_p, apv);
-            fmax_p = fmaxf(fmax_p, apv);
-            const float inv = 1.0f / pv;
-            // scale the column and update the panel's remaining columns: a thread per row, so a
-            // warp instruction covers 32 rows of one column with every lane busy (stride 33:
-            // no bank conflicts; the pivot row is a broadcast)
-            const float *pj = P + j * (kLUNB + 1);
-            for (int r = j + 1 + threadIdx.x; r < m; r += kLU) {
-                float *row = P + r * (kLUNB + 1);
-                const float l = row[j] * inv;
-                row[j] = l;
-                for (int c = j + 1; c < nb; ++c) row[c] -= l * pj[c];
-            }
-            __syncthreads();
         }
         if (!ok) break;
-        // 3. the factored panel back to global memory
-        for (int t = threadIdx.x; t < m * kLUNB; t += kLU) {
-            const int r = t >> 5, c = t & 31;
-            if (c < nb) A[(size_t)(k0 + r) * n1 + k0 + c] = P[r * (kLUNB + 1) + c];
-        }
-        // 4. the panel's row swaps on every other column (a thread per column, swaps in order)
-        for (int c = threadIdx.x; c < n1; c += kLU) {
-            if (c >= k0 && c < k0 + nb) continue;
-            for (int j = 0; j < nb; ++j) {
-                const int p = perm[k0 + j];
-                if (p != k0 + j) {
-                    const float t = A[(size_t)(k0 + j) * n1 + c];
-                    A[(size_t)(k0 + j) * n1 + c] = A[(size_t)p * n1 + c];
-                    A[(size_t)p * n1 + c] = t;
-                }
+        // 3. the factored panel back, rows in their new places; the permutation's entries
+        __syncthreads();
+        if (own) {
+            orig[k0 + pos] = my_orig;
+#pragma unroll
+            for (int c = 0; c < kLUNB; ++c) work[pos * 33 + c] = a[c];
+            if (pos < nb) {
+                sh.src[pos] = k0 + tid;
+                sh.dst[pos] = k0 + pos;
+#pragma unroll
+                for (int c = 0; c < kLUNB; ++c) sh.l11[c][pos] = a[c];
             }
         }
+        if (tid == 0) sh.moved = kLUNB;
         __syncthreads();
-        const int c1 = k0 + nb;
+        for (int r = warp; r < m; r += nw)
+            if (lane < nb) A[(size_t)(k0 + r) * n1 + k0 + lane] = work[r * 33 + lane];
+        if (own && pos >= nb && pos != tid) {
+            const int e = atomicAdd(&sh.moved, 1);  // at most nb rows leave the top
+            sh.src[e] = k0 + tid;
+            sh.dst[e] = k0 + pos;
+        }
+        __syncthreads();
+        // 4. the permutation on the other columns, through shared memory
+        const int moved = sh.moved;
+        for (int e = warp; e < moved; e += nw) {
+            if (e >= nb && e < kLUNB) continue;
+            const bool same = sh.src[e] == sh.dst[e];
+            const float *row = A + (size_t)sh.src[e] * n1;
+            for (int c = (same ? c1 : 0) + lane; c < n1; c += 32)
+                if (c < k0 || c >= c1) S[(size_t)e * ld + c] = row[c];
+        }
+        __syncthreads();
+        for (int e = warp; e < moved; e += nw) {
+            if ((e >= nb && e < kLUNB) || sh.src[e] == sh.dst[e]) continue;
+            float *row = A + (size_t)sh.dst[e] * n1;
+            const int hi = e < kLUNB ? k0 : n1;  // the top rows' right part is U12, below
+            for (int c = lane; c < hi; c += 32)
+                if (c < k0 || c >= c1) row[c] = S[(size_t)e * ld + c];
+        }
         if (c1 >= n1) break;
-        // 5. U12 = L11^-1 A12 (unit lower L11 from the panel), a thread per column
-        for (int c = c1 + threadIdx.x; c < n1; c += kLU) {
+        __syncthreads();  // the displaced rows' copies are no longer needed: L21 takes their place
+        if (own && pos >= nb)
+#pragma unroll
+            for (int j = 0; j < kLUNB; ++j) LT[(size_t)j * ld + pos - nb] = a[j];
+        // 5. U12 = L11^-1 A12 (unit lower L11), a thread per column
+        for (int c = c1 + tid; c < n1; c += nt) {
             float u[kLUNB];
 #pragma unroll
-            for (int j = 0; j < kLUNB; ++j) u[j] = j < nb ? A[(size_t)(k0 + j) * n1 + c] : 0.f;
+            for (int j = 0; j < kLUNB; ++j) u[j] = j < nb ? S[(size_t)j * ld + c] : 0.f;
 #pragma unroll
             for (int j = 0; j < kLUNB; ++j)
 #pragma unroll
-                for (int i = j + 1; i < kLUNB; ++i) u[i] -= P[i * (kLUNB + 1) + j] * u[j];
+                for (int i = j + 1; i < kLUNB; ++i) u[i] = fmaf(-sh.l11[j][i], u[j], u[i]);
 #pragma unroll
             for (int j = 0; j < kLUNB; ++j)
-                if (j < nb) A[(size_t)(k0 + j) * n1 + c] = u[j];
+                if (j < nb) {
+                    S[(size_t)j * ld + c] = u[j];
+                    A[(size_t)(k0 + j) * n1 + c] = u[j];
+                }
         }
         __syncthreads();
-        // 6. A22 -= L21 U12, column tiles of kLUTile staged in shared memory
-        for (int t0 = c1; t0 < n1; t0 += kLUTile) {
-            const int w = min(kLUTile, n1 - t0);
-            for (int t = threadIdx.x; t < kLUNB * kLUTile; t += kLU) {
-                const int j = t / kLUTile, c = t - j * kLUTile;
-                U[t] = (j < nb && c < w) ? A[(size_t)(k0 + j) * n1 + t0 + c] : 0.f;
-            }
-            __syncthreads();
-            const int c = threadIdx.x % kLUTile;
-            if (c < w)
-                for (int r = nb + threadIdx.x / kLUTile; r < m; r += kLU / kLUTile) {
-                    const float *l = P + r * (kLUNB + 1);
-                    float acc = A[(size_t)(k0 + r) * n1 + t0 + c];
-#pragma unroll
-                    for (int j = 0; j < kLUNB; ++j) acc -= l[j] * U[j * kLUTile + c];
-                    A[(size_t)(k0 + r) * n1 + t0 + c] = acc;
-                }
-            __syncthreads();
+        // 6. A22 -= L21 U12
+        const int mr = m - nb, mc = n1 - c1;
+        const int tiles_r = (mr + 7) / 8, tiles_c = (mc + 127) / 128;
+        for (int t = warp; t < tiles_r * tiles_c; t += nw) {
+            const int tc = t / tiles_r, r = (t - tc * tiles_r) * 8, c = tc * 128;
+            const float *l = LT + r, *u = S + c1 + c + lane;
+            const int nc = min(128, mc - c), nr = min(8, mr - r), row = c1 + r, col = c1 + c + lane;
+            if (nc > 96) lu_trailing_tile<4>(A, n1, l, u, nb, row, nr, col, nc, ld);
+            else if (nc > 64) lu_trailing_tile<3>(A, n1, l, u, nb, row, nr, col, nc, ld);
+            else if (nc > 32) lu_trailing_tile<2>(A, n1, l, u, nb, row, nr, col, nc, ld);
+            else lu_trailing_tile<1>(A, n1, l, u, nb, row, nr, col, nc, ld);
         }
     }
     pmin = fmin(pmin, (double)fmin_p);
@@ -394,93 +514,139 @@ __device__ bool lu_factor_f32_blocked(float *A, int *perm, int n1, float *smem, 
     return ok;
 }
 
-// Solve LU x = P y in FP32 (unit lower L, upper U, both in LU), blocked by 32 columns: the
-// 32x32 diagonal block is staged in shared memory and solved by one warp (shuffles, no block
-// barrier), then every warp updates the remaining rows with the block's 32 values (a warp per
-// row, coalesced).  Three block barriers per 32 columns instead of one per column.
-__device__ void lu_apply_f32(const float *__restrict__ LU, const int *__restrict__ perm, int n1, float *y, float *x) {
-    __shared__ float blk[32][33];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __syncthreads();
-    if (threadIdx.x == 0)
-        for (int k = 0; k < n1; ++k) {
-            const int p = perm[k];
-            if (p != k) { const float t = y[k]; y[k] = y[p]; y[p] = t; }
-        }
-    __syncthreads();
-    // forward: L (unit diagonal)
-    for (int c0 = 0; c0 < n1; c0 += 32) {
+// x = K^-1 y in FP32 with the factors (unit lower L, upper U, both in LU; row i of the factors is
+// row orig[i] of K), blocked by 32 columns: the 32x32 diagonal block (fetched to shared memory
+// during the step before) is solved by one warp with shuffles, then every warp updates the
+// remaining rows with the block's 32 values, four rows at a time (coalesced).  Two barriers
+// per 32 columns.
+__device__ void lu_apply_f32(const float *__restrict__ LU, const int *__restrict__ orig, int n1,
+                             const float *__restrict__ y, float *__restrict__ x) {
+    __shared__ float blk[2][32][33];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, nt = blockDim.x;
+    auto fetch = [&](int b, int c0) {
+        if (c0 < 0 || c0 >= n1) return;
         const int bs = min(32, n1 - c0);
-        for (int t = threadIdx.x; t < bs * 32; t += kLU) {
+        for (int t = threadIdx.x; t < bs * 32; t += nt) {
             const int r = t >> 5, c = t & 31;
-            blk[r][c] = c < bs ? LU[(size_t)(c0 + r) * n1 + c0 + c] : 0.f;
+            blk[b][r][c] = c < bs ? LU[(size_t)(c0 + r) * n1 + c0 + c] : 0.f;
         }
-        __syncthreads();
-        if (warp == 0) {
-            float yv = lane < bs ? y[c0 + lane] : 0.f;
+    };
+    // rows r0 .. r1 - 1 less LU[r][c0 ..] times x[c0 .. c0 + bs - 1]: eight rows' products are summed
+    // over the lanes together (each exchange halves the rows a lane keeps), each in the order of
+    // a plain exchange by 16, 8, 4, 2, 1
+    auto update = [&](int r0, int r1, int c0, int bs) {
+        const float xv = lane < bs ? x[c0 + lane] : 0.f;
+        const float *base = LU + c0 + lane;
+        const bool u16 = lane & 16, u8 = lane & 8, u4 = lane & 4;
+        for (int r = r0 + 8 * warp; r < r1; r += 8 * nw) {
+            float t[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) t[k] = (lane < bs && r + k < r1) ? base[(size_t)(r + k) * n1] : 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) t[k] *= xv;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float give = u16 ? t[k] : t[k + 4], keep = u16 ? t[k + 4] : t[k];
+                t[k] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+            }
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const float give = u8 ? t[k] : t[k + 2], keep = u8 ? t[k + 2] : t[k];
+                t[k] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+            }
+            float v = (u4 ? t[1] : t[0]) + __shfl_xor_sync(0xffffffffu, u4 ? t[0] : t[1], 4);
+            for (int o = 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            const int row = r + (u16 ? 4 : 0) + (u8 ? 2 : 0) + (u4 ? 1 : 0);
+            if ((lane & 3) == 0 && row < r1) x[row] -= v;
+        }
+    };
+    // the diagonal block b: its rows' values ahead of the serial chain, in registers
+    auto solve_lower = [&](int b, int c0, int bs) {
+        if (bs < 32) {  // the short block at the end
+            float v = lane < bs ? x[c0 + lane] : 0.f;
             for (int c = 0; c < bs - 1; ++c) {
-                const float yc = __shfl_sync(0xffffffffu, yv, c);
-                if (lane > c && lane < bs) yv -= blk[lane][c] * yc;
+                const float vc = __shfl_sync(0xffffffffu, v, c);
+                if (lane > c && lane < bs) v -= blk[b][lane][c] * vc;
             }
-            if (lane < bs) y[c0 + lane] = yv;
+            if (lane < bs) x[c0 + lane] = v;
+            return;
         }
-        __syncthreads();
-        for (int r = c0 + bs + warp; r < n1; r += kLU / 32) {
-            float t = lane < bs ? LU[(size_t)r * n1 + c0 + lane] * y[c0 + lane] : 0.f;
-            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-            if (lane == 0) y[r] -= t;
+        float l[32];
+#pragma unroll
+        for (int c = 0; c < 32; ++c) l[c] = blk[b][lane][c];
+        float v = x[c0 + lane];
+#pragma unroll
+        for (int c = 0; c < 31; ++c) {
+            const float vc = __shfl_sync(0xffffffffu, v, c);
+            if (lane > c) v -= l[c] * vc;
         }
-        __syncthreads();
-    }
-    // backward: U
-    for (int c1 = n1; c1 > 0; c1 -= 32) {
-        const int c0 = max(0, c1 - 32), bs = c1 - c0;
-        for (int t = threadIdx.x; t < bs * 32; t += kLU) {
-            const int r = t >> 5, c = t & 31;
-            blk[r][c] = c < bs ? LU[(size_t)(c0 + r) * n1 + c0 + c] : 0.f;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            float yv = lane < bs ? y[c0 + lane] : 0.f;
+        x[c0 + lane] = v;
+    };
+    auto solve_upper = [&](int b, int c0, int bs) {
+        if (bs < 32) {
+            float v = lane < bs ? x[c0 + lane] : 0.f;
             for (int c = bs - 1; c >= 0; --c) {
-                if (lane == c) yv = yv / blk[c][c];
-                const float xc = __shfl_sync(0xffffffffu, yv, c);
-                if (lane < c) yv -= blk[lane][c] * xc;
+                if (lane == c) v = v / blk[b][c][c];
+                const float xc = __shfl_sync(0xffffffffu, v, c);
+                if (lane < c) v -= blk[b][lane][c] * xc;
             }
-            if (lane < bs) {
-                y[c0 + lane] = yv;
-                x[c0 + lane] = yv;
-            }
+            if (lane < bs) x[c0 + lane] = v;
+            return;
         }
+        float u[32];
+#pragma unroll
+        for (int c = 0; c < 32; ++c) u[c] = blk[b][lane][c];
+        const float dg = blk[b][lane][lane];
+        float v = x[c0 + lane];
+#pragma unroll
+        for (int c = 31; c >= 0; --c) {
+            if (lane == c) v = v / dg;
+            const float xc = __shfl_sync(0xffffffffu, v, c);
+            if (lane < c) v -= u[c] * xc;
+        }
+        x[c0 + lane] = v;
+    };
+    const int nblk = (n1 + 31) / 32;
+    __syncthreads();
+    fetch(0, 0);
+    for (int t = threadIdx.x; t < n1; t += nt) x[t] = y[orig[t]];
+    __syncthreads();
+    for (int s = 0; s < nblk; ++s) {  // forward: L (unit diagonal)
+        const int c0 = 32 * s, bs = min(32, n1 - c0);
+        if (warp == 0) solve_lower(s & 1, c0, bs);
+        if (s + 1 < nblk) fetch((s + 1) & 1, c0 + 32);
         __syncthreads();
-        for (int r = warp; r < c0; r += kLU / 32) {
-            float t = lane < bs ? LU[(size_t)r * n1 + c0 + lane] * x[c0 + lane] : 0.f;
-            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-            if (lane == 0) y[r] -= t;
-        }
+        update(c0 + bs, n1, c0, bs);
         __syncthreads();
     }
-}
-// sum over the block, fixed order (every thread gets the result)
-__device__ double block_sum(double v, double *sv) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    // backward: U; the blocks end at n1, n1 - 32, ... (the first one, at the top, may be short)
+    fetch(0, max(0, n1 - 32));
     __syncthreads();
-    if ((threadIdx.x & 31) == 0) sv[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double t = 0.0;
-    for (int w = 0; w < kLU / 32; ++w) t += sv[w];
-    return t;
+    for (int s = 0; s < nblk; ++s) {
+        const int e = n1 - 32 * s, c0 = max(0, e - 32), bs = e - c0;
+        if (warp == 0) solve_upper(s & 1, c0, bs);
+        if (s + 1 < nblk) {
+            const int e2 = e - 32, d0 = max(0, e2 - 32);
+            for (int t = threadIdx.x; t < (e2 - d0) * 32; t += nt) {
+                const int r = t >> 5, c = t & 31;
+                blk[(s + 1) & 1][r][c] = c < e2 - d0 ? LU[(size_t)(d0 + r) * n1 + d0 + c] : 0.f;
+            }
+        }
+        __syncthreads();
+        update(0, c0, c0, bs);
+        __syncthreads();
+    }
 }
 
 // d.r <- K^{-1} d.r with the factors that solved the system: FP32 (in the first half of As,
 // through the FP32 shared vectors ys/xs) or FP64 (in As).  Non-finite FP32 results (a system
 // far beyond FP32) read as 1e300.
-__device__ void apply_inverse(const SolveDesc &d, int n1, bool f32, float *ys, float *xs) {
+__device__ void apply_inverse(const SolveDesc &d, int n1, bool f32, float *ys, float *xs, const int *orig) {
     if (f32) {
         __syncthreads();
-        for (int t = threadIdx.x; t < n1; t += kLU) ys[t] = (float)d.r[t];
-        lu_apply_f32(reinterpret_cast<const float *>(d.As), d.perm, n1, ys, xs);
-        for (int t = threadIdx.x; t < n1; t += kLU) {
+        for (int t = threadIdx.x; t < n1; t += blockDim.x) ys[t] = (float)d.r[t];
+        lu_apply_f32(reinterpret_cast<const float *>(d.As), orig, n1, ys, xs);
+        for (int t = threadIdx.x; t < n1; t += blockDim.x) {
             const float v = xs[t];
             d.r[t] = isfinite(v) ? (double)v : 1e300;
         }
@@ -496,47 +662,47 @@ __device__ void apply_inverse(const SolveDesc &d, int n1, bool f32, float *ys, f
 // 311-316) with Higham's extra test vector (N. J. Higham, ACM TOMS 14 (1988) 381-396),
 // at most four sign iterations.  A lower bound that is almost always within a small factor.
 // Uses d.r as the work vector.
-__device__ double inverse_norm1_estimate(const SolveDesc &d, int n1, bool f32, float *fsh, double *sv, int *si,
+__device__ double inverse_norm1_estimate(const SolveDesc &d, int n1, bool f32, float *fsh, const int *orig, double *sv, int *si,
                                          double *piv_v, int *piv_i) {
     float *ys = fsh, *xs = fsh + n1;
-    for (int t = threadIdx.x; t < n1; t += kLU) d.r[t] = 1.0 / (double)n1;
-    apply_inverse(d, n1, f32, ys, xs);
+    for (int t = threadIdx.x; t < n1; t += blockDim.x) d.r[t] = 1.0 / (double)n1;
+    apply_inverse(d, n1, f32, ys, xs, orig);
     double a = 0.0;
-    for (int t = threadIdx.x; t < n1; t += kLU) a += fabs(d.r[t]);
-    double est = block_sum(a, sv);
+    for (int t = threadIdx.x; t < n1; t += blockDim.x) a += fabs(d.r[t]);
+    double est = block_sum(a, n1, sv);
     int jprev = -1;
     for (int it = 0; it < 4; ++it) {
-        for (int t = threadIdx.x; t < n1; t += kLU) d.r[t] = d.r[t] >= 0.0 ? 1.0 : -1.0;
-        apply_inverse(d, n1, f32, ys, xs);  // z = K^{-T} sign(y)
+        for (int t = threadIdx.x; t < n1; t += blockDim.x) d.r[t] = d.r[t] >= 0.0 ? 1.0 : -1.0;
+        apply_inverse(d, n1, f32, ys, xs, orig);  // z = K^{-T} sign(y)
         double best = -1.0, zsum = 0.0;
         int bi = 0x7fffffff;
-        for (int t = threadIdx.x; t < n1; t += kLU) {
+        for (int t = threadIdx.x; t < n1; t += blockDim.x) {
             const double v = fabs(d.r[t]);
             zsum += d.r[t];
             if (v > best || (v == best && t < bi)) { best = v; bi = t; }
         }
-        zsum = block_sum(zsum, sv);
+        zsum = block_sum(zsum, n1, sv);
         block_argmax(best, bi, sv, si, piv_v, piv_i);
         const double zmax = *piv_v;
         const int j = *piv_i;
         const double ztx = jprev < 0 ? zsum / (double)n1 : d.r[jprev];
         __syncthreads();
         if (!(zmax > ztx)) break;  // uniform: every thread read the same values
-        for (int t = threadIdx.x; t < n1; t += kLU) d.r[t] = t == j ? 1.0 : 0.0;
-        apply_inverse(d, n1, f32, ys, xs);
+        for (int t = threadIdx.x; t < n1; t += blockDim.x) d.r[t] = t == j ? 1.0 : 0.0;
+        apply_inverse(d, n1, f32, ys, xs, orig);
         double b = 0.0;
-        for (int t = threadIdx.x; t < n1; t += kLU) b += fabs(d.r[t]);
-        b = block_sum(b, sv);
+        for (int t = threadIdx.x; t < n1; t += blockDim.x) b += fabs(d.r[t]);
+        b = block_sum(b, n1, sv);
         if (!(b > est)) break;
         est = b;
         jprev = j;
     }
-    for (int t = threadIdx.x; t < n1; t += kLU)
+    for (int t = threadIdx.x; t < n1; t += blockDim.x)
         d.r[t] = ((t & 1) ? -1.0 : 1.0) * (1.0 + (double)t / (double)max(n1 - 1, 1));
-    apply_inverse(d, n1, f32, ys, xs);
+    apply_inverse(d, n1, f32, ys, xs, orig);
     double c = 0.0;
-    for (int t = threadIdx.x; t < n1; t += kLU) c += fabs(d.r[t]);
-    c = 2.0 * block_sum(c, sv) / (3.0 * (double)n1);
+    for (int t = threadIdx.x; t < n1; t += blockDim.x) c += fabs(d.r[t]);
+    c = 2.0 * block_sum(c, n1, sv) / (3.0 * (double)n1);
     est = fmax(est, c);
     return est < 1e300 ? est : 1e300;
 }
@@ -552,88 +718,117 @@ constexpr int kLUWideMin = 768;
 constexpr int kLUHost64Min = 256;
 constexpr int kLUWideMax = (int)((225 * 1024) / (sizeof(float) * 5));
 
-// r = bs - A0 x in FP64: a warp per row, lanes along the row, fixed-order shuffle sum
+// r = bs - A0 x in FP64: a warp per eight rows, lanes along the row.  The rows' sums over the lanes
+// are reduced together (each exchange halves the rows a lane keeps), in the order of a plain
+// exchange by 16, 8, 4, 2, 1: 9 additions for 8 rows instead of 40 on the slow FP64 pipe.
 __device__ void residual(const SolveDesc &d, int n1) {
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    for (int rr = threadIdx.x >> 5; rr < n1; rr += kLU / 32) {
-        const double *row = d.A0 + (size_t)rr * n1;
-        double s = 0.0;
-        for (int c = lane; c < n1; c += 32) s += row[c] * d.x[c];
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) d.r[rr] = d.bs[rr] - s;
+    const bool u16 = lane & 16, u8 = lane & 8, u4 = lane & 4;
+    for (int r = 8 * (threadIdx.x >> 5); r < n1; r += 8 * (blockDim.x >> 5)) {
+        double s[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s[k] = 0.0;
+        const double *row = d.A0 + (size_t)r * n1;
+        for (int c = lane; c < n1; c += 32) {
+            const double xv = d.x[c];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (r + k < n1) s[k] += row[(size_t)k * n1 + c] * xv;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const double give = u16 ? s[k] : s[k + 4], keep = u16 ? s[k + 4] : s[k];
+            s[k] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const double give = u8 ? s[k] : s[k + 2], keep = u8 ? s[k + 2] : s[k];
+            s[k] = keep + __shfl_xor_sync(0xffffffffu, give, 8);
+        }
+        double v = (u4 ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, u4 ? s[0] : s[1], 4);
+        for (int o = 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        const int rr = r + (u16 ? 4 : 0) + (u8 ? 2 : 0) + (u4 ? 1 : 0);
+        if ((lane & 3) == 0 && rr < n1) d.r[rr] = d.bs[rr] - v;
     }
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kLU) lu_solve_refine_kernel(const SolveDesc *__restrict__ descs) {
+__global__ void __launch_bounds__(kSolve) lu_solve_refine_kernel(const SolveDesc *__restrict__ descs) {
     const SolveDesc d = descs[blockIdx.x];
     if (d.wide64 || d.host32) return;  // refined on the host path (factor_refine_wide64, refine_wide32)
     const int n1 = d.n + 1;
-    extern __shared__ __align__(16) float fsh[];  // [2 * n1]: right-hand side / correction in FP32 (or n1 doubles)
+    // [2 n1] right-hand side / correction in FP32 (or n1 doubles), [n1] row order, then the work
+    // area of the blocked factorisation
+    extern __shared__ __align__(16) float fsh[];
     float *ys = fsh, *xs = fsh + n1;
-    __shared__ double sv[kLU / 32];
+    int *orig = reinterpret_cast<int *>(fsh + 2 * n1);
+    __shared__ double sv[33];
     __shared__ int si[kLU / 32];
     __shared__ double piv_v;
     __shared__ int piv_i;
+    __shared__ LuShared lus;
     double pmin = 1e308, pmax = 0.0, res = 0.0;
     int singular = 0, steps = 0;
     bool done = false;
 
     // ---- FP32 LU + FP64-residual refinement
-    if (!d.wide64) {
-        float *L = reinterpret_cast<float *>(d.As);  // the first half of the FP64 work matrix
-        const bool wide32 = d.pre && !d.host64;  // FP32 factors from across the GPU
-        if (!wide32)
-            for (long long t = threadIdx.x; t < (long long)n1 * n1; t += kLU) L[t] = (float)d.A0[t];
-        for (int t = threadIdx.x; t < n1; t += kLU) {
+    double an, anorm;  // max row sums of |K| and |A| (prepare_kernel)
+    {
+        double u = 0.0, v = 0.0;
+        for (int t = threadIdx.x; t < n1; t += blockDim.x) {
+            u = fmax(u, d.r[t]);
+            v = fmax(v, d.x[t]);
+        }
+        an = block_max(u, n1, sv);
+        anorm = block_max(v, n1, sv);
+    }
+    {
+        float *L = reinterpret_cast<float *>(d.As);  // the first half of the FP64 work matrix (prepare_kernel's copy)
+        for (int t = threadIdx.x; t < n1; t += blockDim.x) {
             d.x[t] = 0.0;
             d.r[t] = d.bs[t];
         }
-        __syncthreads();
         bool factored;
-        if (wide32) {  // factored across the GPU before this launch (lu_wide_factor)
-            factored = d.pre[0] == 0.0;
-            if (factored) {
-                pmin = fmin(pmin, d.pre[1]);
-                pmax = fmax(pmax, d.pre[2]);
-            }
+        if (n1 <= kLUBlockedMax) {
+            float *work = fsh + ((3 * n1 + 3) & ~3);
+            factored = lu_factor_f32_blocked(L, orig, n1, work, lus, pmin, pmax);
         } else {
-            factored = n1 <= kLUBlockedMax ? lu_factor_f32_blocked(L, d.perm, n1, fsh, reinterpret_cast<float *>(sv),
-                                                                   si, &piv_i, pmin, pmax)
-                                           : lu_factor_f32(L, d.perm, n1, sv, si, &piv_v, &piv_i, pmin, pmax);
+            factored = lu_factor_f32(L, d.perm, n1, sv, si, &piv_v, &piv_i, pmin, pmax);
+            if (threadIdx.x == 0) {  // the interchanges as a row order
+                for (int k = 0; k < n1; ++k) orig[k] = k;
+                for (int k = 0; factored && k < n1; ++k) {
+                    const int p = d.perm[k], o = orig[k];
+                    orig[k] = orig[p];
+                    orig[p] = o;
+                }
+            }
+            __syncthreads();
         }
         if (factored) {
-            double an = 0.0;  // |A| (max row sum)
-            for (int rr = threadIdx.x; rr < n1; rr += kLU) {
-                double s = 0.0;
-                for (int c = 0; c < n1; ++c) s += fabs(d.A0[(size_t)rr * n1 + c]);
-                an = fmax(an, s);
-            }
-            an = block_max(an, sv);
             double rprev = 1e308;
             for (int it = 0; it < kRefineMax && !done; ++it) {
                 double rm = 0.0;
-                for (int t = threadIdx.x; t < n1; t += kLU) rm = fmax(rm, fabs(d.r[t]));
-                rm = block_max(rm, sv);
+                for (int t = threadIdx.x; t < n1; t += blockDim.x) rm = fmax(rm, fabs(d.r[t]));
+                rm = block_max(rm, n1, sv);
                 if (rm == 0.0) {
                     done = true;
                     break;
                 }
                 const double inv = 1.0 / rm;
                 ++steps;
-                for (int t = threadIdx.x; t < n1; t += kLU) ys[t] = (float)(d.r[t] * inv);
-                lu_apply_f32(L, d.perm, n1, ys, xs);
-                for (int t = threadIdx.x; t < n1; t += kLU) d.x[t] += (double)xs[t] * rm;
+                for (int t = threadIdx.x; t < n1; t += blockDim.x) ys[t] = (float)(d.r[t] * inv);
+                lu_apply_f32(L, orig, n1, ys, xs);
+                for (int t = threadIdx.x; t < n1; t += blockDim.x) d.x[t] += (double)xs[t] * rm;
                 __syncthreads();
                 double rn = 0.0, xn = 0.0;
                 residual(d, n1);
-                for (int rr = threadIdx.x; rr < n1; rr += kLU) {
+                for (int rr = threadIdx.x; rr < n1; rr += blockDim.x) {
                     rn = fmax(rn, fabs(d.r[rr]));
                     xn = fmax(xn, fabs(d.x[rr]));
                 }
-                rn = block_max(rn, sv);
-                xn = block_max(xn, sv);
+                rn = block_max(rn, n1, sv);
+                xn = block_max(xn, n1, sv);
                 res = rn;
                 if (rn <= (double)n1 * 1.1102230246251565e-16 * an * xn) done = true;
                 // stalled (cond(A) near 1/eps32 or beyond): no use refining further, FP64 takes over
@@ -656,22 +851,22 @@ __global__ void __launch_bounds__(kLU) lu_solve_refine_kernel(const SolveDesc *_
     if (!done) {
         double *A = d.As;
         {
-        for (long long t = threadIdx.x; t < (long long)n1 * n1; t += kLU) A[t] = d.A0[t];
+        for (long long t = threadIdx.x; t < (long long)n1 * n1; t += blockDim.x) A[t] = d.A0[t];
         __syncthreads();
         pmin = 1e308;
         pmax = 0.0;
         for (int k = 0; k < n1; ++k) {
             double best = -1.0;
             int bi = 0x7fffffff;
-            for (int r = k + threadIdx.x; r < n1; r += kLU) {
+            for (int r = k + threadIdx.x; r < n1; r += blockDim.x) {
                 double v = fabs(A[(size_t)r * n1 + k]);
                 if (v > best || (v == best && r < bi)) { best = v; bi = r; }
             }
             block_argmax(best, bi, sv, si, &piv_v, &piv_i);
-            const int p = piv_i;
+            const int p = piv_i < n1 ? piv_i : k;  // no candidate (NaN): stay
             if (threadIdx.x == 0) d.perm[k] = p;
             if (p != k)
-                for (int c = threadIdx.x; c < n1; c += kLU) {
+                for (int c = threadIdx.x; c < n1; c += blockDim.x) {
                     double t = A[(size_t)k * n1 + c];
                     A[(size_t)k * n1 + c] = A[(size_t)p * n1 + c];
                     A[(size_t)p * n1 + c] = t;
@@ -688,10 +883,10 @@ __global__ void __launch_bounds__(kLU) lu_solve_refine_kernel(const SolveDesc *_
             }
             __syncthreads();
             const double inv = 1.0 / pv;
-            for (int r = k + 1 + threadIdx.x; r < n1; r += kLU) A[(size_t)r * n1 + k] *= inv;
+            for (int r = k + 1 + threadIdx.x; r < n1; r += blockDim.x) A[(size_t)r * n1 + k] *= inv;
             __syncthreads();
             const double *prow = A + (size_t)k * n1;
-            for (int rr = k + 1 + (threadIdx.x >> 5); rr < n1; rr += kLU / 32) {
+            for (int rr = k + 1 + (threadIdx.x >> 5); rr < n1; rr += (blockDim.x >> 5)) {
                 double *row = A + (size_t)rr * n1;
                 const double l = row[k];
                 for (int cc = k + 1 + (threadIdx.x & 31); cc < n1; cc += 32) row[cc] -= l * prow[cc];
@@ -699,38 +894,31 @@ __global__ void __launch_bounds__(kLU) lu_solve_refine_kernel(const SolveDesc *_
             __syncthreads();
         }
         }
-        for (int t = threadIdx.x; t < n1; t += kLU) d.x[t] = d.bs[t];
+        for (int t = threadIdx.x; t < n1; t += blockDim.x) d.x[t] = d.bs[t];
         lu_apply(A, d.perm, n1, d.x, reinterpret_cast<double *>(fsh));
-        for (int rr = threadIdx.x; rr < n1; rr += kLU) {
+        for (int rr = threadIdx.x; rr < n1; rr += blockDim.x) {
             double s = d.bs[rr];
             const double *row = d.A0 + (size_t)rr * n1;
             for (int c = 0; c < n1; ++c) s -= row[c] * d.x[c];
             d.r[rr] = s;
         }
         lu_apply(A, d.perm, n1, d.r, reinterpret_cast<double *>(fsh));
-        for (int t = threadIdx.x; t < n1; t += kLU) d.x[t] += d.r[t];
+        for (int t = threadIdx.x; t < n1; t += blockDim.x) d.x[t] += d.r[t];
         __syncthreads();
         double rmax = 0.0;
-        for (int rr = threadIdx.x; rr < n1; rr += kLU) {
+        for (int rr = threadIdx.x; rr < n1; rr += blockDim.x) {
             double s = d.bs[rr];
             const double *row = d.A0 + (size_t)rr * n1;
             for (int c = 0; c < n1; ++c) s -= row[c] * d.x[c];
             rmax = fmax(rmax, fabs(s));
         }
-        res = block_max(rmax, sv);
+        res = block_max(rmax, n1, sv);
     }
     // ---- conditioning: kappa = ||A||_1 ||K^{-1}||_1 with A the folded normal matrix (RESP
     // included, the border excluded) and K the bordered matrix.  A relative error e in A moves
     // the solution by about e * kappa * |q| at worst, so kappa says how much of the Gram's
     // rounding reaches the charges (the fit escalates a mixed-precision cube beyond a limit).
-    double anorm = 0.0;
-    for (int c = threadIdx.x; c < d.n; c += kLU) {
-        double sacc = 0.0;
-        for (int rr = 0; rr < d.n; ++rr) sacc += fabs(d.A0[(size_t)rr * n1 + c]);
-        anorm = fmax(anorm, sacc);
-    }
-    anorm = block_max(anorm, sv);
-    const double kinv = inverse_norm1_estimate(d, n1, f32_solved, fsh, sv, si, &piv_v, &piv_i);
+    const double kinv = inverse_norm1_estimate(d, n1, f32_solved, fsh, orig, sv, si, &piv_v, &piv_i);
     if (threadIdx.x == 0) {
         d.info[0] = res;
         d.info[1] = pmin;
@@ -739,11 +927,11 @@ __global__ void __launch_bounds__(kLU) lu_solve_refine_kernel(const SolveDesc *_
         d.info[4] = fmin(anorm * kinv, 1e300);
         d.info[5] = n1;
         d.info[6] = steps;
-        d.info[7] = f32_solved ? ((d.pre && !d.host64) ? 1.0 : 0.0) : 2.0;
+        d.info[7] = f32_solved ? 0.0 : 2.0;
     }
     __syncthreads();
     // expand to all atoms
-    for (int i = threadIdx.x; i < d.N; i += kLU) d.q[i] = d.x[d.map[i]];
+    for (int i = threadIdx.x; i < d.N; i += blockDim.x) d.q[i] = d.x[d.map[i]];
 }
 
 // ---------------------------------------------------------------------------
@@ -794,7 +982,6 @@ __global__ void __launch_bounds__(kLU) lu_panel_kernel(T *__restrict__ A, int *_
     __shared__ int piv_i;
     __shared__ double piv_v;
     const int m = n1 - k0, nb = min(NB, m), ld = NB + 1;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int t = threadIdx.x; t < m * NB; t += kLU) {
         const int r = t / NB, c = t - r * NB;
         P[r * ld + c] = c < nb ? A[(size_t)(k0 + r) * n1 + k0 + c] : T(0);
@@ -813,7 +1000,7 @@ __global__ void __launch_bounds__(kLU) lu_panel_kernel(T *__restrict__ A, int *_
             block_argmax_f(best, bi, reinterpret_cast<float *>(svd), si, &piv_i);
         else
             block_argmax(best, bi, svd, si, &piv_v, &piv_i);
-        const int p = piv_i;
+        const int p = piv_i < m ? piv_i : j;  // no candidate (NaN): stay
         if (threadIdx.x == 0) perm[k0 + j] = k0 + p;
         if (p != j && threadIdx.x < NB) {
             const T t = P[j * ld + threadIdx.x];
@@ -896,19 +1083,21 @@ __global__ void __launch_bounds__(256) lu_trsm_kernel(T *__restrict__ A, int n1,
         if (j < nb) A[(size_t)(k0 + j) * n1 + c] = u[j];
 }
 
-// dynamic shared memory of lu_solve_refine_kernel: the right-hand side and correction in
-// FP32 (2 n1 floats) and, for the blocked factorisation, the panel and the U12 tile
+// dynamic shared memory of lu_solve_refine_kernel: the right-hand side, the correction and the row
+// order, and for the blocked factorisation 64 rows of a panel's neighbours (or its own rows,
+// 33 floats each)
 size_t solve_smem_bytes(int n1) {
-    size_t b = sizeof(float) * 2 * (size_t)n1;
-    if (n1 <= kLUBlockedMax) b = std::max(b, sizeof(float) * ((size_t)n1 * (kLUNB + 1) + kLUNB * kLUTile));
-    return b;
+    size_t f = (3 * (size_t)n1 + 3) & ~(size_t)3;
+    if (n1 <= kLUBlockedMax) f += 64 * (((size_t)n1 + 3) & ~(size_t)3);
+    return sizeof(float) * f;
 }
+// threads: at least a row each for the blocked factorisation; 24 warps from 100 unknowns on (0.33
+// against 0.38 ms at 151 unknowns, 1.37 against 1.48 at 425), 8 below (fewer to a barrier: 0.06
+// against 0.09 ms at 10)
+int solve_threads(int n1) { return n1 <= 100 ? 256 : kSolve; }
 
-// the launch's shared memory opt-in, raised once to the largest the kernel can ask for
-void lu_smem_optin() {
-    smem_optin((const void *)lu_solve_refine_kernel,
-               std::max(solve_smem_bytes(kLUBlockedMax), solve_smem_bytes(1)));
-}
+// the launch's shared memory opt-in, raised once to the largest the kernel is launched with
+void lu_smem_optin() { smem_optin((const void *)lu_solve_refine_kernel, solve_smem_bytes(kLUWideMin - 1)); }
 
 inline cublasStatus_t gemm_nn(cublasHandle_t h, int m, int n, int k, const float *alpha, const float *A, int lda,
                               const float *B, int ldb, const float *beta, float *C, int ldc) {
@@ -1530,7 +1719,6 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
                 hbs[rr] = br[rr] + rsv * rtv;
             }
             hbs[p.n] = J.qtot;
-            RP_CUDA(cudaMemcpyAsync(descs[j].As, hs.data(), sizeof(double) * hs.size(), cudaMemcpyHostToDevice, stream));
             RP_CUDA(cudaMemcpyAsync(descs[j].A0, hs.data(), sizeof(double) * hs.size(), cudaMemcpyHostToDevice, stream));
             RP_CUDA(cudaMemcpyAsync(descs[j].bs, hbs.data(), sizeof(double) * hbs.size(), cudaMemcpyHostToDevice, stream));
             RP_CUDA(cudaStreamSynchronize(stream));
@@ -1553,11 +1741,20 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
     }
     {
         StageTimer tt(ctx, "solve_lu", stream);
-        int n1max = 1;
-        for (const FoldPlan &p : plans) n1max = std::max(n1max, p.n + 1);
-        lu_smem_optin();
-        lu_solve_refine_kernel<<<nj, kLU, solve_smem_bytes(n1max), stream>>>(d_desc);
-        RP_LAUNCH_CHECK();
+        int n1max = 0;  // of the systems solved in their CTAs
+        size_t smem = 0;
+        for (int j = 0; j < nj; ++j) {
+            if (descs[j].wide64 || descs[j].host32) continue;
+            n1max = std::max(n1max, descs[j].n + 1);
+            smem = std::max(smem, solve_smem_bytes(descs[j].n + 1));
+        }
+        if (n1max > 0) {
+            lu_smem_optin();
+            prepare_kernel<<<dim3(ceil_div(n1max, 8), nj), 256, 0, stream>>>(d_desc);
+            RP_LAUNCH_CHECK();
+            lu_solve_refine_kernel<<<nj, solve_threads(n1max), smem, stream>>>(d_desc);
+            RP_LAUNCH_CHECK();
+        }
     }
     for (int j = 0; j < nj; ++j)  // systems known to need FP64 (an escalated fit): getrf, host-driven refinement
         if (descs[j].wide64) factor_refine_wide64(ctx, descs[j], plans[j].n + 1, stream);
@@ -1763,12 +1960,13 @@ extern "C" int rp_solve_noalloc(const double *A_dev, const double *b_dev, int N,
                 hbs[k] = br[k] + rs[k] * rt[k];
             }
             hbs[p.n] = qtot;
-            RP_CUDA(cudaMemcpyAsync(As, hs.data(), sizeof(double) * hs.size(), cudaMemcpyHostToDevice, stream));
             RP_CUDA(cudaMemcpyAsync(A0, hs.data(), sizeof(double) * hs.size(), cudaMemcpyHostToDevice, stream));
             RP_CUDA(cudaMemcpyAsync(bs, hbs.data(), sizeof(double) * hbs.size(), cudaMemcpyHostToDevice, stream));
         }
         lu_smem_optin();
-        lu_solve_refine_kernel<<<1, kLU, solve_smem_bytes(n1), stream>>>(d_desc);
+        prepare_kernel<<<dim3(ceil_div(n1, 8), 1), 256, 0, stream>>>(d_desc);
+        RP_LAUNCH_CHECK();
+        lu_solve_refine_kernel<<<1, solve_threads(n1), solve_smem_bytes(n1), stream>>>(d_desc);
         RP_LAUNCH_CHECK();
         double hinfo[kSolveInfo];
         RP_CUDA(cudaMemcpyAsync(hinfo, d_info, sizeof(hinfo), cudaMemcpyDeviceToHost, stream));

@@ -1,0 +1,50 @@
+"""The bordered solve at the sizes where its blocking can go wrong: one unknown, the 32-column panel's
+edges, the change of thread counts at 100 unknowns, the last size one CTA factors; on matrices that need row
+interchanges in every panel.  Against an FP64 LU of the same bordered system, within the
+bound of the other solve tests (1e-9 of the largest charge)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(A, b, qtot):
+    import scipy.linalg as sl
+    N = len(b)
+    K = np.zeros((N + 1, N + 1))
+    K[:N, :N] = A
+    K[:N, N] = K[N, :N] = 1.0
+    return K, sl.solve(K, np.append(b, qtot))[:N]
+
+
+@pytest.mark.parametrize("N", [1, 2, 30, 31, 32, 33, 62, 63, 64, 65, 99, 100, 255, 256, 513, 766])
+def test_pivoted_systems_at_panel_edges(N, gpu_ctx):
+    """Symmetric indefinite A with a weak diagonal: the pivot is off the diagonal in most columns."""
+    import torch
+    rng = np.random.default_rng(N)
+    A = rng.normal(size=(N, N))
+    A = 0.5 * (A + A.T)
+    A[np.arange(N), np.arange(N)] *= 0.01
+    A += np.diag(np.where(np.arange(N) % 7 == 0, 3.0, 0.0))
+    b = rng.normal(size=N)
+    K, ref = _reference(A, b, 0.25)
+    q, info = gpu_ctx.solve(torch.from_numpy(A).cuda(), torch.from_numpy(b).cuda(), np.full(N, 6), qtot=0.25)
+    q = q.cpu().numpy()
+    tol = max(1e-9, 1e-15 * np.linalg.cond(K) * (N + 1))
+    assert np.abs(q - ref).max() <= tol * max(1.0, np.abs(ref).max())
+    kappa = np.abs(A).sum(axis=0).max() * np.abs(np.linalg.inv(K)).sum(axis=0).max()
+    assert kappa / 3 <= info["kappa"] <= kappa * (1 + 1e-3)
+
+
+@pytest.mark.parametrize("N", [5, 40])
+def test_nan_matrix_is_reported_singular_or_nan(N, gpu_ctx):
+    """A matrix of NaN has no pivot: the solve ends, and returns no finite charge as if it were one."""
+    import torch
+    from pyrepeat_gb300 import _lib
+    A = torch.full((N, N), float("nan"), dtype=torch.float64, device="cuda")
+    b = torch.zeros(N, dtype=torch.float64, device="cuda")
+    try:
+        q, _ = gpu_ctx.solve(A, b, np.full(N, 6))
+    except _lib.RepeatError:
+        return
+    assert not np.isfinite(q.cpu().numpy()).all()
