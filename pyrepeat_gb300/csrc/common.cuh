@@ -490,12 +490,10 @@ void filter_async(rp_ctx *ctx, const rp_grid *grid, const double *atoms, const i
 // Phi^T Phi and r (N) += Phi^T V for Phi rows x N (row-major, ld N) and V (rows).
 void gram_words_fp64(rp_ctx *ctx, const double *P, long long rows, int N, const double *V, double *G, double *r,
                      cudaStream_t stream);
-// separable: the reciprocal sum by the FP64 separable transform and the Gram by
-// gram_words_fp64 (the escalated fit)
-// instead of the flat k-table DGEMM and DSYRK (the plain FP64 comparator)
+// refit: an ill-conditioned mixed fit's (the reciprocal plane and row stages in double-float)
 void gram_fp64(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, const int32_t *kept_idx_dev,
                const double *Vc_dev, int64_t M, double *A_dev, double *b_dev, double *sum_phi_dev,
-               cudaStream_t stream, bool separable = false);
+               cudaStream_t stream, bool refit = false);
 // vstats_dev: the filter's (sum, max |.|) of Vc (only the max is used), or nullptr to
 // compute the max here.  rn (host, N) and clamp_dev (one device counter): the atoms'
 // scaled vdW radii, which bound |Phi| a priori, so Phi goes straight to fixed-point
@@ -576,11 +574,6 @@ struct SolvePending {
 const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, cudaStream_t stream,
                                 const std::string &tag, SolvePending *pend = nullptr, bool fp64_first = false);
 void solve_wide_fp64(rp_ctx *ctx, SolvePending &pd, cudaStream_t stream);  // synchronises stream
-
-// Device table builders (ewald_tables.cu).
-void atom_tables_fp64(const rp_ewald *ew, const double *d_atoms, int N, double *d_B, int ldb, cudaStream_t s);
-void grid_tables_fp64(const rp_ewald *ew, const int32_t *d_kept, int64_t m0, int64_t rows, double *d_T, int ldt,
-                      cudaStream_t s);
 
 // Reciprocal sum by separable lattice phases (recip_sep.cu): E[r][col][n1] for every
 // grid row r = j + l*ny, col = atom (d_q == nullptr) or one charge-weighted column.

@@ -249,58 +249,4 @@ void prune_shifts(const rp_ewald *ew, const double *atoms, int N, std::vector<do
         }
 }
 
-namespace {
-
-__global__ void atom_tables_fp64_kernel(const double *__restrict__ kvec, const double *__restrict__ kcoef, int K,
-                                        const double *__restrict__ atoms, int N, double *__restrict__ B, int ldb) {
-    // B[a][k] = w_k cos(k.r_a), B[a][K+k] = w_k sin(k.r_a)
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)N * K) return;
-    int a = (int)(t / K), k = (int)(t - (long long)a * K);
-    double kr = (atoms[3 * a] * kvec[3 * k] + atoms[3 * a + 1] * kvec[3 * k + 1]) + atoms[3 * a + 2] * kvec[3 * k + 2];
-    double s, c;
-    sincos(kr, &s, &c);
-    B[(size_t)a * ldb + k] = kcoef[k] * c;
-    B[(size_t)a * ldb + K + k] = kcoef[k] * s;
-}
-
-__global__ void grid_tables_fp64_kernel(const int *__restrict__ kidx, int K, int kmax, const double2 *__restrict__ ex,
-                                        const double2 *__restrict__ ey, const double2 *__restrict__ ez, int nx,
-                                        int ny, int nz, const int32_t *__restrict__ kept, long long m0, long long rows,
-                                        double *__restrict__ T, int ldt) {
-    // T[m][k] = cos(k.g_m), T[m][K+k] = sin(k.g_m) from the per-axis tables
-    long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= rows * K) return;
-    long long m = t / K;
-    int k = (int)(t - m * K);
-    int f = kept[m0 + m];
-    int layer = nx * ny;
-    int l = f / layer, rem = f - l * layer, j = rem / nx, i = rem - j * nx;
-    int n1 = kidx[3 * k], n2 = kidx[3 * k + 1], n3 = kidx[3 * k + 2];
-    double2 a = ex[(size_t)n1 * nx + i], b = ey[(size_t)(n2 + kmax) * ny + j], c = ez[(size_t)(n3 + kmax) * nz + l];
-    double re = a.x * b.x - a.y * b.y, im = a.x * b.y + a.y * b.x;
-    double re2 = re * c.x - im * c.y, im2 = re * c.y + im * c.x;
-    T[(size_t)m * ldt + k] = re2;
-    T[(size_t)m * ldt + K + k] = im2;
-}
-
-}  // namespace
-
-void atom_tables_fp64(const rp_ewald *ew, const double *d_atoms, int N, double *d_B, int ldb, cudaStream_t s) {
-    long long n = (long long)N * ew->K;
-    if (n == 0) return;
-    atom_tables_fp64_kernel<<<ceil_div(n, 256), 256, 0, s>>>(ew->d_kvec, ew->d_kcoef, ew->K, d_atoms, N, d_B, ldb);
-    RP_LAUNCH_CHECK();
-}
-
-void grid_tables_fp64(const rp_ewald *ew, const int32_t *d_kept, int64_t m0, int64_t rows, double *d_T, int ldt,
-                      cudaStream_t s) {
-    long long n = (long long)rows * ew->K;
-    if (n == 0) return;
-    grid_tables_fp64_kernel<<<ceil_div(n, 256), 256, 0, s>>>(ew->d_kidx, ew->K, ew->kmax, ew->d_ex, ew->d_ey, ew->d_ez,
-                                                             ew->grid.n_grid[0], ew->grid.n_grid[1], ew->grid.n_grid[2],
-                                                             d_kept, m0, rows, d_T, ldt);
-    RP_LAUNCH_CHECK();
-}
-
 }  // namespace rp

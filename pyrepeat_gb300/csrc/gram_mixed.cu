@@ -1855,7 +1855,6 @@ void gram_words_fp64(rp_ctx *ctx, const double *P, long long rows, int N, const 
     int ntri = 0;
     for (int ti = 0; ti < nt; ++ti) ntri += ntj - 2 * ti;
     const int kb_total = (int)(cols_pad / kBK);
-    RP_CUDA(cudaMemsetAsync(ctx->status_words(), 0, sizeof(int), stream));
     GramArgs g{};
     g.nt = nt;
     g.ntj = ntj;
@@ -1863,7 +1862,7 @@ void gram_words_fp64(rp_ctx *ctx, const double *P, long long rows, int N, const 
     g.kb_total = kb_total;
     g.kb_per_split = kGramSplit;
     g.flush = kGramFlush;
-    g.status = ctx->status_words();
+    g.status = ctx->status_words();  // cleared before and checked after by the caller
     g.budget = ctx->wait_budget;
     gram_totals_init(ctx, "w64_tsum", g, stream);
     const __half *Xq[kGSlices] = {X[0], X[1], X[2], X[3]};
@@ -1873,7 +1872,6 @@ void gram_words_fp64(rp_ctx *ctx, const double *P, long long rows, int N, const 
     RP_LAUNCH_CHECK();
     combine_words_kernel<<<ceil_div((long long)N * Np, 256), 256, 0, stream>>>(G2, N, mx, G, r);
     RP_LAUNCH_CHECK();
-    status_check(ctx, stream);
 }
 
 }  // namespace rp

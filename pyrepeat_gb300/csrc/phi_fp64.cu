@@ -1,16 +1,19 @@
-// Plain FP64 Phi -> normal equations: the "plain FP64 GPU fit" comparator.
+// FP64 Phi -> normal equations: the FP64 fit (--fp64) and the refit of an ill-conditioned mixed one.
 //
 // Per chunk of kept points (Phi is held for one chunk only):
-//   T[m][:]  = [cos(k.g_m) | sin(k.g_m)]            (FP64, exact per-axis phases)
-//   B[a][:]  = [w_k cos(k.r_a) | w_k sin(k.r_a)]    (FP64, once per fit)
-//   Phi      = T B^T                                 (cuBLAS DGEMM, native FP64)
-//   Phi     += sum_s [r <= Rc] erfc(sqrt(alpha) r)/r (FP64 kernel, repeat.py:944-966)
+//   Phi      = the separable reciprocal sum (the transform of recip_sep.cu): the plane stage once
+//              per fit, the row stage for the grid rows that hold points of the chunk, the point
+//              stage.  In FP64 throughout for the FP64 fit; with the plane and row stages in
+//              double-float (~2^-46) for the refit.
+//   Phi     += sum_s [r <= Rc] erfc(sqrt(alpha) r)/r (FP64, repeat.py:944-966)
 //   Phi_c    = Phi - c  (c = column means of the first chunk: a per-column shift,
 //              exactly corrected afterwards, so A needs no large cancellation)
-//   G += Phi_c^T Phi_c, r += Phi_c^T Vc              (cuBLAS DGEMM / DGEMV)
+//   G += Phi_c^T Phi_c, r += Phi_c^T Vc   (exact two-word Gram on the tensor cores, gram_words_fp64)
 // Finally A = G - s s^T / M, b = r - s sum(Vc) / M with s = sum_m Phi_c[m,:]
 // (= sum_phi - M c); this is repeat.py:2266-2276's mean correction written for
 // the shifted columns.
+// (The FP64 fit was a flat k-table DGEMM with an in-place real-space sum and a cuBLAS Gram: 108, 24
+// and 16 ms on 36 M point-atom pairs at K = 754.)
 #include <algorithm>
 #include <cmath>
 
@@ -20,15 +23,84 @@
 namespace rp {
 namespace {
 
+// erfc(s sqrt(u)) / sqrt(u), s = sqrt(alpha), as a Taylor polynomial of degree 9 about the centre of u's
+// interval, 64 intervals per power of two: |u - centre| <= centre / 128, and over the cutoff's
+// range (alpha u <= pi^2) the first term left out is below 2e-18 of the value.  About 10 FP64
+// instructions per term instead of ~75 for erfc, a square root and a division (an FP64
+// instruction holds its pipe for 16 cycles per warp here).  The coefficients follow from the
+// derivative d/du erfc(s sqrt(u)) = -s / sqrt(pi) e^(-s^2 u) u^(-1/2) by products of the series of
+// e^(-s^2 u) and u^(-1/2).
+constexpr int kErfcDeg = 9, kErfcPerOctave = 64;
+constexpr int kErfcLow = -2;  // from u = 2^-2 (half a Bohr); nearer pairs take the functions themselves
+struct ErfcTable {
+    const double *c;  // [intervals][kErfcDeg + 1]; nullptr: the functions themselves (the 1/r basis)
+    int base;         // high word >> 14 of the first interval
+};
+int erfc_intervals(double rc) {  // up to the power of two above Rc^2
+    int e = 0;
+    std::frexp(rc * rc, &e);
+    return std::max(1, e - kErfcLow) * kErfcPerOctave;
+}
+__global__ void erfc_table_kernel(double sa, int n, int base, double *__restrict__ c) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double u = __hiloint2double(((base + i) << 14) | 0x2000, 0);  // the interval's centre
+    double h[kErfcDeg + 1], e[kErfcDeg + 1], g[kErfcDeg + 1];
+    h[0] = 1.0 / sqrt(u);
+    e[0] = exp(-sa * sa * u);
+    for (int k = 1; k <= kErfcDeg; ++k) {
+        h[k] = h[k - 1] * ((0.5 - k) / (k * u));
+        e[k] = e[k - 1] * (-sa * sa / k);
+    }
+    g[0] = erfc(sa * sqrt(u));
+    for (int k = 1; k <= kErfcDeg; ++k) {
+        double t = 0.0;
+        for (int q = 0; q < k; ++q) t += e[q] * h[k - 1 - q];
+        g[k] = -sa * 0.56418958354775628694807945 * t / k;  // 1 / sqrt(pi)
+    }
+    for (int k = 0; k <= kErfcDeg; ++k) {
+        double t = 0.0;
+        for (int q = 0; q <= k; ++q) t += g[q] * h[k - q];
+        c[(size_t)i * (kErfcDeg + 1) + k] = t;
+    }
+}
+__device__ __noinline__ double erfc_term_direct(double d2, double sa) {
+    const double r = sqrt(d2);
+    return erfc(sa * r) / r;
+}
+__device__ __forceinline__ double erfc_term(double d2, const ErfcTable &tab, double sa) {
+    const int hi = __double2hiint(d2), i = (hi >> 14) - tab.base;
+    if (!tab.c || i < 0) return erfc_term_direct(d2, sa);
+    const double2 *c = reinterpret_cast<const double2 *>(tab.c + (size_t)i * (kErfcDeg + 1));
+    const double t = d2 - __hiloint2double((hi & ~0x3fff) | 0x2000, 0);
+    double2 q = c[kErfcDeg / 2];
+    double v = fma(q.y, t, q.x);
+#pragma unroll
+    for (int k = kErfcDeg / 2 - 1; k >= 0; --k) {
+        q = c[k];
+        v = fma(fma(v, t, q.y), t, q.x);
+    }
+    return v;
+}
+// The largest double whose (correctly rounded) square root is at most r: r(d2) <= r and d2 <= this are
+// the same decision, without the square root.
+double square_limit(double r) {
+    double t = r * r;
+    while (std::sqrt(t) > r) t = std::nextafter(t, 0.0);
+    for (double u = std::nextafter(t, 1e308); std::sqrt(u) <= r; u = std::nextafter(u, 1e308)) t = u;
+    return t;
+}
+// a <= b for doubles that are not negative, off the FP64 pipe (their bits order like the values)
+__device__ __forceinline__ bool le_bits(double a, double b) { return __double_as_longlong(a) <= __double_as_longlong(b); }
+
 // Real-space sum in FP64 (repeat.py:944-966) over tiles of kRsPts kept points x kRsAtoms
 // atoms.  For each chunk of up to kRsShiftChunk shifts, the CTA first drops, per atom,
 // every shift whose image lies farther than Rc + 1e-3 Bohr from the bounding box of its
 // points (an FP32 test: FP32 rounding of the coordinates moves a distance by < 1e-4
 // Bohr here, so no image within Rc is dropped).  Each thread then tests the remaining
 // images of each atom against its point in FP32 with the same margin.  QUEUE false: the
-// survivors are evaluated in place (the plain comparator's kept points, in grid order,
-// give tiles of nearby points that reach mostly the same images).  QUEUE true (the
-// escalated fit, whatever the order of its kept points): each thread queues its
+// survivors are evaluated in place (the 1/r basis: one image per atom, reached by every point).
+// QUEUE true (the periodic basis, whatever the order of the kept points): each thread queues its
 // survivors (atom, image) in order, the CTA
 // evaluates the queued pairs in FP64, every lane on one pair, so the FP64 pipe (a small
 // fraction of the FP32 rate on this part, and as slow for one active lane as for 32)
@@ -51,7 +123,7 @@ template <bool QUEUE>
 __global__ void __launch_bounds__(kRsPts) realspace_fp64_kernel(
     const int32_t *__restrict__ kept, long long m0, long long rows, const double *__restrict__ axis, int nx, int ny,
     const double *__restrict__ atoms, int N, const double *__restrict__ shifts, int S, int zero_idx, double rc,
-    double sa, double *__restrict__ phi) {
+    double sa, double d2_in, double d2_self, ErfcTable tab, double *__restrict__ phi) {
     constexpr int kRsShiftChunk = rs_chunk<QUEUE>();
     extern __shared__ float4 rs_cand[];  // [kRsAtoms][kRsShiftChunk] image (x, y, z) in FP32, shift index
     double *qterm = reinterpret_cast<double *>(rs_cand + kRsAtoms * kRsShiftChunk);      // [kRsQueue][kRsPts]
@@ -143,10 +215,10 @@ __global__ void __launch_bounds__(kRsPts) realspace_fp64_kernel(
                         const double ex = g[0] - (pa[0] + shifts[3 * s]);
                         const double ey = g[1] - (pa[1] + shifts[3 * s + 1]);
                         const double ez = g[2] - (pa[2] + shifts[3 * s + 2]);
-                        const double r = sqrt(ex * ex + ey * ey + ez * ez);
-                        if (!(r <= rc)) continue;
-                        if (s == zero_idx && !(r > 1e-10)) continue;
-                        acc += erfc(sa * r) / r;
+                        const double d2 = ex * ex + ey * ey + ez * ez;
+                        if (!le_bits(d2, d2_in)) continue;
+                        if (s == zero_idx && le_bits(d2, d2_self)) continue;
+                        acc += erfc_term(d2, tab, sa);
                     }
                     tile[a][threadIdx.x] = acc;
                 }
@@ -204,9 +276,9 @@ __global__ void __launch_bounds__(kRsPts) realspace_fp64_kernel(
                 const double ex = gs[0][lo] - (pa[0] + shifts[3 * s]);
                 const double ey = gs[1][lo] - (pa[1] + shifts[3 * s + 1]);
                 const double ez = gs[2][lo] - (pa[2] + shifts[3 * s + 2]);
-                const double r = sqrt(ex * ex + ey * ey + ez * ez);
+                const double d2 = ex * ex + ey * ey + ez * ez;
                 double term = 0.0;
-                if ((r <= rc) && !(s == zero_idx && !(r > 1e-10))) term = erfc(sa * r) / r;
+                if (le_bits(d2, d2_in) && !(s == zero_idx && le_bits(d2, d2_self))) term = erfc_term(d2, tab, sa);
                 qterm[k * kRsPts + lo] = term;
             }
             __syncthreads();
@@ -269,29 +341,21 @@ __global__ void finish_kernel(const double *__restrict__ G, const double *__rest
     if (t < N) b[t] = r[t] - s[t] * (*sumV) * invM;
 }
 
-// G (N x N, column-major) holds its upper triangle (row <= column): copy it to the lower
-__global__ void mirror_upper_kernel(double *__restrict__ G, int N) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)N * N) return;
-    const int c = (int)(t / N), r = (int)(t - (long long)c * N);
-    if (r > c) G[t] = G[(size_t)r * N + c];
-}
-
 __global__ void shifted_sums_kernel(const double *__restrict__ sphi, const double *__restrict__ c, long long M,
                                     int N, double *__restrict__ s) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < N) s[t] = sphi[t] - (double)M * c[t];
 }
 
-// ---- FP64 separable reciprocal sum (the escalated fit) ----
-// The transform of recip_sep.cu at FP64-level accuracy: stages A and B in double-float
-// (~2^-46 relative, on the FP32 pipe, whose rate is many times the FP64 pipe's here), the
-// weights and stage C in FP64; with the exact per-axis lattice phases ex, ey, ez of the grid
-// (tables of the Ewald object) and
-// W_a(n) = w_k e^{-i k.r_a},
+// ---- FP64 separable reciprocal sum ----
+// The transform of recip_sep.cu with the exact per-axis lattice phases ex, ey, ez of the grid
+// (tables of the Ewald object) and W_a(n) = w_k e^{-i k.r_a},
 //   F[l][n2][a][n1] = sum_n3 ez[n3][l] W[n2][n3][a][n1]      (every grid plane l)
 //   E[r][a][n1]     = sum_n2 ey[n2][j_r] F[l_r][n2][a][n1]    (the rows r that hold kept points)
 //   Phi[m][a]      += Re sum_n1 ex[n1][i_m] E[r_m][a][n1]     (every kept point)
+// The FP64 fit (Num64) takes every stage in FP64; the refit (NumDf) the first two in double-float
+// (~2^-46 relative, on the FP32 pipe, whose rate is many times the FP64 pipe's here), the
+// weights and stage C in FP64.
 // n1 in [0, P], n2, n3 in [-P, P], P = KMAX - 1 (stored with offset P; the FP64 tables
 // carry offset KMAX).  On the 2000-atom triclinic cube this is ~35 GFLOP instead of the
 // flat k-table's 158 (repeat.py:968-981 evaluated as one DGEMM).
@@ -317,10 +381,40 @@ __device__ __forceinline__ double2 cmul64(double2 x, double2 y) {
     return make_double2(x.x * y.x - x.y * y.y, x.x * y.y + x.y * y.x);
 }
 
+// The numbers of the plane and row stages: how they are stored, and a complex multiply-accumulate
+struct Num64 {
+    using T = double2;
+    struct Acc {
+        double x = 0.0, y = 0.0;
+    };
+    static __device__ __forceinline__ T store(double re, double im) { return make_double2(re, im); }
+    static __device__ __forceinline__ void mac(Acc &a, T p, T q) {
+        a.x = fma(p.x, q.x, a.x);
+        a.x = fma(-p.y, q.y, a.x);
+        a.y = fma(p.x, q.y, a.y);
+        a.y = fma(p.y, q.x, a.y);
+    }
+    static __device__ __forceinline__ T pack(const Acc &a) { return make_double2(a.x, a.y); }
+    static __device__ __forceinline__ double2 value(const Acc &a) { return make_double2(a.x, a.y); }
+};
+struct NumDf {
+    using T = float4;
+    struct Acc {
+        dfa::acc re{0.f, 0.f}, im{0.f, 0.f};
+    };
+    static __device__ __forceinline__ T store(double re, double im) { return dfa::split(re, im); }
+    static __device__ __forceinline__ void mac(Acc &a, const T &p, const T &q) { dfa::cmac(a.re, a.im, p, q); }
+    static __device__ __forceinline__ T pack(const Acc &a) { return dfa::pack(a.re, a.im); }
+    static __device__ __forceinline__ double2 value(const Acc &a) {
+        return make_double2(dfa::to_double(a.re), dfa::to_double(a.im));
+    }
+};
+
 // W[n2'][n3'][a][n1] = w_k e^{-i k.r_a} for the k-set (zero elsewhere: cleared before), from
-// FP64 phase products, stored as double-float for stage A
+// FP64 phase products
+template <class Num>
 __global__ void build_w64_kernel(const int *__restrict__ kidx, const double *__restrict__ kcoef, int K, int N,
-                                 int P, const double2 *__restrict__ U, float4 *__restrict__ W) {
+                                 int P, const double2 *__restrict__ U, typename Num::T *__restrict__ W) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)N * K) return;
     const int a = (int)(t / K), k = (int)(t - (long long)a * K);
@@ -329,39 +423,40 @@ __global__ void build_w64_kernel(const int *__restrict__ kidx, const double *__r
     const double2 *u = U + (size_t)a * 3 * nw;
     const double2 v = cmul64(cmul64(u[n1 + P], u[nw + n2]), u[2 * nw + n3]);
     const double w = kcoef[k];
-    W[(((size_t)n2 * nw + n3) * N + a) * n1c + n1] = dfa::split(w * v.x, w * v.y);
+    W[(((size_t)n2 * nw + n3) * N + a) * n1c + n1] = Num::store(w * v.x, w * v.y);
 }
 
-// stage A: one thread per (l, n2, a, n1), n1 fastest, in double-float (dfa::cmac) from the
-// double-float phases and W; F is stored as double-float for stage B
-__global__ void stage_a64_kernel(const float4 *__restrict__ W, const float4 *__restrict__ ezf, int nz, int N,
-                                 int P, float4 *__restrict__ F) {
+// stage A: one thread per (l, n2, a, n1), n1 fastest
+template <class Num>
+__global__ void stage_a64_kernel(const typename Num::T *__restrict__ W, const typename Num::T *__restrict__ ez, int nz,
+                                 int N, int P, typename Num::T *__restrict__ F) {
     const int nw = 2 * P + 1, n1c = P + 1;
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)nz * nw * N * n1c) return;
     const long long an = (long long)N * n1c;
     const int r = (int)(t % an);           // a n1c + n1
     const int n2 = (int)((t / an) % nw), l = (int)(t / (an * nw));
-    dfa::acc re{0.f, 0.f}, im{0.f, 0.f};
-    for (int n3 = 0; n3 < nw; ++n3) dfa::cmac(re, im, ezf[(size_t)n3 * nz + l], W[((size_t)n2 * nw + n3) * an + r]);
-    F[t] = dfa::pack(re, im);
+    typename Num::Acc acc;
+    for (int n3 = 0; n3 < nw; ++n3) Num::mac(acc, ez[(size_t)n3 * nz + l], W[((size_t)n2 * nw + n3) * an + r]);
+    F[t] = Num::pack(acc);
 }
 
-// stage B over the listed rows (row = j + l ny): one thread per (row, a, n1), n1 fastest.  In
-// double-float on the FP32 pipe (~2^-46 relative, dfa::cmac) from the double-float phases and F:
-// the FP64 pipe is a small fraction of the FP32 rate here, and this stage is most of the sum's
-// work on a sparse cube (29 GFLOP on the 2000-atom triclinic one); E is stored in FP64.
-__global__ void stage_b64_kernel(const float4 *__restrict__ F, const float4 *__restrict__ eyf, int ny, int N,
-                                 int P, const int *__restrict__ rows, int R, double2 *__restrict__ E) {
-    const int nw = 2 * P + 1, n1c = P + 1;
-    const long long an = (long long)N * n1c;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)R * an) return;
-    const int ri = (int)(t / an), r = (int)(t - (long long)ri * an);
-    const int row = rows[ri], l = row / ny, j = row - l * ny;
-    dfa::acc re{0.f, 0.f}, im{0.f, 0.f};
-    for (int n2 = 0; n2 < nw; ++n2) dfa::cmac(re, im, eyf[(size_t)n2 * ny + j], F[((size_t)l * nw + n2) * an + r]);
-    E[t] = make_double2(dfa::to_double(re), dfa::to_double(im));
+// stage B over the listed rows (row = j + l ny, *R of them, a count the host does not wait for): one
+// thread per (a, n1), n1 fastest, the blocks along y striding over the rows; E is stored in FP64.
+template <class Num>
+__global__ void __launch_bounds__(128) stage_b64_kernel(const typename Num::T *__restrict__ F,
+                                                        const typename Num::T *__restrict__ ey, int ny, int N, int P,
+                                                        const int *__restrict__ rows, const int *__restrict__ R,
+                                                        double2 *__restrict__ E) {
+    const int nw = 2 * P + 1, n1c = P + 1, nr = *R;
+    const long long an = (long long)N * n1c, r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= an) return;
+    for (int ri = blockIdx.y; ri < nr; ri += gridDim.y) {
+        const int row = rows[ri], l = row / ny, j = row - l * ny;
+        typename Num::Acc acc;
+        for (int n2 = 0; n2 < nw; ++n2) Num::mac(acc, ey[(size_t)n2 * ny + j], F[((size_t)l * nw + n2) * an + r]);
+        E[ri * an + r] = Num::value(acc);
+    }
 }
 
 // mark the grid rows that hold kept points m0 .. m0+rows-1
@@ -369,6 +464,32 @@ __global__ void mark_rows_kernel(const int32_t *__restrict__ kept, long long m0,
                                  unsigned char *__restrict__ mark) {
     const long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (m < rows) mark[kept[m0 + m] / nx] = 1;
+}
+
+// the marked rows numbered in order (one CTA): rowmap[row] their numbers, rowlist their rows, *R their
+// count
+__global__ void __launch_bounds__(1024) number_rows_kernel(const unsigned char *__restrict__ mark, int nrows,
+                                                           int *__restrict__ rowmap, int *__restrict__ rowlist,
+                                                           int *__restrict__ R) {
+    __shared__ int part[1024];
+    const int t = threadIdx.x, per = (nrows + 1023) / 1024, b0 = min(t * per, nrows), b1 = min(b0 + per, nrows);
+    int c = 0;
+    for (int b = b0; b < b1; ++b) c += mark[b];
+    part[t] = c;
+    __syncthreads();
+    for (int off = 1; off < 1024; off <<= 1) {
+        const int v = t >= off ? part[t - off] : 0;
+        __syncthreads();
+        part[t] += v;
+        __syncthreads();
+    }
+    int run = t == 0 ? 0 : part[t - 1];
+    for (int b = b0; b < b1; ++b)
+        if (mark[b]) {
+            rowmap[b] = run;
+            rowlist[run++] = b;
+        }
+    if (t == 1023) *R = part[1023];
 }
 
 // stage C: phi[m][a] = Re sum_n1 ex[n1][i] E[rowmap[row]][a][n1]  (one thread per (m, a), a fastest)
@@ -414,11 +535,33 @@ void finish_normal_equations(const double *G, const double *r, const double *s_c
     RP_LAUNCH_CHECK();
 }
 
+namespace {
+// W and the plane stage; returns F
+template <class Num>
+typename Num::T *recip_planes64(rp_ctx *ctx, const rp_ewald *ew, const double *d_atoms, int N,
+                                const typename Num::T *ez, cudaStream_t stream) {
+    using T = typename Num::T;
+    const int P = ew->kmax - 1, nw = 2 * P + 1, n1c = P + 1, nz = ew->grid.n_grid[2], K = ew->K;
+    double2 *U = ctx->buf_t<double2>("g64_U", (size_t)N * 3 * nw);
+    T *W = ctx->buf_t<T>("g64_W", (size_t)nw * nw * N * n1c);
+    T *F = ctx->buf_t<T>("g64_F", (size_t)nz * nw * N * n1c);
+    RP_CUDA(cudaMemsetAsync(W, 0, sizeof(T) * (size_t)nw * nw * N * n1c, stream));
+    RecBasis rb;
+    for (int q = 0; q < 9; ++q) rb.rb[q] = ew->rec[q];
+    atom_phases64_kernel<<<ceil_div(N * 3 * nw, 128), 128, 0, stream>>>(d_atoms, N, rb, P, U);
+    RP_LAUNCH_CHECK();
+    build_w64_kernel<Num><<<ceil_div((long long)N * K, 128), 128, 0, stream>>>(ew->d_kidx, ew->d_kcoef, K, N, P, U, W);
+    RP_LAUNCH_CHECK();
+    stage_a64_kernel<Num><<<ceil_div((long long)nz * nw * N * n1c, 128), 128, 0, stream>>>(W, ez, nz, N, P, F);
+    RP_LAUNCH_CHECK();
+    return F;
+}
+}  // namespace
+
 void gram_fp64(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, const int32_t *kept_idx_dev,
                const double *Vc_dev, int64_t M, double *A_dev, double *b_dev, double *sum_phi_dev,
-               cudaStream_t stream, bool separable) {
+               cudaStream_t stream, bool refit) {
     RP_REQUIRE(N > 0 && M > 0, "rp_gram: need N > 0 and M > 0");
-    const int K = ew->K, K2 = 2 * ew->K;
     std::vector<double> sh;
     int zero_idx = -1;
     prune_shifts(ew, atoms, N, sh, zero_idx);
@@ -430,40 +573,24 @@ void gram_fp64(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, cons
     RP_CUDA(cudaMemcpyAsync(d_shifts, sh.data(), sizeof(double) * sh.size(), cudaMemcpyHostToDevice, stream));
     RP_CUDA(cudaMemcpyAsync(d_axis, ew->grid.axis, sizeof(double) * 9, cudaMemcpyHostToDevice, stream));
 
-    // reciprocal part: the flat k-table product (one DGEMM per chunk: the comparator), or
-    // the separable transform in FP64 (the escalated fit): W and the plane stage once per fit
-    const int kp = ew->kmax - 1, nw = 2 * kp + 1, n1c = kp + 1;  // the separable sum's n range
+    // reciprocal part: W and the plane stage once per fit; the FP64 phase tables carry the offset
+    // KMAX on n2 and n3, the sum's range starts at -(KMAX - 1)
+    const int kp = ew->kmax - 1, n1c = kp + 1;  // the separable sum's n range
     const int nx = ew->grid.n_grid[0], ny = ew->grid.n_grid[1], nz = ew->grid.n_grid[2];
-    const bool sep = separable && K > 0 && kp >= 0;
-    double *B = nullptr;
-    float4 *F64 = nullptr;
-    if (sep) {
+    const bool recip = ew->K > 0 && kp >= 0;
+    double2 *F64 = nullptr;
+    float4 *Fdf = nullptr;
+    if (recip) {
         StageTimer tt(ctx, "fp64_recip_sep", stream);
-        double2 *U = ctx->buf_t<double2>("g64_U", (size_t)N * 3 * nw);
-        float4 *W = ctx->buf_t<float4>("g64_W", (size_t)nw * nw * N * n1c);
-        F64 = ctx->buf_t<float4>("g64_F", (size_t)nz * nw * N * n1c);
-        RP_CUDA(cudaMemsetAsync(W, 0, sizeof(float4) * (size_t)nw * nw * N * n1c, stream));
-        RecBasis rb;
-        for (int q = 0; q < 9; ++q) rb.rb[q] = ew->rec[q];
-        atom_phases64_kernel<<<ceil_div(N * 3 * nw, 128), 128, 0, stream>>>(d_atoms, N, rb, kp, U);
-        RP_LAUNCH_CHECK();
-        build_w64_kernel<<<ceil_div((long long)N * K, 128), 128, 0, stream>>>(ew->d_kidx, ew->d_kcoef, K, N, kp, U, W);
-        RP_LAUNCH_CHECK();
-        stage_a64_kernel<<<ceil_div((long long)nz * nw * N * n1c, 128), 128, 0, stream>>>(W, ew->d_ezf, nz, N, kp,
-                                                                                          F64);
-        RP_LAUNCH_CHECK();
-    } else {
-        B = ctx->buf_t<double>("g64_B", (size_t)N * K2);
-        if (K > 0) atom_tables_fp64(ew, d_atoms, N, B, K2, stream);
+        if (refit) Fdf = recip_planes64<NumDf>(ctx, ew, d_atoms, N, ew->d_ezf, stream);
+        else F64 = recip_planes64<Num64>(ctx, ew, d_atoms, N, ew->d_ez + nz, stream);
     }
 
-    // chunk rows so T and Phi stay within ~2 GB together (separable: Phi and the chunk's
-    // reciprocal rows, at most one per point, within ~4 GB)
-    const size_t row_bytes = sep ? sizeof(double) * N + sizeof(double2) * (size_t)N * n1c
-                                 : sizeof(double) * ((size_t)K2 + N);
-    int64_t chunk = std::max<int64_t>(256, (int64_t)((size_t)(sep ? 4 : 2) << 30) / (int64_t)row_bytes);
+    // chunk rows so that Phi and the chunk's reciprocal rows, at most one per point, stay within ~4 GB
+    const size_t nrows = (size_t)ny * nz;
+    const size_t row_bytes = sizeof(double) * N + (recip ? sizeof(double2) * (size_t)N * n1c : 0);
+    int64_t chunk = std::max<int64_t>(256, (int64_t)((size_t)4 << 30) / (int64_t)row_bytes);
     chunk = std::min<int64_t>(chunk, M);
-    double *T = sep ? nullptr : ctx->buf_t<double>("g64_T", (size_t)chunk * K2);
     double *P = ctx->buf_t<double>("g64_P", (size_t)chunk * N);
     double *G = ctx->buf_t<double>("g64_G", (size_t)N * N);
     double *r = ctx->buf_t<double>("g64_r", (size_t)N);
@@ -476,61 +603,59 @@ void gram_fp64(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, cons
     RP_CUDA(cudaMemsetAsync(r, 0, sizeof(double) * N, stream));
     RP_CUDA(cudaMemsetAsync(sphi, 0, sizeof(double) * N, stream));
 
-    const bool syrk = N >= 512;  // the Gram's cuBLAS call (below)
+    // the real-space term's table over the cutoff's range (the 1/r basis has alpha 0 and no cutoff)
+    ErfcTable tab{nullptr, 0};
+    if (recip) {
+        const int n = erfc_intervals(ew->cutoff);
+        double *t = ctx->buf_t<double>("g64_erfc", (size_t)n * (kErfcDeg + 1));
+        const int base = (1023 + kErfcLow) * kErfcPerOctave;  // exponent and six mantissa bits of 2^kErfcLow
+        erfc_table_kernel<<<ceil_div(n, 64), 64, 0, stream>>>(ew->sqrt_alpha, n, base, t);
+        RP_LAUNCH_CHECK();
+        tab = ErfcTable{t, base};
+    }
+    const double d2_in = square_limit(ew->cutoff), d2_self = square_limit(1e-10);
+
     cublasHandle_t h = ctx->blas();
     RP_CUBLAS(cublasSetStream(h, stream));
-    const double one = 1.0, zero = 0.0;
+    const double one = 1.0;
     for (int64_t m0 = 0; m0 < M; m0 += chunk) {
         const int64_t rows = std::min<int64_t>(chunk, M - m0);
-        if (sep) {
+        if (recip) {
             StageTimer tt(ctx, "fp64_recip_sep", stream);
-            // the grid rows of this chunk's points, numbered on the host
-            const size_t nrows = (size_t)ny * nz;
+            // the grid rows of this chunk's points, numbered on the device
+            const int64_t most = std::min<int64_t>((int64_t)nrows, rows);
             unsigned char *mark = ctx->buf_t<unsigned char>("g64_mark", nrows);
+            int *rowmap = ctx->buf_t<int>("g64_rowmap", nrows);
+            int *rowlist = ctx->buf_t<int>("g64_rowlist", (size_t)most + 1);  // the count after the rows
             RP_CUDA(cudaMemsetAsync(mark, 0, nrows, stream));
             mark_rows_kernel<<<ceil_div(rows, 256), 256, 0, stream>>>(kept_idx_dev, m0, rows, nx, mark);
             RP_LAUNCH_CHECK();
-            unsigned char *hmark = static_cast<unsigned char *>(ctx->host_buf("g64_mark", nrows));
-            int *hmap = static_cast<int *>(ctx->host_buf("g64_rowmap", sizeof(int) * nrows * 2));
-            RP_CUDA(cudaMemcpyAsync(hmark, mark, nrows, cudaMemcpyDeviceToHost, stream));
-            RP_CUDA(cudaStreamSynchronize(stream));
-            int R = 0;
-            int *hlist = hmap + nrows;
-            for (size_t r = 0; r < nrows; ++r) {
-                hmap[r] = hmark[r] ? R : -1;
-                if (hmark[r]) hlist[R++] = (int)r;
-            }
-            int *rowmap = ctx->buf_t<int>("g64_rowmap", nrows);
-            int *rowlist = ctx->buf_t<int>("g64_rowlist", (size_t)std::max(R, 1));
-            RP_CUDA(cudaMemcpyAsync(rowmap, hmap, sizeof(int) * nrows, cudaMemcpyHostToDevice, stream));
-            RP_CUDA(cudaMemcpyAsync(rowlist, hlist, sizeof(int) * R, cudaMemcpyHostToDevice, stream));
-            double2 *E64 = ctx->buf_t<double2>("g64_E", (size_t)std::max(R, 1) * N * n1c);
-            stage_b64_kernel<<<ceil_div((long long)R * N * n1c, 128), 128, 0, stream>>>(F64, ew->d_eyf, ny, N, kp,
-                                                                                       rowlist, R, E64);
+            number_rows_kernel<<<1, 1024, 0, stream>>>(mark, (int)nrows, rowmap, rowlist, rowlist + most);
+            RP_LAUNCH_CHECK();
+            double2 *E64 = ctx->buf_t<double2>("g64_E", (size_t)most * N * n1c);
+            // about 32 blocks per SM, or one per row
+            const unsigned bx = ceil_div((long long)N * n1c, 128);
+            const dim3 nb(bx, (unsigned)std::max<int64_t>(1, std::min<int64_t>(most, 32LL * std::max(1, ctx->sm_count) / bx)));
+            if (refit)
+                stage_b64_kernel<NumDf><<<nb, 128, 0, stream>>>(Fdf, ew->d_eyf, ny, N, kp, rowlist, rowlist + most, E64);
+            else
+                stage_b64_kernel<Num64><<<nb, 128, 0, stream>>>(F64, ew->d_ey + ny, ny, N, kp, rowlist, rowlist + most,
+                                                                E64);
             RP_LAUNCH_CHECK();
             stage_c64_kernel<<<ceil_div(rows * N, 128), 128, 0, stream>>>(E64, ew->d_ex, nx, N, kp, kept_idx_dev, m0,
                                                                           rows, rowmap, P);
             RP_LAUNCH_CHECK();
-            // the pinned row arrays are rewritten by the next chunk: its uploads must be done
-            RP_CUDA(cudaStreamSynchronize(stream));
-        } else if (K > 0) {
-            {
-                StageTimer tt(ctx, "fp64_tables", stream);
-                grid_tables_fp64(ew, kept_idx_dev, m0, rows, T, K2, stream);
-            }
-            StageTimer tt(ctx, "fp64_recip_dgemm", stream);
-            RP_CUBLAS(cublasDgemm(h, CUBLAS_OP_T, CUBLAS_OP_N, N, (int)rows, K2, &one, B, K2, T, K2, &zero, P, N));
         } else {  // the non-periodic basis has no reciprocal part
             RP_CUDA(cudaMemsetAsync(P, 0, sizeof(double) * (size_t)rows * N, stream));
         }
         {
             StageTimer t_r(ctx, "fp64_realspace", stream);
-            const size_t smem = realspace_fp64_smem(sep);  // candidates (and the pair queue): 32 or 36 KB
-            auto kern = sep ? realspace_fp64_kernel<true> : realspace_fp64_kernel<false>;
+            const size_t smem = realspace_fp64_smem(recip);  // candidates (and the pair queue): 32 or 36 KB
+            auto kern = recip ? realspace_fp64_kernel<true> : realspace_fp64_kernel<false>;
             smem_optin((const void *)kern, smem);
             kern<<<dim3(ceil_div(rows, kRsPts), ceil_div(N, kRsAtoms)), kRsPts, smem, stream>>>(
-                kept_idx_dev, m0, rows, d_axis, ew->grid.n_grid[0], ew->grid.n_grid[1], d_atoms, N, d_shifts, S,
-                zero_idx, ew->cutoff, ew->sqrt_alpha, P);
+                kept_idx_dev, m0, rows, d_axis, nx, ny, d_atoms, N, d_shifts, S, zero_idx, ew->cutoff, ew->sqrt_alpha,
+                d2_in, d2_self, tab, P);
             RP_LAUNCH_CHECK();
         }
         column_sums_fp64(P, rows, N, N, csum, false, ctx, stream);
@@ -545,31 +670,14 @@ void gram_fp64(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, cons
         }
         shift_columns_kernel<<<ceil_div(rows * N, 256), 256, 0, stream>>>(P, rows, N, c);
         RP_LAUNCH_CHECK();
-        if (sep) {  // the exact two-word Gram on the tensor cores (G full, r included)
-            StageTimer t_g(ctx, "fp64_gram_words", stream);
-            gram_words_fp64(ctx, P, rows, N, Vc_dev + m0, G, r, stream);
-        } else {
-            // column-major view: X = P^T is N x rows with ld N;  G += X X^T,  r += X Vc.  DSYRK
-            // (one triangle, mirrored after the last chunk) halves the work, but for few
-            // columns cuBLAS's rank-k update parallelises poorly over the long k (31 ms for
-            // 77 x 109,682 against ~1.5 ms as a DGEMM), so small systems take the DGEMM.
-            StageTimer t_g(ctx, "fp64_gram_blas", stream);
-            if (syrk)
-                RP_CUBLAS(cublasDsyrk(h, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N, N, (int)rows, &one, P, N, &one, G, N));
-            else
-                RP_CUBLAS(cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_T, N, N, (int)rows, &one, P, N, P, N, &one, G, N));
-            RP_CUBLAS(cublasDgemv(h, CUBLAS_OP_N, N, (int)rows, &one, P, N, Vc_dev + m0, 1, &one, r, 1));
-        }
-    }
-    if (!sep && syrk) {
-        mirror_upper_kernel<<<ceil_div((long long)N * N, 256), 256, 0, stream>>>(G, N);
-        RP_LAUNCH_CHECK();
+        // the exact two-word Gram on the tensor cores (G full, r included)
+        StageTimer t_g(ctx, "fp64_gram_words", stream);
+        gram_words_fp64(ctx, P, rows, N, Vc_dev + m0, G, r, stream);
     }
     column_sums_fp64(Vc_dev, M, 1, 1, sumV, false, ctx, stream);
     shifted_sums_kernel<<<ceil_div(N, 128), 128, 0, stream>>>(sphi, c, M, N, s_c);
     RP_LAUNCH_CHECK();
     finish_normal_equations(G, r, s_c, sumV, M, N, A_dev, b_dev, stream);
-    (void)K;
 }
 
 }  // namespace rp

@@ -398,20 +398,11 @@ void batch_enqueue(rp_ctx *ctx, int n, const rp_fit_desc *descs, const double *c
             }
         const cudaEvent_t inputs = record(copy_lane);
         for (int ln = 0; ln < lanes; ++ln) RP_CUDA(cudaStreamWaitEvent(flane(ln), inputs, 0));
-        // the group's mixed-precision cubes in one launch per filter stage (brick order), the
-        // FP64 ones (flat order, the comparator) one by one
+        // the group's cubes in one launch per filter stage (brick order)
         std::vector<rp::FilterItem> items;
-        for (int i = i0; i < i1; ++i) {
-            const rp_fit_desc &d = descs[i];
-            const double *V = Vsrc[i];
-            if (d.precision == RP_PREC_MIXED) {
-                items.push_back(rp::FilterItem{&plan(i), pl_dev + pl_off[i], V, kept + off_pts[i], Vc + off_pts[i],
-                                               Md + i, vst + 2 * i});
-            } else {
-                rp::filter_launch(ctx, plan(i), pl_dev + pl_off[i], V, kept + off_pts[i], Vc + off_pts[i], Md + i,
-                                  nullptr, flane(i), "#f" + std::to_string(i % lanes), false, vst + 2 * i);
-            }
-        }
+        for (int i = i0; i < i1; ++i)
+            items.push_back(rp::FilterItem{&plan(i), pl_dev + pl_off[i], Vsrc[i], kept + off_pts[i], Vc + off_pts[i],
+                                           Md + i, vst + 2 * i});
         rp::filter_group(ctx, items, flane(g), "#fg" + std::to_string(g));
         for (int ln = 0; ln < lanes; ++ln) RP_CUDA(cudaStreamWaitEvent(stream, record(flane(ln)), 0));
         RP_CUDA(cudaMemcpyAsync(Mh + i0, Md + i0, sizeof(long long) * (i1 - i0), cudaMemcpyDeviceToHost, stream));
@@ -479,8 +470,8 @@ void batch_enqueue(rp_ctx *ctx, int n, const rp_fit_desc *descs, const double *c
     for (int g = 1; g < ngroups; ++g) filter_group_g(g);
     // 3. normal equations, group by group as the kept counts arrive.  Mixed-precision fits
     //    are spread over the gram streams (each with its own scratch), so one cube's small
-    //    kernels and launch gaps overlap another's; the FP64 comparator stays on the
-    //    caller's stream (its cuBLAS handle is shared).  Every cube's result is independent
+    //    kernels and launch gaps overlap another's; FP64 fits stay on the caller's stream
+    //    (they share one set of scratch).  Every cube's result is independent
     //    of the stream it ran on.  A mixed fit takes the single pass (Phi straight to
     //    digits, scaled by the a-priori bounds from the scaled vdW radii); a cube whose
     //    values clamp (a cell the bound's argument does not cover) is redone at completion
@@ -596,8 +587,8 @@ void batch_complete(rp_ctx *ctx, BatchRun &r) {
     rp::status_check(ctx, stream);
     // escalation: a mixed-precision cube whose bordered system is so ill-conditioned that
     // the Gram's rounding (~1e-7 relative) could move its charges visibly (kappa / (n+1)
-    // above the ctx's limit) is fitted again in FP64 (the reciprocal sum by the FP64
-    // separable transform)
+    // above the ctx's limit) is fitted again in FP64 (the reciprocal sum's plane
+    // and row stages in double-float)
     std::vector<int> esc;
     if (ctx->kappa_limit > 0.0)
         for (int i = 0; i < n; ++i)
@@ -611,6 +602,7 @@ void batch_complete(rp_ctx *ctx, BatchRun &r) {
             rp::gram_fp64(ctx, r.ews[i], d.atoms, d.N, r.kept + r.off_pts[i], r.Vc + r.off_pts[i], r.M[i],
                           r.A + r.off_nn[i], r.b + r.off_n[i], nullptr, stream, true);
         }
+        rp::status_check(ctx, stream);
         resolve(esc, RP_FIT_ESCALATED, RP_PREC_FP64);
     }
     if (changed) {
