@@ -1801,38 +1801,37 @@ __global__ void split_words_kernel(const double *__restrict__ P, long long rows,
     }
 }
 
-// G2 (2(N+1) square, row-major) = 2^-54 x the exact tile totals: Gram of the word rows
-__global__ void words_gram_kernel(const unsigned long long *__restrict__ th, const unsigned long long *__restrict__ tl,
-                                  int ntj, int Np2, double *__restrict__ G2) {
-    const int tile = blockIdx.y;
-    int ti, tj;
-    gram_tile_decode(tile, ntj, ti, tj);
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= kBM * kGN) return;
-    const int c = e / kBM, r = e - c * kBM;
-    const int a = ti * kBM + r, b = tj * kGN + c;
-    if (a >= Np2 || b >= Np2) return;
-    const size_t k = (size_t)tile * (kBM * kGN) + e;
+// 2^-54 x the exact total of word rows (r, c), from the tile that holds (min, max)
+__device__ __forceinline__ double tile_total(const unsigned long long *th, const unsigned long long *tl, int ntj,
+                                             int r, int c) {
+    if (r > c) {
+        const int t = r;
+        r = c;
+        c = t;
+    }
+    const int ti = r / kBM, tj = c / kGN;
+    const size_t k = (size_t)(ti * ntj - ti * (ti - 1) + tj - 2 * ti) * (kBM * kGN) + (c % kGN) * kBM + r % kBM;
     long long hi = (long long)th[k], lo = (long long)tl[k];
     hi += lo >> 32;
     lo &= 0xffffffffLL;
-    const double s = ldexp((double)hi * 4294967296.0 + (double)lo, -54);
-    G2[(size_t)a * Np2 + b] = s;
-    G2[(size_t)b * Np2 + a] = s;
+    return ldexp((double)hi * 4294967296.0 + (double)lo, -54);
 }
 
-// G[a][b] (N x N, either order: symmetric) and r[a] (b = N) += the combined words / (s_a s_b)
-__global__ void combine_words_kernel(const double *__restrict__ G2, int N, const unsigned long long *__restrict__ mx,
-                                     double *__restrict__ G, double *__restrict__ r) {
-    const int Np = N + 1, Np2 = 2 * Np;
+// G[a][b] (N x N, either order: symmetric) and r[a] (b = N) += the combined words / (s_a s_b);
+// rows a fastest, as the tiles store them
+__global__ void combine_words_kernel(const unsigned long long *__restrict__ th,
+                                     const unsigned long long *__restrict__ tl, int ntj, int N,
+                                     const unsigned long long *__restrict__ mx, double *__restrict__ G,
+                                     double *__restrict__ r) {
+    const int Np = N + 1;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)N * Np) return;
-    const int a = (int)(t / Np), b = (int)(t - (long long)a * Np);
-    const double g11 = G2[(size_t)a * Np2 + b], g12 = G2[(size_t)a * Np2 + Np + b];
-    const double g21 = G2[(size_t)(Np + a) * Np2 + b], g22 = G2[(size_t)(Np + a) * Np2 + Np + b];
+    const int b = (int)(t / N), a = (int)(t - (long long)b * N);
+    const double g11 = tile_total(th, tl, ntj, a, b), g12 = tile_total(th, tl, ntj, a, Np + b);
+    const double g21 = tile_total(th, tl, ntj, b, Np + a), g22 = tile_total(th, tl, ntj, Np + a, Np + b);
     const double v = (g11 + 7.450580596923828125e-9 * (g12 + g21) + 5.5511151231257827e-17 * g22) /
                      (pow2_scale(mx[a]) * pow2_scale(mx[b]));
-    if (b < N) G[(size_t)a * N + b] += v;
+    if (b < N) G[(size_t)b * N + a] += v;
     else r[a] += v;
 }
 
@@ -1867,10 +1866,7 @@ void gram_words_fp64(rp_ctx *ctx, const double *P, long long rows, int N, const 
     gram_totals_init(ctx, "w64_tsum", g, stream);
     const __half *Xq[kGSlices] = {X[0], X[1], X[2], X[3]};
     launch_gram(ctx, Xq, Np2, cols_pad, g, stream);
-    double *G2 = ctx->buf_t<double>("w64_G2", (size_t)Np2 * Np2);
-    words_gram_kernel<<<dim3(ceil_div(kBM * kGN, 256), ntri), 256, 0, stream>>>(g.out_hi, g.out_lo, ntj, Np2, G2);
-    RP_LAUNCH_CHECK();
-    combine_words_kernel<<<ceil_div((long long)N * Np, 256), 256, 0, stream>>>(G2, N, mx, G, r);
+    combine_words_kernel<<<ceil_div((long long)N * Np, 256), 256, 0, stream>>>(g.out_hi, g.out_lo, ntj, N, mx, G, r);
     RP_LAUNCH_CHECK();
 }
 

@@ -19,79 +19,10 @@
 
 #include "common.cuh"
 #include "df.cuh"
+#include "erfc64.cuh"
 
 namespace rp {
 namespace {
-
-// erfc(s sqrt(u)) / sqrt(u), s = sqrt(alpha), as a Taylor polynomial of degree 9 about the centre of u's
-// interval, 64 intervals per power of two: |u - centre| <= centre / 128, and over the cutoff's
-// range (alpha u <= pi^2) the first term left out is below 2e-18 of the value.  About 10 FP64
-// instructions per term instead of ~75 for erfc, a square root and a division (an FP64
-// instruction holds its pipe for 16 cycles per warp here).  The coefficients follow from the
-// derivative d/du erfc(s sqrt(u)) = -s / sqrt(pi) e^(-s^2 u) u^(-1/2) by products of the series of
-// e^(-s^2 u) and u^(-1/2).
-constexpr int kErfcDeg = 9, kErfcPerOctave = 64;
-constexpr int kErfcLow = -2;  // from u = 2^-2 (half a Bohr); nearer pairs take the functions themselves
-struct ErfcTable {
-    const double *c;  // [intervals][kErfcDeg + 1]; nullptr: the functions themselves (the 1/r basis)
-    int base;         // high word >> 14 of the first interval
-};
-int erfc_intervals(double rc) {  // up to the power of two above Rc^2
-    int e = 0;
-    std::frexp(rc * rc, &e);
-    return std::max(1, e - kErfcLow) * kErfcPerOctave;
-}
-__global__ void erfc_table_kernel(double sa, int n, int base, double *__restrict__ c) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double u = __hiloint2double(((base + i) << 14) | 0x2000, 0);  // the interval's centre
-    double h[kErfcDeg + 1], e[kErfcDeg + 1], g[kErfcDeg + 1];
-    h[0] = 1.0 / sqrt(u);
-    e[0] = exp(-sa * sa * u);
-    for (int k = 1; k <= kErfcDeg; ++k) {
-        h[k] = h[k - 1] * ((0.5 - k) / (k * u));
-        e[k] = e[k - 1] * (-sa * sa / k);
-    }
-    g[0] = erfc(sa * sqrt(u));
-    for (int k = 1; k <= kErfcDeg; ++k) {
-        double t = 0.0;
-        for (int q = 0; q < k; ++q) t += e[q] * h[k - 1 - q];
-        g[k] = -sa * 0.56418958354775628694807945 * t / k;  // 1 / sqrt(pi)
-    }
-    for (int k = 0; k <= kErfcDeg; ++k) {
-        double t = 0.0;
-        for (int q = 0; q <= k; ++q) t += g[q] * h[k - q];
-        c[(size_t)i * (kErfcDeg + 1) + k] = t;
-    }
-}
-__device__ __noinline__ double erfc_term_direct(double d2, double sa) {
-    const double r = sqrt(d2);
-    return erfc(sa * r) / r;
-}
-__device__ __forceinline__ double erfc_term(double d2, const ErfcTable &tab, double sa) {
-    const int hi = __double2hiint(d2), i = (hi >> 14) - tab.base;
-    if (!tab.c || i < 0) return erfc_term_direct(d2, sa);
-    const double2 *c = reinterpret_cast<const double2 *>(tab.c + (size_t)i * (kErfcDeg + 1));
-    const double t = d2 - __hiloint2double((hi & ~0x3fff) | 0x2000, 0);
-    double2 q = c[kErfcDeg / 2];
-    double v = fma(q.y, t, q.x);
-#pragma unroll
-    for (int k = kErfcDeg / 2 - 1; k >= 0; --k) {
-        q = c[k];
-        v = fma(fma(v, t, q.y), t, q.x);
-    }
-    return v;
-}
-// The largest double whose (correctly rounded) square root is at most r: r(d2) <= r and d2 <= this are
-// the same decision, without the square root.
-double square_limit(double r) {
-    double t = r * r;
-    while (std::sqrt(t) > r) t = std::nextafter(t, 0.0);
-    for (double u = std::nextafter(t, 1e308); std::sqrt(u) <= r; u = std::nextafter(u, 1e308)) t = u;
-    return t;
-}
-// a <= b for doubles that are not negative, off the FP64 pipe (their bits order like the values)
-__device__ __forceinline__ bool le_bits(double a, double b) { return __double_as_longlong(a) <= __double_as_longlong(b); }
 
 // Real-space sum in FP64 (repeat.py:944-966) over tiles of kRsPts kept points x kRsAtoms
 // atoms.  For each chunk of up to kRsShiftChunk shifts, the CTA first drops, per atom,
@@ -586,10 +517,18 @@ void gram_fp64(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, cons
         else F64 = recip_planes64<Num64>(ctx, ew, d_atoms, N, ew->d_ez + nz, stream);
     }
 
-    // chunk rows so that Phi and the chunk's reciprocal rows, at most one per point, stay within ~4 GB
+    // chunk rows so that Phi and the chunk's reciprocal rows, at most one per point, stay within
+    // ~4 GB, and with the Gram's digits within what the ctx has left (less a fifth for the rest)
     const size_t nrows = (size_t)ny * nz;
     const size_t row_bytes = sizeof(double) * N + (recip ? sizeof(double2) * (size_t)N * n1c : 0);
-    int64_t chunk = std::max<int64_t>(256, (int64_t)((size_t)4 << 30) / (int64_t)row_bytes);
+    size_t left = ctx->budget > ctx->used ? ctx->budget - ctx->used : 0;
+    for (const char *name : {"g64_P", "g64_E", "w64_X0", "w64_X1", "w64_X2", "w64_X3", "w64_tsum"})
+        left += ctx->scratch[ctx->slot_key(name)].bytes;
+    const size_t tiles = 16 * (size_t)(2 * N + 130) * (2 * N + 194) / 2;  // the Gram's tile totals
+    const size_t room = left > tiles ? (left - tiles) / 5 * 4 : 0;
+    int64_t chunk = std::min<int64_t>((int64_t)((size_t)4 << 30) / (int64_t)row_bytes,
+                                      (int64_t)(room / (row_bytes + 16 * ((size_t)N + 1))));
+    chunk = std::max<int64_t>(256, chunk);
     chunk = std::min<int64_t>(chunk, M);
     double *P = ctx->buf_t<double>("g64_P", (size_t)chunk * N);
     double *G = ctx->buf_t<double>("g64_G", (size_t)N * N);
@@ -604,15 +543,8 @@ void gram_fp64(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, cons
     RP_CUDA(cudaMemsetAsync(sphi, 0, sizeof(double) * N, stream));
 
     // the real-space term's table over the cutoff's range (the 1/r basis has alpha 0 and no cutoff)
-    ErfcTable tab{nullptr, 0};
-    if (recip) {
-        const int n = erfc_intervals(ew->cutoff);
-        double *t = ctx->buf_t<double>("g64_erfc", (size_t)n * (kErfcDeg + 1));
-        const int base = (1023 + kErfcLow) * kErfcPerOctave;  // exponent and six mantissa bits of 2^kErfcLow
-        erfc_table_kernel<<<ceil_div(n, 64), 64, 0, stream>>>(ew->sqrt_alpha, n, base, t);
-        RP_LAUNCH_CHECK();
-        tab = ErfcTable{t, base};
-    }
+    ErfcTable tab{nullptr, 0, 0};
+    if (recip) tab = erfc_table(ctx, "g64_erfc", ew->sqrt_alpha, ew->cutoff, stream);
     const double d2_in = square_limit(ew->cutoff), d2_self = square_limit(1e-10);
 
     cublasHandle_t h = ctx->blas();
