@@ -103,8 +103,9 @@ __device__ __forceinline__ double2 cmul(double2 x, double2 y) {
 __global__ void build_w_kernel(const __grid_constant__ RecipLaunch L) {
     const int jb = recip_job_of(L, blockIdx.x);
     const RecipJob &J = L.job[jb];
-    const long long t = (long long)(blockIdx.x - L.blk[jb]) * blockDim.x + threadIdx.x;
-    const int K = J.K, P = J.P;
+    long long t = (long long)(blockIdx.x - L.blk[jb]) * blockDim.x + threadIdx.x;
+    const int K = J.K, P = J.P, lane = threadIdx.x & 31;
+    if (J.q) t >>= 5;  // the charge-weighted column: a warp per k, its lanes over the atoms
     if (t >= (long long)J.ncols * K) return;
     const int col = (int)(t / K), k = (int)(t - (long long)col * K);
     const int n1c = P + 1, nw = 2 * P + 1;
@@ -127,14 +128,18 @@ __global__ void build_w_kernel(const __grid_constant__ RecipLaunch L) {
         return;
     }
     double2 z = make_double2(0.0, 0.0);
-    for (int a = 0; a < J.N; ++a) {
+    for (int a = lane; a < J.N; a += 32) {
         const double2 *u = J.U + (size_t)a * 3 * nw;
         const double2 v = cmul(cmul(u[n1 + P], u[nw + n2]), u[2 * nw + n3]);
         z.x += J.q[a] * v.x;
         z.y += J.q[a] * v.y;
     }
+    for (int o = 16; o > 0; o >>= 1) {
+        z.x += __shfl_xor_sync(0xffffffffu, z.x, o);
+        z.y += __shfl_xor_sync(0xffffffffu, z.y, o);
+    }
     const double w = J.kcoef[k];
-    *out = make_float2((float)(w * z.x), (float)(w * z.y));
+    if (lane == 0) *out = make_float2((float)(w * z.x), (float)(w * z.y));
 }
 
 // Each stage-A thread produces up to kN1B consecutive n1 outputs of one (plane, n2,
@@ -317,7 +322,7 @@ void recip_rows_group(rp_ctx *ctx, const std::vector<RecipRowsJob> &jobs, cudaSt
             const int nb = (n1c + kN1B - 1) / kN1B;
             const int k = L.n;
             blk[0][k + 1] = blk[0][k] + (int)ceil_div((long long)rj.N * 3 * nw, 128);
-            blk[1][k + 1] = blk[1][k] + (int)ceil_div((long long)ncols * ew->K, 128);
+            blk[1][k + 1] = blk[1][k] + (int)ceil_div((long long)ncols * ew->K, rj.d_q ? 4 : 128);
             blk[2][k + 1] = blk[2][k] + (int)ceil_div((long long)nz * nw * ncols * nb, 128);
             blk[3][k + 1] = blk[3][k] + (int)ceil_div(ncols, J.ab) * nz;
             smem_a = std::max(smem_a, sizeof(float2) * (size_t)nw * nz);
