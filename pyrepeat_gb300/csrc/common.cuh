@@ -553,6 +553,7 @@ struct SolveDesc {
     int wide64;           // As holds wide FP64 factors: skip the FP32 stage and the in-CTA FP64 LU
     int host64;           // FP32 factors in the CTA, but a stalled refinement goes to the host's FP64
                           // factorisation across the GPU (pre holds its flag) instead of an in-CTA FP64 LU
+    int across;           // FP32 factors already in As, their row order in perm and pivot range in pre
     int host32;           // wide FP32 factors refined on the host path (refine_wide32): the kernel skips it
 };
 // Wide systems of a solve launch whose FP32 refinement may not have converged: their flags are

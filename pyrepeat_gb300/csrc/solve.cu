@@ -716,6 +716,7 @@ constexpr int kLUWideMin = 768;
 // when its refinement stalls the FP64 factors come from across the GPU (cuSOLVER getrf): an
 // in-CTA FP64 LU of 425 unknowns takes ~13 ms on one SM's FP64 pipe
 constexpr int kLUHost64Min = 256;
+constexpr int kAcrossTwo = 512;  // least unknowns for two systems of a launch to be factored across the GPU
 constexpr int kLUWideMax = (int)((225 * 1024) / (sizeof(float) * 5));
 
 // r = bs - A0 x in FP64: a warp per eight rows, lanes along the row.  The rows' sums over the lanes
@@ -790,7 +791,13 @@ __global__ void __launch_bounds__(kSolve) lu_solve_refine_kernel(const SolveDesc
             d.r[t] = d.bs[t];
         }
         bool factored;
-        if (n1 <= kLUBlockedMax) {
+        if (d.across) {  // factored across the GPU before this launch
+            factored = d.pre[0] == 0.0;
+            pmin = d.pre[1];
+            pmax = d.pre[2];
+            for (int t = threadIdx.x; t < n1; t += blockDim.x) orig[t] = factored ? d.perm[t] : t;
+            __syncthreads();
+        } else if (n1 <= kLUBlockedMax) {
             float *work = fsh + ((3 * n1 + 3) & ~3);
             factored = lu_factor_f32_blocked(L, orig, n1, work, lus, pmin, pmax);
         } else {
@@ -935,8 +942,8 @@ __global__ void __launch_bounds__(kSolve) lu_solve_refine_kernel(const SolveDesc
 }
 
 // ---------------------------------------------------------------------------
-// Wide factorisation of one large system across the whole GPU, before lu_solve_refine_kernel
-// refines it.  One CTA factoring n1^3 / 3 FMAs alone is SM-bound (20 ms at n1 = 1456 in FP32,
+// Wide factorisation of one system beyond kLUAcrossMax unknowns across the whole GPU, before its
+// refinement.  One CTA factoring n1^3 / 3 FMAs alone is SM-bound (20 ms at n1 = 1456 in FP32,
 // and FP64 runs at 1/64 of the FP32 rate); here only the panels are serial.  A0 is copied into
 // As (FP32 for the first attempt, FP64 when that does not converge), then per panel of nb
 // columns (32, or 16 / 8 / 4 when the panel's rows do not fit shared memory at 32):
@@ -1083,6 +1090,319 @@ __global__ void __launch_bounds__(256) lu_trsm_kernel(T *__restrict__ A, int n1,
         if (j < nb) A[(size_t)(k0 + j) * n1 + c] = u[j];
 }
 
+// ---------------------------------------------------------------------------
+// FP32 factorisation of one system across the whole GPU, for systems of kLUHost64Min unknowns (where
+// one CTA's n1^3 / 3 multiply-adds are SM-bound) to kLUAcrossMax.  Per panel of NB columns:
+//   lu_panel_across_kernel<R>  one CTA: the panel's rows in registers (R rows of NB = 64 / R columns
+//                    per thread, so up to 512 R rows), two barriers per column as in
+//                    lu_factor_f32_blocked.  It writes the panel's rows in their new order
+//                    (LP, for the update), each row to the factors' row of its *input* row
+//                    number (F), and the order itself: no row of earlier panels ever moves.
+//   lu_update_across_kernel   64 x 64 tiles over the GPU: U12 = L11^-1 A12 of the tile's columns
+//                    (by every tile of a column, cheaper than another launch), then
+//                    A22' = A22 - L21 U12 with the rows taken in the new order, from one
+//                    buffer to the other, so that no tile reads what another writes.
+// lu_collect_kernel gathers F's rows into the final order.  d.perm receives that order (row i of
+// the factors is row perm[i] of the input); pre = {flag, min|pivot|, max|pivot|}, flag 1 = zero or
+// non-finite pivot (the later launches return at once).
+// Bounded by the panels' chain of latencies, about 1200 cycles per column (search, publish, pick,
+// update) and 5 us per panel of loads and stores; an update of 2001 x 2001 takes 8 us.  Half as many
+// barriers, eight columns at a time and panels wholly in line (their instruction fetch costs as
+// much) were no faster.  Measured: 7.8 -> 3.5 ms at 2001 unknowns, 2.3 -> 0.83 at 768, 3.6 -> 1.35 at
+// 1101 (against panels in shared memory with four barriers per column, interchanges on one CTA
+// and a cuBLAS rank-32 update).
+constexpr int kLUAcrossMax = 4096;
+constexpr int kPanelT = 512;  // threads of a panel: R rows each, 64 values in registers
+struct LuStep {
+    const float *Ao;   // trailing matrix (rows in the order before this panel)
+    float *An;         // and after it
+    float *LP;         // [rows from k0][32] the panel in its new order
+    float *F;          // factors by input row
+    int *from;         // [n1] new position -> position before this panel
+    const int *id_o;   // position -> input row, before this panel
+    int *id_n;         // and after it
+    int *orig;         // final order
+    double *pre;
+    int n1, k0, nb;
+};
+//   The column loop is not unrolled (a whole panel in line is 60 KB of instructions run once, and
+//   their fetch took 0.7 us per column): column j is always register 0, and the update that
+//   leaves a row shifts it by one.  What is final of a row goes to shared memory on the way.
+template <int R>
+__global__ void __launch_bounds__(kPanelT) lu_panel_across_kernel(LuStep p) {
+    constexpr int NB = 64 / R, LD = NB + 1;
+    extern __shared__ __align__(16) float pst[];  // [m][LD] the panel's rows, then their positions and input rows
+    __shared__ unsigned key[2][16];  // each warp's candidate: its value, position, row of pst ...
+    __shared__ int at_[2][16], row_[2][16];
+    __shared__ __align__(16) float cand[2][16][NB + 4];  // ... and its row from this column on, 1 / pivot for the pivot, which is at NB
+    const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
+    const int n1 = p.n1, k0 = p.k0, nb = p.nb, m = n1 - k0;
+    int *posr = reinterpret_cast<int *>(pst + (size_t)m * LD), *ids = posr + m;
+    if (k0 > 0 && p.pre[0] != 0.0) return;  // an earlier panel met a zero pivot
+    const int sc = lane % NB, sr = warp * (32 / NB) + lane / NB, sn = nw * (32 / NB);  // staging: column, first row, step
+    if (sc < nb)
+        for (int r = sr; r < m; r += sn)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(pst + r * LD + sc)),
+                         "l"(p.Ao + (size_t)(k0 + r) * n1 + k0 + sc) : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    int pos[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        const int t = tid + q * nt;
+        pos[q] = t < m ? t : -1;  // -1: no row
+        if (t < m) ids[t] = p.id_o[k0 + t];
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    float a[R][NB];
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+#pragma unroll
+        for (int c = 0; c < NB; ++c) a[q][c] = pos[q] >= 0 && c < nb ? pst[pos[q] * LD + c] : 0.f;
+    float pmin = 3.0e38f, pmax = 0.f;
+    bool ok = true;
+#pragma unroll
+    for (int seg = 0; seg < NB / 8; ++seg) {
+        const int W = NB - 8 * seg;  // live columns at the segment's start: registers 0 .. W-1
+#pragma unroll 1
+        for (int j = 8 * seg; j < min(8 * seg + 8, nb) && ok; ++j) {
+            const int b = j & 1;
+            unsigned bits = 0u;  // 0: no candidate; a NaN never wins
+            int at = 0x7fffffff;
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                const float v = fabsf(a[q][0]);
+                const unsigned u = pos[q] >= j && v == v ? __float_as_uint(v) + 1u : 0u;
+                if (u > bits || (u == bits && u != 0u && pos[q] < at)) {
+                    bits = u;
+                    at = pos[q];
+                }
+            }
+            unsigned best = __reduce_max_sync(0xffffffffu, bits);
+            unsigned who = __ballot_sync(0xffffffffu, bits == best);
+            bool mine = bits == best;
+            if (__popc(who) != 1) {  // ties: the lowest position
+                const int low = __reduce_min_sync(0xffffffffu, mine ? at : 0x7fffffff);
+                mine = mine && at == low;
+            }
+            if (mine) {  // (with no candidate, any of the lanes: at is the same)
+                key[b][warp] = best;
+                at_[b][warp] = at;
+#pragma unroll
+                for (int q = 0; q < R; ++q)
+                    if (pos[q] == at) {
+                        float *to = cand[b][warp];
+#pragma unroll
+                        for (int c = 4; c < W; c += 4)
+                            *reinterpret_cast<float4 *>(to + c) = make_float4(a[q][c], a[q][c + 1], a[q][c + 2], a[q][c + 3]);
+                        *reinterpret_cast<float4 *>(to) = make_float4(1.0f / a[q][0], a[q][1], a[q][2], a[q][3]);
+                        to[NB] = a[q][0];
+                        row_[b][warp] = tid + q * nt;
+                    }
+            }
+            __syncthreads();
+            const unsigned kb = lane < nw ? key[b][lane] : 0u;
+            best = __reduce_max_sync(0xffffffffu, kb);
+            who = __ballot_sync(0xffffffffu, kb == best);
+            const float apv = __uint_as_float(best - 1u);
+            if (best <= 1u || !(apv <= 3.402823466e38f)) {
+                ok = false;  // uniform: zero, infinite or no pivot
+                break;
+            }
+            if (__popc(who) != 1) {
+                const int ka = kb == best ? at_[b][lane] : 0x7fffffff;  // (best > 1: such lanes are below nw)
+                const int low = __reduce_min_sync(0xffffffffu, ka);
+                who = __ballot_sync(0xffffffffu, ka == low);
+            }
+            const int w = __ffs(who) - 1;
+            const float *prow = cand[b][w];
+            at = at_[b][w];
+            pmin = fminf(pmin, apv);
+            pmax = fmaxf(pmax, apv);
+            const float inv = prow[0];
+            float l[R];
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                l[q] = a[q][0] * inv;
+                if (pos[q] == at) pos[q] = j;  // the pivot row and position j trade places
+                else if (pos[q] == j) pos[q] = at;
+                if (pos[q] > j) pst[(tid + q * nt) * LD + j] = l[q];
+            }
+#pragma unroll
+            for (int c = 1; c < W; ++c) {  // (rows that are done take part: nothing reads them again)
+                const float pc = prow[c];
+#pragma unroll
+                for (int q = 0; q < R; ++q) a[q][c - 1] = fmaf(-l[q], pc, a[q][c]);
+            }
+            if (warp == j % nw && lane < NB - j) pst[row_[b][w] * LD + j + lane] = prow[lane ? lane : NB];
+        }
+    }
+    if (!ok) {
+        if (tid == 0) p.pre[0] = 1.0;
+        return;
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        if (pos[q] < 0) continue;
+        const int t = tid + q * nt, id = ids[t];
+        posr[t] = pos[q];
+        p.from[k0 + pos[q]] = k0 + t;
+        p.id_n[k0 + pos[q]] = id;
+        if (pos[q] < nb) p.orig[k0 + pos[q]] = id;
+    }
+    if (tid == 0) {
+        p.pre[1] = k0 == 0 ? (double)pmin : fmin(p.pre[1], (double)pmin);
+        p.pre[2] = k0 == 0 ? (double)pmax : fmax(p.pre[2], (double)pmax);
+    }
+    __syncthreads();
+    if (sc < nb)
+#pragma unroll 8
+        for (int r = sr; r < m; r += sn) {
+            const float v = pst[r * LD + sc];
+            p.LP[(size_t)posr[r] * 32 + sc] = v;
+            p.F[(size_t)ids[r] * n1 + k0 + sc] = v;
+        }
+}
+
+constexpr int kUpd = 64;  // tile edge of the update
+// SUM: the 32 products are summed and subtracted once, as a matrix product rounds (the wide
+// systems); otherwise subtracted one by one, as the factorisation in one CTA rounds.
+template <bool SUM>
+__global__ void __launch_bounds__(256, 3) lu_update_across_kernel(LuStep p) {
+    __shared__ __align__(16) float lt[kLUNB][kUpd + 4];    // L21 of the tile's rows, by columns
+    __shared__ __align__(16) float l11[kLUNB][kLUNB + 4];  // L11 by columns
+    __shared__ float u[kLUNB][kUpd];
+    const int n1 = p.n1, k0 = p.k0, nb = p.nb, c1 = k0 + nb;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int r0 = c1 + blockIdx.y * kUpd, q0 = c1 + blockIdx.x * kUpd;  // the tile's rows and columns
+    const int tr = (tid >> 4) * 4, tc = tid & 15;  // rows tr .. tr+3, columns tc + 16 i
+    const double flag = p.pre[0];
+    const int top = lane < nb ? p.from[k0 + lane] : k0;
+    int fr[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) fr[k] = p.from[min(r0 + tr + k, n1 - 1)];
+#pragma unroll
+    for (int t = tid; t < kLUNB * kLUNB; t += 256) {
+        const int i = t >> 5, j = t & 31;
+        l11[j][i] = i < nb && j < nb ? p.LP[(size_t)i * 32 + j] : 0.f;
+    }
+#pragma unroll
+    for (int r = warp; r < kUpd; r += 8) lt[lane][r] = r0 + r < n1 && lane < nb ? p.LP[(size_t)(r0 + r - k0) * 32 + lane] : 0.f;
+    if (flag != 0.0) return;  // (the row order is whole only after a whole panel)
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const int j = warp + 8 * h;
+        const float *row = p.Ao + (size_t)__shfl_sync(0xffffffffu, top, j) * n1 + q0;
+        u[j][lane] = j < nb && q0 + lane < n1 ? row[lane] : 0.f;
+        u[j][lane + 32] = j < nb && q0 + lane + 32 < n1 ? row[lane + 32] : 0.f;
+    }
+    __syncthreads();
+    // the tile's own values are in flight while U12 is formed
+    float old[4][4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float *row = p.Ao + (size_t)fr[k] * n1 + q0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) old[k][i] = r0 + tr + k < n1 && q0 + tc + 16 * i < n1 ? row[tc + 16 * i] : 0.f;
+    }
+    if (tid < kUpd) {  // U12 = L11^-1 A12 (unit lower L11), a thread per column
+        float v[kLUNB];
+#pragma unroll
+        for (int j = 0; j < kLUNB; ++j) v[j] = u[j][tid];
+#pragma unroll
+        for (int j = 0; j < kLUNB; ++j)
+#pragma unroll
+            for (int i = j + 1; i < kLUNB; ++i) v[i] = fmaf(-l11[j][i], v[j], v[i]);
+#pragma unroll
+        for (int j = 0; j < kLUNB; ++j) u[j][tid] = v[j];
+    }
+    __syncthreads();
+    if (blockIdx.y == 0)
+        for (int j = warp; j < nb; j += 8) {
+            float *row = p.F + (size_t)p.orig[k0 + j] * n1;
+            for (int c = lane; c < kUpd && q0 + c < n1; c += 32) row[q0 + c] = u[j][c];
+        }
+    float acc[4][4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[k][i] = SUM ? 0.f : old[k][i];
+#pragma unroll 4
+    for (int j = 0; j < nb; ++j) {
+        const float4 l4 = *reinterpret_cast<const float4 *>(&lt[j][tr]);
+        const float l[4] = {l4.x, l4.y, l4.z, l4.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float w = u[j][tc + 16 * i];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[k][i] = fmaf(SUM ? l[k] : -l[k], w, acc[k][i]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = r0 + tr + k, c = q0 + tc + 16 * i;
+            if (r < n1 && c < n1) p.An[(size_t)r * n1 + c] = SUM ? old[k][i] - acc[k][i] : acc[k][i];
+        }
+}
+
+__global__ void lu_collect_kernel(const float *__restrict__ F, const int *__restrict__ orig, int n1,
+                                  const double *__restrict__ pre, float *__restrict__ LU) {
+    if (pre[0] != 0.0) return;
+    const int i = blockIdx.x;
+    const float *src = F + (size_t)orig[i] * n1;
+    for (int c = threadIdx.x; c < n1; c += blockDim.x) LU[(size_t)i * n1 + c] = src[c];
+}
+__global__ void iota_kernel(int *__restrict__ v, int n) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) v[t] = t;
+}
+
+// The FP32 matrix is in the first half of d.As, the second half is the other buffer.
+void lu_factor_across(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &tag, cudaStream_t stream) {
+    float *buf[2] = {reinterpret_cast<float *>(d.As), reinterpret_cast<float *>(d.As) + (size_t)n1 * n1};
+    LuStep p{};
+    p.F = ctx->buf_t<float>("s_luF" + tag, (size_t)n1 * n1);
+    p.LP = ctx->buf_t<float>("s_luLP" + tag, (size_t)n1 * 32);
+    int *idx = ctx->buf_t<int>("s_luidx" + tag, 3 * (size_t)n1);  // order, two generations; then from
+    p.from = idx + 2 * (size_t)n1;
+    p.orig = d.perm;
+    p.pre = d.pre;
+    p.n1 = n1;
+    iota_kernel<<<ceil_div(n1, 256), 256, 0, stream>>>(idx, n1);
+    RP_LAUNCH_CHECK();
+    const size_t most = sizeof(float) * 4096 * 11;  // (8 columns of 4096 rows; 16 of 2048 and 32 of 1024 take less)
+    smem_optin((const void *)lu_panel_across_kernel<2>, most);
+    smem_optin((const void *)lu_panel_across_kernel<4>, most);
+    smem_optin((const void *)lu_panel_across_kernel<8>, most);
+    int step = 0;
+    for (int k0 = 0; k0 < n1; ++step) {
+        const int m = n1 - k0, R = m <= 2 * kPanelT ? 2 : m <= 4 * kPanelT ? 4 : 8, NB = 64 / R;
+        p.Ao = buf[step & 1];
+        p.An = buf[(step + 1) & 1];
+        p.id_o = idx + (size_t)(step & 1) * n1;
+        p.id_n = idx + (size_t)((step + 1) & 1) * n1;
+        p.k0 = k0;
+        p.nb = std::min(NB, m);
+        const int nt = (int)ceil_div(ceil_div(m, R), 32) * 32;
+        const size_t smem = sizeof(float) * (size_t)m * (NB + 3);
+        if (R == 2) lu_panel_across_kernel<2><<<1, nt, smem, stream>>>(p);
+        else if (R == 4) lu_panel_across_kernel<4><<<1, nt, smem, stream>>>(p);
+        else lu_panel_across_kernel<8><<<1, nt, smem, stream>>>(p);
+        RP_LAUNCH_CHECK();
+        k0 += p.nb;
+        if (k0 < n1) {
+            const unsigned t = ceil_div(n1 - k0, kUpd);
+            if (n1 >= kLUWideMin) lu_update_across_kernel<true><<<dim3(t, t), 256, 0, stream>>>(p);
+            else lu_update_across_kernel<false><<<dim3(t, t), 256, 0, stream>>>(p);
+            RP_LAUNCH_CHECK();
+        }
+    }
+    lu_collect_kernel<<<n1, 256, 0, stream>>>(p.F, d.perm, n1, d.pre, buf[0]);
+    RP_LAUNCH_CHECK();
+}
+
 // dynamic shared memory of lu_solve_refine_kernel: the right-hand side, the correction and the row
 // order, and for the blocked factorisation 64 rows of a panel's neighbours (or its own rows,
 // 33 floats each)
@@ -1102,10 +1422,6 @@ void lu_smem_optin() { smem_optin((const void *)lu_solve_refine_kernel, solve_sm
 inline cublasStatus_t gemm_nn(cublasHandle_t h, int m, int n, int k, const float *alpha, const float *A, int lda,
                               const float *B, int ldb, const float *beta, float *C, int ldc) {
     return cublasSgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-}
-inline cublasStatus_t gemm_nn(cublasHandle_t h, int m, int n, int k, const double *alpha, const double *A, int lda,
-                              const double *B, int ldb, const double *beta, double *C, int ldc) {
-    return cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
 }
 
 // ---- FP64 wide factorisation by cuSOLVER's getrf
@@ -1317,18 +1633,28 @@ __global__ void from_f32_kernel(const float *__restrict__ y, int n, double scale
     if (mode == 0) x[t] += (double)y[t] * scale;
     else x[t] = isfinite(y[t]) ? (double)y[t] : 1e300;
 }
-// the factorisation's row interchanges applied to y in order (one CTA, in shared memory)
-__global__ void __launch_bounds__(1024) swap_rows_kernel(float *__restrict__ y, const int *__restrict__ perm, int n) {
-    extern __shared__ float ysm[];
-    for (int t = threadIdx.x; t < n; t += blockDim.x) ysm[t] = y[t];
+// y[i] = v[order[i]]: the factorisation's row order
+__global__ void gather_rows_kernel(const float *__restrict__ v, const int *__restrict__ order, int n,
+                                   float *__restrict__ y) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) y[t] = v[order[t]];
+}
+// interchanges in order (perm[k]: the row that came to k) to a row order, in place; one CTA
+__global__ void __launch_bounds__(1024) order_of_swaps_kernel(int *__restrict__ perm, int n) {
+    extern __shared__ int osm[];  // [n] interchanges, [n] order
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+        osm[t] = perm[t];
+        osm[n + t] = t;
+    }
     __syncthreads();
     if (threadIdx.x == 0)
         for (int k = 0; k < n; ++k) {
-            const int p = perm[k];
-            if (p != k) { const float v = ysm[k]; ysm[k] = ysm[p]; ysm[p] = v; }
+            const int q = osm[k], o = osm[n + k];
+            osm[n + k] = osm[n + q];
+            osm[n + q] = o;
         }
     __syncthreads();
-    for (int t = threadIdx.x; t < n; t += blockDim.x) y[t] = ysm[t];
+    for (int t = threadIdx.x; t < n; t += blockDim.x) perm[t] = osm[n + t];
 }
 // max row sum |A0| (the backward-error bound's ||A||)
 __global__ void rowabs_max_kernel(const double *__restrict__ A0, int n1, unsigned long long *__restrict__ out) {
@@ -1345,7 +1671,7 @@ bool refine_wide32(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t stream)
     const float *LU = reinterpret_cast<const float *>(d.As);
     cublasHandle_t hb = ctx->blas();
     RP_CUBLAS(cublasSetStream(hb, stream));
-    float *ys = ctx->buf_t<float>("s_r32_y", (size_t)n1);
+    float *ys = ctx->buf_t<float>("s_r32_y", (size_t)n1), *yv = ctx->buf_t<float>("s_r32_v", (size_t)n1);
     unsigned long long *bits = ctx->buf_t<unsigned long long>("s_r32_bits", 2);
     const int nb = (int)ceil_div(n1, 256);
     // pivot range and zero-pivot flag of the wide FP32 factorisation, ||A0|| (rows)
@@ -1365,8 +1691,8 @@ bool refine_wide32(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t stream)
     double an, anorm;
     std::memcpy(&an, &hbits[0], sizeof(an));
     std::memcpy(&anorm, &hbits[1], sizeof(anorm));
-    auto apply = [&]() {  // ys = (P L U)^-1 ys in FP32
-        swap_rows_kernel<<<1, 1024, sizeof(float) * (size_t)n1, stream>>>(ys, d.perm, n1);
+    auto apply = [&]() {  // ys = (P L U)^-1 yv in FP32
+        gather_rows_kernel<<<nb, 256, 0, stream>>>(yv, d.perm, n1, ys);
         RP_LAUNCH_CHECK();
         RP_CUBLAS(cublasStrsv(hb, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_T, CUBLAS_DIAG_UNIT, n1, LU, n1, ys, 1));
         RP_CUBLAS(cublasStrsv(hb, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, CUBLAS_DIAG_NON_UNIT, n1, LU, n1, ys, 1));
@@ -1392,7 +1718,7 @@ bool refine_wide32(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t stream)
             break;
         }
         ++steps;
-        to_f32_kernel<<<nb, 256, 0, stream>>>(d.r, n1, rm, ys);
+        to_f32_kernel<<<nb, 256, 0, stream>>>(d.r, n1, rm, yv);
         RP_LAUNCH_CHECK();
         apply();
         from_f32_kernel<<<nb, 256, 0, stream>>>(ys, n1, rm, 0, d.x);
@@ -1408,7 +1734,7 @@ bool refine_wide32(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t stream)
     if (!done) return false;
     // Hager's estimate of ||K^-1||_1 with the FP32 factors (lu_solve_refine_kernel's steps)
     auto solve_r = [&]() {
-        to_f32_kernel<<<nb, 256, 0, stream>>>(d.r, n1, 0.0, ys);
+        to_f32_kernel<<<nb, 256, 0, stream>>>(d.r, n1, 0.0, yv);
         RP_LAUNCH_CHECK();
         apply();
         from_f32_kernel<<<nb, 256, 0, stream>>>(ys, n1, 0.0, 1, d.r);
@@ -1466,12 +1792,16 @@ bool refine_wide32(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t stream)
 }
 
 template <typename T>
-void lu_wide_factor(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t stream) {
-    smem_optin((const void *)lu_panel_kernel<T>, kPanelSmem);
+void lu_wide_factor(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &tag, cudaStream_t stream) {
     T *L = reinterpret_cast<T *>(d.As);
     const long long nn = (long long)n1 * n1;
     lu_copy_kernel<T><<<(int)std::min<long long>(ceil_div(nn, 256), 4096), 256, 0, stream>>>(d.A0, L, nn, d.pre);
     RP_LAUNCH_CHECK();
+    if (n1 <= kLUAcrossMax) {
+        lu_factor_across(ctx, d, n1, tag, stream);
+        return;
+    }
+    smem_optin((const void *)lu_panel_kernel<T>, kPanelSmem);
     cublasHandle_t h = ctx->blas();
     RP_CUBLAS(cublasSetStream(h, stream));
     const T minus_one = T(-1), one = T(1);
@@ -1494,6 +1824,9 @@ void lu_wide_factor(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t stream
         }
         k0 = c1;
     }
+    smem_optin((const void *)order_of_swaps_kernel, 2 * sizeof(int) * kLUWideMax);
+    order_of_swaps_kernel<<<1, 1024, 2 * sizeof(int) * (size_t)n1, stream>>>(d.perm, n1);
+    RP_LAUNCH_CHECK();
 }
 
 }  // namespace
@@ -1664,6 +1997,17 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         }
         if (plans[j].disjoint) disjoint.push_back(j);
     }
+    // One system of kLUHost64Min unknowns or more is factored across the GPU (0.44 ms at 425
+    // unknowns against 0.74 in one CTA, 0.76 against 2.0 at 720), two of them one after the other
+    // from kAcrossTwo; more run side by side, each in its CTA.
+    int mid = 0, least = kLUWideMin;
+    for (int j = 0; j < nj; ++j)
+        if (descs[j].host64 && !descs[j].wide64) {
+            ++mid;
+            least = std::min(least, plans[j].n + 1);
+        }
+    if (mid == 1 || (mid == 2 && least >= kAcrossTwo))
+        for (int j = 0; j < nj; ++j) descs[j].across = descs[j].host64 && !descs[j].wide64;
     // the small tables go up from one pinned staging block per tag (asynchronous copies that
     // never wait for the stream; a later solve with another tag cannot overwrite them)
     const size_t st_bytes[7] = {sizeof(int) * n_map, sizeof(int) * n_mptr, sizeof(int) * n_midx,
@@ -1735,7 +2079,7 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
             any_wide = true;  // its flag is read after the launch, as a wide system's
         } else {
             StageTimer tt(ctx, "solve_lu_wide", stream);
-            lu_wide_factor<float>(ctx, descs[j], plans[j].n + 1, stream);
+            lu_wide_factor<float>(ctx, descs[j], plans[j].n + 1, tag, stream);
             any_wide = true;
         }
     }
@@ -1752,6 +2096,11 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
             lu_smem_optin();
             prepare_kernel<<<dim3(ceil_div(n1max, 8), nj), 256, 0, stream>>>(d_desc);
             RP_LAUNCH_CHECK();
+            for (int j = 0; j < nj; ++j)
+                if (descs[j].across) {
+                    StageTimer ta(ctx, "solve_lu_across", stream);
+                    lu_factor_across(ctx, descs[j], plans[j].n + 1, tag, stream);
+                }
             lu_solve_refine_kernel<<<nj, solve_threads(n1max), smem, stream>>>(d_desc);
             RP_LAUNCH_CHECK();
         }

@@ -48,3 +48,38 @@ def test_nan_matrix_is_reported_singular_or_nan(N, gpu_ctx):
     except _lib.RepeatError:
         return
     assert not np.isfinite(q.cpu().numpy()).all()
+
+
+@pytest.mark.parametrize("N", [767, 800, 1023, 1055, 2047, 2049, 2600, 4095, 4096])
+def test_wide_pivoted_systems(N, gpu_ctx):
+    """The factorisation across the GPU: the changes of its panel width at 1024 and 2048 rows, its last
+    size and the first beyond it.  The bound of the test above, with the 1-norm condition number."""
+    import torch
+    rng = np.random.default_rng(N)
+    A = rng.normal(size=(N, N))
+    A = 0.5 * (A + A.T)
+    A[np.arange(N), np.arange(N)] *= 0.01
+    b = rng.normal(size=N)
+    K, ref = _reference(A, b, 0.25)
+    q, _ = gpu_ctx.solve(torch.from_numpy(A).cuda(), torch.from_numpy(b).cuda(), np.full(N, 6), qtot=0.25)
+    q = q.cpu().numpy()
+    kinv = np.abs(np.linalg.inv(K)).sum(axis=0).max()
+    tol = max(1e-9, 1e-15 * np.abs(K).sum(axis=0).max() * kinv * (N + 1))
+    assert np.abs(q - ref).max() <= tol * max(1.0, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("N", [300, 800])
+def test_singular_systems_across_the_gpu(N, gpu_ctx):
+    """Two equal rows and columns: refused as singular, or solved with a residual that says so."""
+    import torch
+    from pyrepeat_gb300 import _lib
+    rng = np.random.default_rng(N)
+    A = rng.normal(size=(N, N))
+    A = A @ A.T / N
+    A[:, N // 2] = A[:, 3]
+    A[N // 2, :] = A[3, :]
+    try:
+        _, info = gpu_ctx.solve(torch.from_numpy(A).cuda(), torch.from_numpy(rng.normal(size=N)).cuda(), np.full(N, 6))
+    except _lib.RepeatError:
+        return
+    assert info["kappa"] > 1e12
