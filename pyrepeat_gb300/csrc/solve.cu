@@ -21,13 +21,17 @@
 // refinement stalls (a step that does not halve the residual, or kRefineMax steps:
 // cond(A) near 1/eps32), the system is factored again in FP64 with one step of FP64
 // refinement.  Either way the refined residual and the pivot range are reported.
-// Systems of kLUWideMin or more unknowns are factored across the whole GPU instead
-// of by their CTA (lu_wide_factor), in FP32 and, when that stalls, in FP64.
+// Systems of kLUWideMin or more unknowns, and single ones of kLUHost64Min or more, are factored and
+// refined across the whole GPU instead of by their CTA (lu_wide_factor, refine_across), in FP32
+// and, when that stalls, in FP64 (factor_refine_wide64).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
 #include <set>
+#include <utility>
+
+#include <cooperative_groups.h>
 
 #include "common.cuh"
 
@@ -88,7 +92,7 @@ __global__ void __launch_bounds__(256) prepare_kernel(const SolveDesc *__restric
     double s = 0.0;
     for (int c = lane; c < n1; c += 32) {
         const double v = row[c];
-        L[c] = (float)v;
+        if (!d.across) L[c] = (float)v;  // (factors from across the GPU stay)
         s += c < d.n ? fabs(v) : 0.0;
     }
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -712,8 +716,8 @@ constexpr int kRefineMax = 30;  // and stop early once a step no longer halves t
 // that fit shared memory at 4 columns; FP64 by cuSOLVER when the FP32 refinement does not
 // converge): n1 in [kLUWideMin, kLUWideMax]
 constexpr int kLUWideMin = 768;
-// systems of kLUHost64Min to kLUWideMin unknowns keep their FP32 factorisation in the CTA, but
-// when its refinement stalls the FP64 factors come from across the GPU (cuSOLVER getrf): an
+// systems of kLUHost64Min to kLUWideMin unknowns keep their FP32 factorisation in the CTA when a
+// launch holds several, but when its refinement stalls the FP64 factors come from across the GPU (cuSOLVER getrf): an
 // in-CTA FP64 LU of 425 unknowns takes ~13 ms on one SM's FP64 pipe
 constexpr int kLUHost64Min = 256;
 constexpr int kAcrossTwo = 512;  // least unknowns for two systems of a launch to be factored across the GPU
@@ -757,7 +761,7 @@ __device__ void residual(const SolveDesc &d, int n1) {
 
 __global__ void __launch_bounds__(kSolve) lu_solve_refine_kernel(const SolveDesc *__restrict__ descs) {
     const SolveDesc d = descs[blockIdx.x];
-    if (d.wide64 || d.host32) return;  // refined on the host path (factor_refine_wide64, refine_wide32)
+    if (d.wide64 || d.host32) return;  // factor_refine_wide64, refine_across
     const int n1 = d.n + 1;
     // [2 n1] right-hand side / correction in FP32 (or n1 doubles), [n1] row order, then the work
     // area of the blocked factorisation
@@ -1613,25 +1617,470 @@ void factor_refine_wide64(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t 
     RP_CUDA(cudaStreamSynchronize(stream));  // the pinned info words are reused by the next system
 }
 
-// ---- host-driven refinement with wide FP32 factors
+// ---- refinement across the GPU with wide FP32 factors
 // The refinement of lu_solve_refine_kernel for a system whose FP32 factors were computed across
 // the GPU (lu_wide_factor<float>): the same steps (scaled FP32 corrections, FP64 residuals, the
-// backward-error stop, the stall rule) and the same condition estimate, with cuBLAS DGEMV
-// residuals and STRSV solves across the GPU instead of one CTA's (whose FP64 residual alone takes
-// ~1 ms on one SM's FP64 pipe at 2001 unknowns).  Returns false when the refinement stalls: the
-// caller then factors the system in FP64 (factor_refine_wide64).  Waits.
+// backward-error stop) and the same condition estimate, as rounds of three
+// launches that decide on the device and return at once when there is nothing left to do:
+//   across_control_kernel   one CTA: what the last round's results mean for the refinement and
+//                           for Hager's estimate, and the next right-hand sides;
+//   across_apply_kernel     (P L U)^-1 of all of them at once, in one cluster;
+//   across_residual_kernel  x += correction and r = bs - A0 x in FP64, rows over the GPU.
+// The refinement, the estimate and its extra test vector do not depend on one another, so
+// round k carries correction k, the estimate's vector k and (round 0) the extra vector: four
+// rounds instead of eight triangular solves one after the other.
+// Measured, refinement and estimate: 2.46 -> 0.95 ms at 2001 unknowns and 1.3 -> 0.45 at 768 (against
+// cuBLAS solves and residuals with a look by the host after each), 1.56 -> 0.41 at 767 and 0.70 ->
+// 0.31 at 425 (against one CTA, whose FP64 residual alone takes 154 us per step at 767).
+constexpr int kAcB = 128;     // unknowns of a block, whose diagonal blocks of L and U are inverted once
+constexpr int kAcCTAs = 8;    // CTAs of the cluster, 16 rows of each block each
+constexpr int kAcT = 512;     // their threads
+constexpr int kAcRounds = 6;  // rounds launched ahead of a look at the outcome
+// A step that leaves more than this share of the residual: the solution that three such steps
+// give then depends at the tenth digit on how the triangular solves round, and the system goes
+// to substitution.  (Shares of 1e-6 to 3.6e-4 at fits and QEq systems of 260 to 2001 unknowns of
+// ordinary cells, whose charges agree with substitution's to 3e-10; 6.8e-4 to 2.5e-3 at dense cells
+// of 830 to 920, where they differ by 1e-9 to 1e-7.)
+constexpr double kInvRate = 4e-4;
 
-// y (FP32) = v / scale, or v with non-finite values as they are (scale 0: plain conversion)
+struct AcrossState {
+    unsigned long long an_bits, anorm_bits;  // max row sums of |K| and of |A|
+    unsigned long long rn_bits, xn_bits;     // max |r|, max |x| of the round's residual
+    double rm, rprev, res, est, alt;
+    int steps, phase;       // phase 0: refining, 1: converged, 2: left to substitution, 3: zero pivot
+    int hstate, hit, jprev, jcur;  // 0: uniform vector under way, 1: signs, 2: a unit vector, 3: estimate done
+    int xsel, finished;     // which x holds the solution; nothing left to do
+};
+struct AcrossRun {
+    const float *LU;        // factors
+    float *inv;             // inverses of their diagonal blocks, L's then U's, and behind them the blocks
+    float *V, *Y;           // [3][n1] right-hand sides and solutions
+    double *x[2];           // solution before and after a round
+    AcrossState *st;
+    SolveDesc d;
+    int n1, nblk;
+    double path;            // info's factorisation path
+};
+
+// max row sums of |K| and |A| (K symmetric), a warp per row; st cleared before
+__global__ void __launch_bounds__(256) across_norms_kernel(AcrossRun p) {
+    const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, n1 = p.n1;
+    if (r >= n1) return;
+    const double *row = p.d.A0 + (size_t)r * n1;
+    double s = 0.0;
+    for (int c = lane; c < n1 - 1; c += 32) s += fabs(row[c]);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) {  // (non-negative: the bits order like the values)
+        atomicMax(&p.st->an_bits, (unsigned long long)__double_as_longlong(s + fabs(row[n1 - 1])));
+        if (r < n1 - 1) atomicMax(&p.st->anorm_bits, (unsigned long long)__double_as_longlong(s));
+    }
+}
+
+// Inverses of the diagonal blocks: blockIdx.x the block, blockIdx.y 0 for L (unit), 1 for U, taken
+// with rows and columns reversed, as a lower triangle too.  Four threads per column of the inverse
+// hold 32 of its rows each in registers (rows 16 g + 4 q + 0..3), column by column of the triangle: 16
+// steps in line, then the registers move up by 16 rows, so the code stays small.  (Dot products
+// from shared memory, row by row, took 100 us at any size.)  Rows past the end: identity.
+constexpr int kInvLD = kAcB + 4, kInvCols = 64, kInvT = 4 * kInvCols;  // blockIdx.z: which 64 columns
+__global__ void __launch_bounds__(kInvT) across_invert_kernel(AcrossRun p) {
+    extern __shared__ __align__(16) float ash[];
+    float *B = ash, *dinv = ash + kAcB * kInvLD;  // B[k][i]: column k below the diagonal
+    if (p.d.pre[0] != 0.0) return;
+    const int n1 = p.n1, b0 = blockIdx.x * kAcB, tid = threadIdx.x, lane = tid & 31, c = blockIdx.z * kInvCols + (tid >> 2), q = tid & 3;
+    const bool rev = blockIdx.y == 1;
+#pragma unroll 16
+    for (int t = tid; t < kAcB * kAcB; t += kInvT) {
+        const int i = t / kAcB, j = t % kAcB;
+        const float v = b0 + i < n1 && b0 + j < n1 ? p.LU[(size_t)(b0 + i) * n1 + b0 + j] : (i == j ? 1.f : 0.f);
+        const int r = rev ? kAcB - 1 - i : i, k = rev ? kAcB - 1 - j : j;
+        B[k * kInvLD + r] = r > k ? v : 0.f;
+        if (r == k) dinv[k] = rev ? 1.f / v : 1.f;
+    }
+    __syncthreads();
+    float x[32];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) x[j] = 16 * (j >> 2) + 4 * q + (j & 3) == c ? 1.f : 0.f;
+    float *out = p.inv + ((size_t)blockIdx.y * p.nblk + blockIdx.x) * kAcB * kAcB;
+    float *tri = out + 2 * (size_t)p.nblk * kAcB * kAcB;  // the block's own triangle, zeros elsewhere
+    for (int t = tid; t < kAcB * kInvCols; t += kInvT) {
+        const int i = t / kInvCols, j = blockIdx.z * kInvCols + t % kInvCols;
+        float v = i == j ? 1.f : 0.f;
+        if ((rev ? j >= i : j < i) && b0 + i < n1 && b0 + j < n1) v = p.LU[(size_t)(b0 + i) * n1 + b0 + j];
+        tri[i * kAcB + j] = v;
+    }
+#pragma unroll 1
+    for (int t = 0; t < 8; ++t) {
+#pragma unroll
+        for (int kk = 0; kk < 16; ++kk) {
+            const int k = 16 * t + kk;
+            const float xk = __shfl_sync(0xffffffffu, x[kk & 3], (lane & ~3) | (kk >> 2)) * dinv[k];
+            if (q == kk >> 2) out[(rev ? kAcB - 1 - k : k) * kAcB + (rev ? kAcB - 1 - c : c)] = xk;
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+                if (t + g < 8) {
+                    const float4 b = *reinterpret_cast<const float4 *>(B + k * kInvLD + 16 * (t + g) + 4 * q);
+                    x[4 * g + 0] = fmaf(-b.x, xk, x[4 * g + 0]);
+                    x[4 * g + 1] = fmaf(-b.y, xk, x[4 * g + 1]);
+                    x[4 * g + 2] = fmaf(-b.z, xk, x[4 * g + 2]);
+                    x[4 * g + 3] = fmaf(-b.w, xk, x[4 * g + 3]);
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < 28; ++j) x[j] = x[j + 4];
+    }
+}
+
+// pre[0] at the end (last): 0 solved, 2 zero pivot, 3 not finished, 4 substitution (with the estimate
+// in info); 3 is taken back by the rounds that follow
+__global__ void __launch_bounds__(1024) across_control_kernel(AcrossRun p, int round, int last) {
+    __shared__ double sv[33], piv_v;
+    __shared__ int si[32], piv_i;
+    __shared__ AcrossState st;
+    const int tid = threadIdx.x, n1 = p.n1, nt = blockDim.x;
+    if (tid == 0) st = *p.st;
+    __syncthreads();
+    if (st.finished) return;
+    if (round == 0) {
+        double m = 0.0;
+        for (int t = tid; t < n1; t += nt) {
+            const double b = p.d.bs[t];
+            p.d.r[t] = b;
+            p.x[0][t] = 0.0;
+            m = fmax(m, fabs(b));
+        }
+        m = block_max(m, n1, sv);
+        if (tid == 0) {
+            st.rm = m;
+            st.rprev = 1e308;
+            st.res = 0.0;
+            st.steps = st.hit = st.hstate = st.xsel = 0;
+            st.jprev = -1;
+            st.est = st.alt = 0.0;
+            st.phase = p.d.pre[0] != 0.0 ? 3 : m == 0.0 ? 1 : 0;
+        }
+        for (int t = tid; t < n1; t += nt) {
+            p.V[n1 + t] = (float)(1.0 / (double)n1);
+            p.V[2 * (size_t)n1 + t] = (float)(((t & 1) ? -1.0 : 1.0) * (1.0 + (double)t / (double)max(n1 - 1, 1)));
+        }
+    } else {
+        if (tid == 0 && st.phase == 0) {
+            const double rn = __longlong_as_double((long long)st.rn_bits), xn = __longlong_as_double((long long)st.xn_bits),
+                         an = __longlong_as_double((long long)st.an_bits);
+            st.res = rn;
+            ++st.steps;
+            st.xsel = round & 1;
+            if (rn <= (double)n1 * 1.1102230246251565e-16 * an * xn) st.phase = 1;
+            else if (!(rn < 1e300) || (st.steps >= 2 && rn > kInvRate * st.rprev)) st.phase = 2;  // substitution takes over
+            st.rprev = st.rm = rn;
+        }
+        if (st.hstate != 3) {
+            const float *y = p.Y + n1;
+            auto val = [&](float v) { return isfinite(v) ? (double)v : 1e300; };
+            if (st.hstate == 1) {
+                double best = -1.0, sum = 0.0;
+                int bi = 0x7fffffff;
+                for (int t = tid; t < n1; t += nt) {
+                    const double z = val(y[t]), v = fabs(z);
+                    sum += z;
+                    if (v > best || (v == best && t < bi)) {
+                        best = v;
+                        bi = t;
+                    }
+                }
+                sum = block_sum(sum, n1, sv);
+                block_argmax(best, bi, sv, si, &piv_v, &piv_i);
+                if (tid == 0) {
+                    const double ztx = st.jprev < 0 ? sum / (double)n1 : val(y[st.jprev]);
+                    st.jcur = piv_i;
+                    st.hstate = piv_v > ztx ? 2 : 3;
+                }
+            } else {
+                double a = 0.0;
+                for (int t = tid; t < n1; t += nt) a += fabs(val(y[t]));
+                a = block_sum(a, n1, sv);
+                if (tid == 0) {
+                    if (st.hstate == 0) {
+                        st.est = a;
+                        st.hstate = 1;
+                    } else if (a > st.est) {
+                        st.est = a;
+                        st.jprev = st.jcur;
+                        st.hstate = ++st.hit < 4 ? 1 : 3;
+                    } else {
+                        st.hstate = 3;
+                    }
+                }
+            }
+            __syncthreads();
+            for (int t = tid; t < n1; t += nt)
+                p.V[n1 + t] = st.hstate == 2 ? (t == st.jcur ? 1.f : 0.f) : (y[t] >= 0.f || !isfinite(y[t])) ? 1.f : -1.f;
+        }
+        if (round == 1) {
+            double a = 0.0;
+            for (int t = tid; t < n1; t += nt) {
+                const float v = p.Y[2 * (size_t)n1 + t];
+                a += isfinite(v) ? fabs((double)v) : 1e300;
+            }
+            a = block_sum(a, n1, sv);
+            if (tid == 0) st.alt = 2.0 * a / (3.0 * (double)n1);
+        }
+    }
+    __syncthreads();
+    if (st.phase == 0) {
+        const double rm = st.rm;
+        for (int t = tid; t < n1; t += nt) p.V[t] = (float)(p.d.r[t] / rm);
+    }
+    const bool solved = st.hstate == 3 && (st.phase == 1 || st.phase == 2);
+    if (solved && st.phase == 1) {  // the solution, expanded to all atoms
+        const double *x = p.x[st.xsel];
+        for (int i = tid; i < p.d.N; i += nt) p.d.q[i] = x[p.d.map[i]];
+    }
+    if (tid == 0) {
+        if (solved) {
+            const double est = fmax(st.est, st.alt), kinv = est < 1e300 ? est : 1e300;
+            p.d.info[0] = st.res;
+            p.d.info[1] = p.d.pre[1];
+            p.d.info[2] = p.d.pre[2];
+            p.d.info[3] = 0.0;
+            p.d.info[4] = fmin(__longlong_as_double((long long)st.anorm_bits) * kinv, 1e300);
+            p.d.info[5] = n1;
+            p.d.info[6] = st.steps;
+            p.d.info[7] = p.path;
+        }
+        st.finished = solved || st.phase == 3;
+        if (st.phase == 3) p.d.pre[0] = 2.0;
+        else if (solved) p.d.pre[0] = st.phase == 2 ? 4.0 : 0.0;
+        else if (last) p.d.pre[0] = 3.0;
+        st.rn_bits = st.xn_bits = 0;
+        *p.st = st;
+    }
+}
+
+// Y = U^-1 L^-1 P V for NR right-hand sides, in one cluster: a block of 128 unknowns at a time.  Each CTA
+// keeps the whole solution; its 16 warps hold a row of the block each (of 128 rows, 16 per CTA),
+// whose product with the unknowns known so far they form while the cluster waits for the
+// previous block.  The rows' values go to every CTA's shared memory, and every CTA multiplies
+// them by the inverted diagonal block: one cluster barrier per block.
+// Bounded by those steps' latency (16 + 16 of them at 2001 unknowns) and by the factors' way from
+// L2 to eight SMs (2 MB each there).
+template <int NR>
+__global__ void __cluster_dims__(kAcCTAs, 1, 1) __launch_bounds__(kAcT) across_apply_kernel(AcrossRun p) {
+    namespace cg = cooperative_groups;
+    constexpr int NS = NR == 3 ? 4 : NR;  // floats per unknown in shared memory
+    extern __shared__ __align__(16) float ash[];
+    float *xs = ash;                                    // [nblk * 128][NS]
+    float *wb = ash + (size_t)p.nblk * kAcB * NS;       // [2][128][NS] the block's rows
+    float *rb = wb + 2 * kAcB * NS;                     // [128][NS] what they leave
+    cg::cluster_group cl = cg::this_cluster();
+    if (p.st->finished) return;  // (the same for the whole cluster)
+    const int rank = (int)cl.block_rank(), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int n1 = p.n1, nblk = p.nblk, rl = rank * (kAcB / kAcCTAs) + warp;  // the warp's row of each block
+    for (int t = tid; t < nblk * kAcB; t += kAcT) {
+        const int o = t < n1 ? p.d.perm[t] : 0;
+#pragma unroll
+        for (int q = 0; q < NR; ++q) xs[t * NS + q] = t < n1 ? p.V[(size_t)q * n1 + o] : 0.f;
+    }
+    cl.sync();  // every CTA runs and holds its right-hand sides
+    const int mr = tid >> 2, mp = tid & 3;  // a diagonal block: a row's quarter of the columns
+    auto times = [&](const float4 (&m)[8], const float *w, float (&v)[NR]) {  // its row times w, in all four threads
+#pragma unroll
+        for (int q = 0; q < NR; ++q) v[q] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float e[4] = {m[j].x, m[j].y, m[j].z, m[j].w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int q = 0; q < NR; ++q) v[q] = fmaf(e[i], w[(16 * j + 4 * mp + i) * NS + q], v[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < NR; ++q) {
+            v[q] += __shfl_xor_sync(0xffffffffu, v[q], 1);
+            v[q] += __shfl_xor_sync(0xffffffffu, v[q], 2);
+        }
+    };
+#pragma unroll 1
+    for (int dir = 0; dir < 2; ++dir) {
+        const float *inv = p.inv + (size_t)dir * nblk * kAcB * kAcB + (size_t)mr * kAcB + 4 * mp;
+        float acc[NR];
+#pragma unroll
+        for (int q = 0; q < NR; ++q) acc[q] = 0.f;
+#pragma unroll 1
+        for (int s = 0; s < nblk; ++s) {
+            const int b = dir ? nblk - 1 - s : s, nb_ = dir ? b - 1 : b + 1, buf = s & 1;
+            // this block's rows, to every CTA
+#pragma unroll
+            for (int q = 0; q < NR; ++q) {
+                float v = acc[q];
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                v = xs[(b * kAcB + rl) * NS + q] - v;
+                if (lane < kAcCTAs) *cl.map_shared_rank(wb + (buf * kAcB + rl) * NS + q, lane) = v;
+                acc[q] = 0.f;
+            }
+            __syncwarp();
+            cg::cluster_group::arrival_token tok = cl.barrier_arrive();
+            // while they travel: the inverted block, and the next block's rows times what is known
+            float4 iv[8];
+            {
+                const float *src = inv + (size_t)b * kAcB * kAcB;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) iv[j] = *reinterpret_cast<const float4 *>(src + 16 * j);
+            }
+            float near_[4] = {0.f, 0.f, 0.f, 0.f};  // the next rows' part of this block's columns
+            const int nrow = nb_ * kAcB + rl;
+            if (s + 1 < nblk && nrow < n1) {
+                const float *row = p.LU + (size_t)nrow * n1;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int c = b * kAcB + lane + 32 * i;
+                    near_[i] = c < n1 ? row[c] : 0.f;
+                }
+                const int c0 = dir ? (b + 1) * kAcB : 0, c1 = dir ? n1 : b * kAcB;
+                for (int cc = c0 + lane; cc - lane < c1; cc += 512) {  // 16 loads in flight, none left over
+                    float l[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) l[i] = cc + 32 * i < c1 ? row[cc + 32 * i] : 0.f;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const float *x = xs + (cc + 32 * i < c1 ? cc + 32 * i : cc) * NS;
+#pragma unroll
+                        for (int q = 0; q < NR; ++q) acc[q] = fmaf(l[i], x[q], acc[q]);
+                    }
+                }
+            }
+            cl.barrier_wait(std::move(tok));
+            // x = inv w, then once more on what w - B x leaves: as exact as substitution
+            float v[NR], u[NR];
+            times(iv, wb + buf * kAcB * NS, v);
+            float4 bv[8];
+            {
+                const float *src = inv + (2 * (size_t)nblk + b) * kAcB * kAcB;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) bv[j] = *reinterpret_cast<const float4 *>(src + 16 * j);
+            }
+#pragma unroll
+            for (int q = 0; q < NR; ++q)
+                if (mp == 0) xs[(b * kAcB + mr) * NS + q] = v[q];
+            __syncthreads();
+            times(bv, xs + b * kAcB * NS, u);
+#pragma unroll
+            for (int q = 0; q < NR; ++q)
+                if (mp == 0) rb[mr * NS + q] = wb[(buf * kAcB + mr) * NS + q] - u[q];
+            __syncthreads();
+            times(iv, rb, u);
+#pragma unroll
+            for (int q = 0; q < NR; ++q)
+                if (mp == 0) xs[(b * kAcB + mr) * NS + q] = v[q] + u[q];
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int q = 0; q < NR; ++q) acc[q] = fmaf(near_[i], xs[(b * kAcB + lane + 32 * i) * NS + q], acc[q]);
+        }
+    }
+    for (int t = rank * kAcT + tid; t < n1; t += kAcCTAs * kAcT)
+#pragma unroll
+        for (int q = 0; q < NR; ++q) p.Y[(size_t)q * n1 + t] = xs[t * NS + q];
+    cl.sync();  // no CTA leaves while another may still write to it
+}
+
+// x' = x + rm y (kept by the first CTA) and r = bs - A0 x' with its largest element, a warp per row
+__global__ void __launch_bounds__(256) across_residual_kernel(AcrossRun p, int round) {
+    extern __shared__ double xd[];
+    __shared__ unsigned long long top[2];
+    if (p.st->finished || p.st->phase != 0) return;
+    const int n1 = p.n1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double rm = p.st->rm, *xo = p.x[round & 1];
+    double *xn = p.x[(round + 1) & 1];
+    if (threadIdx.x < 2) top[threadIdx.x] = 0;
+    __syncthreads();
+    double m = 0.0;
+    for (int t = threadIdx.x; t < n1; t += 256) {
+        const double v = xo[t] + (double)p.Y[t] * rm;
+        xd[t] = v;
+        if (blockIdx.x == 0) {
+            xn[t] = v;
+            m = fmax(m, fabs(v));
+        }
+    }
+    if (blockIdx.x == 0) atomicMax(&top[1], (unsigned long long)__double_as_longlong(m));
+    __syncthreads();
+    for (int r = blockIdx.x * 8 + warp; r < n1; r += gridDim.x * 8) {
+        const double *row = p.d.A0 + (size_t)r * n1;
+        double s = 0.0;
+#pragma unroll 8
+        for (int c = lane; c < n1; c += 32) s = fma(row[c], xd[c], s);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) {
+            const double v = p.d.bs[r] - s;
+            p.d.r[r] = v;
+            atomicMax(&top[0], (unsigned long long)__double_as_longlong(fabs(v)));
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicMax(&p.st->rn_bits, top[0]);
+        if (blockIdx.x == 0) p.st->xn_bits = top[1];
+    }
+}
+
+// Launches rounds first .. first + rounds - 1 of system j of its launch (whose state is kept for the
+// rounds that may follow), then looks at the outcome: pre[0] = 0 (solved: q and info written), 2
+// (zero pivot: FP64 factors), 3 (not finished) or 4 (substitution).
+void refine_across(rp_ctx *ctx, const SolveDesc &d, int n1, int first, int rounds, const std::string &key, cudaStream_t stream) {
+    StageTimer tt(ctx, "solve_refine32", stream);
+    AcrossRun p{};
+    p.n1 = n1;
+    p.nblk = (int)ceil_div(n1, kAcB);
+    p.LU = reinterpret_cast<const float *>(d.As);
+    p.d = d;
+    p.inv = ctx->buf_t<float>("s_ac_inv" + key, 4 * (size_t)p.nblk * kAcB * kAcB);
+    p.V = ctx->buf_t<float>("s_ac_V" + key, 6 * (size_t)n1);
+    p.Y = p.V + 3 * (size_t)n1;
+    p.x[0] = d.x;
+    p.x[1] = ctx->buf_t<double>("s_ac_x" + key, (size_t)n1);
+    p.st = ctx->buf_t<AcrossState>("s_ac_st" + key, 1);
+    p.path = n1 < kLUWideMin ? 0.0 : 1.0;
+    if (first == 0) {
+        RP_CUDA(cudaMemsetAsync(p.st, 0, sizeof(AcrossState), stream));
+        across_norms_kernel<<<(int)ceil_div(n1, 8), 256, 0, stream>>>(p);
+        RP_LAUNCH_CHECK();
+        const size_t inv_smem = sizeof(float) * (kAcB * kInvLD + kAcB);
+        smem_optin((const void *)across_invert_kernel, inv_smem);
+        across_invert_kernel<<<dim3(p.nblk, 2, kAcB / kInvCols), kInvT, inv_smem, stream>>>(p);
+        RP_LAUNCH_CHECK();
+        across_control_kernel<<<1, 1024, 0, stream>>>(p, 0, 0);
+        RP_LAUNCH_CHECK();
+    }
+    const size_t np = (size_t)p.nblk * kAcB, res_smem = sizeof(double) * n1;
+    const size_t most = sizeof(float) * 4 * (((size_t)kLUWideMax + kAcB - 1) / kAcB * kAcB + 3 * kAcB);
+    smem_optin((const void *)across_apply_kernel<3>, most);
+    smem_optin((const void *)across_apply_kernel<2>, most / 2);
+    smem_optin((const void *)across_residual_kernel, sizeof(double) * kLUWideMax);
+    for (int k = first; k < first + rounds; ++k) {
+        if (k == 0) across_apply_kernel<3><<<kAcCTAs, kAcT, sizeof(float) * 4 * (np + 3 * kAcB), stream>>>(p);
+        else across_apply_kernel<2><<<kAcCTAs, kAcT, sizeof(float) * 2 * (np + 3 * kAcB), stream>>>(p);
+        RP_LAUNCH_CHECK();
+        across_residual_kernel<<<(int)std::min<long long>(ceil_div(n1, 8), 304), 256, res_smem, stream>>>(p, k);
+        RP_LAUNCH_CHECK();
+        across_control_kernel<<<1, 1024, 0, stream>>>(p, k + 1, k + 1 == first + rounds);
+        RP_LAUNCH_CHECK();
+    }
+}
+
+// ---- the same by substitution, driven by the host
+// For a wide system that converges too slowly for the inverted blocks (kInvRate): cuBLAS STRSV
+// solves and DGEMV residuals across the GPU, a look at the outcome after each step.  Returns
+// false when the refinement stalls: the caller then factors the system in FP64
+// (factor_refine_wide64).  Waits.
+
 __global__ void to_f32_kernel(const double *__restrict__ v, int n, double scale, float *__restrict__ y) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) y[t] = (float)(scale != 0.0 ? v[t] / scale : v[t]);
+    if (t < n) y[t] = (float)(v[t] / scale);
 }
-// mode 0: x += y * scale;  mode 1: x = finite(y) ? y : 1e300 (the estimate's solves)
-__global__ void from_f32_kernel(const float *__restrict__ y, int n, double scale, int mode, double *__restrict__ x) {
+__global__ void add_f32_kernel(const float *__restrict__ y, int n, double scale, double *__restrict__ x) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    if (mode == 0) x[t] += (double)y[t] * scale;
-    else x[t] = isfinite(y[t]) ? (double)y[t] : 1e300;
+    if (t < n) x[t] += (double)y[t] * scale;
 }
 // y[i] = v[order[i]]: the factorisation's row order
 __global__ void gather_rows_kernel(const float *__restrict__ v, const int *__restrict__ order, int n,
@@ -1639,58 +2088,22 @@ __global__ void gather_rows_kernel(const float *__restrict__ v, const int *__res
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) y[t] = v[order[t]];
 }
-// interchanges in order (perm[k]: the row that came to k) to a row order, in place; one CTA
-__global__ void __launch_bounds__(1024) order_of_swaps_kernel(int *__restrict__ perm, int n) {
-    extern __shared__ int osm[];  // [n] interchanges, [n] order
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        osm[t] = perm[t];
-        osm[n + t] = t;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-        for (int k = 0; k < n; ++k) {
-            const int q = osm[k], o = osm[n + k];
-            osm[n + k] = osm[n + q];
-            osm[n + q] = o;
-        }
-    __syncthreads();
-    for (int t = threadIdx.x; t < n; t += blockDim.x) perm[t] = osm[n + t];
-}
-// max row sum |A0| (the backward-error bound's ||A||)
-__global__ void rowabs_max_kernel(const double *__restrict__ A0, int n1, unsigned long long *__restrict__ out) {
-    const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (r >= n1) return;
-    double s = 0.0;
-    for (int c = lane; c < n1; c += 32) s += fabs(A0[(size_t)r * n1 + c]);
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) atomicMax(out, (unsigned long long)__double_as_longlong(s));
-}
-
-bool refine_wide32(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t stream) {
+bool refine_wide32(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &key, cudaStream_t stream) {
     StageTimer tt(ctx, "solve_refine32", stream);
     const float *LU = reinterpret_cast<const float *>(d.As);
     cublasHandle_t hb = ctx->blas();
     RP_CUBLAS(cublasSetStream(hb, stream));
     float *ys = ctx->buf_t<float>("s_r32_y", (size_t)n1), *yv = ctx->buf_t<float>("s_r32_v", (size_t)n1);
-    unsigned long long *bits = ctx->buf_t<unsigned long long>("s_r32_bits", 2);
     const int nb = (int)ceil_div(n1, 256);
-    // pivot range and zero-pivot flag of the wide FP32 factorisation, ||A0|| (rows)
-    double pre[3];
+    // pivot range of the factorisation, norms of the matrix and the estimate of refine_across
+    double pre[3], kappa;
+    AcrossState st{};
     RP_CUDA(cudaMemcpyAsync(pre, d.pre, sizeof(pre), cudaMemcpyDeviceToHost, stream));
-    RP_CUDA(cudaMemsetAsync(bits, 0, 2 * sizeof(unsigned long long), stream));
-    rowabs_max_kernel<<<(int)ceil_div(n1, 8), 256, 0, stream>>>(d.A0, n1, bits);
-    RP_LAUNCH_CHECK();
-    if (d.n > 0) {
-        anorm1_kernel<<<(int)ceil_div(d.n, 256), 256, 0, stream>>>(d.A0, d.n, n1, bits + 1);
-        RP_LAUNCH_CHECK();
-    }
-    unsigned long long hbits[2] = {0, 0};
-    RP_CUDA(cudaMemcpyAsync(hbits, bits, sizeof(hbits), cudaMemcpyDeviceToHost, stream));
+    RP_CUDA(cudaMemcpyAsync(&kappa, d.info + 4, sizeof(kappa), cudaMemcpyDeviceToHost, stream));
+    RP_CUDA(cudaMemcpyAsync(&st, ctx->buf_t<AcrossState>("s_ac_st" + key, 1), sizeof(st), cudaMemcpyDeviceToHost, stream));
     RP_CUDA(cudaStreamSynchronize(stream));
-    if (pre[0] != 0.0) return false;  // a zero FP32 pivot: FP64 takes over
-    double an, anorm;
-    std::memcpy(&an, &hbits[0], sizeof(an));
-    std::memcpy(&anorm, &hbits[1], sizeof(anorm));
+    double an;
+    std::memcpy(&an, &st.an_bits, sizeof(an));
     auto apply = [&]() {  // ys = (P L U)^-1 yv in FP32
         gather_rows_kernel<<<nb, 256, 0, stream>>>(yv, d.perm, n1, ys);
         RP_LAUNCH_CHECK();
@@ -1721,7 +2134,7 @@ bool refine_wide32(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t stream)
         to_f32_kernel<<<nb, 256, 0, stream>>>(d.r, n1, rm, yv);
         RP_LAUNCH_CHECK();
         apply();
-        from_f32_kernel<<<nb, 256, 0, stream>>>(ys, n1, rm, 0, d.x);
+        add_f32_kernel<<<nb, 256, 0, stream>>>(ys, n1, rm, d.x);
         RP_LAUNCH_CHECK();
         RP_CUDA(cudaMemcpyAsync(d.r, d.bs, sizeof(double) * n1, cudaMemcpyDeviceToDevice, stream));
         RP_CUBLAS(cublasDgemv(hb, CUBLAS_OP_T, n1, n1, &minus_one, d.A0, n1, d.x, 1, &one, d.r, 1));
@@ -1732,55 +2145,12 @@ bool refine_wide32(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t stream)
         rprev = rn;
     }
     if (!done) return false;
-    // Hager's estimate of ||K^-1||_1 with the FP32 factors (lu_solve_refine_kernel's steps)
-    auto solve_r = [&]() {
-        to_f32_kernel<<<nb, 256, 0, stream>>>(d.r, n1, 0.0, yv);
-        RP_LAUNCH_CHECK();
-        apply();
-        from_f32_kernel<<<nb, 256, 0, stream>>>(ys, n1, 0.0, 1, d.r);
-        RP_LAUNCH_CHECK();
-    };
-    auto asum = [&]() {
-        double v = 0.0;
-        RP_CUBLAS(cublasDasum(hb, n1, d.r, 1, &v));
-        return v;
-    };
-    double *ones = ctx->buf_t<double>("s_ones", (size_t)n1);
-    vec_fill_kernel<<<nb, 256, 0, stream>>>(ones, n1, 4, 0);
-    vec_fill_kernel<<<nb, 256, 0, stream>>>(d.r, n1, 0, 0);
-    solve_r();
-    double est = asum();
-    int jprev = -1;
-    for (int it = 0; it < 4; ++it) {
-        vec_fill_kernel<<<nb, 256, 0, stream>>>(d.r, n1, 1, 0);
-        solve_r();
-        int jm = 0;
-        RP_CUBLAS(cublasIdamax(hb, n1, d.r, 1, &jm));
-        const int j = jm - 1;
-        double zj = 0.0, ztx = 0.0, zsum = 0.0;
-        RP_CUDA(cudaMemcpyAsync(&zj, d.r + j, sizeof(double), cudaMemcpyDeviceToHost, stream));
-        if (jprev >= 0) RP_CUDA(cudaMemcpyAsync(&ztx, d.r + jprev, sizeof(double), cudaMemcpyDeviceToHost, stream));
-        RP_CUBLAS(cublasDdot(hb, n1, d.r, 1, ones, 1, &zsum));
-        RP_CUDA(cudaStreamSynchronize(stream));
-        if (jprev < 0) ztx = zsum / (double)n1;
-        if (!(std::fabs(zj) > ztx)) break;
-        vec_fill_kernel<<<nb, 256, 0, stream>>>(d.r, n1, 2, j);
-        solve_r();
-        const double bval = asum();
-        if (!(bval > est)) break;
-        est = bval;
-        jprev = j;
-    }
-    vec_fill_kernel<<<nb, 256, 0, stream>>>(d.r, n1, 3, 0);
-    solve_r();
-    est = std::max(est, 2.0 * asum() / (3.0 * (double)n1));
-    const double kinv = est < 1e300 ? est : 1e300;
     double *hinfo = static_cast<double *>(ctx->host_buf("s_info32", sizeof(double) * kSolveInfo));
     hinfo[0] = res;
     hinfo[1] = pre[1];
     hinfo[2] = pre[2];
     hinfo[3] = 0.0;
-    hinfo[4] = std::fmin(anorm * kinv, 1e300);
+    hinfo[4] = kappa;
     hinfo[5] = n1;
     hinfo[6] = steps;
     hinfo[7] = 1.0;  // FP32 factors from across the GPU
@@ -1791,6 +2161,23 @@ bool refine_wide32(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t stream)
     return true;
 }
 
+// interchanges in order (perm[k]: the row that came to k) to a row order, in place; one CTA
+__global__ void __launch_bounds__(1024) order_of_swaps_kernel(int *__restrict__ perm, int n) {
+    extern __shared__ int osm[];  // [n] interchanges, [n] order
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+        osm[t] = perm[t];
+        osm[n + t] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int k = 0; k < n; ++k) {
+            const int q = osm[k], o = osm[n + k];
+            osm[n + k] = osm[n + q];
+            osm[n + q] = o;
+        }
+    __syncthreads();
+    for (int t = threadIdx.x; t < n; t += blockDim.x) perm[t] = osm[n + t];
+}
 template <typename T>
 void lu_wide_factor(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &tag, cudaStream_t stream) {
     T *L = reinterpret_cast<T *>(d.As);
@@ -1826,6 +2213,22 @@ void lu_wide_factor(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &
     }
     smem_optin((const void *)order_of_swaps_kernel, 2 * sizeof(int) * kLUWideMax);
     order_of_swaps_kernel<<<1, 1024, 2 * sizeof(int) * (size_t)n1, stream>>>(d.perm, n1);
+    RP_LAUNCH_CHECK();
+}
+
+// the refinement of lu_solve_refine_kernel alone, on FP32 factors from across the GPU; pre[0] = 2 when
+// it stalls
+void refine_in_cta(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t stream) {
+    StageTimer tt(ctx, "solve_refine32", stream);
+    SolveDesc *one = ctx->buf_t<SolveDesc>("s_desc1", 1), h = d;
+    h.host32 = 0;
+    h.across = 1;
+    RP_CUDA(cudaMemsetAsync(d.pre, 0, sizeof(double), stream));
+    RP_CUDA(cudaMemcpyAsync(one, &h, sizeof(h), cudaMemcpyHostToDevice, stream));
+    lu_smem_optin();
+    prepare_kernel<<<(int)ceil_div(n1, 8), 256, 0, stream>>>(one);
+    RP_LAUNCH_CHECK();
+    lu_solve_refine_kernel<<<1, solve_threads(n1), solve_smem_bytes(n1), stream>>>(one);
     RP_LAUNCH_CHECK();
 }
 
@@ -1997,9 +2400,9 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         }
         if (plans[j].disjoint) disjoint.push_back(j);
     }
-    // One system of kLUHost64Min unknowns or more is factored across the GPU (0.44 ms at 425
-    // unknowns against 0.74 in one CTA, 0.76 against 2.0 at 720), two of them one after the other
-    // from kAcrossTwo; more run side by side, each in its CTA.
+    // One system of kLUHost64Min unknowns or more is solved across the GPU (0.44 + 0.31 ms at 425
+    // unknowns, factors and refinement, against 0.74 + 0.70 in one CTA; 0.76 + 0.4 against 2.0 + 1.4
+    // at 720), two of them one after the other from kAcrossTwo; more run side by side, each in its CTA.
     int mid = 0, least = kLUWideMin;
     for (int j = 0; j < nj; ++j)
         if (descs[j].host64 && !descs[j].wide64) {
@@ -2007,7 +2410,11 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
             least = std::min(least, plans[j].n + 1);
         }
     if (mid == 1 || (mid == 2 && least >= kAcrossTwo))
-        for (int j = 0; j < nj; ++j) descs[j].across = descs[j].host64 && !descs[j].wide64;
+        for (int j = 0; j < nj; ++j)
+            if (descs[j].host64 && !descs[j].wide64) {
+                descs[j].host64 = 0;
+                descs[j].host32 = 1;
+            }
     // the small tables go up from one pinned staging block per tag (asynchronous copies that
     // never wait for the stream; a later solve with another tag cannot overwrite them)
     const size_t st_bytes[7] = {sizeof(int) * n_map, sizeof(int) * n_mptr, sizeof(int) * n_midx,
@@ -2078,8 +2485,11 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         if (descs[j].host64) {
             any_wide = true;  // its flag is read after the launch, as a wide system's
         } else {
-            StageTimer tt(ctx, "solve_lu_wide", stream);
-            lu_wide_factor<float>(ctx, descs[j], plans[j].n + 1, tag, stream);
+            {
+                StageTimer tt(ctx, "solve_lu_wide", stream);
+                lu_wide_factor<float>(ctx, descs[j], plans[j].n + 1, tag, stream);
+            }
+            refine_across(ctx, descs[j], plans[j].n + 1, 0, kAcRounds, tag + "#" + std::to_string(j), stream);
             any_wide = true;
         }
     }
@@ -2096,20 +2506,12 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
             lu_smem_optin();
             prepare_kernel<<<dim3(ceil_div(n1max, 8), nj), 256, 0, stream>>>(d_desc);
             RP_LAUNCH_CHECK();
-            for (int j = 0; j < nj; ++j)
-                if (descs[j].across) {
-                    StageTimer ta(ctx, "solve_lu_across", stream);
-                    lu_factor_across(ctx, descs[j], plans[j].n + 1, tag, stream);
-                }
             lu_solve_refine_kernel<<<nj, solve_threads(n1max), smem, stream>>>(d_desc);
             RP_LAUNCH_CHECK();
         }
     }
     for (int j = 0; j < nj; ++j)  // systems known to need FP64 (an escalated fit): getrf, host-driven refinement
         if (descs[j].wide64) factor_refine_wide64(ctx, descs[j], plans[j].n + 1, stream);
-    std::vector<int> refine32;
-    for (int j = 0; j < nj; ++j)
-        if (descs[j].host32) refine32.push_back(j);
     double *h_info = static_cast<double *>(ctx->host_buf("s_info" + tag, sizeof(double) * kSolveInfo * nj));
     if (any_wide) {
         // wide systems whose FP32 refinement did not converge (flag 2) are factored again in FP64:
@@ -2127,7 +2529,6 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         pd.descs = descs;
         pd.n1.resize((size_t)nj);
         for (int j = 0; j < nj; ++j) pd.n1[j] = plans[j].n + 1;
-        pd.refine32 = refine32;
         if (!pend) {
             RP_CUDA(cudaStreamSynchronize(stream));
             solve_wide_fp64(ctx, pd, stream);
@@ -2142,15 +2543,27 @@ void solve_wide_fp64(rp_ctx *ctx, SolvePending &pd, cudaStream_t stream) {
     pd.any_wide = false;
     const int nj = (int)pd.descs.size();
     bool any = false;
-    for (int j : pd.refine32) {  // wide FP32 factors: refined here, FP64 factors when that stalls
-        if (!refine_wide32(ctx, pd.descs[j], pd.n1[j], stream)) factor_refine_wide64(ctx, pd.descs[j], pd.n1[j], stream);
-        any = true;
-    }
-    pd.refine32.clear();
     for (int j = 0; j < nj; ++j) {
-        if (!pd.descs[j].pre || pd.descs[j].host32 || pd.h_pre[3 * j] != 2.0) continue;
-        factor_refine_wide64(ctx, pd.descs[j], pd.n1[j], stream);
+        if (!pd.descs[j].pre || pd.h_pre[3 * j] < 2.0) continue;
+        double flag = pd.h_pre[3 * j];
         any = true;
+        for (int first = kAcRounds; flag == 3.0; first += 4) {  // not finished: more rounds
+            refine_across(ctx, pd.descs[j], pd.n1[j], first, 4, pd.tag + "#" + std::to_string(j), stream);
+            RP_CUDA(cudaMemcpyAsync(&flag, pd.descs[j].pre, sizeof(flag), cudaMemcpyDeviceToHost, stream));
+            RP_CUDA(cudaStreamSynchronize(stream));
+        }
+        if (flag == 0.0) continue;
+        if (flag == 4.0) {  // by substitution
+            if (pd.n1[j] >= kLUWideMin) {
+                if (refine_wide32(ctx, pd.descs[j], pd.n1[j], pd.tag + "#" + std::to_string(j), stream)) continue;
+            } else {
+                refine_in_cta(ctx, pd.descs[j], pd.n1[j], stream);
+                RP_CUDA(cudaMemcpyAsync(&flag, pd.descs[j].pre, sizeof(flag), cudaMemcpyDeviceToHost, stream));
+                RP_CUDA(cudaStreamSynchronize(stream));
+                if (flag == 0.0) continue;
+            }
+        }
+        factor_refine_wide64(ctx, pd.descs[j], pd.n1[j], stream);
     }
     if (!any) return;
     RP_CUDA(cudaMemcpyAsync(pd.h_info, pd.d_info, sizeof(double) * kSolveInfo * nj, cudaMemcpyDeviceToHost, stream));

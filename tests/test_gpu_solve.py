@@ -83,3 +83,41 @@ def test_singular_systems_across_the_gpu(N, gpu_ctx):
     except _lib.RepeatError:
         return
     assert info["kappa"] > 1e12
+
+
+@pytest.mark.parametrize("N", [255, 382, 383, 384, 511, 766, 1151, 1152])
+def test_refinement_across_the_gpu(N, gpu_ctx):
+    """One system refined across the GPU, at the edges of its 128-unknown blocks, for a matrix whose
+    solution and condition estimate are checked against FP64.  The estimate is Hager's with FP32
+    solves, whose relative error is below n eps32 kappa."""
+    import torch
+    rng = np.random.default_rng(N)
+    X = rng.normal(size=(3 * N, N))
+    A = X.T @ X / (3 * N)
+    b = rng.normal(size=N)
+    K, ref = _reference(A, b, -1.5)
+    q, info = gpu_ctx.solve(torch.from_numpy(A).cuda(), torch.from_numpy(b).cuda(), np.full(N, 6), qtot=-1.5)
+    q = q.cpu().numpy()
+    kinv = np.abs(np.linalg.inv(K)).sum(axis=0).max()
+    kk = np.abs(K).sum(axis=0).max() * kinv
+    assert np.abs(q - ref).max() <= max(1e-12, 1e-15 * kk * (N + 1)) * max(1.0, np.abs(ref).max())
+    kappa = np.abs(A).sum(axis=0).max() * kinv
+    assert kappa / 3 <= info["kappa"] <= kappa * (1 + (N + 1) * 2.0**-24 * kk)
+    xmax = np.abs(np.linalg.solve(K, np.append(b, -1.5))).max()
+    assert info["residual"] <= 2 * (N + 1) * 2.0**-53 * np.abs(K).sum(axis=0).max() * xmax
+
+
+@pytest.mark.parametrize("N", [400, 900])
+def test_slow_refinement(N, gpu_ctx):
+    """kappa towards 1/eps32: refinement with inverted blocks, by substitution, and FP64 factors."""
+    import torch
+    rng = np.random.default_rng(7)
+    U, _ = np.linalg.qr(rng.normal(size=(N, N)))
+    for top in (1e5, 1e6, 1e7, 1e9):
+        A = (U * np.geomspace(1.0 / top, 1.0, N)) @ U.T
+        A = 0.5 * (A + A.T)
+        b = rng.normal(size=N)
+        K, ref = _reference(A, b, 0.0)
+        q, info = gpu_ctx.solve(torch.from_numpy(A).cuda(), torch.from_numpy(b).cuda(), np.full(N, 6), qtot=0.0)
+        tol = max(1e-12, 1e-15 * np.linalg.cond(K) * (N + 1))
+        assert np.abs(q.cpu().numpy() - ref).max() <= tol * max(1.0, np.abs(ref).max())
