@@ -523,11 +523,14 @@ struct SolveJob {
     const double *resp_s, *resp_t;
     double qtot;
     double *q;
+    int refit = 0;  // an escalated fit's system: 1 FP32 factors and refinement beyond convergence, 2 FP64
+                    // factors at once
 };
-// fp64_first: wide systems (known ill-conditioned, e.g. an escalated fit) are factored in
-// FP64 at once instead of after a stalled FP32 attempt
-void solve_batch(rp_ctx *ctx, const std::vector<SolveJob> &jobs, std::vector<double> &info, cudaStream_t stream,
-                 bool fp64_first = false);
+// The largest kappa of an escalated fit's system that is refined with FP32 factors (refit = 1).  A step
+// then leaves 1.5e-10 kappa of the residual (1e-4 at 6.8e5, 3.6e-4 at 2.1e6, 1e-3 at 9.2e6): three and
+// the extra one reach what FP64 factors do, in 1.2 ms instead of 6.3 at 710 unknowns.
+constexpr double kRefitKappa32 = 2e6;
+void solve_batch(rp_ctx *ctx, const std::vector<SolveJob> &jobs, std::vector<double> &info, cudaStream_t stream);
 // One bordered system of the solve kernel (device-side descriptor).
 struct SolveDesc {
     const double *A;      // N x N input
@@ -550,6 +553,7 @@ struct SolveDesc {
     double *info;         // kSolveInfo out: residual inf-norm, min|piv|, max|piv|, singular flag,
                           // kappa, unknowns n+1, refinement steps, factorisation path
     double *pre;          // null, or {flag, min|piv|, max|piv|} of a wide factorisation already in As
+    int refit;            // SolveJob's
     int wide64;           // As holds wide FP64 factors: skip the FP32 stage and the in-CTA FP64 LU
     int host64;           // FP32 factors in the CTA, but a stalled refinement goes to the host's FP64
                           // factorisation across the GPU (pre holds its flag) instead of an in-CTA FP64 LU
@@ -572,7 +576,7 @@ struct SolvePending {
 // are final after it); without, the call waits for them.  (Systems with overlapping symmetry
 // groups are folded on the host, which waits.)
 const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, cudaStream_t stream,
-                                const std::string &tag, SolvePending *pend = nullptr, bool fp64_first = false);
+                                const std::string &tag, SolvePending *pend = nullptr);
 void solve_wide_fp64(rp_ctx *ctx, SolvePending &pd, cudaStream_t stream);  // synchronises stream
 
 // Reciprocal sum by separable lattice phases (recip_sep.cu): E[r][col][n1] for every

@@ -560,10 +560,13 @@ void batch_complete(rp_ctx *ctx, BatchRun &r) {
         }
     auto resolve = [&](const std::vector<int> &cubes, int flag, int precision) {
         std::vector<rp::SolveJob> jobs;
-        for (int i : cubes) jobs.push_back(r.job(i));
+        for (int i : cubes) {
+            jobs.push_back(r.job(i));
+            if (flag == RP_FIT_ESCALATED)  // refined to the end, or FP64 factors at once, by its mixed fit's kappa
+                jobs.back().refit = info[(size_t)W * i + 4] <= rp::kRefitKappa32 ? 1 : 2;
+        }
         std::vector<double> rinfo;
-        // an escalated cube's system is known to be beyond FP32 refinement: FP64 factors at once
-        rp::solve_batch(ctx, jobs, rinfo, stream, flag == RP_FIT_ESCALATED);
+        rp::solve_batch(ctx, jobs, rinfo, stream);
         for (size_t t = 0; t < cubes.size(); ++t) {
             take(cubes[t], rinfo.data() + (size_t)rp::kSolveInfo * t);
             info[(size_t)W * cubes[t] + 6] = precision;

@@ -938,7 +938,7 @@ __global__ void __launch_bounds__(kSolve) lu_solve_refine_kernel(const SolveDesc
         d.info[4] = fmin(anorm * kinv, 1e300);
         d.info[5] = n1;
         d.info[6] = steps;
-        d.info[7] = f32_solved ? 0.0 : 2.0;
+        d.info[7] = f32_solved ? (d.across ? 1.0 : 0.0) : 2.0;
     }
     __syncthreads();
     // expand to all atoms
@@ -1626,6 +1626,9 @@ void factor_refine_wide64(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t 
 //                           for Hager's estimate, and the next right-hand sides;
 //   across_apply_kernel     (P L U)^-1 of all of them at once, in one cluster;
 //   across_residual_kernel  x += correction and r = bs - A0 x in FP64, rows over the GPU.
+// An escalated fit's system (SolveJob::refit = 1) gets one correction beyond convergence, kept when
+// the residual falls: FP64's accuracy from FP32 factors (charges 2.1e-12 from 64 bits either way, 1.2 ms
+// instead of getrf's 3.9 and its refinement's 2.4 at 710 unknowns).
 // The refinement, the estimate and its extra test vector do not depend on one another, so
 // round k carries correction k, the estimate's vector k and (round 0) the extra vector: four
 // rounds instead of eight triangular solves one after the other.
@@ -1649,6 +1652,7 @@ struct AcrossState {
     double rm, rprev, res, est, alt;
     int steps, phase;       // phase 0: refining, 1: converged, 2: left to substitution, 3: zero pivot
     int hstate, hit, jprev, jcur;  // 0: uniform vector under way, 1: signs, 2: a unit vector, 3: estimate done
+    int extra;              // a refit: the correction beyond convergence is under way
     int xsel, finished;     // which x holds the solution; nothing left to do
 };
 struct AcrossRun {
@@ -1659,7 +1663,6 @@ struct AcrossRun {
     AcrossState *st;
     SolveDesc d;
     int n1, nblk;
-    double path;            // info's factorisation path
 };
 
 // max row sums of |K| and |A| (K symmetric), a warp per row; st cleared before
@@ -1753,7 +1756,7 @@ __global__ void __launch_bounds__(1024) across_control_kernel(AcrossRun p, int r
             st.rm = m;
             st.rprev = 1e308;
             st.res = 0.0;
-            st.steps = st.hit = st.hstate = st.xsel = 0;
+            st.steps = st.hit = st.hstate = st.xsel = st.extra = 0;
             st.jprev = -1;
             st.est = st.alt = 0.0;
             st.phase = p.d.pre[0] != 0.0 ? 3 : m == 0.0 ? 1 : 0;
@@ -1766,11 +1769,24 @@ __global__ void __launch_bounds__(1024) across_control_kernel(AcrossRun p, int r
         if (tid == 0 && st.phase == 0) {
             const double rn = __longlong_as_double((long long)st.rn_bits), xn = __longlong_as_double((long long)st.xn_bits),
                          an = __longlong_as_double((long long)st.an_bits);
-            st.res = rn;
-            ++st.steps;
-            st.xsel = round & 1;
-            if (rn <= (double)n1 * 1.1102230246251565e-16 * an * xn) st.phase = 1;
-            else if (!(rn < 1e300) || (st.steps >= 2 && rn > kInvRate * st.rprev)) st.phase = 2;  // substitution takes over
+            if (st.extra) {  // kept if the residual fell
+                if (rn < st.res) {
+                    st.res = rn;
+                    ++st.steps;
+                    st.xsel = round & 1;
+                }
+                st.phase = 1;
+            } else {
+                st.res = rn;
+                ++st.steps;
+                st.xsel = round & 1;
+                if (rn <= (double)n1 * 1.1102230246251565e-16 * an * xn) {
+                    if (p.d.refit && rn > 0.0) st.extra = 1;
+                    else st.phase = 1;
+                } else if (!(rn < 1e300) || (st.steps >= 2 && rn > kInvRate * st.rprev)) {
+                    st.phase = 2;  // substitution takes over
+                }
+            }
             st.rprev = st.rm = rn;
         }
         if (st.hstate != 3) {
@@ -1845,7 +1861,7 @@ __global__ void __launch_bounds__(1024) across_control_kernel(AcrossRun p, int r
             p.d.info[4] = fmin(__longlong_as_double((long long)st.anorm_bits) * kinv, 1e300);
             p.d.info[5] = n1;
             p.d.info[6] = st.steps;
-            p.d.info[7] = p.path;
+            p.d.info[7] = 1.0;  // FP32 factors from across the GPU
         }
         st.finished = solved || st.phase == 3;
         if (st.phase == 3) p.d.pre[0] = 2.0;
@@ -2040,7 +2056,6 @@ void refine_across(rp_ctx *ctx, const SolveDesc &d, int n1, int first, int round
     p.x[0] = d.x;
     p.x[1] = ctx->buf_t<double>("s_ac_x" + key, (size_t)n1);
     p.st = ctx->buf_t<AcrossState>("s_ac_st" + key, 1);
-    p.path = n1 < kLUWideMin ? 0.0 : 1.0;
     if (first == 0) {
         RP_CUDA(cudaMemsetAsync(p.st, 0, sizeof(AcrossState), stream));
         across_norms_kernel<<<(int)ceil_div(n1, 8), 256, 0, stream>>>(p);
@@ -2327,7 +2342,7 @@ static void host_fold(int N, const std::vector<double> &A, const std::vector<dou
 }
 
 const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, cudaStream_t stream,
-                                const std::string &tag, SolvePending *pend, bool fp64_first) {
+                                const std::string &tag, SolvePending *pend) {
     const int nj = (int)jobs.size();
     if (nj == 0) return nullptr;
     std::vector<FoldPlan> plans((size_t)nj);
@@ -2381,6 +2396,7 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         d.resp_s = J.resp_s ? d_rs + o_red : nullptr; d.resp_t = J.resp_s ? d_rt + o_red : nullptr;
         d.map = d_map + o_map; d.qtot = J.qtot;
         d.As = As + o_sq; d.A0 = A0 + o_sq; d.bs = bs + o_red; d.x = x + o_red; d.r = r + o_red;
+        d.refit = J.refit;
         d.perm = perm + o_red; d.q = J.q; d.info = d_info + kSolveInfo * (size_t)j;
         o_map += J.N;
         o_mptr += p.mem_ptr.size();
@@ -2394,9 +2410,9 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         const int n1 = plans[j].n + 1;
         if (n1 >= kLUHost64Min && n1 <= kLUWideMax) {
             descs[j].pre = d_pre + 3 * (size_t)j;
-            descs[j].host64 = n1 < kLUWideMin;
-            if (fp64_first) descs[j].wide64 = 1;
-            else if (n1 >= kLUWideMin) descs[j].host32 = 1;
+            if (jobs[j].refit == 2) descs[j].wide64 = 1;
+            else if (jobs[j].refit == 1 || n1 >= kLUWideMin) descs[j].host32 = 1;
+            else descs[j].host64 = 1;
         }
         if (plans[j].disjoint) disjoint.push_back(j);
     }
@@ -2405,13 +2421,13 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
     // at 720), two of them one after the other from kAcrossTwo; more run side by side, each in its CTA.
     int mid = 0, least = kLUWideMin;
     for (int j = 0; j < nj; ++j)
-        if (descs[j].host64 && !descs[j].wide64) {
+        if (descs[j].host64) {
             ++mid;
             least = std::min(least, plans[j].n + 1);
         }
     if (mid == 1 || (mid == 2 && least >= kAcrossTwo))
         for (int j = 0; j < nj; ++j)
-            if (descs[j].host64 && !descs[j].wide64) {
+            if (descs[j].host64) {
                 descs[j].host64 = 0;
                 descs[j].host32 = 1;
             }
@@ -2553,7 +2569,7 @@ void solve_wide_fp64(rp_ctx *ctx, SolvePending &pd, cudaStream_t stream) {
             RP_CUDA(cudaStreamSynchronize(stream));
         }
         if (flag == 0.0) continue;
-        if (flag == 4.0) {  // by substitution
+        if (flag == 4.0 && pd.descs[j].refit == 0) {  // by substitution
             if (pd.n1[j] >= kLUWideMin) {
                 if (refine_wide32(ctx, pd.descs[j], pd.n1[j], pd.tag + "#" + std::to_string(j), stream)) continue;
             } else {
@@ -2570,12 +2586,11 @@ void solve_wide_fp64(rp_ctx *ctx, SolvePending &pd, cudaStream_t stream) {
     RP_CUDA(cudaStreamSynchronize(stream));
 }
 
-void solve_batch(rp_ctx *ctx, const std::vector<SolveJob> &jobs, std::vector<double> &info, cudaStream_t stream,
-                 bool fp64_first) {
+void solve_batch(rp_ctx *ctx, const std::vector<SolveJob> &jobs, std::vector<double> &info, cudaStream_t stream) {
     const int nj = (int)jobs.size();
     info.assign((size_t)nj * kSolveInfo, 0.0);
     if (nj == 0) return;
-    const double *h = solve_batch_async(ctx, jobs, stream, "", nullptr, fp64_first);
+    const double *h = solve_batch_async(ctx, jobs, stream, "");
     RP_CUDA(cudaStreamSynchronize(stream));
     std::copy(h, h + kSolveInfo * (size_t)nj, info.begin());
 }

@@ -172,3 +172,21 @@ def test_tric_full_size_mixed_against_fp64(gpu_ctx):
     qm, _, im = _batch(gpu_ctx, cube, _lib.PREC_MIXED)
     assert im["escalated"]
     assert np.abs(qm - q64).max() <= 1e-3
+
+
+@pytest.mark.parametrize("n_atoms", [150, 330, 1000, 1400])
+def test_escalated_fits_by_kappa_and_size(n_atoms, gpu_ctx):
+    """Escalated by a low limit, so that kappa decides between FP32 factors refined to the end (below 2e6)
+    and FP64 factors, at sizes solved in one CTA, and across the GPU below and above 768 unknowns: the
+    charges of the plain FP64 fit, within n eps64 kappa of the largest."""
+    from pyrepeat_gb300 import _lib, synth
+    cube = synth.make_tric(seed=n_atoms, n_grid=(72, 70, 75), n_atoms=n_atoms, ctx=gpu_ctx)
+    ref, M, info = _batch(gpu_ctx, cube, _lib.PREC_FP64)
+    gpu_ctx.set_kappa_limit(1e-3)
+    try:
+        q, Me, einfo = _batch(gpu_ctx, cube, _lib.PREC_MIXED)
+    finally:
+        gpu_ctx.set_kappa_limit(_lib.DEFAULT_KAPPA_LIMIT)
+    assert einfo["escalated"] and M == Me
+    n1 = n_atoms + 1
+    assert np.abs(q - ref).max() <= 4 * n1 * 2.0**-53 * info["kappa"] * max(1.0, np.abs(ref).max())
