@@ -42,6 +42,7 @@
 
 #include "common.cuh"
 #include "df.cuh"
+#include "f32x2.cuh"
 #include "tc.cuh"
 
 namespace rp {
@@ -463,34 +464,6 @@ __device__ __forceinline__ float erfc_nr2(float xs) {
     return t * ex2_ftz(fmaf(-xs, xs, p));
 }
 
-// Pairs of FP32 values in one 64-bit register, for the packed instructions of this part: one
-// issue slot does the IEEE operation of both halves, each rounded as the scalar instruction
-// rounds it.  (The Phi kernel is bound by instruction issue, not by the FP32 pipe.)
-using f2 = unsigned long long;
-__device__ __forceinline__ f2 pack2(float a, float b) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ f2 dup2(float a) { return pack2(a, a); }
-__device__ __forceinline__ void unpack2(f2 v, float &a, float &b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f2 add2(f2 a, f2 b) {
-    f2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
 __device__ __forceinline__ f2 sub2(f2 a, f2 b) { return fma2(b, dup2(-1.0f), a); }  // one rounding, as a - b
 // a + b as s + e exactly, both halves (dfa::two_sum)
 __device__ __forceinline__ void two_sum2(f2 a, f2 b, f2 &s, f2 &e) {

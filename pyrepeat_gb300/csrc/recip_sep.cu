@@ -9,8 +9,8 @@
 //   phi_recip(g, a) = Re sum_n1 ex[n1][i] sum_n2 ey[n2][j] sum_n3 ez[n3][l] W_a(n)
 //
 // is a three-stage separable transform, evaluated as
-//   stage A   F[l][n2][a][n1] = sum_n3 ez[n3][l] W[a][n2][n3][n1]       (every grid plane l)
-//   stage B   E[r][a][n1]     = sum_n2 ey[n2][j] F[l][n2][a][n1]         (every grid row r = j + l n_y)
+//   stage A   F[l][a][n2][n1] = sum_n3 ez[n3][l] W[a][n3][n2][n1]       (every grid plane l)
+//   stage B   E[r][a][n1]     = sum_n2 ey[n2][j] F[l][a][n2][n1]         (every grid row r = j + l n_y)
 //   stage C   phi_recip(m, a) = Re sum_n1 ex[n1][i_m] E[r_m][a][n1]      (per kept point, fused into
 //                                                                        the real-space kernel)
 // Stage C costs 2 KMAX real multiply-adds per point-atom instead of the 4 K of a dense
@@ -26,6 +26,7 @@
 
 #include "common.cuh"
 #include "df.cuh"
+#include "f32x2.cuh"
 
 namespace rp {
 namespace {
@@ -46,6 +47,7 @@ struct RecipJob {
     float2 *W, *F, *E;
     double rb[9];          // reciprocal basis (rows)
     int N, ncols, K, P, ny, nz, ab;
+    int ea, ra;            // stage A: (n2, n1) entries and planes of a CTA
     int ecols;             // columns of E's rows (recip_cols)
 };
 constexpr int kRecipJobs = 64;
@@ -95,7 +97,7 @@ __device__ __forceinline__ double2 cmul(double2 x, double2 y) {
     return make_double2(x.x * y.x - x.y * y.y, x.x * y.y + x.y * y.x);
 }
 
-// W[col][n2'][n3'][n1] = w_k e^{-i k.r} (col = atom), or sum_a q_a w_k e^{-i k.r_a} (one
+// W[col][n3'][n2'][n1] = w_k e^{-i k.r} (col = atom), or sum_a q_a w_k e^{-i k.r_a} (one
 // charge-weighted column when q != nullptr), stored rounded to FP32.  Per atom the two
 // phase products and the weight are double-float products on the FP32 pipe (~2^-44
 // relative); the charge-weighted sum stays FP64.  (W is zero outside the k-set: the host
@@ -110,7 +112,7 @@ __global__ void build_w_kernel(const __grid_constant__ RecipLaunch L) {
     const int col = (int)(t / K), k = (int)(t - (long long)col * K);
     const int n1c = P + 1, nw = 2 * P + 1;
     const int n1 = J.kidx[3 * k], n2 = J.kidx[3 * k + 1] + P, n3 = J.kidx[3 * k + 2] + P;
-    float2 *out = J.W + (((long long)col * nw + n2) * nw + n3) * n1c + n1;
+    float2 *out = J.W + (((long long)col * nw + n3) * nw + n2) * n1c + n1;
     if (J.q == nullptr) {
         const float4 *u = J.Udf + (size_t)col * 3 * nw;
         dfa::acc re{0.f, 0.f}, im{0.f, 0.f};
@@ -142,122 +144,132 @@ __global__ void build_w_kernel(const __grid_constant__ RecipLaunch L) {
     if (lane == 0) *out = make_float2((float)(w * z.x), (float)(w * z.y));
 }
 
-// Each stage-A thread produces up to kN1B consecutive n1 outputs of one (plane, n2,
-// column): kN1B independent accumulator chains, and the shared phase factor is
-// loaded once per term.
-constexpr int kN1B = 8;
-
-// Stage A, one thread per (n2, column, n1 block, plane l) with l fastest: a warp reads
-// one W row (broadcast) and consecutive ez phases (coalesced); FP32 products.
-__global__ void recip_stage_a_kernel(const __grid_constant__ RecipLaunch L) {
-    extern __shared__ float2 ezs[];  // the job's ez table [nw][nz] (FP32), read once per CTA
-    const int jb = recip_job_of(L, blockIdx.x);
-    const RecipJob &J = L.job[jb];
-    const int P = J.P, nz = J.nz, ncols = J.ncols;
-    const int n1c = P + 1, nw = 2 * P + 1, nb = (n1c + kN1B - 1) / kN1B;
-    for (int q = threadIdx.x; q < nw * nz; q += blockDim.x) {
-        const float4 e = J.EZ[q];
-        ezs[q] = make_float2(e.x, e.z);
+// Stages A and B are the same product, out[row][r] = sum_k t[k][row] f[k][r] (complex), with the planes
+// and ez, or a plane's rows and ey, as rows.  f and the phases t, split into cosines and sines, sit
+// in shared memory.  A thread owns kJB consecutive rows of two entries r: per k it reads two values
+// of f and eight rows of phases (warp broadcasts) for 32 packed FMAs, two rows to an
+// instruction, in the order of k and with the roundings of a scalar loop; a warp's stores of a row are
+// consecutive in r.
+// Bound by the FMA pipe, which a packed FMA holds for two cycles.  Measured per launch against one
+// thread per eight n1 reading W through L1 (stage A) and one entry per thread with scalar FMAs
+// (stage B, 60 instructions per k for 32 FMAs): 99 us from 291 and 359 from 587
+// (424 atoms, 128^3, KMAX 12: 0.08 and 7.7 G multiply-adds, 667 MB of E; the FMA pipe is 66 % busy in stage
+// B).  Several planes per stage B CTA, for one load of the phases, were slower (406 us).
+constexpr int kJB = 8, kRecipT = 128;
+__device__ __forceinline__ void rows_load_table(float *cs, float *sn, int np, const float4 *T, int nk, int rows, int r0, int n) {
+    for (int q = threadIdx.x; q < nk * np; q += kRecipT) {
+        const int k = q / np, j = q - k * np;
+        const float4 y = j < n ? T[k * rows + r0 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
+        cs[q] = y.x;
+        sn[q] = y.z;
     }
-    __syncthreads();
-    long long t = (long long)(blockIdx.x - L.blk[jb]) * blockDim.x + threadIdx.x;
-    if (t >= (long long)nz * nw * ncols * nb) return;
-    const int l = (int)(t % nz);
-    t /= nz;
-    const int b = (int)(t % nb);
-    t /= nb;
-    const int a = (int)(t % ncols);
-    const int n2 = (int)(t / ncols);
-    const int n10 = b * kN1B, cnt = min(kN1B, n1c - n10);
-    float re[kN1B], im[kN1B];
-#pragma unroll
-    for (int u = 0; u < kN1B; ++u) re[u] = im[u] = 0.f;
-    const float2 *w = J.W + ((long long)a * nw + n2) * nw * n1c + n10;
-    for (int n3 = 0; n3 < nw; ++n3) {
-        const float2 z = ezs[n3 * nz + l];
-        const float2 *wr = w + (long long)n3 * n1c;
-#pragma unroll
-        for (int u = 0; u < kN1B; ++u)
-            if (u < cnt) {
-                const float2 v = wr[u];
-                re[u] = fmaf(z.x, v.x, re[u]);
-                re[u] = fmaf(-z.y, v.y, re[u]);
-                im[u] = fmaf(z.x, v.y, im[u]);
-                im[u] = fmaf(z.y, v.x, im[u]);
-            }
-    }
-    float2 *o = J.F + (((long long)l * nw + n2) * ncols + a) * n1c + n10;
-#pragma unroll
-    for (int u = 0; u < kN1B; ++u)
-        if (u < cnt) o[u] = make_float2(re[u], im[u]);
 }
-
-// Stage B, one CTA per (plane l, block of `ab` columns) of a job.  The plane's F slab for
-// those columns ([n2][a][n1], FP32) and the ey phases ([n2][j], rows padded to kJB) sit in
-// shared memory.  A thread owns one (column, n1) and kJB consecutive rows j: its F value is
-// one load per n2, the ey values are warp broadcasts read two rows at a time, and a warp's
-// stores of E land on consecutive (column, n1) of one row, contiguous in memory.
-constexpr int kJB = 8;
-__global__ void __launch_bounds__(128) recip_stage_b_kernel(const __grid_constant__ RecipLaunch L) {
-    extern __shared__ float4 smem_b[];
-    const int jb = recip_job_of(L, blockIdx.x);
-    const RecipJob &J = L.job[jb];
-    const int P = J.P, ncols = J.ncols, ny = J.ny, ab = J.ab;
-    const int n1c = P + 1, nw = 2 * P + 1;
-    const int nbx = (ncols + ab - 1) / ab, bloc = blockIdx.x - L.blk[jb];
-    const int l = bloc / nbx, a0 = (bloc - l * nbx) * ab, na = min(ab, ncols - a0);
-    const int an = na * n1c;                                  // (column, n1) pairs of the CTA
-    const int nyp = (ny + kJB - 1) / kJB * kJB;
-    float2 *fs = reinterpret_cast<float2 *>(smem_b);          // [nw][an]
-    float2 *eys = fs + ((nw * ab * n1c + 1) & ~1);           // [nw][nyp], 16-byte aligned rows
-    for (int t = threadIdx.x; t < nw * an; t += blockDim.x) {
-        const int n2 = t / an, r = t - n2 * an;
-        fs[t] = J.F[(((long long)l * nw + n2) * ncols + a0) * n1c + r];
-    }
-    for (int q = threadIdx.x; q < nw * nyp; q += blockDim.x) {
-        const int n2 = q / nyp, j = q - n2 * nyp;
-        const float4 y = j < ny ? J.EY[n2 * ny + j] : make_float4(0.f, 0.f, 0.f, 0.f);
-        eys[q] = make_float2(y.x, y.z);
-    }
-    __syncthreads();
-    const int tasks = an * (nyp / kJB);
-    for (int task = threadIdx.x; task < tasks; task += blockDim.x) {
-        const int jj = task / an, r = task - jj * an;  // r = a n1c + n1
-        float re[kJB], im[kJB];
+// entry r is at f[off(r) + k fk]; rows r0 .. r0 + n of out, entries 0 .. an
+template <class Off>
+__device__ __forceinline__ void rows_product(const float2 *f, int fk, Off off, int an, const float *cs, const float *sn, int np,
+                                             int nk, int n, float2 *out, long long stride) {
+    const int half = (an + 1) >> 1, tasks = half * (np / kJB);
+    for (int task = threadIdx.x; task < tasks; task += kRecipT) {
+        const int jj = task / half, r = task - jj * half;
+        const bool two = r + half < an;
+        const float2 *fa = f + off(r), *fb = f + off(two ? r + half : r);
+        const float *c = cs + jj * kJB, *s = sn + jj * kJB;
+        f2 re[2][kJB / 2], im[2][kJB / 2];
 #pragma unroll
-        for (int u = 0; u < kJB; ++u) re[u] = im[u] = 0.f;
-        for (int n2 = 0; n2 < nw; ++n2) {
-            const float2 f = fs[n2 * an + r];
-            const float4 *yp = reinterpret_cast<const float4 *>(eys + n2 * nyp + jj * kJB);
+        for (int u = 0; u < kJB / 2; ++u) re[0][u] = re[1][u] = im[0][u] = im[1][u] = 0ull;
+#pragma unroll 2
+        for (int k = 0; k < nk; ++k) {
+            const float2 v[2] = {*fa, *fb};
+            const ulonglong2 c0 = *reinterpret_cast<const ulonglong2 *>(c), c1 = *reinterpret_cast<const ulonglong2 *>(c + 4);
+            const ulonglong2 s0 = *reinterpret_cast<const ulonglong2 *>(s), s1 = *reinterpret_cast<const ulonglong2 *>(s + 4);
+            const f2 cc[kJB / 2] = {c0.x, c0.y, c1.x, c1.y}, ss[kJB / 2] = {s0.x, s0.y, s1.x, s1.y};
 #pragma unroll
-            for (int u = 0; u < kJB / 2; ++u) {
-                const float4 y = yp[u];  // rows 2u and 2u+1: (re, im, re, im)
-                re[2 * u] = fmaf(y.x, f.x, re[2 * u]);
-                re[2 * u] = fmaf(-y.y, f.y, re[2 * u]);
-                im[2 * u] = fmaf(y.x, f.y, im[2 * u]);
-                im[2 * u] = fmaf(y.y, f.x, im[2 * u]);
-                re[2 * u + 1] = fmaf(y.z, f.x, re[2 * u + 1]);
-                re[2 * u + 1] = fmaf(-y.w, f.y, re[2 * u + 1]);
-                im[2 * u + 1] = fmaf(y.z, f.y, im[2 * u + 1]);
-                im[2 * u + 1] = fmaf(y.w, f.x, im[2 * u + 1]);
+            for (int e = 0; e < 2; ++e) {
+                const f2 x = dup2(v[e].x), y = dup2(v[e].y), ny = dup2(-v[e].y);
+#pragma unroll
+                for (int u = 0; u < kJB / 2; ++u) {
+                    re[e][u] = fma2(cc[u], x, re[e][u]);
+                    im[e][u] = fma2(cc[u], y, im[e][u]);
+                }
+#pragma unroll
+                for (int u = 0; u < kJB / 2; ++u) {
+                    re[e][u] = fma2(ss[u], ny, re[e][u]);
+                    im[e][u] = fma2(ss[u], x, im[e][u]);
+                }
+            }
+            fa += fk;
+            fb += fk;
+            c += np;
+            s += np;
+        }
+        float2 *o = out + jj * kJB * stride + r;
+#pragma unroll
+        for (int u = 0; u < kJB / 2; ++u) {
+            float2 a, b;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                if (e == 1 && !two) continue;
+                unpack2(re[e][u], a.x, b.x);
+                unpack2(im[e][u], a.y, b.y);
+                if (jj * kJB + 2 * u < n) o[2 * u * stride + e * half] = a;
+                if (jj * kJB + 2 * u + 1 < n) o[(2 * u + 1) * stride + e * half] = b;
             }
         }
-        float2 *o = J.E + (((long long)l * ny + jj * kJB) * J.ecols + a0) * n1c + r;
-        const long long row_stride = (long long)J.ecols * n1c;
-#pragma unroll
-        for (int u = 0; u < kJB; ++u)
-            if (jj * kJB + u < ny) o[u * row_stride] = make_float2(re[u], im[u]);
     }
 }
 
-// stage B's columns per CTA: as many as fit 48 KB of shared memory (at most 16)
+// Stage A, one CTA per (column, J.ea of its (n2, n1) entries, J.ra planes).
+__global__ void __launch_bounds__(kRecipT) recip_stage_a_kernel(const __grid_constant__ RecipLaunch L) {
+    extern __shared__ __align__(16) float smem_r[];
+    const int jb = recip_job_of(L, blockIdx.x);
+    const RecipJob &J = L.job[jb];
+    const int n1c = J.P + 1, nw = 2 * J.P + 1, ne = nw * n1c, nc = (ne + J.ea - 1) / J.ea, nr = (J.nz + J.ra - 1) / J.ra;
+    int b = blockIdx.x - L.blk[jb];
+    const int l0 = (b % nr) * J.ra, n = min(J.ra, J.nz - l0);
+    b /= nr;
+    const int e0 = (b % nc) * J.ea, an = min(J.ea, ne - e0), a = b / nc;
+    const int np = (n + kJB - 1) / kJB * kJB;
+    float *cs = smem_r, *sn = cs + nw * np;  // np is a multiple of 8
+    float2 *f = reinterpret_cast<float2 *>(sn + nw * np);
+    const float2 *w = J.W + (long long)a * nw * ne + e0;
+    for (int k = 0; k < nw; ++k)
+        for (int r = threadIdx.x; r < an; r += kRecipT) f[k * an + r] = w[k * ne + r];
+    rows_load_table(cs, sn, np, J.EZ, nw, J.nz, l0, n);
+    __syncthreads();
+    rows_product(f, an, [](int r) { return r; }, an, cs, sn, np, nw, n,
+                 J.F + ((long long)l0 * J.ncols + a) * ne + e0, (long long)J.ncols * ne);
+}
+
+// Stage B, one CTA per (plane l, block of `ab` columns) of a job: the plane's F of those columns is one
+// contiguous slab [a][n2][n1].
+__global__ void __launch_bounds__(kRecipT) recip_stage_b_kernel(const __grid_constant__ RecipLaunch L) {
+    extern __shared__ __align__(16) float smem_r[];
+    const int jb = recip_job_of(L, blockIdx.x);
+    const RecipJob &J = L.job[jb];
+    const int ncols = J.ncols, ny = J.ny, ab = J.ab;
+    const int n1c = J.P + 1, nw = 2 * J.P + 1, ne = nw * n1c;
+    const int nbx = (ncols + ab - 1) / ab, bloc = blockIdx.x - L.blk[jb];
+    const int l = bloc / nbx, a0 = (bloc - l * nbx) * ab, na = min(ab, ncols - a0);
+    const int np = (ny + kJB - 1) / kJB * kJB;
+    float *cs = smem_r, *sn = cs + nw * np;
+    float2 *f = reinterpret_cast<float2 *>(sn + nw * np);
+    const float2 *F = J.F + ((long long)l * ncols + a0) * ne;
+#pragma unroll 4
+    for (int t = threadIdx.x; t < na * ne; t += kRecipT) f[t] = F[t];
+    rows_load_table(cs, sn, np, J.EY, nw, ny, 0, ny);
+    __syncthreads();
+    rows_product(f, n1c, [=](int r) { return r / n1c * ne + r % n1c; }, na * n1c, cs, sn, np, nw, ny,
+                 J.E + ((long long)l * ny * J.ecols + a0) * n1c, (long long)J.ecols * n1c);
+}
+
+// stage B's columns per CTA: as many as fit 24 KB of shared memory (at most 16)
 int stage_b_columns(int P) {
     const size_t col_bytes = sizeof(float2) * (size_t)(2 * P + 1) * (P + 1);
-    return (int)std::max<size_t>(1, std::min<size_t>(16, (48u << 10) / col_bytes));
+    return (int)std::max<size_t>(1, std::min<size_t>(16, (24u << 10) / col_bytes));
 }
+size_t table_bytes(int P, int rows) { return sizeof(float2) * (size_t)(2 * P + 1) * ((rows + kJB - 1) / kJB * kJB); }
 size_t stage_b_smem(int P, int ny, int ab) {
-    const size_t nw = 2 * P + 1, n1c = P + 1, nyp = (size_t)(ny + kJB - 1) / kJB * kJB;
-    return sizeof(float2) * (((size_t)nw * ab * n1c + 1) & ~(size_t)1) + sizeof(float2) * nw * nyp;
+    return table_bytes(P, ny) + sizeof(float2) * (size_t)(2 * P + 1) * ab * (P + 1);
 }
 
 }  // namespace
@@ -299,6 +311,10 @@ void recip_rows_group(rp_ctx *ctx, const std::vector<RecipRowsJob> &jobs, cudaSt
         const size_t j1 = std::min(nj, j0 + kRecipJobs);
         RecipLaunch L{};
         int blk[4][kRecipJobs + 1] = {};
+        // stage A's planes are split over CTAs where the columns alone would leave the GPU idle
+        long long cols = 0;
+        for (size_t j = j0; j < j1; ++j) cols += jobs[j].d_q ? 1 : jobs[j].N;
+        const int splits = (int)std::min<long long>(4, ceil_div(456, std::max<long long>(cols, 1)));
         size_t smem_a = 0, smem_b = 0;
         L.n = 0;
         for (size_t j = j0; j < j1; ++j) {
@@ -319,18 +335,23 @@ void recip_rows_group(rp_ctx *ctx, const std::vector<RecipRowsJob> &jobs, cudaSt
             for (int q = 0; q < 9; ++q) J.rb[q] = ew->rec[q];
             J.N = rj.N; J.ncols = ncols; J.K = ew->K; J.P = P; J.ny = ny; J.nz = nz; J.ab = stage_b_columns(P);
             J.ecols = rj.d_q ? 1 : recip_cols(ncols);
-            const int nb = (n1c + kN1B - 1) / kN1B;
+            // stage A's slab of W: up to 32 KB beside the phases (a column of KMAX 7 is 9.5 KB)
+            const int ne = nw * n1c;
+            RP_REQUIRE(sizeof(float2) * (size_t)nw * nz <= (200u << 10), "recip_rows: grid too large along z for KMAX");
+            const size_t room = std::min<size_t>(32u << 10, (224u << 10) - table_bytes(P, nz));
+            const int chunks = (int)ceil_div(ne, std::max<long long>(1, room / (sizeof(float2) * nw)));
+            J.ea = (int)ceil_div(ne, chunks);
+            J.ra = (int)ceil_div(ceil_div(nz, splits), kJB) * kJB;
             const int k = L.n;
             blk[0][k + 1] = blk[0][k] + (int)ceil_div((long long)rj.N * 3 * nw, 128);
             blk[1][k + 1] = blk[1][k] + (int)ceil_div((long long)ncols * ew->K, rj.d_q ? 4 : 128);
-            blk[2][k + 1] = blk[2][k] + (int)ceil_div((long long)nz * nw * ncols * nb, 128);
+            blk[2][k + 1] = blk[2][k] + ncols * (int)ceil_div(ne, J.ea) * (int)ceil_div(nz, J.ra);
             blk[3][k + 1] = blk[3][k] + (int)ceil_div(ncols, J.ab) * nz;
-            smem_a = std::max(smem_a, sizeof(float2) * (size_t)nw * nz);
+            smem_a = std::max(smem_a, table_bytes(P, std::min(J.ra, nz)) + sizeof(float2) * (size_t)nw * J.ea);
             smem_b = std::max(smem_b, stage_b_smem(P, ny, J.ab));
             ++L.n;
         }
         if (L.n == 0) continue;
-        RP_REQUIRE(smem_a <= (200u << 10), "recip_rows: grid too large along z for KMAX");
         RP_REQUIRE(smem_b <= (200u << 10), "recip_rows: KMAX too large");
         smem_optin((const void *)recip_stage_a_kernel, smem_a);
         smem_optin((const void *)recip_stage_b_kernel, smem_b);
@@ -345,10 +366,10 @@ void recip_rows_group(rp_ctx *ctx, const std::vector<RecipRowsJob> &jobs, cudaSt
         build_w_kernel<<<g, 128, 0, stream>>>(L);
         RP_LAUNCH_CHECK();
         g = with(2);
-        recip_stage_a_kernel<<<g, 128, smem_a, stream>>>(L);
+        recip_stage_a_kernel<<<g, kRecipT, smem_a, stream>>>(L);
         RP_LAUNCH_CHECK();
         g = with(3);
-        recip_stage_b_kernel<<<g, 128, smem_b, stream>>>(L);
+        recip_stage_b_kernel<<<g, kRecipT, smem_b, stream>>>(L);
         RP_LAUNCH_CHECK();
     }
 }

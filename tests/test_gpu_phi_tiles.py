@@ -79,3 +79,15 @@ def test_phi_small_cell_overflows_the_image_table(n, gpu_ctx, oracle_mod):
         far &= (np.linalg.norm(p[:, None] - (atoms + s)[None], axis=2) > 1.0).all(axis=1)
     idx = idx[far]
     _check(_phi(gpu_ctx, cube, atoms, idx, 7), _reference(oracle_mod, cube, atoms, idx, 7))
+
+
+@pytest.mark.parametrize("kmax", [1, 2, 6, 12, 20])
+@pytest.mark.parametrize("n", [1, 17, 34])
+def test_phi_over_kmax(n, kmax, gpu_ctx, oracle_mod):
+    """The reciprocal rows' stages: columns of more entries than one CTA's slab, an odd and an even number
+    of columns, one n1, rows that are no multiple of eight."""
+    cube, g = load_golden("tricmini")
+    atoms = np.ascontiguousarray(cube.atom_pos[:n], dtype=np.float64)
+    idx = np.random.default_rng(kmax).permutation(cube.n_points)[:300].astype(np.int64)
+    idx = idx[g["mask"].ravel()[idx] != 0]
+    _check(_phi(gpu_ctx, cube, atoms, idx, kmax), _reference(oracle_mod, cube, atoms, idx, kmax))
