@@ -593,9 +593,13 @@ struct RecipRowsJob {
     const double *d_q;
     int N;
     float2 *E;
+    // kept points (count in device memory, both there once the group's event has passed): only grid
+    // rows near them are written to E; null: every row
+    const int32_t *kept = nullptr;
+    const long long *kept_count = nullptr;
 };
 void recip_rows_group(rp_ctx *ctx, const std::vector<RecipRowsJob> &jobs, cudaStream_t stream,
-                      const std::string &tag);
+                      const std::string &tag, cudaEvent_t kept_ready = nullptr);
 
 // Shared epilogue kernels (phi_fp64.cu).
 void column_sums_fp64(const double *X, int64_t rows, int cols, int ld, double *out, bool accumulate,

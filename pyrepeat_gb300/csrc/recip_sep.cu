@@ -49,6 +49,7 @@ struct RecipJob {
     int N, ncols, K, P, ny, nz, ab;
     int ea, ra;            // stage A: (n2, n1) entries and planes of a CTA
     int ecols;             // columns of E's rows (recip_cols)
+    const uint8_t *marks;  // [nz][ny / kJB, rounded up] whether stage B writes those rows, or null: all
 };
 constexpr int kRecipJobs = 64;
 struct RecipLaunch {
@@ -164,13 +165,14 @@ __device__ __forceinline__ void rows_load_table(float *cs, float *sn, int np, co
         sn[q] = y.z;
     }
 }
-// entry r is at f[off(r) + k fk]; rows r0 .. r0 + n of out, entries 0 .. an
-template <class Off>
-__device__ __forceinline__ void rows_product(const float2 *f, int fk, Off off, int an, const float *cs, const float *sn, int np,
+// entry r is at f[off(r) + k fk]; rows 0 .. n of out, of these the groups of kJB rows that group() lists,
+// entries 0 .. an
+template <class Off, class Group>
+__device__ __forceinline__ void rows_product(const float2 *f, int fk, Off off, int ngroups, Group group, int an, const float *cs, const float *sn, int np,
                                              int nk, int n, float2 *out, long long stride) {
-    const int half = (an + 1) >> 1, tasks = half * (np / kJB);
+    const int half = (an + 1) >> 1, tasks = half * ngroups;
     for (int task = threadIdx.x; task < tasks; task += kRecipT) {
-        const int jj = task / half, r = task - jj * half;
+        const int t = task / half, r = task - t * half, jj = group(t);
         const bool two = r + half < an;
         const float2 *fa = f + off(r), *fb = f + off(two ? r + half : r);
         const float *c = cs + jj * kJB, *s = sn + jj * kJB;
@@ -236,13 +238,24 @@ __global__ void __launch_bounds__(kRecipT) recip_stage_a_kernel(const __grid_con
         for (int r = threadIdx.x; r < an; r += kRecipT) f[k * an + r] = w[k * ne + r];
     rows_load_table(cs, sn, np, J.EZ, nw, J.nz, l0, n);
     __syncthreads();
-    rows_product(f, an, [](int r) { return r; }, an, cs, sn, np, nw, n,
+    rows_product(f, an, [](int r) { return r; }, np / kJB, [](int t) { return t; }, an, cs, sn, np, nw, n,
                  J.F + ((long long)l0 * J.ncols + a) * ne + e0, (long long)J.ncols * ne);
+}
+
+// marks[l][j / kJB] = 1 for every kept point's row (j, l) (the host clears them)
+__global__ void recip_mark_kernel(const int32_t *__restrict__ kept, const long long *__restrict__ count, int nx, int ny,
+                                  uint8_t *__restrict__ marks) {
+    const int ng = (ny + kJB - 1) / kJB;
+    const long long M = *count;
+    for (long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x; m < M; m += (long long)gridDim.x * blockDim.x) {
+        const int row = kept[m] / nx, l = row / ny;
+        marks[(long long)l * ng + (row - l * ny) / kJB] = 1;
+    }
 }
 
 // Stage B, one CTA per (plane l, block of `ab` columns) of a job: the plane's F of those columns is one
 // contiguous slab [a][n2][n1].
-__global__ void __launch_bounds__(kRecipT) recip_stage_b_kernel(const __grid_constant__ RecipLaunch L) {
+__global__ void __launch_bounds__(kRecipT, 6) recip_stage_b_kernel(const __grid_constant__ RecipLaunch L) {
     extern __shared__ __align__(16) float smem_r[];
     const int jb = recip_job_of(L, blockIdx.x);
     const RecipJob &J = L.job[jb];
@@ -250,16 +263,29 @@ __global__ void __launch_bounds__(kRecipT) recip_stage_b_kernel(const __grid_con
     const int n1c = J.P + 1, nw = 2 * J.P + 1, ne = nw * n1c;
     const int nbx = (ncols + ab - 1) / ab, bloc = blockIdx.x - L.blk[jb];
     const int l = bloc / nbx, a0 = (bloc - l * nbx) * ab, na = min(ab, ncols - a0);
-    const int np = (ny + kJB - 1) / kJB * kJB;
+    const int np = (ny + kJB - 1) / kJB * kJB, ng = np / kJB;
     float *cs = smem_r, *sn = cs + nw * np;
     float2 *f = reinterpret_cast<float2 *>(sn + nw * np);
+    int *live = reinterpret_cast<int *>(f + na * ne), nlive = ng;  // the groups to write
+    if (J.marks) {
+        nlive = 0;
+        const uint8_t *m = J.marks + (long long)l * ng;
+        for (int t0 = 0; t0 < ng; t0 += 32) {  // (every warp forms the same list)
+            const int t = t0 + (threadIdx.x & 31);
+            const unsigned on = __ballot_sync(0xffffffffu, t < ng && m[t]);
+            if (on >> (threadIdx.x & 31) & 1) live[nlive + __popc(on & ((1u << (threadIdx.x & 31)) - 1))] = t;
+            nlive += __popc(on);
+        }
+        if (nlive == 0) return;
+    }
     const float2 *F = J.F + ((long long)l * ncols + a0) * ne;
 #pragma unroll 4
     for (int t = threadIdx.x; t < na * ne; t += kRecipT) f[t] = F[t];
     rows_load_table(cs, sn, np, J.EY, nw, ny, 0, ny);
     __syncthreads();
-    rows_product(f, n1c, [=](int r) { return r / n1c * ne + r % n1c; }, na * n1c, cs, sn, np, nw, ny,
-                 J.E + ((long long)l * ny * J.ecols + a0) * n1c, (long long)J.ecols * n1c);
+    const bool all = J.marks == nullptr;
+    rows_product(f, n1c, [=](int r) { return r / n1c * ne + r % n1c; }, nlive, [=](int t) { return all ? t : live[t]; },
+                 na * n1c, cs, sn, np, nw, ny, J.E + ((long long)l * ny * J.ecols + a0) * n1c, (long long)J.ecols * n1c);
 }
 
 // stage B's columns per CTA: as many as fit 24 KB of shared memory (at most 16)
@@ -269,7 +295,7 @@ int stage_b_columns(int P) {
 }
 size_t table_bytes(int P, int rows) { return sizeof(float2) * (size_t)(2 * P + 1) * ((rows + kJB - 1) / kJB * kJB); }
 size_t stage_b_smem(int P, int ny, int ab) {
-    return table_bytes(P, ny) + sizeof(float2) * (size_t)(2 * P + 1) * ab * (P + 1);
+    return table_bytes(P, ny) + sizeof(float2) * (size_t)(2 * P + 1) * ab * (P + 1) + sizeof(int) * ((ny + kJB - 1) / kJB);
 }
 
 }  // namespace
@@ -285,8 +311,15 @@ size_t recip_rows_bytes(const rp_ewald *ew, int ncols) {
 }
 
 void recip_rows_group(rp_ctx *ctx, const std::vector<RecipRowsJob> &jobs, cudaStream_t stream,
-                      const std::string &tag) {
+                      const std::string &tag, cudaEvent_t kept_ready) {
     if (jobs.empty()) return;
+    // marks of the jobs that write only the rows near kept points
+    std::vector<size_t> oM(jobs.size() + 1, 0);
+    for (size_t j = 0; j < jobs.size(); ++j) {
+        const int *g = jobs[j].ew->grid.n_grid;
+        oM[j + 1] = oM[j] + (jobs[j].kept && jobs[j].ew->K > 0 ? (size_t)g[2] * ceil_div(g[1], kJB) : 0);
+    }
+    uint8_t *marks = oM.back() ? ctx->buf_t<uint8_t>("rs_marks" + tag, oM.back()) : nullptr;
     // scratch of every job in one arena per kind; the W arena is cleared with one memset
     std::vector<size_t> oW(jobs.size() + 1, 0), oF(jobs.size() + 1, 0), oU(jobs.size() + 1, 0),
         oK(jobs.size() + 1, 0);
@@ -332,6 +365,7 @@ void recip_rows_group(rp_ctx *ctx, const std::vector<RecipRowsJob> &jobs, cudaSt
             J.EY = ew->d_eyf; J.EZ = ew->d_ezf;
             J.U = U + oU[j]; J.Udf = Udf + oU[j]; J.kdf = kdf + oK[j]; J.W = W + oW[j]; J.F = F + oF[j];
             J.E = rj.E;
+            J.marks = rj.kept ? marks + oM[j] : nullptr;
             for (int q = 0; q < 9; ++q) J.rb[q] = ew->rec[q];
             J.N = rj.N; J.ncols = ncols; J.K = ew->K; J.P = P; J.ny = ny; J.nz = nz; J.ab = stage_b_columns(P);
             J.ecols = rj.d_q ? 1 : recip_cols(ncols);
@@ -368,6 +402,16 @@ void recip_rows_group(rp_ctx *ctx, const std::vector<RecipRowsJob> &jobs, cudaSt
         g = with(2);
         recip_stage_a_kernel<<<g, kRecipT, smem_a, stream>>>(L);
         RP_LAUNCH_CHECK();
+        if (oM[j1] > oM[j0]) {
+            RP_CUDA(cudaStreamWaitEvent(stream, kept_ready, 0));
+            RP_CUDA(cudaMemsetAsync(marks + oM[j0], 0, oM[j1] - oM[j0], stream));
+            for (size_t j = j0; j < j1; ++j)
+                if (oM[j + 1] > oM[j]) {
+                    const int *n = jobs[j].ew->grid.n_grid;
+                    recip_mark_kernel<<<152, 256, 0, stream>>>(jobs[j].kept, jobs[j].kept_count, n[0], n[1], marks + oM[j]);
+                    RP_LAUNCH_CHECK();
+                }
+        }
         g = with(3);
         recip_stage_b_kernel<<<g, kRecipT, smem_b, stream>>>(L);
         RP_LAUNCH_CHECK();

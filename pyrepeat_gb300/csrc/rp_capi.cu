@@ -454,16 +454,38 @@ void batch_enqueue(rp_ctx *ctx, int n, const rp_fit_desc *descs, const double *c
         e_off[i + 1] = e_off[i] + (descs[i].precision == RP_PREC_MIXED
                                        ? recip_rows_bytes(r.ews[i], descs[i].N) / sizeof(float2) : 0);
     float2 *E_all = ctx->buf_t<float2>("fit_E", std::max<size_t>(e_off[n], 1));
+    // In a crowded cell the kept points sit in few pockets, and most grid rows hold none: stage B
+    // then waits for the filter and writes only the rows near kept points.  The line: the atoms' spheres
+    // together fill the cell 2.5 times over (3.8 to 4.0 in the MOF-like and triclinic cells, where
+    // 20 to 33 % of the groups of eight rows are needed; below 1.6 in cells of 90 Bohr^3 per atom, where
+    // 99 % are and the wait would cost what the filter takes).
+    auto crowded = [](const rp_fit_desc &d) {
+        const double *a = d.grid.axis;
+        double det = a[0] * (a[4] * a[8] - a[5] * a[7]) - a[1] * (a[3] * a[8] - a[5] * a[6]) + a[2] * (a[3] * a[7] - a[4] * a[6]);
+        det = std::fabs(det) * d.grid.n_grid[0] * d.grid.n_grid[1] * d.grid.n_grid[2];
+        double fill = 0.0;
+        for (int t = 0; t < d.N; ++t) {
+            const double rad = d.vdw_factor * rp::radius_of(d.Z[t]);
+            fill += 4.0 / 3.0 * M_PI * rad * rad * rad;
+        }
+        return fill >= 2.5 * det;
+    };
     std::vector<cudaEvent_t> rows_ready((size_t)ngroups);
     for (int g = 0; g < ngroups; ++g) {
         std::vector<rp::RecipRowsJob> rj;
         for (int i = g0[g]; i < g0[g + 1]; ++i)
-            if (descs[i].precision == RP_PREC_MIXED)
+            if (descs[i].precision == RP_PREC_MIXED) {
                 rj.push_back(rp::RecipRowsJob{r.ews[i], atoms_dev + 3 * off_n[i], nullptr, descs[i].N,
                                               E_all + e_off[i]});
+                // (the first group's filters are queued already, the others' are not)
+                if (g == 0 && crowded(descs[i])) {
+                    rj.back().kept = kept + off_pts[i];
+                    rj.back().kept_count = Md + i;
+                }
+            }
         {
             StageTimer tt(ctx, "recip_rows", recip_lane);
-            rp::recip_rows_group(ctx, rj, recip_lane, "#r" + std::to_string(g));
+            rp::recip_rows_group(ctx, rj, recip_lane, "#r" + std::to_string(g), kept_ready[0]);
         }
         rows_ready[g] = record(recip_lane);
     }

@@ -91,3 +91,24 @@ def test_phi_over_kmax(n, kmax, gpu_ctx, oracle_mod):
     idx = np.random.default_rng(kmax).permutation(cube.n_points)[:300].astype(np.int64)
     idx = idx[g["mask"].ravel()[idx] != 0]
     _check(_phi(gpu_ctx, cube, atoms, idx, kmax), _reference(oracle_mod, cube, atoms, idx, kmax))
+
+
+@pytest.mark.parametrize("n_grid,n_atoms", [((80, 85, 90), 300), ((96, 75, 64), 200), ((110, 121, 63), 420)])
+def test_fits_of_crowded_cells(n_grid, n_atoms, gpu_ctx):
+    """A batch writes only the grid rows near kept points in a crowded cell.  The mixed fit against the
+    FP64 fit of the same cube, after a fit of another cube has left its rows in the scratch, within
+    ten times the usual distance of the two (2e-11 kappa / (n + 1) e)."""
+    from pyrepeat_gb300 import _lib, synth
+    s = (n_atoms / 2000.0) ** (1 / 3)
+    cubes = [synth.make_tric(seed=k, n_grid=n_grid, n_atoms=n_atoms, n_groups=10,
+                             lengths=(40.0 * s, 42.0 * s, 45.0 * s), ctx=gpu_ctx) for k in (5, 6)]
+    gpu_ctx.set_kappa_limit(0.0)
+    try:
+        q = []
+        for c, prec in ((cubes[1], _lib.PREC_MIXED), (cubes[0], _lib.PREC_MIXED), (cubes[0], _lib.PREC_FP64)):
+            r, _, info = gpu_ctx.fit_batch([c], prec, V_dev=[c.V_dev] if c.V is None else None)
+            q.append(np.asarray(r[0]).copy())
+    finally:
+        gpu_ctx.set_kappa_limit(_lib.DEFAULT_KAPPA_LIMIT)
+    kappa = _lib.fit_info(info[0])["kappa"]
+    assert np.abs(q[1] - q[2]).max() <= max(1e-5, 2e-10 * kappa / (n_atoms + 1)) * max(1.0, np.abs(q[2]).max())
