@@ -1112,7 +1112,7 @@ __global__ void __launch_bounds__(256) lu_trsm_kernel(T *__restrict__ A, int n1,
 // Bounded by the panels' chain of latencies, about 1200 cycles per column (search, publish, pick,
 // update) and 5 us per panel of loads and stores; an update of 2001 x 2001 takes 8 us.  Half as many
 // barriers, eight columns at a time and panels wholly in line (their instruction fetch costs as
-// much) were no faster.  Measured: 7.8 -> 3.5 ms at 2001 unknowns, 2.3 -> 0.83 at 768, 3.6 -> 1.35 at
+// much) were no faster.  Measured: 7.8 -> 3.1 ms at 2001 unknowns, 2.3 -> 0.75 at 768, 3.6 -> 1.2 at
 // 1101 (against panels in shared memory with four barriers per column, interchanges on one CTA
 // and a cuBLAS rank-32 update).
 constexpr int kLUAcrossMax = 4096;
@@ -1132,6 +1132,30 @@ struct LuStep {
 //   The column loop is not unrolled (a whole panel in line is 60 KB of instructions run once, and
 //   their fetch took 0.7 us per column): column j is always register 0, and the update that
 //   leaves a row shifts it by one.  What is final of a row goes to shared memory on the way.
+// Launches of one factorisation or refinement overlap their start-up with the end of the kernel before
+// (programmatic dependent launch): each lets its successor begin when all its CTAs run, and waits
+// for its predecessor's end, and so for all before it, ahead of its first access to memory.
+// (A factorisation is two short launches per panel: 3.5 -> 3.1 ms at 2001 unknowns, 0.44 -> 0.38 at 425.)
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+void launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = dim3((unsigned)threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    RP_CUDA(cudaLaunchKernelEx(&c, kernel, P(args)...));
+    RP_LAUNCH_CHECK();
+}
+
 template <int R>
 __global__ void __launch_bounds__(kPanelT) lu_panel_across_kernel(LuStep p) {
     constexpr int NB = 64 / R, LD = NB + 1;
@@ -1142,6 +1166,7 @@ __global__ void __launch_bounds__(kPanelT) lu_panel_across_kernel(LuStep p) {
     const int tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
     const int n1 = p.n1, k0 = p.k0, nb = p.nb, m = n1 - k0;
     int *posr = reinterpret_cast<int *>(pst + (size_t)m * LD), *ids = posr + m;
+    chain_begin();
     if (k0 > 0 && p.pre[0] != 0.0) return;  // an earlier panel met a zero pivot
     const int sc = lane % NB, sr = warp * (32 / NB) + lane / NB, sn = nw * (32 / NB);  // staging: column, first row, step
     if (sc < nb)
@@ -1280,6 +1305,7 @@ __global__ void __launch_bounds__(256, 3) lu_update_across_kernel(LuStep p) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int r0 = c1 + blockIdx.y * kUpd, q0 = c1 + blockIdx.x * kUpd;  // the tile's rows and columns
     const int tr = (tid >> 4) * 4, tc = tid & 15;  // rows tr .. tr+3, columns tc + 16 i
+    chain_begin();
     const double flag = p.pre[0];
     const int top = lane < nb ? p.from[k0 + lane] : k0;
     int fr[4];
@@ -1353,6 +1379,7 @@ __global__ void __launch_bounds__(256, 3) lu_update_across_kernel(LuStep p) {
 
 __global__ void lu_collect_kernel(const float *__restrict__ F, const int *__restrict__ orig, int n1,
                                   const double *__restrict__ pre, float *__restrict__ LU) {
+    chain_begin();
     if (pre[0] != 0.0) return;
     const int i = blockIdx.x;
     const float *src = F + (size_t)orig[i] * n1;
@@ -1391,20 +1418,15 @@ void lu_factor_across(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string
         p.nb = std::min(NB, m);
         const int nt = (int)ceil_div(ceil_div(m, R), 32) * 32;
         const size_t smem = sizeof(float) * (size_t)m * (NB + 3);
-        if (R == 2) lu_panel_across_kernel<2><<<1, nt, smem, stream>>>(p);
-        else if (R == 4) lu_panel_across_kernel<4><<<1, nt, smem, stream>>>(p);
-        else lu_panel_across_kernel<8><<<1, nt, smem, stream>>>(p);
-        RP_LAUNCH_CHECK();
+        launch_chained(R == 2 ? lu_panel_across_kernel<2> : R == 4 ? lu_panel_across_kernel<4> : lu_panel_across_kernel<8>, dim3(1), nt, smem,
+                       stream, p);
         k0 += p.nb;
         if (k0 < n1) {
             const unsigned t = ceil_div(n1 - k0, kUpd);
-            if (n1 >= kLUWideMin) lu_update_across_kernel<true><<<dim3(t, t), 256, 0, stream>>>(p);
-            else lu_update_across_kernel<false><<<dim3(t, t), 256, 0, stream>>>(p);
-            RP_LAUNCH_CHECK();
+            launch_chained(n1 >= kLUWideMin ? lu_update_across_kernel<true> : lu_update_across_kernel<false>, dim3(t, t), 256, 0, stream, p);
         }
     }
-    lu_collect_kernel<<<n1, 256, 0, stream>>>(p.F, d.perm, n1, d.pre, buf[0]);
-    RP_LAUNCH_CHECK();
+    launch_chained(lu_collect_kernel, dim3(n1), 256, 0, stream, p.F, d.perm, n1, d.pre, buf[0]);
 }
 
 // dynamic shared memory of lu_solve_refine_kernel: the right-hand side, the correction and the row
@@ -1688,6 +1710,7 @@ constexpr int kInvLD = kAcB + 4, kInvCols = 64, kInvT = 4 * kInvCols;  // blockI
 __global__ void __launch_bounds__(kInvT) across_invert_kernel(AcrossRun p) {
     extern __shared__ __align__(16) float ash[];
     float *B = ash, *dinv = ash + kAcB * kInvLD;  // B[k][i]: column k below the diagonal
+    chain_begin();
     if (p.d.pre[0] != 0.0) return;
     const int n1 = p.n1, b0 = blockIdx.x * kAcB, tid = threadIdx.x, lane = tid & 31, c = blockIdx.z * kInvCols + (tid >> 2), q = tid & 3;
     const bool rev = blockIdx.y == 1;
@@ -1740,6 +1763,7 @@ __global__ void __launch_bounds__(1024) across_control_kernel(AcrossRun p, int r
     __shared__ int si[32], piv_i;
     __shared__ AcrossState st;
     const int tid = threadIdx.x, n1 = p.n1, nt = blockDim.x;
+    chain_begin();
     if (tid == 0) st = *p.st;
     __syncthreads();
     if (st.finished) return;
@@ -1888,6 +1912,7 @@ __global__ void __cluster_dims__(kAcCTAs, 1, 1) __launch_bounds__(kAcT) across_a
     float *wb = ash + (size_t)p.nblk * kAcB * NS;       // [2][128][NS] the block's rows
     float *rb = wb + 2 * kAcB * NS;                     // [128][NS] what they leave
     cg::cluster_group cl = cg::this_cluster();
+    chain_begin();
     if (p.st->finished) return;  // (the same for the whole cluster)
     const int rank = (int)cl.block_rank(), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n1 = p.n1, nblk = p.nblk, rl = rank * (kAcB / kAcCTAs) + warp;  // the warp's row of each block
@@ -2004,6 +2029,7 @@ __global__ void __cluster_dims__(kAcCTAs, 1, 1) __launch_bounds__(kAcT) across_a
 __global__ void __launch_bounds__(256) across_residual_kernel(AcrossRun p, int round) {
     extern __shared__ double xd[];
     __shared__ unsigned long long top[2];
+    chain_begin();
     if (p.st->finished || p.st->phase != 0) return;
     const int n1 = p.n1, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const double rm = p.st->rm, *xo = p.x[round & 1];
@@ -2062,10 +2088,8 @@ void refine_across(rp_ctx *ctx, const SolveDesc &d, int n1, int first, int round
         RP_LAUNCH_CHECK();
         const size_t inv_smem = sizeof(float) * (kAcB * kInvLD + kAcB);
         smem_optin((const void *)across_invert_kernel, inv_smem);
-        across_invert_kernel<<<dim3(p.nblk, 2, kAcB / kInvCols), kInvT, inv_smem, stream>>>(p);
-        RP_LAUNCH_CHECK();
-        across_control_kernel<<<1, 1024, 0, stream>>>(p, 0, 0);
-        RP_LAUNCH_CHECK();
+        launch_chained(across_invert_kernel, dim3(p.nblk, 2, kAcB / kInvCols), kInvT, inv_smem, stream, p);
+        launch_chained(across_control_kernel, dim3(1), 1024, 0, stream, p, 0, 0);
     }
     const size_t np = (size_t)p.nblk * kAcB, res_smem = sizeof(double) * n1;
     const size_t most = sizeof(float) * 4 * (((size_t)kLUWideMax + kAcB - 1) / kAcB * kAcB + 3 * kAcB);
@@ -2073,13 +2097,10 @@ void refine_across(rp_ctx *ctx, const SolveDesc &d, int n1, int first, int round
     smem_optin((const void *)across_apply_kernel<2>, most / 2);
     smem_optin((const void *)across_residual_kernel, sizeof(double) * kLUWideMax);
     for (int k = first; k < first + rounds; ++k) {
-        if (k == 0) across_apply_kernel<3><<<kAcCTAs, kAcT, sizeof(float) * 4 * (np + 3 * kAcB), stream>>>(p);
-        else across_apply_kernel<2><<<kAcCTAs, kAcT, sizeof(float) * 2 * (np + 3 * kAcB), stream>>>(p);
-        RP_LAUNCH_CHECK();
-        across_residual_kernel<<<(int)std::min<long long>(ceil_div(n1, 8), 304), 256, res_smem, stream>>>(p, k);
-        RP_LAUNCH_CHECK();
-        across_control_kernel<<<1, 1024, 0, stream>>>(p, k + 1, k + 1 == first + rounds);
-        RP_LAUNCH_CHECK();
+        if (k == 0) launch_chained(across_apply_kernel<3>, dim3(kAcCTAs), kAcT, sizeof(float) * 4 * (np + 3 * kAcB), stream, p);
+        else launch_chained(across_apply_kernel<2>, dim3(kAcCTAs), kAcT, sizeof(float) * 2 * (np + 3 * kAcB), stream, p);
+        launch_chained(across_residual_kernel, dim3((unsigned)std::min<long long>(ceil_div(n1, 8), 304)), 256, res_smem, stream, p, k);
+        launch_chained(across_control_kernel, dim3(1), 1024, 0, stream, p, k + 1, (int)(k + 1 == first + rounds));
     }
 }
 
@@ -2416,8 +2437,8 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         }
         if (plans[j].disjoint) disjoint.push_back(j);
     }
-    // One system of kLUHost64Min unknowns or more is solved across the GPU (0.44 + 0.31 ms at 425
-    // unknowns, factors and refinement, against 0.74 + 0.70 in one CTA; 0.76 + 0.4 against 2.0 + 1.4
+    // One system of kLUHost64Min unknowns or more is solved across the GPU (0.38 + 0.29 ms at 425
+    // unknowns, factors and refinement, against 0.74 + 0.70 in one CTA; 0.68 + 0.4 against 2.0 + 1.4
     // at 720), two of them one after the other from kAcrossTwo; more run side by side, each in its CTA.
     int mid = 0, least = kLUWideMin;
     for (int j = 0; j < nj; ++j)
