@@ -1661,12 +1661,13 @@ constexpr int kAcB = 128;     // unknowns of a block, whose diagonal blocks of L
 constexpr int kAcCTAs = 8;    // CTAs of the cluster, 16 rows of each block each
 constexpr int kAcT = 512;     // their threads
 constexpr int kAcRounds = 6;  // rounds launched ahead of a look at the outcome
-// A step that leaves more than this share of the residual: the solution that three such steps
-// give then depends at the tenth digit on how the triangular solves round, and the system goes
-// to substitution.  (Shares of 1e-6 to 3.6e-4 at fits and QEq systems of 260 to 2001 unknowns of
-// ordinary cells, whose charges agree with substitution's to 3e-10; 6.8e-4 to 2.5e-3 at dense cells
-// of 830 to 920, where they differ by 1e-9 to 1e-7.)
-constexpr double kInvRate = 4e-4;
+// When a system goes to substitution instead.  What the last correction leaves of itself, its largest
+// element times the rate at which the residual fell, says how far the solution still depends on
+// how the triangular solves round: at 3 steps the charges differ from substitution's by up to 4 times
+// that (1e-10 to 2e-10 at the triclinic cells' 2e-11 to 1.4e-10, 3.5e-10 to 7.6e-8 at 4e-10 to 2e-7 of
+// dense cells of 830 to 920 unknowns), at 2 steps by up to 0.45 times (QEq systems of 479 to 2001).
+constexpr double kInvLeft2 = 1e-9, kInvLeft = 2e-10;
+constexpr double kInvRate = 1e-2;  // a slower system is not waited for
 
 struct AcrossState {
     unsigned long long an_bits, anorm_bits;  // max row sums of |K| and of |A|
@@ -1790,6 +1791,11 @@ __global__ void __launch_bounds__(1024) across_control_kernel(AcrossRun p, int r
             p.V[2 * (size_t)n1 + t] = (float)(((t & 1) ? -1.0 : 1.0) * (1.0 + (double)t / (double)max(n1 - 1, 1)));
         }
     } else {
+        double ym = 0.0;  // the correction's largest element, in units of rm
+        if (st.phase == 0) {
+            for (int t = tid; t < n1; t += nt) ym = fmax(ym, fabs((double)p.Y[t]));
+            ym = block_max(ym, n1, sv);
+        }
         if (tid == 0 && st.phase == 0) {
             const double rn = __longlong_as_double((long long)st.rn_bits), xn = __longlong_as_double((long long)st.xn_bits),
                          an = __longlong_as_double((long long)st.an_bits);
@@ -1805,8 +1811,9 @@ __global__ void __launch_bounds__(1024) across_control_kernel(AcrossRun p, int r
                 ++st.steps;
                 st.xsel = round & 1;
                 if (rn <= (double)n1 * 1.1102230246251565e-16 * an * xn) {
+                    // (ym st.rm the correction, rn / st.rm the rate)
                     if (p.d.refit && rn > 0.0) st.extra = 1;
-                    else st.phase = 1;
+                    else st.phase = p.d.refit || !(ym * rn > (st.steps <= 2 ? kInvLeft2 : kInvLeft) * xn) ? 1 : 2;
                 } else if (!(rn < 1e300) || (st.steps >= 2 && rn > kInvRate * st.rprev)) {
                     st.phase = 2;  // substitution takes over
                 }
@@ -2105,7 +2112,7 @@ void refine_across(rp_ctx *ctx, const SolveDesc &d, int n1, int first, int round
 }
 
 // ---- the same by substitution, driven by the host
-// For a wide system that converges too slowly for the inverted blocks (kInvRate): cuBLAS STRSV
+// For a system that the inverted blocks leave too far from it (kInvLeft, kInvRate): cuBLAS STRSV
 // solves and DGEMV residuals across the GPU, a look at the outcome after each step.  Returns
 // false when the refinement stalls: the caller then factors the system in FP64
 // (factor_refine_wide64).  Waits.
