@@ -401,8 +401,8 @@ def qeq_cell(n_atoms: int, seed: int):
 
 def qeq_arm(args, world, rank, local):
     """QEq charges (repeat.py:2539-2634) of one periodic cell per step through rp_qeq, from
-    host atoms and parameters to host charges: the Coulomb matrix (per-atom k tables, one
-    FP64 DGEMM, the real-space pair kernel over all 27+ images) and the equalisation solve.
+    host atoms and parameters to host charges: the Coulomb matrix (per-atom k tables, their
+    exact Gram, the real-space pair kernel over all 27+ images) and the equalisation solve.
     CPU baseline: the oracle's NumPy Coulomb matrix on a bounded block of rows,
     extrapolated in pairs, plus its full solve."""
     import torch
