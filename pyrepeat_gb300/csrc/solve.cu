@@ -1390,6 +1390,12 @@ __global__ void iota_kernel(int *__restrict__ v, int n) {
     if (t < n) v[t] = t;
 }
 
+// Whether a system is factored across the GPU: its size, and room in the scratch budget for the factors by
+// input row (a quarter of what the system holds already; without it, panels in shared memory or
+// the system's CTA as before)
+bool across_fits(rp_ctx *ctx, int n1, const std::string &tag) {
+    return n1 <= kLUAcrossMax && ctx->fits("s_luF" + tag, sizeof(float) * ((size_t)n1 * n1 + 64 * (size_t)n1 + (1 << 20)));
+}
 // The FP32 matrix is in the first half of d.As, the second half is the other buffer.
 void lu_factor_across(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &tag, cudaStream_t stream) {
     float *buf[2] = {reinterpret_cast<float *>(d.As), reinterpret_cast<float *>(d.As) + (size_t)n1 * n1};
@@ -2083,8 +2089,13 @@ void refine_across(rp_ctx *ctx, const SolveDesc &d, int n1, int first, int round
     p.nblk = (int)ceil_div(n1, kAcB);
     p.LU = reinterpret_cast<const float *>(d.As);
     p.d = d;
-    p.inv = ctx->buf_t<float>("s_ac_inv" + key, 4 * (size_t)p.nblk * kAcB * kAcB);
-    p.V = ctx->buf_t<float>("s_ac_V" + key, 6 * (size_t)n1);
+    // inverses, blocks and vectors go to the second half of As, which is free once the factors are
+    // collected, where they fit there
+    const size_t need = sizeof(float) * (4 * (size_t)p.nblk * kAcB * kAcB + 6 * (size_t)n1), half = sizeof(float) * (size_t)n1 * n1;
+    const uintptr_t free_half = (reinterpret_cast<uintptr_t>(p.LU) + half + 255) & ~(uintptr_t)255;
+    p.inv = need + 255 <= half ? reinterpret_cast<float *>(free_half)
+                               : static_cast<float *>(ctx->buf("s_ac_inv" + key, need));
+    p.V = p.inv + 4 * (size_t)p.nblk * kAcB * kAcB;
     p.Y = p.V + 3 * (size_t)n1;
     p.x[0] = d.x;
     p.x[1] = ctx->buf_t<double>("s_ac_x" + key, (size_t)n1);
@@ -2227,7 +2238,7 @@ void lu_wide_factor(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &
     const long long nn = (long long)n1 * n1;
     lu_copy_kernel<T><<<(int)std::min<long long>(ceil_div(nn, 256), 4096), 256, 0, stream>>>(d.A0, L, nn, d.pre);
     RP_LAUNCH_CHECK();
-    if (n1 <= kLUAcrossMax) {
+    if (across_fits(ctx, n1, tag)) {
         lu_factor_across(ctx, d, n1, tag, stream);
         return;
     }
@@ -2455,7 +2466,7 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         }
     if (mid == 1 || (mid == 2 && least >= kAcrossTwo))
         for (int j = 0; j < nj; ++j)
-            if (descs[j].host64) {
+            if (descs[j].host64 && across_fits(ctx, plans[j].n + 1, tag)) {
                 descs[j].host64 = 0;
                 descs[j].host32 = 1;
             }

@@ -121,3 +121,19 @@ def test_slow_refinement(N, gpu_ctx):
         q, info = gpu_ctx.solve(torch.from_numpy(A).cuda(), torch.from_numpy(b).cuda(), np.full(N, 6), qtot=0.0)
         tol = max(1e-12, 1e-15 * np.linalg.cond(K) * (N + 1))
         assert np.abs(q.cpu().numpy() - ref).max() <= tol * max(1.0, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("N", [400, 900])
+def test_solve_within_a_tight_scratch_budget(N):
+    """Room for the system and its copy, not for the factors' extra buffer: solved by the ways that need none."""
+    import torch
+    from pyrepeat_gb300.fit import Context
+    rng = np.random.default_rng(N)
+    X = rng.normal(size=(3 * N, N))
+    A = X.T @ X / (3 * N)
+    b = rng.normal(size=N)
+    K, ref = _reference(A, b, 0.5)
+    ctx = Context(0, hbm_budget=16 * (N + 1) ** 2 + (2 << 20))
+    q, _ = ctx.solve(torch.from_numpy(A).cuda(), torch.from_numpy(b).cuda(), np.full(N, 6), qtot=0.5)
+    tol = max(1e-12, 1e-15 * np.linalg.cond(K) * (N + 1))
+    assert np.abs(q.cpu().numpy() - ref).max() <= tol * max(1.0, np.abs(ref).max())
