@@ -1112,7 +1112,7 @@ __global__ void __launch_bounds__(256) lu_trsm_kernel(T *__restrict__ A, int n1,
 // Bounded by the panels' chain of latencies, about 1200 cycles per column (search, publish, pick,
 // update) and 5 us per panel of loads and stores; an update of 2001 x 2001 takes 8 us.  Half as many
 // barriers, eight columns at a time and panels wholly in line (their instruction fetch costs as
-// much) were no faster.  Measured: 7.8 -> 3.1 ms at 2001 unknowns, 2.3 -> 0.75 at 768, 3.6 -> 1.2 at
+// much) were no faster.  Measured: 7.8 -> 2.9 ms at 2001 unknowns, 2.3 -> 0.68 at 768, 3.6 -> 1.1 at
 // 1101 (against panels in shared memory with four barriers per column, interchanges on one CTA
 // and a cuBLAS rank-32 update).
 constexpr int kLUAcrossMax = 4096;
@@ -1248,7 +1248,10 @@ __global__ void __launch_bounds__(kPanelT) lu_panel_across_kernel(LuStep p) {
             at = at_[b][w];
             pmin = fminf(pmin, apv);
             pmax = fmaxf(pmax, apv);
-            const float inv = prow[0];
+            float4 pv[NB / 4];  // the pivot row, by vector loads (word by word: 3.1 ms at 2001 unknowns)
+#pragma unroll
+            for (int c = 0; c < W / 4; ++c) pv[c] = reinterpret_cast<const float4 *>(prow)[c];
+            const float inv = pv[0].x;
             float l[R];
 #pragma unroll
             for (int q = 0; q < R; ++q) {
@@ -1259,7 +1262,8 @@ __global__ void __launch_bounds__(kPanelT) lu_panel_across_kernel(LuStep p) {
             }
 #pragma unroll
             for (int c = 1; c < W; ++c) {  // (rows that are done take part: nothing reads them again)
-                const float pc = prow[c];
+                const float4 &v4 = pv[c / 4];
+                const float pc = c % 4 == 0 ? v4.x : c % 4 == 1 ? v4.y : c % 4 == 2 ? v4.z : v4.w;
 #pragma unroll
                 for (int q = 0; q < R; ++q) a[q][c - 1] = fmaf(-l[q], pc, a[q][c]);
             }
@@ -2455,8 +2459,8 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         }
         if (plans[j].disjoint) disjoint.push_back(j);
     }
-    // One system of kLUHost64Min unknowns or more is solved across the GPU (0.38 + 0.29 ms at 425
-    // unknowns, factors and refinement, against 0.74 + 0.70 in one CTA; 0.68 + 0.4 against 2.0 + 1.4
+    // One system of kLUHost64Min unknowns or more is solved across the GPU (0.34 + 0.29 ms at 425
+    // unknowns, factors and refinement, against 0.74 + 0.70 in one CTA; 0.62 + 0.4 against 2.0 + 1.4
     // at 720), two of them one after the other from kAcrossTwo; more run side by side, each in its CTA.
     int mid = 0, least = kLUWideMin;
     for (int j = 0; j < nj; ++j)
