@@ -1965,7 +1965,10 @@ __global__ void __cluster_dims__(kAcCTAs, 1, 1) __launch_bounds__(kAcT) across_a
         for (int q = 0; q < NR; ++q) acc[q] = 0.f;
 #pragma unroll 1
         for (int s = 0; s < nblk; ++s) {
-            const int b = dir ? nblk - 1 - s : s, nb_ = dir ? b - 1 : b + 1, buf = s & 1;
+            // (the buffers take turns over both sweeps: with an odd number of blocks, turns counted per
+            // sweep would let a CTA that is ahead write the second sweep's first rows over the first's
+            // last ones while another still reads them)
+            const int b = dir ? nblk - 1 - s : s, nb_ = dir ? b - 1 : b + 1, buf = (dir * nblk + s) & 1;
             // this block's rows, to every CTA
 #pragma unroll
             for (int q = 0; q < NR; ++q) {

@@ -107,6 +107,30 @@ def test_refinement_across_the_gpu(N, gpu_ctx):
     assert info["residual"] <= 2 * (N + 1) * 2.0**-53 * np.abs(K).sum(axis=0).max() * xmax
 
 
+@pytest.mark.parametrize("N", [769, 830, 895, 1025, 1100, 1151, 1281])
+def test_repeated_solves_agree_on_a_busy_gpu(N, gpu_ctx):
+    """Odd numbers of 128-unknown blocks, whose two sweeps meet in one exchange buffer: charges and kappa of
+    repeated solves are the same bits while another stream keeps the SMs busy."""
+    import torch
+    rng = np.random.default_rng(N)
+    X = rng.normal(size=(2 * N, N))
+    A = torch.from_numpy(X.T @ X / (2 * N)).cuda()
+    b = torch.from_numpy(rng.normal(size=N)).cuda()
+    side = torch.cuda.Stream()
+    a = torch.rand(1 << 22, device="cuda")
+    m = torch.rand(1536, 1536, device="cuda")
+    seen = []
+    for rep in range(12):
+        with torch.cuda.stream(side):
+            for _ in range(4 * (rep % 4)):
+                a = a * 0.999 + 0.001
+                m = (m @ m).clamp_(0.0, 1.0)
+        q, info = gpu_ctx.solve(A, b, np.full(N, 6), qtot=0.5)
+        seen.append((q.cpu().numpy().tobytes(), info["kappa"]))
+    torch.cuda.synchronize()
+    assert len(set(seen)) == 1
+
+
 @pytest.mark.parametrize("N", [400, 900])
 def test_slow_refinement(N, gpu_ctx):
     """kappa towards 1/eps32: refinement with inverted blocks, by substitution, and FP64 factors."""
