@@ -2222,9 +2222,12 @@ bool refine_wide32(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &k
     return true;
 }
 
-// interchanges in order (perm[k]: the row that came to k) to a row order, in place; one CTA
-__global__ void __launch_bounds__(1024) order_of_swaps_kernel(int *__restrict__ perm, int n) {
+// interchanges in order (perm[k]: the row that came to k) to a row order, in place; one CTA.  After a
+// zero pivot the later panels wrote no interchanges: nothing is read then.
+__global__ void __launch_bounds__(1024) order_of_swaps_kernel(int *__restrict__ perm, int n,
+                                                              const double *__restrict__ pre) {
     extern __shared__ int osm[];  // [n] interchanges, [n] order
+    if (pre[0] != 0.0) return;
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
         osm[t] = perm[t];
         osm[n + t] = t;
@@ -2273,7 +2276,7 @@ void lu_wide_factor(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &
         k0 = c1;
     }
     smem_optin((const void *)order_of_swaps_kernel, 2 * sizeof(int) * kLUWideMax);
-    order_of_swaps_kernel<<<1, 1024, 2 * sizeof(int) * (size_t)n1, stream>>>(d.perm, n1);
+    order_of_swaps_kernel<<<1, 1024, 2 * sizeof(int) * (size_t)n1, stream>>>(d.perm, n1, d.pre);
     RP_LAUNCH_CHECK();
 }
 

@@ -85,6 +85,32 @@ def test_singular_systems_across_the_gpu(N, gpu_ctx):
     assert info["kappa"] > 1e12
 
 
+@pytest.mark.parametrize("where", [5, 2000, 4190])
+def test_zero_pivot_in_the_panels_beyond_the_register_panels(where, gpu_ctx):
+    """Two atoms without any normal-equation entries leave an exactly zero pivot, here in the first, a middle
+    and the last panel of a system factored by panels in shared memory, whose later panels then write no
+    interchanges: reported singular, and the context solves the next system."""
+    import torch
+    from pyrepeat_gb300 import _lib
+    N = 4200
+    g = torch.Generator(device="cuda").manual_seed(where)
+    A = torch.randn(N, N, generator=g, dtype=torch.float64, device="cuda") / N
+    A = A + A.T + 10.0 * torch.eye(N, dtype=torch.float64, device="cuda")  # (the border is no pivot but theirs)
+    good = A.clone()
+    for i in (where, where + 3):
+        A[i, :] = 0.0
+        A[:, i] = 0.0
+    b = torch.randn(N, generator=g, dtype=torch.float64, device="cuda")
+    with pytest.raises(_lib.RepeatError):
+        gpu_ctx.solve(A, b, np.full(N, 6))
+    q, _ = gpu_ctx.solve(good, b, np.full(N, 6))
+    K = torch.ones(N + 1, N + 1, dtype=torch.float64, device="cuda")
+    K[:N, :N] = good
+    K[N, N] = 0.0
+    ref = torch.linalg.solve(K, torch.cat([b, b.new_zeros(1)]))[:N]
+    assert float((q - ref).abs().max()) <= 1e-10 * float(ref.abs().max())
+
+
 @pytest.mark.parametrize("N", [255, 382, 383, 384, 511, 766, 1151, 1152])
 def test_refinement_across_the_gpu(N, gpu_ctx):
     """One system refined across the GPU, at the edges of its 128-unknown blocks, for a matrix whose
