@@ -529,13 +529,8 @@ struct SolveJob {
     const double *resp_s, *resp_t;
     double qtot;
     double *q;
-    int refit = 0;  // an escalated fit's system: 1 FP32 factors and refinement beyond convergence, 2 FP64
-                    // factors at once
+    bool fp64 = false;  // an escalated fit's system: FP64 factors at once where they come from across the GPU
 };
-// The largest kappa of an escalated fit's system that is refined with FP32 factors (refit = 1).  A step
-// then leaves 1.5e-10 kappa of the residual (1e-4 at 6.8e5, 3.6e-4 at 2.1e6, 1e-3 at 9.2e6): three and
-// the extra one reach what FP64 factors do, in 1.2 ms instead of 6.3 at 710 unknowns.
-constexpr double kRefitKappa32 = 2e6;
 void solve_batch(rp_ctx *ctx, const std::vector<SolveJob> &jobs, std::vector<double> &info, cudaStream_t stream);
 // One bordered system of the solve kernel (device-side descriptor).
 struct SolveDesc {
@@ -559,7 +554,6 @@ struct SolveDesc {
     double *info;         // kSolveInfo out: residual inf-norm, min|piv|, max|piv|, singular flag,
                           // kappa, unknowns n+1, refinement steps, factorisation path
     double *pre;          // null, or {flag, min|piv|, max|piv|} of a wide factorisation already in As
-    int refit;            // SolveJob's
     int wide64;           // As holds wide FP64 factors: skip the FP32 stage and the in-CTA FP64 LU
     int host64;           // FP32 factors in the CTA, but a stalled refinement goes to the host's FP64
                           // factorisation across the GPU (pre holds its flag) instead of an in-CTA FP64 LU

@@ -584,8 +584,7 @@ void batch_complete(rp_ctx *ctx, BatchRun &r) {
         std::vector<rp::SolveJob> jobs;
         for (int i : cubes) {
             jobs.push_back(r.job(i));
-            if (flag == RP_FIT_ESCALATED)  // refined to the end, or FP64 factors at once, by its mixed fit's kappa
-                jobs.back().refit = info[(size_t)W * i + 4] <= rp::kRefitKappa32 ? 1 : 2;
+            jobs.back().fp64 = flag == RP_FIT_ESCALATED;  // known to be ill-conditioned
         }
         std::vector<double> rinfo;
         rp::solve_batch(ctx, jobs, rinfo, stream);

@@ -1658,9 +1658,6 @@ void factor_refine_wide64(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t 
 //                           for Hager's estimate, and the next right-hand sides;
 //   across_apply_kernel     (P L U)^-1 of all of them at once, in one cluster;
 //   across_residual_kernel  x += correction and r = bs - A0 x in FP64, rows over the GPU.
-// An escalated fit's system (SolveJob::refit = 1) gets one correction beyond convergence, kept when
-// the residual falls: FP64's accuracy from FP32 factors (charges 2.1e-12 from 64 bits either way, 1.2 ms
-// instead of getrf's 3.9 and its refinement's 2.4 at 710 unknowns).
 // The refinement, the estimate and its extra test vector do not depend on one another, so
 // round k carries correction k, the estimate's vector k and (round 0) the extra vector: four
 // rounds instead of eight triangular solves one after the other.
@@ -1685,7 +1682,6 @@ struct AcrossState {
     double rm, rprev, res, est, alt;
     int steps, phase;       // phase 0: refining, 1: converged, 2: left to substitution, 3: zero pivot
     int hstate, hit, jprev, jcur;  // 0: uniform vector under way, 1: signs, 2: a unit vector, 3: estimate done
-    int extra;              // a refit: the correction beyond convergence is under way
     int xsel, finished;     // which x holds the solution; nothing left to do
 };
 struct AcrossRun {
@@ -1791,7 +1787,7 @@ __global__ void __launch_bounds__(1024) across_control_kernel(AcrossRun p, int r
             st.rm = m;
             st.rprev = 1e308;
             st.res = 0.0;
-            st.steps = st.hit = st.hstate = st.xsel = st.extra = 0;
+            st.steps = st.hit = st.hstate = st.xsel = 0;
             st.jprev = -1;
             st.est = st.alt = 0.0;
             st.phase = p.d.pre[0] != 0.0 ? 3 : m == 0.0 ? 1 : 0;
@@ -1809,24 +1805,14 @@ __global__ void __launch_bounds__(1024) across_control_kernel(AcrossRun p, int r
         if (tid == 0 && st.phase == 0) {
             const double rn = __longlong_as_double((long long)st.rn_bits), xn = __longlong_as_double((long long)st.xn_bits),
                          an = __longlong_as_double((long long)st.an_bits);
-            if (st.extra) {  // kept if the residual fell
-                if (rn < st.res) {
-                    st.res = rn;
-                    ++st.steps;
-                    st.xsel = round & 1;
-                }
-                st.phase = 1;
-            } else {
-                st.res = rn;
-                ++st.steps;
-                st.xsel = round & 1;
-                if (rn <= (double)n1 * 1.1102230246251565e-16 * an * xn) {
-                    // (ym st.rm the correction, rn / st.rm the rate)
-                    if (p.d.refit && rn > 0.0) st.extra = 1;
-                    else st.phase = p.d.refit || !(ym * rn > (st.steps <= 2 ? kInvLeft2 : kInvLeft) * xn) ? 1 : 2;
-                } else if (!(rn < 1e300) || (st.steps >= 2 && rn > kInvRate * st.rprev)) {
-                    st.phase = 2;  // substitution takes over
-                }
+            st.res = rn;
+            ++st.steps;
+            st.xsel = round & 1;
+            if (rn <= (double)n1 * 1.1102230246251565e-16 * an * xn) {
+                // (ym st.rm the correction, rn / st.rm the rate)
+                st.phase = !(ym * rn > (st.steps <= 2 ? kInvLeft2 : kInvLeft) * xn) ? 1 : 2;
+            } else if (!(rn < 1e300) || (st.steps >= 2 && rn > kInvRate * st.rprev)) {
+                st.phase = 2;  // substitution takes over
             }
             st.rprev = st.rm = rn;
         }
@@ -2445,7 +2431,6 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         d.resp_s = J.resp_s ? d_rs + o_red : nullptr; d.resp_t = J.resp_s ? d_rt + o_red : nullptr;
         d.map = d_map + o_map; d.qtot = J.qtot;
         d.As = As + o_sq; d.A0 = A0 + o_sq; d.bs = bs + o_red; d.x = x + o_red; d.r = r + o_red;
-        d.refit = J.refit;
         d.perm = perm + o_red; d.q = J.q; d.info = d_info + kSolveInfo * (size_t)j;
         o_map += J.N;
         o_mptr += p.mem_ptr.size();
@@ -2459,8 +2444,8 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         const int n1 = plans[j].n + 1;
         if (n1 >= kLUHost64Min && n1 <= kLUWideMax) {
             descs[j].pre = d_pre + 3 * (size_t)j;
-            if (jobs[j].refit == 2) descs[j].wide64 = 1;
-            else if (jobs[j].refit == 1 || n1 >= kLUWideMin) descs[j].host32 = 1;
+            if (jobs[j].fp64) descs[j].wide64 = 1;
+            else if (n1 >= kLUWideMin) descs[j].host32 = 1;
             else descs[j].host64 = 1;
         }
         if (plans[j].disjoint) disjoint.push_back(j);
@@ -2618,7 +2603,7 @@ void solve_wide_fp64(rp_ctx *ctx, SolvePending &pd, cudaStream_t stream) {
             RP_CUDA(cudaStreamSynchronize(stream));
         }
         if (flag == 0.0) continue;
-        if (flag == 4.0 && pd.descs[j].refit == 0) {  // by substitution
+        if (flag == 4.0) {  // by substitution
             if (pd.n1[j] >= kLUWideMin) {
                 if (refine_wide32(ctx, pd.descs[j], pd.n1[j], pd.tag + "#" + std::to_string(j), stream)) continue;
             } else {

@@ -190,3 +190,21 @@ def test_escalated_fits_by_kappa_and_size(n_atoms, gpu_ctx):
     assert einfo["escalated"] and M == Me
     n1 = n_atoms + 1
     assert np.abs(q - ref).max() <= 4 * n1 * 2.0**-53 * info["kappa"] * max(1.0, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("n_atoms", [430, 700])
+def test_every_escalated_system_gets_fp64_factors(n_atoms, gpu_ctx):
+    """Whatever its kappa: a system that FP32 factors would solve too (below 2e6, by RESP on every element), sent
+    to FP64 by a low limit."""
+    from pyrepeat_gb300 import _lib, synth
+    cube = synth.make_tric(seed=n_atoms, n_grid=(72, 70, 75), n_atoms=n_atoms, ctx=gpu_ctx)
+    cube.symm_groups = None
+    cube.resp = {s: (0.1, 0.0) for s in ("H", "C", "N", "O", "S", "Zn")}
+    _, _, info = _batch(gpu_ctx, cube, _lib.PREC_MIXED)
+    assert not info["escalated"] and info["kappa"] < 2e6
+    gpu_ctx.set_kappa_limit(1e-3)
+    try:
+        _, _, einfo = _batch(gpu_ctx, cube, _lib.PREC_MIXED)
+    finally:
+        gpu_ctx.set_kappa_limit(_lib.DEFAULT_KAPPA_LIMIT)
+    assert einfo["escalated"] and einfo["solve_path"] == 3
