@@ -268,12 +268,6 @@ struct rp_ctx {
         used += bytes;
         return b.ptr;
     }
-    // whether buf(name, bytes) would stay within the budget
-    bool fits(const std::string &name, size_t bytes) const {
-        const auto it = scratch.find(slot_key(name));
-        const size_t have = it == scratch.end() ? 0 : it->second.bytes;
-        return have >= bytes || used - have + bytes <= budget;
-    }
     template <class T>
     T *buf_t(const std::string &name, size_t count) {
         return static_cast<T *>(buf(name, count * sizeof(T)));

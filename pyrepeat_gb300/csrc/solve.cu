@@ -1098,31 +1098,28 @@ __global__ void __launch_bounds__(256) lu_trsm_kernel(T *__restrict__ A, int n1,
 // FP32 factorisation of one system across the whole GPU, for systems of kLUHost64Min unknowns (where
 // one CTA's n1^3 / 3 multiply-adds are SM-bound) to kLUAcrossMax.  Per panel of NB columns:
 //   lu_panel_across_kernel<R>  one CTA: the panel's rows in registers (R rows of NB = 64 / R columns
-//                    per thread, so up to 512 R rows), two barriers per column as in
-//                    lu_factor_f32_blocked.  It writes the panel's rows in their new order
-//                    (LP, for the update), each row to the factors' row of its *input* row
-//                    number (F), and the order itself: no row of earlier panels ever moves.
+//                    per thread, so up to 512 R rows), one barrier per column.  It writes the panel's rows in their new order
+//                    (LP, for the update), each row to the factors' row of its input row's number
+//                    (F), and the order itself: no row ever moves.
 //   lu_update_across_kernel   64 x 64 tiles over the GPU: U12 = L11^-1 A12 of the tile's columns
 //                    (by every tile of a column, cheaper than another launch), then
-//                    A22' = A22 - L21 U12 with the rows taken in the new order, from one
-//                    buffer to the other, so that no tile reads what another writes.
+//                    A22 -= L21 U12 in place, the rows taken in the new order; the pivot rows,
+//                    which every tile of a column reads, are not written again.
 // lu_collect_kernel gathers F's rows into the final order.  d.perm receives that order (row i of
 // the factors is row perm[i] of the input); pre = {flag, min|pivot|, max|pivot|}, flag 1 = zero or
 // non-finite pivot (the later launches return at once).
 // Bounded by the panels' chain of latencies, about 1200 cycles per column (search, publish, pick,
-// update) and 5 us per panel of loads and stores; an update of 2001 x 2001 takes 8 us.  Half as many
-// barriers, eight columns at a time and panels wholly in line (their instruction fetch costs as
-// much) were no faster.  Measured: 7.8 -> 2.9 ms at 2001 unknowns, 2.3 -> 0.68 at 768, 3.6 -> 1.1 at
+// update) and 5 us per panel of loads and stores; an update of 2001 x 2001 takes 8 us.  Two barriers
+// per column took 5 % longer; eight columns at a time and panels wholly in line (their instruction
+// fetch costs as much) were no faster.  Measured: 7.8 -> 2.9 ms at 2001 unknowns, 2.3 -> 0.68 at 768, 3.6 -> 1.1 at
 // 1101 (against panels in shared memory with four barriers per column, interchanges on one CTA
 // and a cuBLAS rank-32 update).
 constexpr int kLUAcrossMax = 4096;
 constexpr int kPanelT = 512;  // threads of a panel: R rows each, 64 values in registers
 struct LuStep {
-    const float *Ao;   // trailing matrix (rows in the order before this panel)
-    float *An;         // and after it
-    float *LP;         // [rows from k0][32] the panel in its new order
+    float *A;          // the matrix, updated in place: row id stays where it is
     float *F;          // factors by input row
-    int *from;         // [n1] new position -> position before this panel
+    float *LP;         // [rows from k0][32] the panel in its new order
     const int *id_o;   // position -> input row, before this panel
     int *id_n;         // and after it
     int *orig;         // final order
@@ -1169,17 +1166,30 @@ __global__ void __launch_bounds__(kPanelT) lu_panel_across_kernel(LuStep p) {
     chain_begin();
     if (k0 > 0 && p.pre[0] != 0.0) return;  // an earlier panel met a zero pivot
     const int sc = lane % NB, sr = warp * (32 / NB) + lane / NB, sn = nw * (32 / NB);  // staging: column, first row, step
-    if (sc < nb)
-        for (int r = sr; r < m; r += sn)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(pst + r * LD + sc)),
-                         "l"(p.Ao + (size_t)(k0 + r) * n1 + k0 + sc) : "memory");
+    constexpr int RB = 32 / NB;  // rows of a staging step; a lane holds the input row of NB steps ahead
+    int idl[64 / NB];
+#pragma unroll
+    for (int h = 0; h < 64 / NB; ++h) {
+        const int r = warp * RB + lane % RB + (h * NB + lane / RB) * sn;
+        idl[h] = r < m ? p.id_o[k0 + r] : 0;
+    }
+#pragma unroll
+    for (int h = 0; h < 64 / NB; ++h) {
+        const int own = warp * RB + lane % RB + (h * NB + lane / RB) * sn;
+        if (own < m) ids[own] = idl[h];
+        for (int it = 0; it < NB && warp * RB + (h * NB + it) * sn < m; ++it) {
+            const int id = __shfl_sync(0xffffffffu, idl[h], it * RB + lane / NB), r = sr + (h * NB + it) * sn;
+            if (r < m && sc < nb)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(pst + r * LD + sc)),
+                             "l"(p.A + (size_t)id * n1 + k0 + sc) : "memory");
+        }
+    }
     asm volatile("cp.async.commit_group;" ::: "memory");
     int pos[R];
 #pragma unroll
     for (int q = 0; q < R; ++q) {
         const int t = tid + q * nt;
         pos[q] = t < m ? t : -1;  // -1: no row
-        if (t < m) ids[t] = p.id_o[k0 + t];
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
@@ -1279,7 +1289,6 @@ __global__ void __launch_bounds__(kPanelT) lu_panel_across_kernel(LuStep p) {
         if (pos[q] < 0) continue;
         const int t = tid + q * nt, id = ids[t];
         posr[t] = pos[q];
-        p.from[k0 + pos[q]] = k0 + t;
         p.id_n[k0 + pos[q]] = id;
         if (pos[q] < nb) p.orig[k0 + pos[q]] = id;
     }
@@ -1311,10 +1320,10 @@ __global__ void __launch_bounds__(256, 3) lu_update_across_kernel(LuStep p) {
     const int tr = (tid >> 4) * 4, tc = tid & 15;  // rows tr .. tr+3, columns tc + 16 i
     chain_begin();
     const double flag = p.pre[0];
-    const int top = lane < nb ? p.from[k0 + lane] : k0;
+    const int top = lane < nb ? p.orig[k0 + lane] : 0;
     int fr[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) fr[k] = p.from[min(r0 + tr + k, n1 - 1)];
+    for (int k = 0; k < 4; ++k) fr[k] = p.id_n[min(r0 + tr + k, n1 - 1)];
 #pragma unroll
     for (int t = tid; t < kLUNB * kLUNB; t += 256) {
         const int i = t >> 5, j = t & 31;
@@ -1326,7 +1335,7 @@ __global__ void __launch_bounds__(256, 3) lu_update_across_kernel(LuStep p) {
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
         const int j = warp + 8 * h;
-        const float *row = p.Ao + (size_t)__shfl_sync(0xffffffffu, top, j) * n1 + q0;
+        const float *row = p.A + (size_t)__shfl_sync(0xffffffffu, top, j) * n1 + q0;
         u[j][lane] = j < nb && q0 + lane < n1 ? row[lane] : 0.f;
         u[j][lane + 32] = j < nb && q0 + lane + 32 < n1 ? row[lane + 32] : 0.f;
     }
@@ -1335,7 +1344,7 @@ __global__ void __launch_bounds__(256, 3) lu_update_across_kernel(LuStep p) {
     float old[4][4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const float *row = p.Ao + (size_t)fr[k] * n1 + q0;
+        const float *row = p.A + (size_t)fr[k] * n1 + q0;
 #pragma unroll
         for (int i = 0; i < 4; ++i) old[k][i] = r0 + tr + k < n1 && q0 + tc + 16 * i < n1 ? row[tc + 16 * i] : 0.f;
     }
@@ -1377,7 +1386,7 @@ __global__ void __launch_bounds__(256, 3) lu_update_across_kernel(LuStep p) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int r = r0 + tr + k, c = q0 + tc + 16 * i;
-            if (r < n1 && c < n1) p.An[(size_t)r * n1 + c] = SUM ? old[k][i] - acc[k][i] : acc[k][i];
+            if (r < n1 && c < n1) p.A[(size_t)fr[k] * n1 + c] = SUM ? old[k][i] - acc[k][i] : acc[k][i];
         }
 }
 
@@ -1394,20 +1403,15 @@ __global__ void iota_kernel(int *__restrict__ v, int n) {
     if (t < n) v[t] = t;
 }
 
-// Whether a system is factored across the GPU: its size, and room in the scratch budget for the factors by
-// input row (a quarter of what the system holds already; without it, panels in shared memory or
-// the system's CTA as before)
-bool across_fits(rp_ctx *ctx, int n1, const std::string &tag) {
-    return n1 <= kLUAcrossMax && ctx->fits("s_luF" + tag, sizeof(float) * ((size_t)n1 * n1 + 64 * (size_t)n1 + (1 << 20)));
-}
-// The FP32 matrix is in the first half of d.As, the second half is the other buffer.
+// The FP32 matrix is in the first half of d.As; the second half takes the factors by input row.  (A buffer of
+// n1^2 floats more, so that rows can move with their positions, made it 5 % faster, but a system
+// would then be factored one way or another by what the scratch budget has left.)
 void lu_factor_across(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &tag, cudaStream_t stream) {
-    float *buf[2] = {reinterpret_cast<float *>(d.As), reinterpret_cast<float *>(d.As) + (size_t)n1 * n1};
     LuStep p{};
-    p.F = ctx->buf_t<float>("s_luF" + tag, (size_t)n1 * n1);
+    p.A = reinterpret_cast<float *>(d.As);
+    p.F = p.A + (size_t)n1 * n1;
     p.LP = ctx->buf_t<float>("s_luLP" + tag, (size_t)n1 * 32);
-    int *idx = ctx->buf_t<int>("s_luidx" + tag, 3 * (size_t)n1);  // order, two generations; then from
-    p.from = idx + 2 * (size_t)n1;
+    int *idx = ctx->buf_t<int>("s_luidx" + tag, 2 * (size_t)n1);  // the rows' order, two generations
     p.orig = d.perm;
     p.pre = d.pre;
     p.n1 = n1;
@@ -1420,8 +1424,6 @@ void lu_factor_across(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string
     int step = 0;
     for (int k0 = 0; k0 < n1; ++step) {
         const int m = n1 - k0, R = m <= 2 * kPanelT ? 2 : m <= 4 * kPanelT ? 4 : 8, NB = 64 / R;
-        p.Ao = buf[step & 1];
-        p.An = buf[(step + 1) & 1];
         p.id_o = idx + (size_t)(step & 1) * n1;
         p.id_n = idx + (size_t)((step + 1) & 1) * n1;
         p.k0 = k0;
@@ -1436,7 +1438,7 @@ void lu_factor_across(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string
             launch_chained(n1 >= kLUWideMin ? lu_update_across_kernel<true> : lu_update_across_kernel<false>, dim3(t, t), 256, 0, stream, p);
         }
     }
-    launch_chained(lu_collect_kernel, dim3(n1), 256, 0, stream, p.F, d.perm, n1, d.pre, buf[0]);
+    launch_chained(lu_collect_kernel, dim3(n1), 256, 0, stream, p.F, d.perm, n1, d.pre, p.A);
 }
 
 // dynamic shared memory of lu_solve_refine_kernel: the right-hand side, the correction and the row
@@ -2234,7 +2236,7 @@ void lu_wide_factor(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &
     const long long nn = (long long)n1 * n1;
     lu_copy_kernel<T><<<(int)std::min<long long>(ceil_div(nn, 256), 4096), 256, 0, stream>>>(d.A0, L, nn, d.pre);
     RP_LAUNCH_CHECK();
-    if (across_fits(ctx, n1, tag)) {
+    if (n1 <= kLUAcrossMax) {
         lu_factor_across(ctx, d, n1, tag, stream);
         return;
     }
@@ -2461,7 +2463,7 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         }
     if (mid == 1 || (mid == 2 && least >= kAcrossTwo))
         for (int j = 0; j < nj; ++j)
-            if (descs[j].host64 && across_fits(ctx, plans[j].n + 1, tag)) {
+            if (descs[j].host64) {
                 descs[j].host64 = 0;
                 descs[j].host32 = 1;
             }

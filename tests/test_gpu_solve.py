@@ -187,3 +187,18 @@ def test_solve_within_a_tight_scratch_budget(N):
     q, _ = ctx.solve(torch.from_numpy(A).cuda(), torch.from_numpy(b).cuda(), np.full(N, 6), qtot=0.5)
     tol = max(1e-12, 1e-15 * np.linalg.cond(K) * (N + 1))
     assert np.abs(q.cpu().numpy() - ref).max() <= tol * max(1.0, np.abs(ref).max())
+
+
+@pytest.mark.parametrize("N", [420, 900, 2040])
+def test_charges_do_not_depend_on_the_scratch_left(N, gpu_ctx):
+    """The same system in a context with room for it alone and in one with all of the memory: the same bits."""
+    import torch
+    from pyrepeat_gb300.fit import Context
+    rng = np.random.default_rng(N)
+    A = rng.normal(size=(N, N))
+    A = 0.5 * (A + A.T) + np.diag(np.where(np.arange(N) % 5 == 0, 40.0, 0.0))
+    A, b = torch.from_numpy(A).cuda(), torch.from_numpy(rng.normal(size=N)).cuda()
+    tight = Context(0, hbm_budget=16 * (N + 1) ** 2 + (2 << 20))
+    out = [(q.cpu().numpy().tobytes(), info["kappa"])
+           for q, info in (c.solve(A, b, np.full(N, 6), qtot=0.25) for c in (tight, gpu_ctx))]
+    assert out[0] == out[1]
