@@ -21,9 +21,10 @@
 // refinement stalls (a step that does not halve the residual, or kRefineMax steps:
 // cond(A) near 1/eps32), the system is factored again in FP64 with one step of FP64
 // refinement.  Either way the refined residual and the pivot range are reported.
-// Systems of kLUWideMin or more unknowns, and single ones of kLUHost64Min or more, are factored and
-// refined across the whole GPU instead of by their CTA (lu_wide_factor, refine_across), in FP32
-// and, when that stalls, in FP64 (factor_refine_wide64).
+// Systems of kLUWideMin or more unknowns are factored and refined across the whole GPU instead of by
+// their CTA (lu_wide_factor, refine_across), in FP32 and, when that stalls, in FP64
+// (factor_refine_wide64).  A single one of kLUHost64Min or more is factored across the GPU, to the
+// same factors as its CTA's, and refined by its CTA.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -938,7 +939,7 @@ __global__ void __launch_bounds__(kSolve) lu_solve_refine_kernel(const SolveDesc
         d.info[4] = fmin(anorm * kinv, 1e300);
         d.info[5] = n1;
         d.info[6] = steps;
-        d.info[7] = f32_solved ? (d.across ? 1.0 : 0.0) : 2.0;
+        d.info[7] = f32_solved ? 0.0 : 2.0;
     }
     __syncthreads();
     // expand to all atoms
@@ -2268,22 +2269,6 @@ void lu_wide_factor(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &
     RP_LAUNCH_CHECK();
 }
 
-// the refinement of lu_solve_refine_kernel alone, on FP32 factors from across the GPU; pre[0] = 2 when
-// it stalls
-void refine_in_cta(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t stream) {
-    StageTimer tt(ctx, "solve_refine32", stream);
-    SolveDesc *one = ctx->buf_t<SolveDesc>("s_desc1", 1), h = d;
-    h.host32 = 0;
-    h.across = 1;
-    RP_CUDA(cudaMemsetAsync(d.pre, 0, sizeof(double), stream));
-    RP_CUDA(cudaMemcpyAsync(one, &h, sizeof(h), cudaMemcpyHostToDevice, stream));
-    lu_smem_optin();
-    prepare_kernel<<<(int)ceil_div(n1, 8), 256, 0, stream>>>(one);
-    RP_LAUNCH_CHECK();
-    lu_solve_refine_kernel<<<1, solve_threads(n1), solve_smem_bytes(n1), stream>>>(one);
-    RP_LAUNCH_CHECK();
-}
-
 }  // namespace
 
 // Host side: reduced-index maps (repeat.py:2445-2470 semantics).
@@ -2452,9 +2437,9 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         }
         if (plans[j].disjoint) disjoint.push_back(j);
     }
-    // One system of kLUHost64Min unknowns or more is solved across the GPU (0.34 + 0.29 ms at 425
-    // unknowns, factors and refinement, against 0.74 + 0.70 in one CTA; 0.62 + 0.4 against 2.0 + 1.4
-    // at 720), two of them one after the other from kAcrossTwo; more run side by side, each in its CTA.
+    // A single system of kLUHost64Min to kLUWideMin unknowns is factored across the GPU, two of them one after the
+    // other from kAcrossTwo; more are factored side by side, each in its CTA.  Both give the same factors, bit
+    // for bit, and its CTA refines it either way, so that charges do not depend on the batch.
     int mid = 0, least = kLUWideMin;
     for (int j = 0; j < nj; ++j)
         if (descs[j].host64) {
@@ -2462,11 +2447,7 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
             least = std::min(least, plans[j].n + 1);
         }
     if (mid == 1 || (mid == 2 && least >= kAcrossTwo))
-        for (int j = 0; j < nj; ++j)
-            if (descs[j].host64) {
-                descs[j].host64 = 0;
-                descs[j].host32 = 1;
-            }
+        for (int j = 0; j < nj; ++j) descs[j].across = descs[j].host64;
     // the small tables go up from one pinned staging block per tag (asynchronous copies that
     // never wait for the stream; a later solve with another tag cannot overwrite them)
     const size_t st_bytes[7] = {sizeof(int) * n_map, sizeof(int) * n_mptr, sizeof(int) * n_midx,
@@ -2534,16 +2515,13 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
     if (any_pre) RP_CUDA(cudaMemsetAsync(d_pre, 0, sizeof(double) * 3 * nj, stream));
     for (int j = 0; j < nj; ++j) {
         if (!descs[j].pre || descs[j].wide64) continue;  // wide64: factored and refined after the launch
-        if (descs[j].host64) {
-            any_wide = true;  // its flag is read after the launch, as a wide system's
-        } else {
-            {
-                StageTimer tt(ctx, "solve_lu_wide", stream);
-                lu_wide_factor<float>(ctx, descs[j], plans[j].n + 1, tag, stream);
-            }
-            refine_across(ctx, descs[j], plans[j].n + 1, 0, kAcRounds, tag + "#" + std::to_string(j), stream);
-            any_wide = true;
+        any_wide = true;  // its flag is read after the launch
+        if (descs[j].host64 && !descs[j].across) continue;
+        {
+            StageTimer tt(ctx, "solve_lu_wide", stream);
+            lu_wide_factor<float>(ctx, descs[j], plans[j].n + 1, tag, stream);
         }
+        if (descs[j].host32) refine_across(ctx, descs[j], plans[j].n + 1, 0, kAcRounds, tag + "#" + std::to_string(j), stream);
     }
     {
         StageTimer tt(ctx, "solve_lu", stream);
@@ -2606,14 +2584,7 @@ void solve_wide_fp64(rp_ctx *ctx, SolvePending &pd, cudaStream_t stream) {
         }
         if (flag == 0.0) continue;
         if (flag == 4.0) {  // by substitution
-            if (pd.n1[j] >= kLUWideMin) {
-                if (refine_wide32(ctx, pd.descs[j], pd.n1[j], pd.tag + "#" + std::to_string(j), stream)) continue;
-            } else {
-                refine_in_cta(ctx, pd.descs[j], pd.n1[j], stream);
-                RP_CUDA(cudaMemcpyAsync(&flag, pd.descs[j].pre, sizeof(flag), cudaMemcpyDeviceToHost, stream));
-                RP_CUDA(cudaStreamSynchronize(stream));
-                if (flag == 0.0) continue;
-            }
+            if (refine_wide32(ctx, pd.descs[j], pd.n1[j], pd.tag + "#" + std::to_string(j), stream)) continue;
         }
         factor_refine_wide64(ctx, pd.descs[j], pd.n1[j], stream);
     }
