@@ -277,6 +277,7 @@ struct rp_ctx {
     std::unordered_map<std::string, rp::Buffer> host_scratch;
     double bound_scale = 1.0;  // factor on the single-pass Phi bounds (tests shrink it to force clamps)
     long long chunk_cap = 0;   // cap on the staged mixed Gram's points per chunk (tests; 0 = none)
+    bool solve_in_memory = false;  // the in-CTA solves keep their vectors in memory whatever the size (tests)
     long long wait_budget = 4000000000LL;  // clock budget of the Gram pipeline's waits (tests shorten it)
     std::unique_ptr<rp::HostPool> pool;  // host workers (created on first use)
     std::unique_ptr<rp::BatchServer> server;  // asynchronous batches (created on first submit)
@@ -551,6 +552,7 @@ struct SolveDesc {
     int wide64;           // As holds wide FP64 factors: skip the FP32 stage and the in-CTA FP64 LU
     int host64;           // FP32 factors in the CTA, but a stalled refinement goes to the host's FP64
                           // factorisation across the GPU (pre holds its flag) instead of an in-CTA FP64 LU
+    int big;              // the in-CTA solve's vectors are kept in memory
     int across;           // FP32 factors already in As, their row order in perm and pivot range in pre
     int host32;           // factored and refined across the GPU (lu_wide_factor, refine_across): the kernel skips it
 };

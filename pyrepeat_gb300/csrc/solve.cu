@@ -170,9 +170,8 @@ __device__ double block_sum(double v, int active, double *sv) {
     return sv[32];
 }
 
-__device__ void lu_apply(const double *__restrict__ LU, const int *__restrict__ perm, int n1, double *__restrict__ y,
-                         double *__restrict__ ysh) {
-    // solve (P L U) z = y in place (y global; ysh: n1 doubles of shared memory), blocked by 32
+__device__ void lu_apply(const double *__restrict__ LU, const int *__restrict__ perm, int n1, double *y, double *ysh) {
+    // solve (P L U) z = y in place (y global; ysh: n1 doubles of shared memory, or y itself), blocked by 32
     // columns: the diagonal block is solved by one warp with shuffles, then every thread
     // updates one remaining row with the block's 32 values (a warp instruction covers 32 rows:
     // the FP64 pipe takes as long for one lane as for 32).  The row interchanges run in
@@ -644,9 +643,9 @@ __device__ void lu_apply_f32(const float *__restrict__ LU, const int *__restrict
 }
 
 // d.r <- K^{-1} d.r with the factors that solved the system: FP32 (in the first half of As,
-// through the FP32 shared vectors ys/xs) or FP64 (in As).  Non-finite FP32 results (a system
+// through the FP32 vectors ys/xs) or FP64 (in As, through y64).  Non-finite FP32 results (a system
 // far beyond FP32) read as 1e300.
-__device__ void apply_inverse(const SolveDesc &d, int n1, bool f32, float *ys, float *xs, const int *orig) {
+__device__ void apply_inverse(const SolveDesc &d, int n1, bool f32, float *ys, float *xs, const int *orig, double *y64) {
     if (f32) {
         __syncthreads();
         for (int t = threadIdx.x; t < n1; t += blockDim.x) ys[t] = (float)d.r[t];
@@ -657,7 +656,7 @@ __device__ void apply_inverse(const SolveDesc &d, int n1, bool f32, float *ys, f
         }
         __syncthreads();
     } else {
-        lu_apply(d.As, d.perm, n1, d.r, reinterpret_cast<double *>(ys));
+        lu_apply(d.As, d.perm, n1, d.r, y64);
         __syncthreads();
     }
 }
@@ -667,18 +666,17 @@ __device__ void apply_inverse(const SolveDesc &d, int n1, bool f32, float *ys, f
 // 311-316) with Higham's extra test vector (N. J. Higham, ACM TOMS 14 (1988) 381-396),
 // at most four sign iterations.  A lower bound that is almost always within a small factor.
 // Uses d.r as the work vector.
-__device__ double inverse_norm1_estimate(const SolveDesc &d, int n1, bool f32, float *fsh, const int *orig, double *sv, int *si,
-                                         double *piv_v, int *piv_i) {
-    float *ys = fsh, *xs = fsh + n1;
+__device__ double inverse_norm1_estimate(const SolveDesc &d, int n1, bool f32, float *ys, float *xs, const int *orig, double *y64,
+                                         double *sv, int *si, double *piv_v, int *piv_i) {
     for (int t = threadIdx.x; t < n1; t += blockDim.x) d.r[t] = 1.0 / (double)n1;
-    apply_inverse(d, n1, f32, ys, xs, orig);
+    apply_inverse(d, n1, f32, ys, xs, orig, y64);
     double a = 0.0;
     for (int t = threadIdx.x; t < n1; t += blockDim.x) a += fabs(d.r[t]);
     double est = block_sum(a, n1, sv);
     int jprev = -1;
     for (int it = 0; it < 4; ++it) {
         for (int t = threadIdx.x; t < n1; t += blockDim.x) d.r[t] = d.r[t] >= 0.0 ? 1.0 : -1.0;
-        apply_inverse(d, n1, f32, ys, xs, orig);  // z = K^{-T} sign(y)
+        apply_inverse(d, n1, f32, ys, xs, orig, y64);  // z = K^{-T} sign(y)
         double best = -1.0, zsum = 0.0;
         int bi = 0x7fffffff;
         for (int t = threadIdx.x; t < n1; t += blockDim.x) {
@@ -694,7 +692,7 @@ __device__ double inverse_norm1_estimate(const SolveDesc &d, int n1, bool f32, f
         __syncthreads();
         if (!(zmax > ztx)) break;  // uniform: every thread read the same values
         for (int t = threadIdx.x; t < n1; t += blockDim.x) d.r[t] = t == j ? 1.0 : 0.0;
-        apply_inverse(d, n1, f32, ys, xs, orig);
+        apply_inverse(d, n1, f32, ys, xs, orig, y64);
         double b = 0.0;
         for (int t = threadIdx.x; t < n1; t += blockDim.x) b += fabs(d.r[t]);
         b = block_sum(b, n1, sv);
@@ -704,7 +702,7 @@ __device__ double inverse_norm1_estimate(const SolveDesc &d, int n1, bool f32, f
     }
     for (int t = threadIdx.x; t < n1; t += blockDim.x)
         d.r[t] = ((t & 1) ? -1.0 : 1.0) * (1.0 + (double)t / (double)max(n1 - 1, 1));
-    apply_inverse(d, n1, f32, ys, xs, orig);
+    apply_inverse(d, n1, f32, ys, xs, orig, y64);
     double c = 0.0;
     for (int t = threadIdx.x; t < n1; t += blockDim.x) c += fabs(d.r[t]);
     c = 2.0 * block_sum(c, n1, sv) / (3.0 * (double)n1);
@@ -760,6 +758,9 @@ __device__ void residual(const SolveDesc &d, int n1) {
     __syncthreads();
 }
 
+// BIG: a launch with a system beyond kLUWideMax, whose vectors do not fit shared memory: they follow the FP32
+// factors in the work matrix (3 n1 of its n1^2 words there), or the FP64 solves run on the vector itself.
+template <bool BIG>
 __global__ void __launch_bounds__(kSolve) lu_solve_refine_kernel(const SolveDesc *__restrict__ descs) {
     const SolveDesc d = descs[blockIdx.x];
     if (d.wide64 || d.host32) return;  // factor_refine_wide64, refine_across
@@ -767,8 +768,9 @@ __global__ void __launch_bounds__(kSolve) lu_solve_refine_kernel(const SolveDesc
     // [2 n1] right-hand side / correction in FP32 (or n1 doubles), [n1] row order, then the work
     // area of the blocked factorisation
     extern __shared__ __align__(16) float fsh[];
-    float *ys = fsh, *xs = fsh + n1;
-    int *orig = reinterpret_cast<int *>(fsh + 2 * n1);
+    const bool big = BIG && d.big;
+    float *ys = big ? reinterpret_cast<float *>(d.As) + (size_t)n1 * n1 : fsh, *xs = ys + n1;
+    int *orig = reinterpret_cast<int *>(xs + n1);
     __shared__ double sv[33];
     __shared__ int si[kLU / 32];
     __shared__ double piv_v;
@@ -802,7 +804,7 @@ __global__ void __launch_bounds__(kSolve) lu_solve_refine_kernel(const SolveDesc
             pmax = d.pre[2];
             for (int t = threadIdx.x; t < n1; t += blockDim.x) orig[t] = factored ? d.perm[t] : t;
             __syncthreads();
-        } else if (n1 <= kLUBlockedMax) {
+        } else if (n1 <= kLUBlockedMax && !big) {
             float *work = fsh + ((3 * n1 + 3) & ~3);
             factored = lu_factor_f32_blocked(L, orig, n1, work, lus, pmin, pmax);
         } else {
@@ -907,14 +909,14 @@ __global__ void __launch_bounds__(kSolve) lu_solve_refine_kernel(const SolveDesc
         }
         }
         for (int t = threadIdx.x; t < n1; t += blockDim.x) d.x[t] = d.bs[t];
-        lu_apply(A, d.perm, n1, d.x, reinterpret_cast<double *>(fsh));
+        lu_apply(A, d.perm, n1, d.x, big ? d.x : reinterpret_cast<double *>(fsh));
         for (int rr = threadIdx.x; rr < n1; rr += blockDim.x) {
             double s = d.bs[rr];
             const double *row = d.A0 + (size_t)rr * n1;
             for (int c = 0; c < n1; ++c) s -= row[c] * d.x[c];
             d.r[rr] = s;
         }
-        lu_apply(A, d.perm, n1, d.r, reinterpret_cast<double *>(fsh));
+        lu_apply(A, d.perm, n1, d.r, big ? d.r : reinterpret_cast<double *>(fsh));
         for (int t = threadIdx.x; t < n1; t += blockDim.x) d.x[t] += d.r[t];
         __syncthreads();
         double rmax = 0.0;
@@ -930,7 +932,7 @@ __global__ void __launch_bounds__(kSolve) lu_solve_refine_kernel(const SolveDesc
     // included, the border excluded) and K the bordered matrix.  A relative error e in A moves
     // the solution by about e * kappa * |q| at worst, so kappa says how much of the Gram's
     // rounding reaches the charges (the fit escalates a mixed-precision cube beyond a limit).
-    const double kinv = inverse_norm1_estimate(d, n1, f32_solved, fsh, orig, sv, si, &piv_v, &piv_i);
+    const double kinv = inverse_norm1_estimate(d, n1, f32_solved, ys, xs, orig, big ? d.r : reinterpret_cast<double *>(fsh), sv, si, &piv_v, &piv_i);
     if (threadIdx.x == 0) {
         d.info[0] = res;
         d.info[1] = pmin;
@@ -1444,8 +1446,9 @@ void lu_factor_across(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string
 
 // dynamic shared memory of lu_solve_refine_kernel: the right-hand side, the correction and the row
 // order, and for the blocked factorisation 64 rows of a panel's neighbours (or its own rows,
-// 33 floats each)
-size_t solve_smem_bytes(int n1) {
+// 33 floats each); none beyond kLUWideMax (BIG)
+size_t solve_smem_bytes(int n1, bool big = false) {
+    if (big) return 0;
     size_t f = (3 * (size_t)n1 + 3) & ~(size_t)3;
     if (n1 <= kLUBlockedMax) f += 64 * (((size_t)n1 + 3) & ~(size_t)3);
     return sizeof(float) * f;
@@ -1456,7 +1459,10 @@ size_t solve_smem_bytes(int n1) {
 int solve_threads(int n1) { return n1 <= 100 ? 256 : kSolve; }
 
 // the launch's shared memory opt-in, raised once to the largest the kernel is launched with
-void lu_smem_optin() { smem_optin((const void *)lu_solve_refine_kernel, solve_smem_bytes(kLUWideMin - 1)); }
+void lu_smem_optin() {
+    smem_optin((const void *)lu_solve_refine_kernel<false>, solve_smem_bytes(kLUWideMin - 1));
+    smem_optin((const void *)lu_solve_refine_kernel<true>, solve_smem_bytes(kLUWideMin - 1));
+}
 
 inline cublasStatus_t gemm_nn(cublasHandle_t h, int m, int n, int k, const float *alpha, const float *A, int lda,
                               const float *B, int ldb, const float *beta, float *C, int ldc) {
@@ -2418,6 +2424,7 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         d.resp_s = J.resp_s ? d_rs + o_red : nullptr; d.resp_t = J.resp_s ? d_rt + o_red : nullptr;
         d.map = d_map + o_map; d.qtot = J.qtot;
         d.As = As + o_sq; d.A0 = A0 + o_sq; d.bs = bs + o_red; d.x = x + o_red; d.r = r + o_red;
+        d.big = n1 > kLUWideMax || (ctx->solve_in_memory && n1 >= 4);
         d.perm = perm + o_red; d.q = J.q; d.info = d_info + kSolveInfo * (size_t)j;
         o_map += J.N;
         o_mptr += p.mem_ptr.size();
@@ -2527,16 +2534,19 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         StageTimer tt(ctx, "solve_lu", stream);
         int n1max = 0;  // of the systems solved in their CTAs
         size_t smem = 0;
+        bool big = false;
         for (int j = 0; j < nj; ++j) {
             if (descs[j].wide64 || descs[j].host32) continue;
             n1max = std::max(n1max, descs[j].n + 1);
-            smem = std::max(smem, solve_smem_bytes(descs[j].n + 1));
+            smem = std::max(smem, solve_smem_bytes(descs[j].n + 1, descs[j].big));
+            big |= descs[j].big != 0;
         }
         if (n1max > 0) {
             lu_smem_optin();
             prepare_kernel<<<dim3(ceil_div(n1max, 8), nj), 256, 0, stream>>>(d_desc);
             RP_LAUNCH_CHECK();
-            lu_solve_refine_kernel<<<nj, solve_threads(n1max), smem, stream>>>(d_desc);
+            auto kernel = big ? lu_solve_refine_kernel<true> : lu_solve_refine_kernel<false>;
+            kernel<<<nj, solve_threads(n1max), smem, stream>>>(d_desc);
             RP_LAUNCH_CHECK();
         }
     }
@@ -2750,7 +2760,7 @@ extern "C" int rp_solve_noalloc(const double *A_dev, const double *b_dev, int N,
         lu_smem_optin();
         prepare_kernel<<<dim3(ceil_div(n1, 8), 1), 256, 0, stream>>>(d_desc);
         RP_LAUNCH_CHECK();
-        lu_solve_refine_kernel<<<1, solve_threads(n1), solve_smem_bytes(n1), stream>>>(d_desc);
+        lu_solve_refine_kernel<false><<<1, solve_threads(n1), solve_smem_bytes(n1), stream>>>(d_desc);
         RP_LAUNCH_CHECK();
         double hinfo[kSolveInfo];
         RP_CUDA(cudaMemcpyAsync(hinfo, d_info, sizeof(hinfo), cudaMemcpyDeviceToHost, stream));
@@ -2767,4 +2777,12 @@ extern "C" int rp_solve_noalloc(const double *A_dev, const double *b_dev, int N,
     } catch (const std::exception &) {
         return RP_E_ARG;
     }
+}
+
+// Diagnostics (not part of the public ABI): solve systems of any size in their CTA with the vectors in
+// memory, as those beyond kLUWideMax are (on != 0)
+extern "C" int rp_debug_solve_in_memory(rp_ctx *ctx, int on) {
+    if (!ctx) return RP_E_ARG;
+    ctx->solve_in_memory = on != 0;
+    return RP_OK;
 }

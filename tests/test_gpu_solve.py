@@ -202,3 +202,27 @@ def test_charges_do_not_depend_on_the_scratch_left(N, gpu_ctx):
     out = [(q.cpu().numpy().tobytes(), info["kappa"])
            for q, info in (c.solve(A, b, np.full(N, 6), qtot=0.25) for c in (tight, gpu_ctx))]
     assert out[0] == out[1]
+
+
+@pytest.mark.parametrize("N", [3, 40, 200])
+@pytest.mark.parametrize("top", [1e2, 1e10])
+def test_systems_with_their_vectors_in_memory(N, top, gpu_ctx):
+    """What systems beyond 11520 unknowns run (their vectors do not fit shared memory), at sizes that take no
+    minutes: by FP32 factors and refinement, and by FP64 factors.  The bound of the first test."""
+    import ctypes
+    import torch
+    hook = gpu_ctx.lib.rp_debug_solve_in_memory
+    hook.restype, hook.argtypes = ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]
+    rng = np.random.default_rng(N)
+    U, _ = np.linalg.qr(rng.normal(size=(N, N)))
+    A = (U * np.geomspace(1.0 / top, 1.0, N)) @ U.T
+    A = 0.5 * (A + A.T)
+    b = rng.normal(size=N)
+    K, ref = _reference(A, b, 0.25)
+    assert hook(gpu_ctx.ptr, 1) == 0
+    try:
+        q, info = gpu_ctx.solve(torch.from_numpy(A).cuda(), torch.from_numpy(b).cuda(), np.full(N, 6), qtot=0.25)
+    finally:
+        hook(gpu_ctx.ptr, 0)
+    tol = max(1e-9, 1e-15 * np.linalg.cond(K) * (N + 1))
+    assert np.abs(q.cpu().numpy() - ref).max() <= tol * max(1.0, np.abs(ref).max())
