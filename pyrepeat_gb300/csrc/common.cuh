@@ -268,6 +268,15 @@ struct rp_ctx {
         used += bytes;
         return b.ptr;
     }
+    // what the named buffers may grow to within the budget, all of them together
+    size_t room(std::initializer_list<const char *> names) const {
+        size_t have = budget > used ? budget - used : 0;
+        for (const char *name : names) {
+            const auto it = scratch.find(slot_key(name));
+            if (it != scratch.end()) have += it->second.bytes;
+        }
+        return have;
+    }
     template <class T>
     T *buf_t(const std::string &name, size_t count) {
         return static_cast<T *>(buf(name, count * sizeof(T)));
@@ -488,9 +497,17 @@ void filter_async(rp_ctx *ctx, const rp_grid *grid, const double *atoms, const i
                   uint8_t *mask_dev, cudaStream_t stream, const std::string &tag, bool brick_order,
                   double *vstats_dev);
 // Exact Gram of a chunk of FP64 columns on the tensor cores (gram_mixed.cu): G (N x N) +=
-// Phi^T Phi and r (N) += Phi^T V for Phi rows x N (row-major, ld N) and V (rows).
+// Phi^T Phi and r (N) += Phi^T V for Phi rows x N (row-major, ld N) and V (rows).  `scratch`: what its digits
+// and tile totals may take (GramWordsScratch); less than the whole is made up for by blocks of columns
+// and of rows, to the same bits.
 void gram_words_fp64(rp_ctx *ctx, const double *P, long long rows, int N, const double *V, double *G, double *r,
-                     cudaStream_t stream);
+                     size_t scratch, cudaStream_t stream);
+size_t gram_words_bytes(rp_ctx *ctx, long long rows, int N);  // digits and totals of the whole in one piece
+// What a stage may take of the ctx's budget: a quarter of what the named buffers could grow to (the rest is
+// for the stages that follow), and at least `need`
+inline size_t scratch_share(rp_ctx *ctx, std::initializer_list<const char *> names, size_t need) {
+    return std::max(need, ctx->room(names) / 4);
+}
 // refit: an ill-conditioned mixed fit's (the reciprocal plane and row stages in double-float)
 void gram_fp64(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, const int32_t *kept_idx_dev,
                const double *Vc_dev, int64_t M, double *A_dev, double *b_dev, double *sum_phi_dev,

@@ -1477,10 +1477,12 @@ int gram_units_per_launch(const rp_ctx *ctx) { return std::max(1, ctx->sm_count)
 
 // Zeroed tile totals (high and low halves, 2 x ntri x 128 x 64 words) with one work counter
 // per launch after them, in one buffer cleared by one memset on the stream
+size_t gram_launches(const rp_ctx *ctx, const GramArgs &g) { return (size_t)ceil_div(gram_units_total(g), gram_units_per_launch(ctx)); }
+size_t gram_totals_words(const rp_ctx *ctx, const GramArgs &g) {
+    return 2 * (size_t)g.ntri * kBM * kGN + (gram_launches(ctx, g) + 1) / 2 + 1;
+}
 void gram_totals_init(rp_ctx *ctx, const std::string &name, GramArgs &g, cudaStream_t s) {
-    const size_t n = (size_t)g.ntri * kBM * kGN;
-    const size_t nl = (size_t)ceil_div(gram_units_total(g), gram_units_per_launch(ctx));
-    const size_t words = 2 * n + (nl + 1) / 2 + 1;
+    const size_t n = (size_t)g.ntri * kBM * kGN, words = gram_totals_words(ctx, g);
     unsigned long long *t = ctx->buf_t<unsigned long long>(name, words);
     RP_CUDA(cudaMemsetAsync(t, 0, sizeof(unsigned long long) * words, s));
     g.out_hi = t;
@@ -1724,7 +1726,18 @@ void gram_mixed(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, con
 //   G[a][b] += (G11 + 2^-27 (G12 + G21) + 2^-54 G22)[a][b] / (s_a s_b)
 // with the ESP as column N (G[a][N] = (Phi^T V)[a]).  An FP64-accurate Gram from the
 // tensor cores: 4x the work of the mixed path's Gram, instead of DSYRK at the FP64 rate.
+// Where its digits (16 bytes per point and column) and tile totals (32 per pair of columns) have no
+// room, the columns are taken two blocks at a time and the points block by block: the scales are of the
+// whole columns and the totals exact integers, so every entry of G has the same bits.
 namespace {
+
+// The columns of a Gram: block I (i0 .. i0 + ni - 1) and then block J of the N + 1
+struct WordCols {
+    int i0, ni, j0, nj;
+    int own_i, own_j;  // whether the products within I and within J are this Gram's to add
+    __host__ __device__ int n() const { return ni + nj; }
+    __device__ int global(int c) const { return c < ni ? i0 + c : j0 + c - ni; }
+};
 
 // max |x| of each column (N of Phi, then the ESP as column N), as order-preserving bits
 __global__ void colmax_fp64_kernel(const double *__restrict__ P, long long rows, int N, const double *__restrict__ V,
@@ -1744,33 +1757,33 @@ __device__ __forceinline__ double pow2_scale(unsigned long long mbits) {
     return ldexp(1.0, -e - 1);
 }
 
-// two 28-bit words of each value, as four 7-bit digits each: column c < N and the ESP
-// (c = N) to rows c and c + N + 1 of the slices; a 32 x 32 tile per CTA through shared
+// two 28-bit words of each value, as four 7-bit digits each: column c < n of the block (the ESP
+// is column N) to rows c and c + n of the slices; a 32 x 32 tile per CTA through shared
 // memory, so both the reads of Phi and the writes of the slices coalesce
-__global__ void split_words_kernel(const double *__restrict__ P, long long rows, long long cols_pad, int N,
+__global__ void split_words_kernel(const double *__restrict__ P, long long rows, long long cols_pad, int N, WordCols wc,
                                    const double *__restrict__ V, const unsigned long long *__restrict__ mx,
                                    __half *__restrict__ X0, __half *__restrict__ X1, __half *__restrict__ X2,
                                    __half *__restrict__ X3) {
     __shared__ double t[32][33];
     const long long m0 = (long long)blockIdx.x * 32;
-    const int c0 = blockIdx.y * 32;
+    const int c0 = blockIdx.y * 32, n = wc.n();
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {  // t[point][column]
         const long long m = m0 + k;
-        const int c = c0 + threadIdx.x;
+        const int c = c0 + threadIdx.x, g = wc.global(c);
         double v = 0.0;
-        if (m < rows && c <= N) v = c < N ? P[m * N + c] : V[m];
+        if (m < rows && c < n) v = g < N ? P[m * N + g] : V[m];
         t[k][threadIdx.x] = v;
     }
     __syncthreads();
     for (int k = threadIdx.y; k < 32; k += blockDim.y) {  // column c0 + k, point m0 + x
         const int c = c0 + k;
         const long long m = m0 + threadIdx.x;
-        if (c > N || m >= cols_pad) continue;
-        const double x = t[threadIdx.x][k] * pow2_scale(mx[c]) * 134217728.0;  // |x| < 2^26
+        if (c >= n || m >= cols_pad) continue;
+        const double x = t[threadIdx.x][k] * pow2_scale(mx[wc.global(c)]) * 134217728.0;  // |x| < 2^26
         const double i1 = rint(x);
         const double i2 = rint((x - i1) * 134217728.0);                          // |x - i1| <= 1/2
         digits4((int)i1, X0, X1, X2, X3, (long long)c * cols_pad + m);
-        digits4((int)i2, X0, X1, X2, X3, (long long)(c + N + 1) * cols_pad + m);
+        digits4((int)i2, X0, X1, X2, X3, (long long)(c + n) * cols_pad + m);
     }
 }
 
@@ -1793,54 +1806,97 @@ __device__ __forceinline__ double tile_total(const unsigned long long *th, const
 // G[a][b] (N x N, either order: symmetric) and r[a] (b = N) += the combined words / (s_a s_b);
 // rows a fastest, as the tiles store them
 __global__ void combine_words_kernel(const unsigned long long *__restrict__ th,
-                                     const unsigned long long *__restrict__ tl, int ntj, int N,
+                                     const unsigned long long *__restrict__ tl, int ntj, int N, WordCols wc,
                                      const unsigned long long *__restrict__ mx, double *__restrict__ G,
                                      double *__restrict__ r) {
-    const int Np = N + 1;
+    const int n = wc.n();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)N * Np) return;
-    const int b = (int)(t / N), a = (int)(t - (long long)b * N);
-    const double g11 = tile_total(th, tl, ntj, a, b), g12 = tile_total(th, tl, ntj, a, Np + b);
-    const double g21 = tile_total(th, tl, ntj, b, Np + a), g22 = tile_total(th, tl, ntj, Np + a, Np + b);
+    if (t >= (long long)n * n) return;
+    const int lb = (int)(t / n), la = (int)(t - (long long)lb * n), a = wc.global(la), b = wc.global(lb);
+    if (a >= N || (la < wc.ni && lb < wc.ni && !wc.own_i) || (la >= wc.ni && lb >= wc.ni && !wc.own_j)) return;
+    const double g11 = tile_total(th, tl, ntj, la, lb), g12 = tile_total(th, tl, ntj, la, n + lb);
+    const double g21 = tile_total(th, tl, ntj, lb, n + la), g22 = tile_total(th, tl, ntj, n + la, n + lb);
     const double v = (g11 + 7.450580596923828125e-9 * (g12 + g21) + 5.5511151231257827e-17 * g22) /
                      (pow2_scale(mx[a]) * pow2_scale(mx[b]));
     if (b < N) G[(size_t)b * N + a] += v;
     else r[a] += v;
 }
 
-}  // namespace
-
-void gram_words_fp64(rp_ctx *ctx, const double *P, long long rows, int N, const double *V, double *G, double *r,
-                     cudaStream_t stream) {
-    const int Np = N + 1, Np2 = 2 * Np;
-    const long long cols_pad = round_up(rows, kKPad);
-    unsigned long long *mx = ctx->buf_t<unsigned long long>("w64_mx", (size_t)Np);
-    RP_CUDA(cudaMemsetAsync(mx, 0, sizeof(unsigned long long) * Np, stream));
-    colmax_fp64_kernel<<<dim3(ceil_div(Np, 256), ceil_div(rows, 256)), 256, 0, stream>>>(P, rows, N, V, mx);
-    RP_LAUNCH_CHECK();
-    __half *X[kGSlices];
-    for (int q = 0; q < kGSlices; ++q) X[q] = ctx->buf_t<__half>("w64_X" + std::to_string(q), (size_t)Np2 * cols_pad);
-    split_words_kernel<<<dim3(ceil_div(cols_pad, 32), ceil_div(Np, 32)), dim3(32, 8), 0, stream>>>(
-        P, rows, cols_pad, N, V, mx, X[0], X[1], X[2], X[3]);
-    RP_LAUNCH_CHECK();
-    const int nt = (int)ceil_div(Np2, kBM), ntj = (int)ceil_div(Np2, kGN);
-    int ntri = 0;
-    for (int ti = 0; ti < nt; ++ti) ntri += ntj - 2 * ti;
-    const int kb_total = (int)(cols_pad / kBK);
+// the Gram of the word rows of n columns over cols points
+GramArgs words_args(rp_ctx *ctx, int n, long long cols) {
     GramArgs g{};
-    g.nt = nt;
-    g.ntj = ntj;
-    g.ntri = ntri;
-    g.kb_total = kb_total;
+    g.nt = (int)ceil_div(2 * n, kBM);
+    g.ntj = (int)ceil_div(2 * n, kGN);
+    for (int ti = 0; ti < g.nt; ++ti) g.ntri += g.ntj - 2 * ti;
+    g.kb_total = (int)(cols / kBK);
     g.kb_per_split = kGramSplit;
     g.flush = kGramFlush;
     g.status = ctx->status_words();  // cleared before and checked after by the caller
     g.budget = ctx->wait_budget;
-    gram_totals_init(ctx, "w64_tsum", g, stream);
-    const __half *Xq[kGSlices] = {X[0], X[1], X[2], X[3]};
-    launch_gram(ctx, Xq, Np2, cols_pad, g, stream);
-    combine_words_kernel<<<ceil_div((long long)N * Np, 256), 256, 0, stream>>>(g.out_hi, g.out_lo, ntj, N, mx, G, r);
+    return g;
+}
+size_t words_totals_bytes(rp_ctx *ctx, int n, long long cols) {
+    return sizeof(unsigned long long) * gram_totals_words(ctx, words_args(ctx, n, cols));
+}
+size_t words_digit_bytes(int n, long long cols) { return sizeof(__half) * kGSlices * 2 * (size_t)n * (size_t)cols; }
+
+}  // namespace
+
+size_t gram_words_bytes(rp_ctx *ctx, long long rows, int N) {
+    const long long cols = round_up(rows, kKPad);
+    return words_totals_bytes(ctx, N + 1, cols) + words_digit_bytes(N + 1, cols);
+}
+
+void gram_words_fp64(rp_ctx *ctx, const double *P, long long rows, int N, const double *V, double *G, double *r,
+                     size_t scratch, cudaStream_t stream) {
+    const int Np = N + 1;
+    unsigned long long *mx = ctx->buf_t<unsigned long long>("w64_mx", (size_t)Np);
+    RP_CUDA(cudaMemsetAsync(mx, 0, sizeof(unsigned long long) * Np, stream));
+    colmax_fp64_kernel<<<dim3(ceil_div(Np, 256), ceil_div(rows, 256)), 256, 0, stream>>>(P, rows, N, V, mx);
     RP_LAUNCH_CHECK();
+    // Blocks: the whole where it fits; else the largest blocks of columns whose totals leave room for the digits
+    // of 4096 points (fewer, longer runs of the pipeline), down to 16 columns, and the points that then fit.
+    long long cols = round_up(rows, kKPad);
+    int block = Np, n = Np;
+    if (words_totals_bytes(ctx, n, cols) + words_digit_bytes(n, cols) > scratch) {
+        size_t totals = 0;
+        for (int nb = 1;; ++nb) {
+            block = (int)ceil_div(Np, nb);
+            n = std::min(Np, nb == 1 ? block : 2 * block);
+            totals = words_totals_bytes(ctx, n, cols);
+            if (block <= 16 || totals + words_digit_bytes(n, std::min<long long>(cols, 4096)) <= scratch) break;
+        }
+        const size_t left = scratch > totals ? scratch - totals : 0;
+        cols = std::min<long long>(cols, std::max<long long>(kKPad, (long long)(left / words_digit_bytes(n, kKPad)) * kKPad));
+    }
+    __half *X[kGSlices];
+    for (int q = 0; q < kGSlices; ++q) X[q] = ctx->buf_t<__half>("w64_X" + std::to_string(q), 2 * (size_t)n * cols);
+    const __half *Xq[kGSlices] = {X[0], X[1], X[2], X[3]};
+    const int nb = (int)ceil_div(Np, block);
+    auto gram = [&](const WordCols &wc) {
+        GramArgs g = words_args(ctx, wc.n(), cols);
+        gram_totals_init(ctx, "w64_tsum", g, stream);
+        for (long long m0 = 0; m0 < rows; m0 += cols) {
+            const long long part = std::min<long long>(cols, rows - m0), pad = round_up(part, kKPad);
+            if (m0 > 0) {  // more points into the same totals, with fresh work counters
+                g.kb_total = (int)(pad / kBK);
+                RP_CUDA(cudaMemsetAsync(g.next_unit, 0, sizeof(int) * gram_launches(ctx, g), stream));
+            }
+            split_words_kernel<<<dim3(ceil_div(pad, 32), ceil_div(wc.n(), 32)), dim3(32, 8), 0, stream>>>(
+                P + m0 * N, part, pad, N, wc, V + m0, mx, X[0], X[1], X[2], X[3]);
+            RP_LAUNCH_CHECK();
+            launch_gram(ctx, Xq, 2 * wc.n(), pad, g, stream);
+        }
+        combine_words_kernel<<<ceil_div((long long)wc.n() * wc.n(), 256), 256, 0, stream>>>(g.out_hi, g.out_lo, g.ntj, N,
+                                                                                           wc, mx, G, r);
+        RP_LAUNCH_CHECK();
+    };
+    auto first = [&](int b) { return b * block; };
+    auto size = [&](int b) { return std::min(block, Np - b * block); };
+    if (nb == 1) gram(WordCols{0, Np, 0, 0, 1, 0});
+    for (int i = 0; i < nb; ++i)  // each pair once; a block's own products with its successor, the last's with its predecessor
+        for (int j = i + 1; j < nb; ++j)
+            gram(WordCols{first(i), size(i), first(j), size(j), j == i + 1, j == nb - 1 && j == i + 1});
 }
 
 }  // namespace rp

@@ -604,7 +604,7 @@ void gram_fp64(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, cons
         RP_LAUNCH_CHECK();
         // the exact two-word Gram on the tensor cores (G full, r included)
         StageTimer t_g(ctx, "fp64_gram_words", stream);
-        gram_words_fp64(ctx, P, rows, N, Vc_dev + m0, G, r, stream);
+        gram_words_fp64(ctx, P, rows, N, Vc_dev + m0, G, r, gram_words_bytes(ctx, rows, N), stream);
     }
     column_sums_fp64(Vc_dev, M, 1, 1, sumV, false, ctx, stream);
     shifted_sums_kernel<<<ceil_div(N, 128), 128, 0, stream>>>(sphi, c, M, N, s_c);

@@ -149,7 +149,10 @@ void qeq_run(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, const 
         RP_CUDA(cudaMemsetAsync(d_J, 0, sizeof(double) * N * N, stream));
         RP_CUDA(cudaMemsetAsync(rz, 0, sizeof(double) * N, stream));
         status_clear(ctx, stream);
-        gram_words_fp64(ctx, X, K2, N, zero, d_J, rz, stream);
+        // (at least what this stage's tables and matrix took as a cuBLAS product)
+        const size_t need = (size_t)N * (16 * (size_t)K + 8 * (size_t)N);
+        gram_words_fp64(ctx, X, K2, N, zero, d_J, rz,
+                        scratch_share(ctx, {"w64_X0", "w64_X1", "w64_X2", "w64_X3", "w64_tsum"}, need), stream);
     }
     if (ew->sqrt_alpha > 0.0) tab = erfc_table(ctx, "qeq_erfc", ew->sqrt_alpha, 7.1 / ew->sqrt_alpha, stream);
     {
