@@ -423,10 +423,11 @@ __global__ void __launch_bounds__(1024) number_rows_kernel(const unsigned char *
     if (t == 1023) *R = part[1023];
 }
 
-// stage C: phi[m][a] = Re sum_n1 ex[n1][i] E[rowmap[row]][a][n1]  (one thread per (m, a), a fastest)
+// stage C: phi[m][a] = Re sum_n1 ex[n1][i] E[rowmap[row]][a][n1], rows of phi ld apart  (one thread per
+// (m, a), a fastest)
 __global__ void stage_c64_kernel(const double2 *__restrict__ E, const double2 *__restrict__ ex, int nx, int N,
                                  int P, const int32_t *__restrict__ kept, long long m0, long long rows,
-                                 const int *__restrict__ rowmap, double *__restrict__ phi) {
+                                 const int *__restrict__ rowmap, double *__restrict__ phi, int ld) {
     const int n1c = P + 1;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= rows * N) return;
@@ -439,7 +440,7 @@ __global__ void stage_c64_kernel(const double2 *__restrict__ E, const double2 *_
         const double2 x = ex[(size_t)n1 * nx + i], v = e[n1];
         s += x.x * v.x - x.y * v.y;
     }
-    phi[t] = s;
+    phi[m * ld + a] = s;
 }
 
 }  // namespace
@@ -504,32 +505,57 @@ void gram_fp64(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, cons
     RP_CUDA(cudaMemcpyAsync(d_shifts, sh.data(), sizeof(double) * sh.size(), cudaMemcpyHostToDevice, stream));
     RP_CUDA(cudaMemcpyAsync(d_axis, ew->grid.axis, sizeof(double) * 9, cudaMemcpyHostToDevice, stream));
 
-    // reciprocal part: W and the plane stage once per fit; the FP64 phase tables carry the offset
-    // KMAX on n2 and n3, the sum's range starts at -(KMAX - 1)
-    const int kp = ew->kmax - 1, n1c = kp + 1;  // the separable sum's n range
-    const int nx = ew->grid.n_grid[0], ny = ew->grid.n_grid[1], nz = ew->grid.n_grid[2];
-    const bool recip = ew->K > 0 && kp >= 0;
+    // reciprocal part: the FP64 phase tables carry the offset KMAX on n2 and n3, the sum's range
+    // starts at -(KMAX - 1)
+    const int kp = ew->kmax - 1, n1c = kp + 1, nw = 2 * kp + 1;  // the separable sum's n range
+    const int nx = ew->grid.n_grid[0], ny = ew->grid.n_grid[1], nz = ew->grid.n_grid[2], K = ew->K;
+    const bool recip = K > 0 && kp >= 0;
+    const size_t nrows = (size_t)ny * nz;
+
+    // Points of a chunk, by the sizes alone (each chunk's Gram is rounded once, so what is left of the
+    // scratch budget must not choose it): Phi and the reciprocal rows, at most one per point, within 4 GB;
+    // without them Phi and the Gram's digits within 2 GB.
+    const size_t point = sizeof(double) * (size_t)N, point_words = 16 * ((size_t)N + 1);
+    const size_t per_point = recip ? point + sizeof(double2) * (size_t)N * n1c : point + point_words;
+    int64_t chunk = std::max<int64_t>(256, (int64_t)(((size_t)(recip ? 4 : 2) << 30) / per_point));
+    chunk = std::min<int64_t>(chunk, M);
+
+    // Atoms of a block of the reciprocal sum, whose planes (W, F) and rows (E) are held at a time: all where
+    // they fit, else fewer, with the planes formed again for every chunk.  Each atom's column is its own,
+    // so the blocks do not change it.  The share is at least what an FP64 fit with a flat table of the
+    // K wave vectors holds (the tables of a chunk of points and of the atoms), and for the refit the whole but
+    // for the reciprocal rows that the points cannot need and a copy of the Gram's 2 (N + 1) columns.
+    const size_t most_rows = std::min<size_t>(nrows, (size_t)chunk);
+    auto recip_bytes = [&](size_t atoms_, size_t rows_) {
+        return recip ? 16 * atoms_ * n1c * ((size_t)nw * nw + (size_t)nz * nw + rows_) + 48 * atoms_ * nw : 0;
+    };
+    const size_t words = gram_words_bytes(ctx, chunk, N), whole = recip_bytes(N, most_rows) + point * chunk + words;
+    size_t need;
+    if (refit) {
+        need = recip_bytes(N, (size_t)ceil_div(chunk, nx)) + point * chunk + words + 32 * ((size_t)N + 1) * (N + 1);
+    } else {
+        const size_t flat = 16 * (size_t)K + point, flat_chunk = std::min<size_t>((size_t)M, std::max<size_t>(256, ((size_t)2 << 30) / flat));
+        need = 16 * (size_t)K * N + flat * flat_chunk;
+    }
+    const size_t share = scratch_share(ctx, {"g64_U", "g64_W", "g64_F", "g64_E", "g64_P", "w64_X0", "w64_X1", "w64_X2", "w64_X3", "w64_tsum"}, need);
+    int block = N;
+    size_t words_share = words;
+    if (whole > share) {
+        const size_t rest = share > point * chunk ? share - point * chunk : 0;
+        if (recip) block = (int)std::min<size_t>(N, std::max<size_t>(1, rest / 2 / recip_bytes(1, most_rows)));
+        words_share = rest > recip_bytes(block, most_rows) ? rest - recip_bytes(block, most_rows) : 0;
+        words_share = std::max<size_t>(words_share, 4 << 20);  // (64 columns and 3700 points at a time)
+    }
     double2 *F64 = nullptr;
     float4 *Fdf = nullptr;
-    if (recip) {
+    auto planes = [&](int a0, int na) {
+        if (refit) Fdf = recip_planes64<NumDf>(ctx, ew, d_atoms + 3 * (size_t)a0, na, ew->d_ezf, stream);
+        else F64 = recip_planes64<Num64>(ctx, ew, d_atoms + 3 * (size_t)a0, na, ew->d_ez + nz, stream);
+    };
+    if (recip && block == N) {
         StageTimer tt(ctx, "fp64_recip_sep", stream);
-        if (refit) Fdf = recip_planes64<NumDf>(ctx, ew, d_atoms, N, ew->d_ezf, stream);
-        else F64 = recip_planes64<Num64>(ctx, ew, d_atoms, N, ew->d_ez + nz, stream);
+        planes(0, N);
     }
-
-    // chunk rows so that Phi and the chunk's reciprocal rows, at most one per point, stay within
-    // ~4 GB, and with the Gram's digits within what the ctx has left (less a fifth for the rest)
-    const size_t nrows = (size_t)ny * nz;
-    const size_t row_bytes = sizeof(double) * N + (recip ? sizeof(double2) * (size_t)N * n1c : 0);
-    size_t left = ctx->budget > ctx->used ? ctx->budget - ctx->used : 0;
-    for (const char *name : {"g64_P", "g64_E", "w64_X0", "w64_X1", "w64_X2", "w64_X3", "w64_tsum"})
-        left += ctx->scratch[ctx->slot_key(name)].bytes;
-    const size_t tiles = 16 * (size_t)(2 * N + 130) * (2 * N + 194) / 2;  // the Gram's tile totals
-    const size_t room = left > tiles ? (left - tiles) / 5 * 4 : 0;
-    int64_t chunk = std::min<int64_t>((int64_t)((size_t)4 << 30) / (int64_t)row_bytes,
-                                      (int64_t)(room / (row_bytes + 16 * ((size_t)N + 1))));
-    chunk = std::max<int64_t>(256, chunk);
-    chunk = std::min<int64_t>(chunk, M);
     double *P = ctx->buf_t<double>("g64_P", (size_t)chunk * N);
     double *G = ctx->buf_t<double>("g64_G", (size_t)N * N);
     double *r = ctx->buf_t<double>("g64_r", (size_t)N);
@@ -564,19 +590,23 @@ void gram_fp64(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, cons
             RP_LAUNCH_CHECK();
             number_rows_kernel<<<1, 1024, 0, stream>>>(mark, (int)nrows, rowmap, rowlist, rowlist + most);
             RP_LAUNCH_CHECK();
-            double2 *E64 = ctx->buf_t<double2>("g64_E", (size_t)most * N * n1c);
-            // about 32 blocks per SM, or one per row
-            const unsigned bx = ceil_div((long long)N * n1c, 128);
-            const dim3 nb(bx, (unsigned)std::max<int64_t>(1, std::min<int64_t>(most, 32LL * std::max(1, ctx->sm_count) / bx)));
-            if (refit)
-                stage_b64_kernel<NumDf><<<nb, 128, 0, stream>>>(Fdf, ew->d_eyf, ny, N, kp, rowlist, rowlist + most, E64);
-            else
-                stage_b64_kernel<Num64><<<nb, 128, 0, stream>>>(F64, ew->d_ey + ny, ny, N, kp, rowlist, rowlist + most,
-                                                                E64);
-            RP_LAUNCH_CHECK();
-            stage_c64_kernel<<<ceil_div(rows * N, 128), 128, 0, stream>>>(E64, ew->d_ex, nx, N, kp, kept_idx_dev, m0,
-                                                                          rows, rowmap, P);
-            RP_LAUNCH_CHECK();
+            double2 *E64 = ctx->buf_t<double2>("g64_E", (size_t)most * block * n1c);
+            for (int a0 = 0; a0 < N; a0 += block) {
+                const int na = std::min(block, N - a0);
+                if (block < N) planes(a0, na);
+                // about 32 blocks per SM, or one per row
+                const unsigned bx = ceil_div((long long)na * n1c, 128);
+                const dim3 nb(bx, (unsigned)std::max<int64_t>(1, std::min<int64_t>(most, 32LL * std::max(1, ctx->sm_count) / bx)));
+                if (refit)
+                    stage_b64_kernel<NumDf><<<nb, 128, 0, stream>>>(Fdf, ew->d_eyf, ny, na, kp, rowlist, rowlist + most, E64);
+                else
+                    stage_b64_kernel<Num64><<<nb, 128, 0, stream>>>(F64, ew->d_ey + ny, ny, na, kp, rowlist, rowlist + most,
+                                                                    E64);
+                RP_LAUNCH_CHECK();
+                stage_c64_kernel<<<ceil_div(rows * na, 128), 128, 0, stream>>>(E64, ew->d_ex, nx, na, kp, kept_idx_dev, m0,
+                                                                               rows, rowmap, P + a0, N);
+                RP_LAUNCH_CHECK();
+            }
         } else {  // the non-periodic basis has no reciprocal part
             RP_CUDA(cudaMemsetAsync(P, 0, sizeof(double) * (size_t)rows * N, stream));
         }
@@ -604,7 +634,7 @@ void gram_fp64(rp_ctx *ctx, const rp_ewald *ew, const double *atoms, int N, cons
         RP_LAUNCH_CHECK();
         // the exact two-word Gram on the tensor cores (G full, r included)
         StageTimer t_g(ctx, "fp64_gram_words", stream);
-        gram_words_fp64(ctx, P, rows, N, Vc_dev + m0, G, r, gram_words_bytes(ctx, rows, N), stream);
+        gram_words_fp64(ctx, P, rows, N, Vc_dev + m0, G, r, words_share, stream);
     }
     column_sums_fp64(Vc_dev, M, 1, 1, sumV, false, ctx, stream);
     shifted_sums_kernel<<<ceil_div(N, 128), 128, 0, stream>>>(sphi, c, M, N, s_c);
