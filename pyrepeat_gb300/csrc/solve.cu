@@ -949,26 +949,23 @@ __global__ void __launch_bounds__(kSolve) lu_solve_refine_kernel(const SolveDesc
 }
 
 // ---------------------------------------------------------------------------
-// Wide factorisation of one system beyond kLUAcrossMax unknowns across the whole GPU, before its
-// refinement.  One CTA factoring n1^3 / 3 FMAs alone is SM-bound (20 ms at n1 = 1456 in FP32,
-// and FP64 runs at 1/64 of the FP32 rate); here only the panels are serial.  A0 is copied into
-// As (FP32 for the first attempt, FP64 when that does not converge), then per panel of nb
-// columns (32, or 16 / 8 / 4 when the panel's rows do not fit shared memory at 32):
+// FP32 factorisation of one system beyond kLUAcrossMax unknowns across the whole GPU, before its
+// refinement.  One CTA factoring n1^3 / 3 FMAs alone is SM-bound (20 ms at n1 = 1456); here only the
+// panels are serial.  A0 is copied into As in FP32, then per panel of nb columns (32, or 16 / 8 / 4
+// when the panel's rows do not fit shared memory at 32):
 //   lu_panel_kernel   one CTA: the panel in shared memory, factored with the partial pivoting
-//                     of the one-CTA factorisations (perm[k] = pivot row, full-row swaps; in
-//                     FP64 a pivot below 1e-300 is replaced and flagged, as there), written
-//                     back, its swaps applied to every other column;
+//                     of the one-CTA factorisations (perm[k] = pivot row, full-row swaps),
+//                     written back, its swaps applied to every other column;
 //   lu_trsm_kernel    U12 = L11^-1 A12, a thread per column over many CTAs;
-//   cuBLAS GEMM       A22 -= L21 U12 (SGEMM or DGEMM, plain GEMM).
-// pre = {flag, min|pivot|, max|pivot|}.  FP32: flag 1 = zero or non-finite pivot (the later
-// panels return at once), set to 2 by lu_solve_refine_kernel when the refinement does not
-// converge.  FP64: flag 1 = a pivot was replaced (singular).
+//   cuBLAS SGEMM      A22 -= L21 U12 (a plain product).
+// pre = {flag, min|pivot|, max|pivot|}: flag 1 = zero or non-finite pivot (the later panels return at
+// once).  refine_across refines; refine_wide32 by substitution or factor_refine_wide64 in FP64 take
+// over when it says so.
 constexpr size_t kPanelSmem = 225 * 1024;
 
-template <typename T>
 int wide_panel_nb(int m) {
     for (int nb = 32; nb >= 4; nb /= 2)
-        if (sizeof(T) * (size_t)m * (nb + 1) <= kPanelSmem) return nb;
+        if (sizeof(float) * (size_t)m * (nb + 1) <= kPanelSmem) return nb;
     return 0;
 }
 
@@ -984,67 +981,48 @@ __global__ void lu_copy_kernel(const double *__restrict__ A0, T *__restrict__ L,
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kLU) lu_panel_kernel(T *__restrict__ A, int *__restrict__ perm, int n1, int k0,
+__global__ void __launch_bounds__(kLU) lu_panel_kernel(float *__restrict__ A, int *__restrict__ perm, int n1, int k0,
                                                        int NB, double *__restrict__ pre) {
-    constexpr bool f32 = sizeof(T) == 4;
-    if (f32 && pre[0] != 0.0) return;  // an earlier panel met a zero pivot
-    extern __shared__ __align__(16) unsigned char panel_raw[];
-    T *P = reinterpret_cast<T *>(panel_raw);  // [m][NB + 1] panel rows k0..n1-1
-    __shared__ double svd[kLU / 32];
+    if (pre[0] != 0.0) return;  // an earlier panel met a zero pivot
+    extern __shared__ __align__(16) float P[];  // [m][NB + 1] panel rows k0..n1-1
+    __shared__ double sv[kLU / 32];
     __shared__ int si[kLU / 32];
     __shared__ int piv_i;
-    __shared__ double piv_v;
     const int m = n1 - k0, nb = min(NB, m), ld = NB + 1;
     for (int t = threadIdx.x; t < m * NB; t += kLU) {
         const int r = t / NB, c = t - r * NB;
-        P[r * ld + c] = c < nb ? A[(size_t)(k0 + r) * n1 + k0 + c] : T(0);
+        P[r * ld + c] = c < nb ? A[(size_t)(k0 + r) * n1 + k0 + c] : 0.f;
     }
     __syncthreads();
     double pmin_l = 1e308, pmax_l = 0.0;
-    bool sing = false;
     for (int j = 0; j < nb; ++j) {
-        T best = T(-1);
+        float best = -1.f;
         int bi = 0x7fffffff;
         for (int r = j + threadIdx.x; r < m; r += kLU) {
-            const T v = fabs(P[r * ld + j]);
+            const float v = fabsf(P[r * ld + j]);
             if (v > best || (v == best && r < bi)) { best = v; bi = r; }
         }
-        if constexpr (f32)
-            block_argmax_f(best, bi, reinterpret_cast<float *>(svd), si, &piv_i);
-        else
-            block_argmax(best, bi, svd, si, &piv_v, &piv_i);
+        block_argmax_f(best, bi, reinterpret_cast<float *>(sv), si, &piv_i);
         const int p = piv_i < m ? piv_i : j;  // no candidate (NaN): stay
         if (threadIdx.x == 0) perm[k0 + j] = k0 + p;
         if (p != j && threadIdx.x < NB) {
-            const T t = P[j * ld + threadIdx.x];
+            const float t = P[j * ld + threadIdx.x];
             P[j * ld + threadIdx.x] = P[p * ld + threadIdx.x];
             P[p * ld + threadIdx.x] = t;
         }
         __syncthreads();
-        T pv = P[j * ld + j];
-        const T apv = fabs(pv);
-        if constexpr (f32) {
-            if (!(apv > 0.f) || !isfinite(pv)) {  // uniform: every thread read the same pivot
-                if (threadIdx.x == 0) pre[0] = 1.0;
-                return;
-            }
-        } else {
-            if (!(apv > 1e-300)) {  // exactly singular: a tiny pivot, flagged (as the one-CTA FP64 LU)
-                sing = true;
-                pv = pv < 0 ? T(-1e-300) : T(1e-300);
-                if (threadIdx.x == 0) P[j * ld + j] = pv;
-            }
+        const float pv = P[j * ld + j], apv = fabsf(pv);
+        if (!(apv > 0.f) || !isfinite(pv)) {  // uniform: every thread read the same pivot
+            if (threadIdx.x == 0) pre[0] = 1.0;
+            return;
         }
         pmin_l = fmin(pmin_l, (double)apv);
         pmax_l = fmax(pmax_l, (double)apv);
-        const T inv = T(1) / pv;
-        // a thread per row: one warp instruction covers 32 rows of a column, every lane busy
-        // (the FP64 pipe takes the same time for a warp instruction with one lane or 32)
-        const T *pj = P + j * ld;
-        for (int r = j + 1 + threadIdx.x; r < m; r += kLU) {
-            T *row = P + r * ld;
-            const T l = row[j] * inv;
+        const float inv = 1.f / pv;
+        const float *pj = P + j * ld;
+        for (int r = j + 1 + threadIdx.x; r < m; r += kLU) {  // a thread per row
+            float *row = P + r * ld;
+            const float l = row[j] * inv;
             row[j] = l;
             for (int c = j + 1; c < nb; ++c) row[c] -= l * pj[c];
         }
@@ -1059,7 +1037,7 @@ __global__ void __launch_bounds__(kLU) lu_panel_kernel(T *__restrict__ A, int *_
         for (int j = 0; j < nb; ++j) {
             const int p = perm[k0 + j];
             if (p != k0 + j) {
-                const T t = A[(size_t)(k0 + j) * n1 + c];
+                const float t = A[(size_t)(k0 + j) * n1 + c];
                 A[(size_t)(k0 + j) * n1 + c] = A[(size_t)p * n1 + c];
                 A[(size_t)p * n1 + c] = t;
             }
@@ -1068,26 +1046,25 @@ __global__ void __launch_bounds__(kLU) lu_panel_kernel(T *__restrict__ A, int *_
     if (threadIdx.x == 0) {
         pre[1] = fmin(pre[1], pmin_l);
         pre[2] = fmax(pre[2], pmax_l);
-        if (!f32 && sing) pre[0] = 1.0;
     }
 }
 
-template <typename T, int NB>
-__global__ void __launch_bounds__(256) lu_trsm_kernel(T *__restrict__ A, int n1, int k0,
+template <int NB>
+__global__ void __launch_bounds__(256) lu_trsm_kernel(float *__restrict__ A, int n1, int k0,
                                                       const double *__restrict__ pre) {
-    if (sizeof(T) == 4 && pre[0] != 0.0) return;
-    __shared__ T Ls[NB][NB + 1];
+    if (pre[0] != 0.0) return;
+    __shared__ float Ls[NB][NB + 1];
     const int nb = min(NB, n1 - k0), c1 = k0 + nb;
     for (int t = threadIdx.x; t < NB * NB; t += blockDim.x) {
         const int i = t / NB, j = t - i * NB;
-        Ls[i][j] = (i < nb && j < nb) ? A[(size_t)(k0 + i) * n1 + k0 + j] : T(0);
+        Ls[i][j] = (i < nb && j < nb) ? A[(size_t)(k0 + i) * n1 + k0 + j] : 0.f;
     }
     __syncthreads();
     const int c = c1 + blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= n1) return;
-    T u[NB];
+    float u[NB];
 #pragma unroll
-    for (int j = 0; j < NB; ++j) u[j] = j < nb ? A[(size_t)(k0 + j) * n1 + c] : T(0);
+    for (int j = 0; j < NB; ++j) u[j] = j < nb ? A[(size_t)(k0 + j) * n1 + c] : 0.f;
 #pragma unroll
     for (int j = 0; j < NB; ++j)
 #pragma unroll
@@ -1464,11 +1441,6 @@ void lu_smem_optin() {
     smem_optin((const void *)lu_solve_refine_kernel<true>, solve_smem_bytes(kLUWideMin - 1));
 }
 
-inline cublasStatus_t gemm_nn(cublasHandle_t h, int m, int n, int k, const float *alpha, const float *A, int lda,
-                              const float *B, int ldb, const float *beta, float *C, int ldc) {
-    return cublasSgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc);
-}
-
 // ---- FP64 wide factorisation by cuSOLVER's getrf
 // The bordered matrix K is symmetric, so its row-major image is also K read column-major and
 // cuSOLVER's getrf factors it in place (P K = L U, column-major), with its panels across the
@@ -1660,7 +1632,7 @@ void factor_refine_wide64(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t 
 
 // ---- refinement across the GPU with wide FP32 factors
 // The refinement of lu_solve_refine_kernel for a system whose FP32 factors were computed across
-// the GPU (lu_wide_factor<float>): the same steps (scaled FP32 corrections, FP64 residuals, the
+// the GPU (lu_wide_factor): the same steps (scaled FP32 corrections, FP64 residuals, the
 // backward-error stop) and the same condition estimate, as rounds of three
 // launches that decide on the device and return at once when there is nothing left to do:
 //   across_control_kernel   one CTA: what the last round's results mean for the refinement and
@@ -2237,36 +2209,35 @@ __global__ void __launch_bounds__(1024) order_of_swaps_kernel(int *__restrict__ 
     __syncthreads();
     for (int t = threadIdx.x; t < n; t += blockDim.x) perm[t] = osm[n + t];
 }
-template <typename T>
 void lu_wide_factor(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &tag, cudaStream_t stream) {
-    T *L = reinterpret_cast<T *>(d.As);
+    float *L = reinterpret_cast<float *>(d.As);
     const long long nn = (long long)n1 * n1;
-    lu_copy_kernel<T><<<(int)std::min<long long>(ceil_div(nn, 256), 4096), 256, 0, stream>>>(d.A0, L, nn, d.pre);
+    lu_copy_kernel<float><<<(int)std::min<long long>(ceil_div(nn, 256), 4096), 256, 0, stream>>>(d.A0, L, nn, d.pre);
     RP_LAUNCH_CHECK();
     if (n1 <= kLUAcrossMax) {
         lu_factor_across(ctx, d, n1, tag, stream);
         return;
     }
-    smem_optin((const void *)lu_panel_kernel<T>, kPanelSmem);
+    smem_optin((const void *)lu_panel_kernel, kPanelSmem);
     cublasHandle_t h = ctx->blas();
     RP_CUBLAS(cublasSetStream(h, stream));
-    const T minus_one = T(-1), one = T(1);
+    const float minus_one = -1.f, one = 1.f;
     for (int k0 = 0; k0 < n1;) {
-        const int m = n1 - k0, NB = wide_panel_nb<T>(m), nb = std::min(NB, m), c1 = k0 + nb;
-        lu_panel_kernel<T><<<1, kLU, sizeof(T) * (size_t)m * (NB + 1), stream>>>(L, d.perm, n1, k0, NB, d.pre);
+        const int m = n1 - k0, NB = wide_panel_nb(m), nb = std::min(NB, m), c1 = k0 + nb;
+        lu_panel_kernel<<<1, kLU, sizeof(float) * (size_t)m * (NB + 1), stream>>>(L, d.perm, n1, k0, NB, d.pre);
         RP_LAUNCH_CHECK();
         if (c1 < n1) {
             const int w = n1 - c1, grid = (int)ceil_div(w, 256);
             switch (NB) {
-                case 32: lu_trsm_kernel<T, 32><<<grid, 256, 0, stream>>>(L, n1, k0, d.pre); break;
-                case 16: lu_trsm_kernel<T, 16><<<grid, 256, 0, stream>>>(L, n1, k0, d.pre); break;
-                case 8: lu_trsm_kernel<T, 8><<<grid, 256, 0, stream>>>(L, n1, k0, d.pre); break;
-                default: lu_trsm_kernel<T, 4><<<grid, 256, 0, stream>>>(L, n1, k0, d.pre); break;
+                case 32: lu_trsm_kernel<32><<<grid, 256, 0, stream>>>(L, n1, k0, d.pre); break;
+                case 16: lu_trsm_kernel<16><<<grid, 256, 0, stream>>>(L, n1, k0, d.pre); break;
+                case 8: lu_trsm_kernel<8><<<grid, 256, 0, stream>>>(L, n1, k0, d.pre); break;
+                default: lu_trsm_kernel<4><<<grid, 256, 0, stream>>>(L, n1, k0, d.pre); break;
             }
             RP_LAUNCH_CHECK();
             // row-major A22 (w x w) -= L21 (w x nb) U12 (nb x w), as column-major C^T -= U12^T L21^T
-            RP_CUBLAS(gemm_nn(h, w, w, nb, &minus_one, L + (size_t)k0 * n1 + c1, n1, L + (size_t)c1 * n1 + k0, n1,
-                              &one, L + (size_t)c1 * n1 + c1, n1));
+            RP_CUBLAS(cublasSgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, w, w, nb, &minus_one, L + (size_t)k0 * n1 + c1, n1,
+                                  L + (size_t)c1 * n1 + k0, n1, &one, L + (size_t)c1 * n1 + c1, n1));
         }
         k0 = c1;
     }
@@ -2515,7 +2486,7 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
             RP_CUDA(cudaStreamSynchronize(stream));
         }
     }
-    // large systems: factored across the GPU first (lu_solve_refine_kernel then refines them)
+    // large systems: factored across the GPU first (refine_across then refines the wide ones, their CTA the others)
     bool any_wide = false, any_pre = false;
     for (int j = 0; j < nj; ++j) any_pre |= descs[j].pre != nullptr;
     if (pend) *pend = SolvePending{};
@@ -2526,7 +2497,7 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         if (descs[j].host64 && !descs[j].across) continue;
         {
             StageTimer tt(ctx, "solve_lu_wide", stream);
-            lu_wide_factor<float>(ctx, descs[j], plans[j].n + 1, tag, stream);
+            lu_wide_factor(ctx, descs[j], plans[j].n + 1, tag, stream);
         }
         if (descs[j].host32) refine_across(ctx, descs[j], plans[j].n + 1, 0, kAcRounds, tag + "#" + std::to_string(j), stream);
     }
