@@ -49,3 +49,27 @@ def test_kept_points_follow_the_rule(cell, factor, vmax, gpu_ctx):
     kept, _, M, _ = gpu_ctx.filter(n_grid, axis, atoms, Z, V, factor, vmax)
     got = np.sort(kept.cpu().numpy()[:int(M)])
     assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("cell", ["cubic", "slanted", "flat", "far"])
+def test_no_point_is_kept_where_the_rule_keeps_none(cell, gpu_ctx):
+    """The same cells at factors up to spheres that cover them: where the rule rejects every point, so does the
+    filter."""
+    import torch
+    axis = {"cubic": np.diag([0.5, 0.5, 0.5]), "slanted": np.array([[0.5, 0, 0], [-0.3, 0.45, 0], [0.2, -0.25, 0.5]]),
+            "flat": np.diag([0.9, 0.02, 0.7]), "far": np.diag([0.4, 0.5, 0.6])}[cell]
+    n_grid = np.array([23, 18, 27])
+    box = axis * n_grid[:, None]
+    rng = np.random.default_rng(len(cell))
+    atoms = rng.random((5, 3)) @ box
+    if cell == "far":
+        atoms += np.array([2.6, 0.0, -1.4]) @ box
+    Z = np.array([1, 6, 8, 30, 16])
+    radius = np.array([2.72687, 3.63867, 3.30702, 2.61066, 3.81252])
+    V = torch.from_numpy(rng.normal(size=int(np.prod(n_grid)))).cuda()
+    empty = 0
+    for factor, vmax in ((4.0, 1000.0), (8.0, 1000.0), (1.0, 0.9), (4.0, 3.0)):
+        if len(_rule(n_grid, axis, atoms, radius, factor, vmax)) == 0:
+            empty += 1
+            assert gpu_ctx.filter(n_grid, axis, atoms, Z, V, factor, vmax)[2] == 0, (factor, vmax)
+    assert empty > 0
