@@ -53,8 +53,8 @@ extern "C" {
 #define RP_SOLVE_INFO_WORDS 4
 /* Words per cube of rp_fit_batch's (and rp_batch_submit's) info_out: [0] residual,
  * [1] min |pivot|, [2] max |pivot|, [3] singular flag, [4] kappa (as above), [5] the
- * factorisation that solved it (0 FP32 LU in one CTA, 1 FP32 LU across the GPU, 2 FP64 LU in
- * one CTA, 3 FP64 LU across the GPU; FP32 factors are refined with FP64 residuals),
+ * factors that solved it (0 FP32, refined in one CTA, 1 FP32, refined across the GPU, 2 FP64 in
+ * one CTA, 3 FP64 across the GPU; FP32 factors are refined with FP64 residuals),
  * [6] the precision that produced the charges (RP_PREC_*), [7] RP_FIT_* flags. */
 #define RP_FIT_INFO_WORDS 8
 #define RP_FIT_ESCALATED 1 /* mixed-precision cube refitted in FP64: kappa/(n+1) above the limit */

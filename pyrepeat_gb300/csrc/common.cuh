@@ -567,11 +567,10 @@ struct SolveDesc {
                           // kappa, unknowns n+1, refinement steps, factorisation path
     double *pre;          // null, or {flag, min|piv|, max|piv|} of a wide factorisation already in As
     int wide64;           // As holds wide FP64 factors: skip the FP32 stage and the in-CTA FP64 LU
-    int host64;           // FP32 factors in the CTA, but a stalled refinement goes to the host's FP64
-                          // factorisation across the GPU (pre holds its flag) instead of an in-CTA FP64 LU
     int big;              // the in-CTA solve's vectors are kept in memory
     int across;           // FP32 factors already in As, their row order in perm and pivot range in pre
-    int host32;           // factored and refined across the GPU (lu_wide_factor, refine_across): the kernel skips it
+    int factor_only;      // FP32 factors only, for the rounds (refine_across): row order to perm, flag and pivots to pre
+    int host32;           // factored across the GPU for the rounds: the in-CTA kernel skips it
 };
 // Wide systems of a solve launch whose FP32 refinement may not have converged: their flags are
 // on their way to pinned memory; solve_wide_fp64 (after the stream has reached them) factors
@@ -582,6 +581,8 @@ struct SolvePending {
     double *h_pre = nullptr, *h_info = nullptr, *d_info = nullptr;
     std::vector<SolveDesc> descs;
     std::vector<int> n1;
+    std::vector<std::string> keys;  // names of their buffers of the refinement across the GPU
+    bool shared = false;            // ... of which several systems below kLUWideMin share some
 };
 // The same without waiting: returns the pinned host copy of the kSolveInfo words per job, valid
 // once `stream` has reached this point.  `tag` keeps the scratch of solves in flight apart.

@@ -23,8 +23,8 @@
 // refinement.  Either way the refined residual and the pivot range are reported.
 // Systems of kLUWideMin or more unknowns are factored and refined across the whole GPU instead of by
 // their CTA (lu_wide_factor, refine_across), in FP32 and, when that stalls, in FP64
-// (factor_refine_wide64).  A single one of kLUHost64Min or more is factored across the GPU, to the
-// same factors as its CTA's, and refined by its CTA.
+// (factor_refine_wide64).  Those of kLUHost64Min or more are refined across it too, and factored
+// across it when single; several of a launch are factored in their CTAs, to the same bits.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -715,11 +715,14 @@ constexpr int kRefineMax = 30;  // and stop early once a step no longer halves t
 // that fit shared memory at 4 columns; FP64 by cuSOLVER when the FP32 refinement does not
 // converge): n1 in [kLUWideMin, kLUWideMax]
 constexpr int kLUWideMin = 768;
-// systems of kLUHost64Min to kLUWideMin unknowns keep their FP32 factorisation in the CTA when a
-// launch holds several, but when its refinement stalls the FP64 factors come from across the GPU (cuSOLVER getrf): an
-// in-CTA FP64 LU of 425 unknowns takes ~13 ms on one SM's FP64 pipe
+// systems of kLUHost64Min to kLUWideMin unknowns are refined with the wide ones' rounds, and their FP64
+// factors come from across the GPU too (an in-CTA FP64 LU of 425 unknowns takes ~13 ms on one SM's FP64
+// pipe); their FP32 factors come from their CTA when a launch holds several
 constexpr int kLUHost64Min = 256;
-constexpr int kAcrossTwo = 512;  // least unknowns for two systems of a launch to be factored across the GPU
+// least unknowns for two systems of a launch, or one beside smaller ones, to be factored across the GPU one after
+// the other: 0.88 ms for two against 1.06 side by side in their CTAs at 521 unknowns, 0.70 against
+// 0.69 at 421; and a system of 255 takes 0.69 ms in its CTA anyway
+constexpr int kAcrossTwo = 512;
 constexpr int kLUWideMax = (int)((225 * 1024) / (sizeof(float) * 5));
 
 // r = bs - A0 x in FP64: a warp per eight rows, lanes along the row.  The rows' sums over the lanes
@@ -807,6 +810,15 @@ __global__ void __launch_bounds__(kSolve) lu_solve_refine_kernel(const SolveDesc
         } else if (n1 <= kLUBlockedMax && !big) {
             float *work = fsh + ((3 * n1 + 3) & ~3);
             factored = lu_factor_f32_blocked(L, orig, n1, work, lus, pmin, pmax);
+            if (d.factor_only) {  // the rounds refine it
+                for (int t = threadIdx.x; t < n1; t += blockDim.x) d.perm[t] = orig[t];
+                if (threadIdx.x == 0) {
+                    d.pre[0] = factored ? 0.0 : 1.0;
+                    d.pre[1] = pmin;
+                    d.pre[2] = pmax;
+                }
+                return;
+            }
         } else {
             factored = lu_factor_f32(L, d.perm, n1, sv, si, &piv_v, &piv_i, pmin, pmax);
             if (threadIdx.x == 0) {  // the interchanges as a row order
@@ -1666,20 +1678,29 @@ struct AcrossState {
     int xsel, finished;     // which x holds the solution; nothing left to do
 };
 struct AcrossRun {
-    const float *LU;        // factors
+    const float *LU;        // factors, row i of them row perm[i] of K
     float *inv;             // inverses of their diagonal blocks, L's then U's, and behind them the blocks
     float *V, *Y;           // [3][n1] right-hand sides and solutions
     double *x[2];           // solution before and after a round
     AcrossState *st;
-    SolveDesc d;
-    int n1, nblk;
+    const double *A0, *bs;  // SolveDesc's
+    double *r, *q, *info, *pre;
+    const int *perm, *map;
+    int N, n1, nblk;
+};
+// The systems of a launch, one to a row of its grid.  Nothing of one system's work depends on the others, so
+// its results are the same bits in any company.
+constexpr int kAcSystems = 16;
+struct AcrossLaunch {
+    AcrossRun run[kAcSystems];
 };
 
 // max row sums of |K| and |A| (K symmetric), a warp per row; st cleared before
-__global__ void __launch_bounds__(256) across_norms_kernel(AcrossRun p) {
+__global__ void __launch_bounds__(256) across_norms_kernel(const __grid_constant__ AcrossLaunch L) {
+    const AcrossRun &p = L.run[blockIdx.y];
     const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31, n1 = p.n1;
     if (r >= n1) return;
-    const double *row = p.d.A0 + (size_t)r * n1;
+    const double *row = p.A0 + (size_t)r * n1;
     double s = 0.0;
     for (int c = lane; c < n1 - 1; c += 32) s += fabs(row[c]);
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -1694,13 +1715,15 @@ __global__ void __launch_bounds__(256) across_norms_kernel(AcrossRun p) {
 // hold 32 of its rows each in registers (rows 16 g + 4 q + 0..3), column by column of the triangle: 16
 // steps in line, then the registers move up by 16 rows, so the code stays small.  (Dot products
 // from shared memory, row by row, took 100 us at any size.)  Rows past the end: identity.
-constexpr int kInvLD = kAcB + 4, kInvCols = 64, kInvT = 4 * kInvCols;  // blockIdx.z: which 64 columns
-__global__ void __launch_bounds__(kInvT) across_invert_kernel(AcrossRun p) {
+constexpr int kInvLD = kAcB + 4, kInvCols = 64, kInvT = 4 * kInvCols;  // blockIdx.z: the system and which 64 columns
+__global__ void __launch_bounds__(kInvT) across_invert_kernel(const __grid_constant__ AcrossLaunch L) {
+    const AcrossRun &p = L.run[blockIdx.z / (kAcB / kInvCols)];
     extern __shared__ __align__(16) float ash[];
     float *B = ash, *dinv = ash + kAcB * kInvLD;  // B[k][i]: column k below the diagonal
     chain_begin();
-    if (p.d.pre[0] != 0.0) return;
-    const int n1 = p.n1, b0 = blockIdx.x * kAcB, tid = threadIdx.x, lane = tid & 31, c = blockIdx.z * kInvCols + (tid >> 2), q = tid & 3;
+    if ((int)blockIdx.x >= p.nblk || p.pre[0] != 0.0) return;
+    const int half = blockIdx.z % (kAcB / kInvCols);
+    const int n1 = p.n1, b0 = blockIdx.x * kAcB, tid = threadIdx.x, lane = tid & 31, c = half * kInvCols + (tid >> 2), q = tid & 3;
     const bool rev = blockIdx.y == 1;
 #pragma unroll 16
     for (int t = tid; t < kAcB * kAcB; t += kInvT) {
@@ -1717,7 +1740,7 @@ __global__ void __launch_bounds__(kInvT) across_invert_kernel(AcrossRun p) {
     float *out = p.inv + ((size_t)blockIdx.y * p.nblk + blockIdx.x) * kAcB * kAcB;
     float *tri = out + 2 * (size_t)p.nblk * kAcB * kAcB;  // the block's own triangle, zeros elsewhere
     for (int t = tid; t < kAcB * kInvCols; t += kInvT) {
-        const int i = t / kInvCols, j = blockIdx.z * kInvCols + t % kInvCols;
+        const int i = t / kInvCols, j = half * kInvCols + t % kInvCols;
         float v = i == j ? 1.f : 0.f;
         if ((rev ? j >= i : j < i) && b0 + i < n1 && b0 + j < n1) v = p.LU[(size_t)(b0 + i) * n1 + b0 + j];
         tri[i * kAcB + j] = v;
@@ -1746,7 +1769,8 @@ __global__ void __launch_bounds__(kInvT) across_invert_kernel(AcrossRun p) {
 
 // pre[0] at the end (last): 0 solved, 2 zero pivot, 3 not finished, 4 substitution (with the estimate
 // in info); 3 is taken back by the rounds that follow
-__global__ void __launch_bounds__(1024) across_control_kernel(AcrossRun p, int round, int last) {
+__global__ void __launch_bounds__(1024) across_control_kernel(const __grid_constant__ AcrossLaunch L, int round, int last) {
+    const AcrossRun &p = L.run[blockIdx.x];
     __shared__ double sv[33], piv_v;
     __shared__ int si[32], piv_i;
     __shared__ AcrossState st;
@@ -1758,8 +1782,8 @@ __global__ void __launch_bounds__(1024) across_control_kernel(AcrossRun p, int r
     if (round == 0) {
         double m = 0.0;
         for (int t = tid; t < n1; t += nt) {
-            const double b = p.d.bs[t];
-            p.d.r[t] = b;
+            const double b = p.bs[t];
+            p.r[t] = b;
             p.x[0][t] = 0.0;
             m = fmax(m, fabs(b));
         }
@@ -1771,7 +1795,7 @@ __global__ void __launch_bounds__(1024) across_control_kernel(AcrossRun p, int r
             st.steps = st.hit = st.hstate = st.xsel = 0;
             st.jprev = -1;
             st.est = st.alt = 0.0;
-            st.phase = p.d.pre[0] != 0.0 ? 3 : m == 0.0 ? 1 : 0;
+            st.phase = p.pre[0] != 0.0 ? 3 : m == 0.0 ? 1 : 0;
         }
         for (int t = tid; t < n1; t += nt) {
             p.V[n1 + t] = (float)(1.0 / (double)n1);
@@ -1852,29 +1876,29 @@ __global__ void __launch_bounds__(1024) across_control_kernel(AcrossRun p, int r
     __syncthreads();
     if (st.phase == 0) {
         const double rm = st.rm;
-        for (int t = tid; t < n1; t += nt) p.V[t] = (float)(p.d.r[t] / rm);
+        for (int t = tid; t < n1; t += nt) p.V[t] = (float)(p.r[t] / rm);
     }
     const bool solved = st.hstate == 3 && (st.phase == 1 || st.phase == 2);
     if (solved && st.phase == 1) {  // the solution, expanded to all atoms
         const double *x = p.x[st.xsel];
-        for (int i = tid; i < p.d.N; i += nt) p.d.q[i] = x[p.d.map[i]];
+        for (int i = tid; i < p.N; i += nt) p.q[i] = x[p.map[i]];
     }
     if (tid == 0) {
         if (solved) {
             const double est = fmax(st.est, st.alt), kinv = est < 1e300 ? est : 1e300;
-            p.d.info[0] = st.res;
-            p.d.info[1] = p.d.pre[1];
-            p.d.info[2] = p.d.pre[2];
-            p.d.info[3] = 0.0;
-            p.d.info[4] = fmin(__longlong_as_double((long long)st.anorm_bits) * kinv, 1e300);
-            p.d.info[5] = n1;
-            p.d.info[6] = st.steps;
-            p.d.info[7] = 1.0;  // FP32 factors from across the GPU
+            p.info[0] = st.res;
+            p.info[1] = p.pre[1];
+            p.info[2] = p.pre[2];
+            p.info[3] = 0.0;
+            p.info[4] = fmin(__longlong_as_double((long long)st.anorm_bits) * kinv, 1e300);
+            p.info[5] = n1;
+            p.info[6] = st.steps;
+            p.info[7] = 1.0;  // FP32 factors from across the GPU
         }
         st.finished = solved || st.phase == 3;
-        if (st.phase == 3) p.d.pre[0] = 2.0;
-        else if (solved) p.d.pre[0] = st.phase == 2 ? 4.0 : 0.0;
-        else if (last) p.d.pre[0] = 3.0;
+        if (st.phase == 3) p.pre[0] = 2.0;
+        else if (solved) p.pre[0] = st.phase == 2 ? 4.0 : 0.0;
+        else if (last) p.pre[0] = 3.0;
         st.rn_bits = st.xn_bits = 0;
         *p.st = st;
     }
@@ -1888,7 +1912,8 @@ __global__ void __launch_bounds__(1024) across_control_kernel(AcrossRun p, int r
 // Bounded by those steps' latency (16 + 16 of them at 2001 unknowns) and by the factors' way from
 // L2 to eight SMs (2 MB each there).
 template <int NR>
-__global__ void __cluster_dims__(kAcCTAs, 1, 1) __launch_bounds__(kAcT) across_apply_kernel(AcrossRun p) {
+__global__ void __cluster_dims__(kAcCTAs, 1, 1) __launch_bounds__(kAcT) across_apply_kernel(const __grid_constant__ AcrossLaunch L) {
+    const AcrossRun &p = L.run[blockIdx.y];
     namespace cg = cooperative_groups;
     constexpr int NS = NR == 3 ? 4 : NR;  // floats per unknown in shared memory
     extern __shared__ __align__(16) float ash[];
@@ -1901,7 +1926,7 @@ __global__ void __cluster_dims__(kAcCTAs, 1, 1) __launch_bounds__(kAcT) across_a
     const int rank = (int)cl.block_rank(), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int n1 = p.n1, nblk = p.nblk, rl = rank * (kAcB / kAcCTAs) + warp;  // the warp's row of each block
     for (int t = tid; t < nblk * kAcB; t += kAcT) {
-        const int o = t < n1 ? p.d.perm[t] : 0;
+        const int o = t < n1 ? p.perm[t] : 0;
 #pragma unroll
         for (int q = 0; q < NR; ++q) xs[t * NS + q] = t < n1 ? p.V[(size_t)q * n1 + o] : 0.f;
     }
@@ -2013,7 +2038,8 @@ __global__ void __cluster_dims__(kAcCTAs, 1, 1) __launch_bounds__(kAcT) across_a
 }
 
 // x' = x + rm y (kept by the first CTA) and r = bs - A0 x' with its largest element, a warp per row
-__global__ void __launch_bounds__(256) across_residual_kernel(AcrossRun p, int round) {
+__global__ void __launch_bounds__(256) across_residual_kernel(const __grid_constant__ AcrossLaunch L, int round) {
+    const AcrossRun &p = L.run[blockIdx.y];
     extern __shared__ double xd[];
     __shared__ unsigned long long top[2];
     chain_begin();
@@ -2035,14 +2061,14 @@ __global__ void __launch_bounds__(256) across_residual_kernel(AcrossRun p, int r
     if (blockIdx.x == 0) atomicMax(&top[1], (unsigned long long)__double_as_longlong(m));
     __syncthreads();
     for (int r = blockIdx.x * 8 + warp; r < n1; r += gridDim.x * 8) {
-        const double *row = p.d.A0 + (size_t)r * n1;
+        const double *row = p.A0 + (size_t)r * n1;
         double s = 0.0;
 #pragma unroll 8
         for (int c = lane; c < n1; c += 32) s = fma(row[c], xd[c], s);
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) {
-            const double v = p.d.bs[r] - s;
-            p.d.r[r] = v;
+            const double v = p.bs[r] - s;
+            p.r[r] = v;
             atomicMax(&top[0], (unsigned long long)__double_as_longlong(fabs(v)));
         }
     }
@@ -2053,46 +2079,64 @@ __global__ void __launch_bounds__(256) across_residual_kernel(AcrossRun p, int r
     }
 }
 
-// Launches rounds first .. first + rounds - 1 of system j of its launch (whose state is kept for the
+// A system for the rounds, and the name of its buffers
+struct AcrossSystem {
+    const SolveDesc *d;
+    std::string key;
+};
+// what a system needs beside its matrices when the second half of As does not hold it
+size_t across_inv_bytes(int n1) { return sizeof(float) * (4 * (size_t)ceil_div(n1, kAcB) * kAcB * kAcB + 6 * (size_t)n1); }
+
+// Launches rounds first .. first + rounds - 1 of up to kAcSystems systems (whose states are kept for the
 // rounds that may follow), then looks at the outcome: pre[0] = 0 (solved: q and info written), 2
 // (zero pivot: FP64 factors), 3 (not finished) or 4 (substitution).
-void refine_across(rp_ctx *ctx, const SolveDesc &d, int n1, int first, int rounds, const std::string &key, cudaStream_t stream) {
+void refine_across(rp_ctx *ctx, const std::vector<AcrossSystem> &sys, int first, int rounds, cudaStream_t stream) {
     StageTimer tt(ctx, "solve_refine32", stream);
-    AcrossRun p{};
-    p.n1 = n1;
-    p.nblk = (int)ceil_div(n1, kAcB);
-    p.LU = reinterpret_cast<const float *>(d.As);
-    p.d = d;
-    // inverses, blocks and vectors go to the second half of As, which is free once the factors are
-    // collected, where they fit there
-    const size_t need = sizeof(float) * (4 * (size_t)p.nblk * kAcB * kAcB + 6 * (size_t)n1), half = sizeof(float) * (size_t)n1 * n1;
-    const uintptr_t free_half = (reinterpret_cast<uintptr_t>(p.LU) + half + 255) & ~(uintptr_t)255;
-    p.inv = need + 255 <= half ? reinterpret_cast<float *>(free_half)
-                               : static_cast<float *>(ctx->buf("s_ac_inv" + key, need));
-    p.V = p.inv + 4 * (size_t)p.nblk * kAcB * kAcB;
-    p.Y = p.V + 3 * (size_t)n1;
-    p.x[0] = d.x;
-    p.x[1] = ctx->buf_t<double>("s_ac_x" + key, (size_t)n1);
-    p.st = ctx->buf_t<AcrossState>("s_ac_st" + key, 1);
+    AcrossLaunch L{};
+    int n1 = 0;  // the largest
+    for (size_t k = 0; k < sys.size(); ++k) {
+        const SolveDesc &d = *sys[k].d;
+        AcrossRun &p = L.run[k];
+        p.n1 = d.n + 1;
+        p.nblk = (int)ceil_div(p.n1, kAcB);
+        p.LU = reinterpret_cast<const float *>(d.As);
+        p.A0 = d.A0; p.bs = d.bs; p.r = d.r; p.q = d.q; p.info = d.info; p.pre = d.pre; p.perm = d.perm; p.map = d.map;
+        p.N = d.N;
+        // inverses, blocks and vectors go to the second half of As, which is free once the factors are
+        // collected, where they fit there
+        const size_t need = across_inv_bytes(p.n1), half = sizeof(float) * (size_t)p.n1 * p.n1;
+        const uintptr_t free_half = (reinterpret_cast<uintptr_t>(p.LU) + half + 255) & ~(uintptr_t)255;
+        p.inv = need + 255 <= half ? reinterpret_cast<float *>(free_half)
+                                   : static_cast<float *>(ctx->buf("s_ac_inv" + sys[k].key, need));
+        p.V = p.inv + 4 * (size_t)p.nblk * kAcB * kAcB;
+        p.Y = p.V + 3 * (size_t)p.n1;
+        p.x[0] = d.x;
+        p.x[1] = ctx->buf_t<double>("s_ac_x" + sys[k].key, (size_t)p.n1);
+        p.st = ctx->buf_t<AcrossState>("s_ac_st" + sys[k].key, 1);
+        n1 = std::max(n1, p.n1);
+    }
+    const unsigned ns = (unsigned)sys.size();
+    const int nblk = (int)ceil_div(n1, kAcB);
     if (first == 0) {
-        RP_CUDA(cudaMemsetAsync(p.st, 0, sizeof(AcrossState), stream));
-        across_norms_kernel<<<(int)ceil_div(n1, 8), 256, 0, stream>>>(p);
+        for (unsigned k = 0; k < ns; ++k) RP_CUDA(cudaMemsetAsync(L.run[k].st, 0, sizeof(AcrossState), stream));
+        across_norms_kernel<<<dim3(ceil_div(n1, 8), ns), 256, 0, stream>>>(L);
         RP_LAUNCH_CHECK();
         const size_t inv_smem = sizeof(float) * (kAcB * kInvLD + kAcB);
         smem_optin((const void *)across_invert_kernel, inv_smem);
-        launch_chained(across_invert_kernel, dim3(p.nblk, 2, kAcB / kInvCols), kInvT, inv_smem, stream, p);
-        launch_chained(across_control_kernel, dim3(1), 1024, 0, stream, p, 0, 0);
+        launch_chained(across_invert_kernel, dim3(nblk, 2, ns * (kAcB / kInvCols)), kInvT, inv_smem, stream, L);
+        launch_chained(across_control_kernel, dim3(ns), 1024, 0, stream, L, 0, 0);
     }
-    const size_t np = (size_t)p.nblk * kAcB, res_smem = sizeof(double) * n1;
+    const size_t np = (size_t)nblk * kAcB, res_smem = sizeof(double) * n1;
     const size_t most = sizeof(float) * 4 * (((size_t)kLUWideMax + kAcB - 1) / kAcB * kAcB + 3 * kAcB);
     smem_optin((const void *)across_apply_kernel<3>, most);
     smem_optin((const void *)across_apply_kernel<2>, most / 2);
     smem_optin((const void *)across_residual_kernel, sizeof(double) * kLUWideMax);
+    const unsigned rows = (unsigned)std::min<long long>(ceil_div(n1, 8), std::max(304u / ns, 32u));
     for (int k = first; k < first + rounds; ++k) {
-        if (k == 0) launch_chained(across_apply_kernel<3>, dim3(kAcCTAs), kAcT, sizeof(float) * 4 * (np + 3 * kAcB), stream, p);
-        else launch_chained(across_apply_kernel<2>, dim3(kAcCTAs), kAcT, sizeof(float) * 2 * (np + 3 * kAcB), stream, p);
-        launch_chained(across_residual_kernel, dim3((unsigned)std::min<long long>(ceil_div(n1, 8), 304)), 256, res_smem, stream, p, k);
-        launch_chained(across_control_kernel, dim3(1), 1024, 0, stream, p, k + 1, (int)(k + 1 == first + rounds));
+        if (k == 0) launch_chained(across_apply_kernel<3>, dim3(kAcCTAs, ns), kAcT, sizeof(float) * 4 * (np + 3 * kAcB), stream, L);
+        else launch_chained(across_apply_kernel<2>, dim3(kAcCTAs, ns), kAcT, sizeof(float) * 2 * (np + 3 * kAcB), stream, L);
+        launch_chained(across_residual_kernel, dim3(rows, ns), 256, res_smem, stream, L, k);
+        launch_chained(across_control_kernel, dim3(ns), 1024, 0, stream, L, k + 1, (int)(k + 1 == first + rounds));
     }
 }
 
@@ -2244,6 +2288,29 @@ void lu_wide_factor(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &
     smem_optin((const void *)order_of_swaps_kernel, 2 * sizeof(int) * kLUWideMax);
     order_of_swaps_kernel<<<1, 1024, 2 * sizeof(int) * (size_t)n1, stream>>>(d.perm, n1, d.pre);
     RP_LAUNCH_CHECK();
+}
+
+// the refinement of lu_solve_refine_kernel alone, on the FP32 factors that the rounds had; pre[0] = 2 where
+// it stalls
+void refine_in_cta(rp_ctx *ctx, const std::vector<const SolveDesc *> &sys, cudaStream_t stream) {
+    StageTimer tt(ctx, "solve_refine32", stream);
+    std::vector<SolveDesc> h;
+    int n1 = 0;
+    for (const SolveDesc *d : sys) {
+        h.push_back(*d);
+        h.back().host32 = h.back().factor_only = 0;
+        h.back().across = 1;
+        n1 = std::max(n1, d->n + 1);
+        RP_CUDA(cudaMemsetAsync(d->pre, 0, sizeof(double), stream));
+    }
+    SolveDesc *dev = ctx->buf_t<SolveDesc>("s_desc_cta", h.size());
+    RP_CUDA(cudaMemcpyAsync(dev, h.data(), sizeof(SolveDesc) * h.size(), cudaMemcpyHostToDevice, stream));
+    lu_smem_optin();
+    prepare_kernel<<<dim3(ceil_div(n1, 8), (unsigned)h.size()), 256, 0, stream>>>(dev);
+    RP_LAUNCH_CHECK();
+    lu_solve_refine_kernel<false><<<(unsigned)h.size(), solve_threads(n1), solve_smem_bytes(n1), stream>>>(dev);
+    RP_LAUNCH_CHECK();
+    RP_CUDA(cudaStreamSynchronize(stream));
 }
 
 }  // namespace
@@ -2411,21 +2478,28 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
             descs[j].pre = d_pre + 3 * (size_t)j;
             if (jobs[j].fp64) descs[j].wide64 = 1;
             else if (n1 >= kLUWideMin) descs[j].host32 = 1;
-            else descs[j].host64 = 1;
         }
         if (plans[j].disjoint) disjoint.push_back(j);
     }
-    // A single system of kLUHost64Min to kLUWideMin unknowns is factored across the GPU, two of them one after the
-    // other from kAcrossTwo; more are factored side by side, each in its CTA.  Both give the same factors, bit
-    // for bit, and its CTA refines it either way, so that charges do not depend on the batch.
-    int mid = 0, least = kLUWideMin;
-    for (int j = 0; j < nj; ++j)
-        if (descs[j].host64) {
-            ++mid;
-            least = std::min(least, plans[j].n + 1);
+    // Between kLUHost64Min and kLUWideMin unknowns a system alone in its launch is factored across the GPU, from
+    // kAcrossTwo also one or two beside smaller ones; others side by side with them, each in its CTA, to
+    // the same factors bit for bit.  All of a launch are refined together by the rounds, so charges do not depend on the
+    // batch.  (Factors and refinement of 16 systems: 0.71 ms at 256 unknowns, 1.2 at 420, 3.3 at 740, against
+    // 0.76, 1.5 and 4.5 with each refined in its CTA; of one: 0.44, 0.64 and 1.1 against 0.71, 1.2 and 2.6.)
+    std::vector<int> rounds;
+    int least = kLUWideMin;
+    for (int j = 0; j < nj; ++j) {
+        const int n1 = plans[j].n + 1;
+        if (!descs[j].pre || descs[j].wide64 || n1 >= kLUWideMin) continue;
+        rounds.push_back(j);
+        least = std::min(least, n1);
+        descs[j].factor_only = 1;
+    }
+    if (nj == 1 || (rounds.size() <= 2 && least >= kAcrossTwo))
+        for (int j : rounds) {
+            descs[j].across = 1;
+            descs[j].host32 = 1;
         }
-    if (mid == 1 || (mid == 2 && least >= kAcrossTwo))
-        for (int j = 0; j < nj; ++j) descs[j].across = descs[j].host64;
     // the small tables go up from one pinned staging block per tag (asynchronous copies that
     // never wait for the stream; a later solve with another tag cannot overwrite them)
     const size_t st_bytes[7] = {sizeof(int) * n_map, sizeof(int) * n_mptr, sizeof(int) * n_midx,
@@ -2486,7 +2560,7 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
             RP_CUDA(cudaStreamSynchronize(stream));
         }
     }
-    // large systems: factored across the GPU first (refine_across then refines the wide ones, their CTA the others)
+    // large systems: factored across the GPU first, the wide ones refined behind their factors
     bool any_wide = false, any_pre = false;
     for (int j = 0; j < nj; ++j) any_pre |= descs[j].pre != nullptr;
     if (pend) *pend = SolvePending{};
@@ -2494,12 +2568,13 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
     for (int j = 0; j < nj; ++j) {
         if (!descs[j].pre || descs[j].wide64) continue;  // wide64: factored and refined after the launch
         any_wide = true;  // its flag is read after the launch
-        if (descs[j].host64 && !descs[j].across) continue;
+        const bool wide = plans[j].n + 1 >= kLUWideMin;
+        if (!wide && !descs[j].across) continue;
         {
             StageTimer tt(ctx, "solve_lu_wide", stream);
             lu_wide_factor(ctx, descs[j], plans[j].n + 1, tag, stream);
         }
-        if (descs[j].host32) refine_across(ctx, descs[j], plans[j].n + 1, 0, kAcRounds, tag + "#" + std::to_string(j), stream);
+        if (wide) refine_across(ctx, {{&descs[j], tag + "#" + std::to_string(j)}}, 0, kAcRounds, stream);
     }
     {
         StageTimer tt(ctx, "solve_lu", stream);
@@ -2521,6 +2596,19 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
             RP_LAUNCH_CHECK();
         }
     }
+    // the rounds of those below kLUWideMin: as many at a time as a launch takes and a quarter of the scratch left
+    // holds, one set after the other in the same buffers
+    size_t each = 1;
+    for (int j : rounds) each = std::max(each, across_inv_bytes(plans[j].n + 1));
+    const size_t set = std::max<size_t>(1, std::min<size_t>(kAcSystems, ctx->room({}) / 4 / each));
+    std::vector<std::string> keys((size_t)nj);
+    for (int j = 0; j < nj; ++j) keys[j] = tag + "#" + std::to_string(j);
+    for (size_t k = 0; k < rounds.size(); ++k) keys[rounds[k]] = tag + "#m" + std::to_string(k % set);
+    for (size_t k0 = 0; k0 < rounds.size(); k0 += set) {
+        std::vector<AcrossSystem> sys;
+        for (size_t k = k0; k < std::min(rounds.size(), k0 + set); ++k) sys.push_back({&descs[rounds[k]], keys[rounds[k]]});
+        refine_across(ctx, sys, 0, kAcRounds, stream);
+    }
     for (int j = 0; j < nj; ++j)  // systems known to need FP64 (an escalated fit): getrf, host-driven refinement
         if (descs[j].wide64) factor_refine_wide64(ctx, descs[j], plans[j].n + 1, stream);
     double *h_info = static_cast<double *>(ctx->host_buf("s_info" + tag, sizeof(double) * kSolveInfo * nj));
@@ -2538,6 +2626,8 @@ const double *solve_batch_async(rp_ctx *ctx, const std::vector<SolveJob> &jobs, 
         pd.h_info = h_info;
         pd.d_info = d_info;
         pd.descs = descs;
+        pd.keys = keys;
+        pd.shared = rounds.size() > set;
         pd.n1.resize((size_t)nj);
         for (int j = 0; j < nj; ++j) pd.n1[j] = plans[j].n + 1;
         if (!pend) {
@@ -2554,21 +2644,34 @@ void solve_wide_fp64(rp_ctx *ctx, SolvePending &pd, cudaStream_t stream) {
     pd.any_wide = false;
     const int nj = (int)pd.descs.size();
     bool any = false;
+    std::vector<double> flag((size_t)nj, 0.0);
+    auto look = [&](int j) { RP_CUDA(cudaMemcpyAsync(&flag[j], pd.descs[j].pre, sizeof(double), cudaMemcpyDeviceToHost, stream)); };
+    std::vector<int> cta;
     for (int j = 0; j < nj; ++j) {
         if (!pd.descs[j].pre || pd.h_pre[3 * j] < 2.0) continue;
-        double flag = pd.h_pre[3 * j];
+        flag[j] = pd.h_pre[3 * j];
         any = true;
-        for (int first = kAcRounds; flag == 3.0; first += 4) {  // not finished: more rounds
-            refine_across(ctx, pd.descs[j], pd.n1[j], first, 4, pd.tag + "#" + std::to_string(j), stream);
-            RP_CUDA(cudaMemcpyAsync(&flag, pd.descs[j].pre, sizeof(flag), cudaMemcpyDeviceToHost, stream));
+        const bool wide = pd.n1[j] >= kLUWideMin;
+        for (int n = 4; flag[j] == 3.0; n += 4) {  // not finished: more rounds, from the start where a later set took the buffers
+            const bool again = !wide && pd.shared;
+            if (again) RP_CUDA(cudaMemsetAsync(pd.descs[j].pre, 0, sizeof(double), stream));
+            refine_across(ctx, {{&pd.descs[j], pd.keys[j]}}, again ? 0 : kAcRounds + n - 4, again ? kAcRounds + n : 4, stream);
+            look(j);
             RP_CUDA(cudaStreamSynchronize(stream));
         }
-        if (flag == 0.0) continue;
-        if (flag == 4.0) {  // by substitution
-            if (refine_wide32(ctx, pd.descs[j], pd.n1[j], pd.tag + "#" + std::to_string(j), stream)) continue;
-        }
-        factor_refine_wide64(ctx, pd.descs[j], pd.n1[j], stream);
+        if (flag[j] != 4.0) continue;  // 4: by substitution
+        if (!wide) cta.push_back(j);
+        else if (refine_wide32(ctx, pd.descs[j], pd.n1[j], pd.keys[j], stream)) flag[j] = 0.0;
     }
+    if (!cta.empty()) {
+        std::vector<const SolveDesc *> sys;
+        for (int j : cta) sys.push_back(&pd.descs[j]);
+        refine_in_cta(ctx, sys, stream);
+        for (int j : cta) look(j);
+        RP_CUDA(cudaStreamSynchronize(stream));
+    }
+    for (int j = 0; j < nj; ++j)
+        if (flag[j] != 0.0) factor_refine_wide64(ctx, pd.descs[j], pd.n1[j], stream);
     if (!any) return;
     RP_CUDA(cudaMemcpyAsync(pd.h_info, pd.d_info, sizeof(double) * kSolveInfo * nj, cudaMemcpyDeviceToHost, stream));
     RP_CUDA(cudaStreamSynchronize(stream));

@@ -34,3 +34,27 @@ def test_mid_size_systems_alone_and_in_batches(n, gpu_ctx):
         for submit in (False, True):
             for m, got in zip(names, fit(names, submit)):
                 assert got == alone[m], (m, names, submit)
+
+
+@pytest.mark.parametrize("vdw", [1.0, 1.2, 1.3])
+def test_ill_conditioned_systems_alone_and_in_batches(vdw, gpu_ctx):
+    """Systems that need more rounds, substitution or FP64 factors (no escalation), in a launch with more of them
+    than one set of the rounds holds."""
+    from pyrepeat_gb300 import _lib
+    cubes = [_cube(n, gpu_ctx) for n in (270, 411, 440, 520)]
+    for c, t in zip(cubes, (0.1, 1e-3, 1e-5, 0.0)):
+        c.vdw_factor = vdw
+        c.resp = {s: (t, 0.0) for s in RESP} if t else None
+    gpu_ctx.set_kappa_limit(0.0)
+    try:
+        alone = []
+        for c in cubes:
+            q, _, info = gpu_ctx.fit_batch([c], _lib.PREC_MIXED, V_dev=[c.V_dev])
+            alone.append((np.array(q[0]).tobytes(), _lib.fit_info(info[0])["kappa"]))
+        which = [0, 1, 2, 3] * 5 + [2]
+        q, _, info = gpu_ctx.fit_batch([cubes[k] for k in which], _lib.PREC_MIXED, V_dev=[cubes[k].V_dev for k in which])
+    finally:
+        gpu_ctx.set_kappa_limit(_lib.DEFAULT_KAPPA_LIMIT)
+    for k, a, i in zip(which, q, info):
+        assert (np.array(a).tobytes(), _lib.fit_info(i)["kappa"]) == alone[k], k
+    print([_lib.fit_info(i)["solve_path"] for i in info[:4]], ["%.1e" % _lib.fit_info(i)["kappa"] for i in info[:4]])
