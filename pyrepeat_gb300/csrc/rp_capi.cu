@@ -456,9 +456,10 @@ void batch_enqueue(rp_ctx *ctx, int n, const rp_fit_desc *descs, const double *c
     float2 *E_all = ctx->buf_t<float2>("fit_E", std::max<size_t>(e_off[n], 1));
     // In a crowded cell the kept points sit in few pockets, and most grid rows hold none: stage B
     // then waits for the filter and writes only the rows near kept points.  The line: the atoms' spheres
-    // together fill the cell 2.5 times over (3.8 to 4.0 in the MOF-like and triclinic cells, where
-    // 20 to 33 % of the groups of eight rows are needed; below 1.6 in cells of 90 Bohr^3 per atom, where
-    // 99 % are and the wait would cost what the filter takes).
+    // together fill the cell 2.5 times over.  A fit of 800 atoms with and without it: 9.18 against 9.16 ms
+    // at 1.6, 4.63 against 4.66 at 2.2, 3.80 against 3.86 at 2.5, 3.03 against 3.08 at 2.9, 2.55
+    // against 2.66 at 3.4; of 300 atoms: 1.43 both at 1.9, 1.18 both at 2.4, 1.08 against 1.11 at 2.9,
+    // 0.98 against 1.01 at 3.6 (at 4, 20 to 33 % of the groups of eight rows are needed; at 1.6, 99 %).
     auto crowded = [](const rp_fit_desc &d) {
         const double *a = d.grid.axis;
         double det = a[0] * (a[4] * a[8] - a[5] * a[7]) - a[1] * (a[3] * a[8] - a[5] * a[6]) + a[2] * (a[3] * a[7] - a[4] * a[6]);

@@ -1103,7 +1103,7 @@ __global__ void __launch_bounds__(256) lu_trsm_kernel(float *__restrict__ A, int
 // Bounded by the panels' chain of latencies, about 1200 cycles per column (search, publish, pick,
 // update) and 5 us per panel of loads and stores; an update of 2001 x 2001 takes 8 us.  Two barriers
 // per column took 5 % longer; eight columns at a time and panels wholly in line (their instruction
-// fetch costs as much) were no faster.  Measured: 7.8 -> 2.9 ms at 2001 unknowns, 2.3 -> 0.68 at 768, 3.6 -> 1.1 at
+// fetch costs as much) were no faster.  Measured: 7.8 -> 3.05 ms at 2001 unknowns, 2.3 -> 0.67 at 768, 3.6 -> 1.2 at
 // 1101 (against panels in shared memory with four barriers per column, interchanges on one CTA
 // and a cuBLAS rank-32 update).
 constexpr int kLUAcrossMax = 4096;
@@ -1396,8 +1396,9 @@ __global__ void iota_kernel(int *__restrict__ v, int n) {
 }
 
 // The FP32 matrix is in the first half of d.As; the second half takes the factors by input row.  (A buffer of
-// n1^2 floats more, so that rows can move with their positions, made it 5 % faster, but a system
-// would then be factored one way or another by what the scratch budget has left.)
+// n1^2 floats more, so that rows can move with their positions, was up to 5 % faster (2.9 against 3.05 ms at
+// 2001 unknowns), but a system would then be factored one way or another by what the scratch budget
+// has left.)
 void lu_factor_across(rp_ctx *ctx, const SolveDesc &d, int n1, const std::string &tag, cudaStream_t stream) {
     LuStep p{};
     p.A = reinterpret_cast<float *>(d.As);
@@ -1642,21 +1643,21 @@ void factor_refine_wide64(rp_ctx *ctx, const SolveDesc &d, int n1, cudaStream_t 
     RP_CUDA(cudaStreamSynchronize(stream));  // the pinned info words are reused by the next system
 }
 
-// ---- refinement across the GPU with wide FP32 factors
-// The refinement of lu_solve_refine_kernel for a system whose FP32 factors were computed across
-// the GPU (lu_wide_factor): the same steps (scaled FP32 corrections, FP64 residuals, the
-// backward-error stop) and the same condition estimate, as rounds of three
-// launches that decide on the device and return at once when there is nothing left to do:
-//   across_control_kernel   one CTA: what the last round's results mean for the refinement and
-//                           for Hager's estimate, and the next right-hand sides;
-//   across_apply_kernel     (P L U)^-1 of all of them at once, in one cluster;
+// ---- refinement across the GPU with FP32 factors
+// The refinement of lu_solve_refine_kernel for systems of kLUHost64Min or more unknowns: the same steps
+// (scaled FP32 corrections, FP64 residuals, the backward-error stop) and the same condition
+// estimate, as rounds of three launches that decide on the device and return at once when there is
+// nothing left to do, for up to kAcSystems systems:
+//   across_control_kernel   one CTA per system: what the last round's results mean for the refinement
+//                           and for Hager's estimate, and the next right-hand sides;
+//   across_apply_kernel     (P L U)^-1 of all of these at once, in one cluster per system;
 //   across_residual_kernel  x += correction and r = bs - A0 x in FP64, rows over the GPU.
 // The refinement, the estimate and its extra test vector do not depend on one another, so
 // round k carries correction k, the estimate's vector k and (round 0) the extra vector: four
 // rounds instead of eight triangular solves one after the other.
-// Measured, refinement and estimate: 2.46 -> 0.95 ms at 2001 unknowns and 1.3 -> 0.45 at 768 (against
-// cuBLAS solves and residuals with a look by the host after each), 1.56 -> 0.41 at 767 and 0.70 ->
-// 0.31 at 425 (against one CTA, whose FP64 residual alone takes 154 us per step at 767).
+// Measured, refinement and estimate: 2.46 -> 0.95 ms at 2001 unknowns and 1.3 -> 0.38 at 768 (against
+// cuBLAS solves and residuals with a look by the host after each), 1.56 -> 0.39 at 767 and 0.70 ->
+// 0.28 at 425 (against one CTA, whose FP64 residual alone takes 154 us per step at 767).
 constexpr int kAcB = 128;     // unknowns of a block, whose diagonal blocks of L and U are inverted once
 constexpr int kAcCTAs = 8;    // CTAs of the cluster, 16 rows of each block each
 constexpr int kAcT = 512;     // their threads
